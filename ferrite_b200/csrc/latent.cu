@@ -623,6 +623,9 @@ __global__ void __launch_bounds__(256) head_mix_kernel(T* __restrict__ out, long
 // 32-bit.
 // A cache row has 64 NJ columns; values are its first 64 VJ (the rest is a key part). M is 64, or 32 where rows are so wide that two key
 // tiles and 64 queries do not fit.
+// It also serves the multi-head latent attention of the MLA models (512 + 64 columns, 128 heads), whose CUDA-core kernel (mla.cu) has
+// every head read the latents for itself: 6 streams of 1.6K to 4K tokens took 441 us there and 62 us in the merge of its 64 key splits;
+// here the splits are what fills the GPU (6) and the two take 53 and 9 us.
 constexpr int LM_KEYS = 64, LM_THREADS = 256, LM_LDP = LM_KEYS + 8;
 
 __device__ __forceinline__ void lm_cp16(void* smem, const void* gmem, bool valid) {
@@ -645,19 +648,19 @@ __device__ __forceinline__ void lm_mma(float (&c)[4], const uint32_t (&a)[4], ui
 
 template <int NJ>
 struct Lm {
-  static constexpr int LM_M = NJ <= 8 ? 64 : 32, VJ = NJ <= 8 ? NJ : 8;
+  static constexpr int LM_M = NJ <= 8 ? 64 : 32;
   static constexpr int LAT = NJ * 64, LD = LAT + 8;
   static constexpr size_t SMEM = (size_t)(LM_M + 2 * LM_KEYS) * LD * 2 + (size_t)2 * LM_M * LM_LDP * 2 + 6 * LM_M * 4;
 };
 
-template <int NJ>
+template <int NJ, int VJ>
 __global__ void __launch_bounds__(LM_THREADS, 1)
 latent_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ o_part, float* __restrict__ ml_part,
                   const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache, const int* __restrict__ seg_slot,
                   const int* __restrict__ seg_row0, const int* __restrict__ seg_nrows, const int* __restrict__ row_kvlen,
                   const int* __restrict__ block_table, int max_blocks, int kv_block, int heads, int row_base, int tiles_per_seg,
                   int nsplit, float scale_log2, int window, int* status) {
-  constexpr int LAT = Lm<NJ>::LAT, LD = Lm<NJ>::LD, CPR = LAT / 8, LM_M = Lm<NJ>::LM_M, MT = LM_M / 16, VJ = Lm<NJ>::VJ, VL = VJ * 64;
+  constexpr int LAT = Lm<NJ>::LAT, LD = Lm<NJ>::LD, CPR = LAT / 8, LM_M = Lm<NJ>::LM_M, MT = LM_M / 16, VL = VJ * 64;
   extern __shared__ __align__(16) unsigned char lm_smem[];
   __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(lm_smem);           // [M][LD]
   __nv_bfloat16* sK = sQ + LM_M * LD;                                      // [2][KEYS][LD]
@@ -1147,15 +1150,16 @@ extern "C" int fb_latent_mma(void* out, float* o_part, float* ml_part, const voi
                              const int* block_table, int max_blocks, int kv_block, int rows, int row_base, int heads, int lat,
                              int vl, int window, int nsplit, float scale, int* status, cudaStream_t s) {
   if (rows <= 0 || nseg <= 0) return 0;
-  if (lat % 64 || lat > 576 || vl != (lat <= 512 ? lat : 512) || kv_block % LM_KEYS) return -20;
+  const bool key_part = vl == lat - 64 && (lat == 128 || lat == 192 || lat == 576);
+  if (lat % 64 || lat > 576 || (!key_part && (lat > 512 || vl != lat)) || kv_block % LM_KEYS) return -20;
   if (nsplit < 1 || nsplit > 4096 || window < 0) return -1;
   const int m_tile = lat <= 512 ? 64 : 32, tps = (max_rows * heads + m_tile - 1) / m_tile;
   const dim3 grid(nseg * tps, nsplit);
   const float sl = scale * 1.4426950408889634f;
   int rc = 0;
-#define FB_LM(NJ)                                                                                                              \
-  case NJ: {                                                                                                                   \
-    auto kern = latent_mma_kernel<NJ>;                                                                                         \
+#define FB_LM(NJ, VJ)                                                                                                          \
+  case NJ * 16 + VJ: {                                                                                                         \
+    auto kern = latent_mma_kernel<NJ, VJ>;                                                                                     \
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lm<NJ>::SMEM);                \
     if (e != cudaSuccess) return (int)e;                                                                                       \
     rc = (int)launch_pdl(kern, grid, dim3(LM_THREADS), Lm<NJ>::SMEM, s, (bf16*)out, o_part, ml_part, (const bf16*)q,           \
@@ -1163,7 +1167,9 @@ extern "C" int fb_latent_mma(void* out, float* o_part, float* ml_part, const voi
                          row_base, tps, nsplit, sl, window, status);                                                           \
     break;                                                                                                                     \
   }
-  switch (lat / 64) { FB_LM(1) FB_LM(2) FB_LM(3) FB_LM(4) FB_LM(5) FB_LM(6) FB_LM(7) FB_LM(8) FB_LM(9) }
+  switch (lat / 64 * 16 + vl / 64) {
+    FB_LM(1, 1) FB_LM(2, 2) FB_LM(3, 3) FB_LM(4, 4) FB_LM(5, 5) FB_LM(6, 6) FB_LM(7, 7) FB_LM(8, 8) FB_LM(2, 1) FB_LM(3, 2) FB_LM(9, 8)
+  }
 #undef FB_LM
   if (rc || nsplit == 1) return rc;
   return latent_merge<bf16>(out, (long)heads * vl, o_part, ml_part, nullptr, rows, heads, nsplit, vl, s);

@@ -9,7 +9,8 @@
 //   mla_attn      one CTA per (token row, head, key split): warps stride over the keys, online softmax, value = latent;
 //                 rows of a prompt attend causally through their own kvlen
 //   mla_combine   merge of the splits in split order
-// SIMT fp32 throughout: this is the functional path of the MLA model family (prefill cost is quadratic per row here).
+// SIMT fp32 throughout: the path of callers without segment tables and of pages that are no multiple of 64 tokens. The engine's rows run on
+// latent_mma (latent.cu), where heads and rows share the latents they read.
 // Counterparts in the reference: `ds_rope`, `ds_kv_window`, `ds_attn`, `ds_attn16`, `ds_attn_mq(_fin)`
 // (`kernels/k-ds/src`), f32 oracle `crates/fe-dsc/src/refmodel.rs`.
 #include "api_ext.h"

@@ -984,7 +984,8 @@ class Executor:
                     ol = ops.mla_attention(qabs, self.k_cache[i].view(-1, self.ecfg.kv_block, L + R), mv["slot"], mv["kvlen"],
                                            self.block_table, self.ecfg.kv_block, c.n_q, L, R,
                                            1.0 / math.sqrt(c.nope_head_dim + R),
-                                           nsplit=nsplit if max_seg_rows <= FLASH_MIN_ROWS else 1)
+                                           nsplit=nsplit if max_seg_rows <= FLASH_MIN_ROWS else 1,
+                                           segs=(mv["sslot"], mv["srow0"], mv["snrows"], max_seg_rows))
                     o = ops.mla_out(ol, w_uv)
                 x = row(o, w[p + "out_proj"], x)
             else:

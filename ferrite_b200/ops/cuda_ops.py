@@ -16,7 +16,7 @@ import torch
 
 from .._ext import load
 from .extras import CudaExtras
-from .latent import CudaLatent
+from .latent import CudaLatent, SegGroup
 from .mixers import CudaMixers
 from .qweight import Exl3Weight, ExpertsFP4, GgufWeight, QWeight, StackWeight
 
@@ -705,8 +705,14 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
                                    nq, nq, HP, False, max(n for _, _, n in segs))
         return o.view(T, nq, HP)[:, :, :dv].contiguous().view(T, nq * dv)
 
-    def mla_attention(self, qabs, cache, row_slot, row_kvlen, block_table, kv_block, nq, L, R, scale, nsplit=1):
+    def mla_attention(self, qabs, cache, row_slot, row_kvlen, block_table, kv_block, nq, L, R, scale, nsplit=1, segs=None):
+        """Every head attends the cached latents. With `segs` = (seg_slot, seg_row0, seg_nrows, max rows per segment) and pages of whole
+        64-key tiles the tensor-core kernel of the listed models runs: heads and rows of a segment share every pass over the latents, and the
+        key splits are what fills the GPU. Callers without segment tables and other page sizes take the CUDA-core kernel."""
         T = qabs.shape[0]
+        if segs is not None and kv_block % 64 == 0 and R == 64 and L in (64, 128, 512):
+            return self.latent_attention(qabs, cache.view(-1, kv_block, L + R), SegGroup(0, segs[0].numel(), 0, T, segs[3]), row_slot, row_kvlen,
+                                         segs[:3], block_table, kv_block, scale, nsplit, vlat=L)
         out = self.empty(T, nq, L, dtype=self.dtype, device=self.device)
         o_part = self.empty(T * nq * nsplit * L, dtype=torch.float32, device=self.device)
         ml_part = self.empty(T * nq * nsplit * 2, dtype=torch.float32, device=self.device)

@@ -46,6 +46,31 @@ def test_mla_prep_and_attention(ops, L, R, nq, nsplit):
     assert (oa.float() - ob.float()).abs().max().item() < 2e-2
 
 
+@pytest.mark.parametrize("L,R,nq", [(512, 64, 128), (512, 64, 3), (128, 64, 5), (64, 64, 4)])
+@pytest.mark.parametrize("lens,rows,nsplit", [((1, 63, 64, 65), 1, 64), ((700, 129), 3, 4), ((200,), 40, 1)])
+def test_mla_attention_of_segments(ops, L, R, nq, lens, rows, nsplit):
+    """Segments on the tensor-core latent kernel against the CUDA-core kernel and the fp32 statement: contexts at the edges of its 64-key
+    tiles, more splits than tiles, several rows per segment, heads that leave its M tiles ragged."""
+    tops = TorchOps(DEV, torch.float32)
+    g = torch.Generator(device=DEV).manual_seed(L + nq + rows)
+    kvb, nb, S = 64, 12, len(lens)
+    cache = torch.randn(S * nb, kvb, L + R, generator=g, device=DEV).to(torch.bfloat16)
+    bt = torch.randperm(S * nb, generator=g, device=DEV).to(torch.int32).view(S, nb)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    slot = i32([s for s in range(S) for _ in range(rows)])
+    kvlen = i32([max(1, n - rows + 1 + r) for n in lens for r in range(rows)])
+    q = torch.randn(S * rows, nq, L + R, generator=g, device=DEV).to(torch.bfloat16)
+    scale = (L + R) ** -0.5
+    segs = (i32(list(range(S))), i32([s * rows for s in range(S)]), i32([rows] * S), rows)
+    got = ops.mla_attention(q, cache, slot, kvlen, bt, kvb, nq, L, R, scale, nsplit=nsplit, segs=segs).float()
+    want = tops.mla_attention(q, cache, slot, kvlen, bt, kvb, nq, L, R, scale).float()
+    plain = ops.mla_attention(q, cache, slot, kvlen, bt, kvb, nq, L, R, scale, nsplit=nsplit).float()
+    # 32-bit scores and sums, weights of 16 bits (2^-17 relative): what is left is the rounding of the bf16 result, |o| <= 4.5 here
+    for o in (got, plain):
+        assert (o - want).abs().max().item() <= 2 ** -8 * want.abs().max().item()
+    assert ops.status() == 0
+
+
 @pytest.mark.parametrize("T", [1, 6, 8, 19, 300])
 @pytest.mark.parametrize("nh,N,K", [(16, 512, 128), (16, 128, 512), (4, 64, 32), (3, 40, 64)])
 def test_head_linear_row_kernel_and_batched_gemm(ops, T, nh, N, K):
