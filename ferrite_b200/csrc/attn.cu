@@ -411,20 +411,21 @@ __global__ void attn_combine_kernel(__nv_bfloat16* __restrict__ out, const float
   const size_t pbase = ((size_t)row * nq + qh) * nsplit;
   // The first warp turns the splits' (max, sum) pairs into one weight per split (two dependent memory round trips for
   // the whole kernel instead of three per thread); then every thread sums its dimensions over the splits in split order.
-  __shared__ float wgt[ATT_MAX_SPLITS];
+  __shared__ float wgt[ATT_MAX_SPLITS], part[ATT_MAX_SPLITS];
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
     float M = -INFINITY;
     for (int s0 = lane; s0 < nsplit; s0 += 32) M = fmaxf(M, ml_part[(pbase + s0) * 2]);
     M = warp_max(M);
     for (int s0 = lane; s0 < nsplit; s0 += 32) {
-      const float ms = ml_part[(pbase + s0) * 2];
-      wgt[s0] = ms != -INFINITY ? exp2f(ms - M) : 0.f;
+      const float2 ml = *reinterpret_cast<const float2*>(ml_part + (pbase + s0) * 2);
+      wgt[s0] = ml.x != -INFINITY ? exp2f(ml.x - M) : 0.f;
+      part[s0] = ml.y * wgt[s0];
     }
     __syncwarp();
     if (lane == 0) {                                       // the normaliser, summed in split order
       float Ls = 0.f;
-      for (int s0 = 0; s0 < nsplit; ++s0) Ls += ml_part[(pbase + s0) * 2 + 1] * wgt[s0];
+      for (int s0 = 0; s0 < nsplit; ++s0) Ls += part[s0];
       wgt[nsplit] = Ls;                                    // (nsplit < ATT_MAX_SPLITS is checked on the host)
     }
   }
@@ -433,9 +434,10 @@ __global__ void attn_combine_kernel(__nv_bfloat16* __restrict__ out, const float
   const float inv = L > 0.f ? 1.f / L : 0.f;
   for (int d = threadIdx.x; d < HD; d += blockDim.x) {
     float acc = 0.f;
-    for (int s0 = 0; s0 < nsplit; ++s0) {
-      const float e = wgt[s0];
-      if (e != 0.f) acc += o_part[(pbase + s0) * HD + d] * e;
+#pragma unroll 8
+    for (int s0 = 0; s0 < nsplit; ++s0) {                  // several splits' values in flight; an empty split left none
+      const float e = wgt[s0], o = e != 0.f ? o_part[(pbase + s0) * HD + d] : 0.f;
+      acc = fmaf(o, e, acc);
     }
     float v = acc * inv;
     if (gated) v *= sigmoidf_(bf2f(proj[(size_t)row * proj_stride + (size_t)qh * 2 * HD + HD + d]));

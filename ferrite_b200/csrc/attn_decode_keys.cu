@@ -246,8 +246,8 @@ attn_decode_keys_kernel(float* __restrict__ o_part, float* __restrict__ ml_part,
 using namespace fb;
 
 // Records of key splits as fb_attn_decode_mma leaves them (o_part [rows][nq][nsplit][hd], ml_part two floats each); scale of the scores; kb:
-// window, chunk and softcap, or null; pool: means of the blocks before the window, or null. Returns -20 for shapes it does not take: heads of 64
-// or 128 columns, max_rows * (nq / nkv) <= 16 (with means: nq / nkv <= 16), pages of a multiple of 64 keys.
+// window, chunk and softcap, or null; pool: means of the blocks before the window, or null. Returns -20 for shapes it does not take: heads of 64,
+// 128 or (without means) 256 columns, nq / nkv <= 16, pages of a multiple of 64 keys.
 extern "C" int fb_attn_decode_keys(float* o_part, float* ml_part, const void* q, const void* k_cache, const void* v_cache, const int* seg_slot,
                                    const int* seg_row0, const int* seg_nrows, const int* row_kvlen, const int* block_table, int max_blocks,
                                    int kv_block, int nseg, int max_rows, int rows, int nq, int nkv, int hd, int nsplit, float scale,
@@ -255,7 +255,7 @@ extern "C" int fb_attn_decode_keys(float* o_part, float* ml_part, const void* q,
   if (nseg <= 0 || rows <= 0) return 0;
   if (nkv <= 0 || nq % nkv || nsplit < 1) return -1;
   const int G = nq / nkv;
-  if ((hd != 64 && hd != 128) || (pool ? G : (long)max_rows * G) > DK_M || kv_block % DK_KEYS) return -20;
+  if ((hd != 64 && hd != 128 && (hd != 256 || pool)) || G > DK_M || kv_block % DK_KEYS) return -20;
   if (pool && (pool->size < 1 || !kb || !kb->window)) return -1;
   if (kb && (kb->window < 0 || kb->chunk < 0 || (kb->window && kb->chunk) || kb->cap < 0.f)) return -1;
   constexpr float LOG2E = 1.4426950408889634f;
@@ -273,5 +273,5 @@ extern "C" int fb_attn_decode_keys(float* o_part, float* ml_part, const void* q,
                            status);
   };
   if (pool) return hd == 64 ? go(attn_decode_keys_kernel<64, true>) : go(attn_decode_keys_kernel<128, true>);
-  return hd == 64 ? go(attn_decode_keys_kernel<64, false>) : go(attn_decode_keys_kernel<128, false>);
+  return hd == 64 ? go(attn_decode_keys_kernel<64, false>) : hd == 128 ? go(attn_decode_keys_kernel<128, false>) : go(attn_decode_keys_kernel<256, false>);
 }

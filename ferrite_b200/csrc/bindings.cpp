@@ -230,6 +230,23 @@ int64_t attn_decode_mma(Tensor out, Tensor o_part, Tensor ml_part, Tensor q, Ten
                         c10::optional<Tensor> kv_scale) {
   int rc = fb_attn_decode_mma(out.data_ptr(), o_part.data_ptr<float>(), ml_part.data_ptr<float>(), q.data_ptr(),
                               k_cache.data_ptr(), v_cache.data_ptr(), (const float*)cptr(kv_scale), proj.data_ptr(),
+// The same without ancestor masks, keys split over the warps of a CTA.
+int64_t attn_decode_keys(Tensor out, Tensor o_part, Tensor ml_part, Tensor q, Tensor k_cache, Tensor v_cache, Tensor proj, Tensor seg_slot,
+                         Tensor seg_row0, Tensor seg_nrows, int64_t max_rows, Tensor row_kvlen, Tensor block_table, int64_t kv_block, int64_t nq,
+                         int64_t nkv, int64_t hd, int64_t nsplit, bool gated, Tensor status) {
+  const int rows = (int)row_kvlen.numel();
+  TORCH_CHECK(o_part.numel() >= (int64_t)rows * nq * nsplit * hd && ml_part.numel() >= (int64_t)rows * nq * nsplit * 2, "attn_decode_keys: scratch");
+  int rc = fb_attn_decode_keys(o_part.data_ptr<float>(), ml_part.data_ptr<float>(), q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
+                               seg_slot.data_ptr<int>(), seg_row0.data_ptr<int>(), seg_nrows.data_ptr<int>(), row_kvlen.data_ptr<int>(),
+                               block_table.data_ptr<int>(), (int)block_table.size(1), (int)kv_block, (int)seg_slot.numel(), (int)max_rows, rows, (int)nq,
+                               (int)nkv, (int)hd, (int)nsplit, 1.f / sqrtf((float)hd), nullptr, nullptr, 0, status.data_ptr<int>(), cur_stream());
+  if (rc == -20) return rc;
+  check(rc, "attn_decode_keys");
+  check(fb_attn_combine(out.data_ptr(), o_part.data_ptr<float>(), ml_part.data_ptr<float>(), proj.data_ptr(), (long)proj.stride(0), rows, (int)nq, (int)hd,
+                        (int)nsplit, gated ? 1 : 0, cur_stream()), "attn_combine");
+  return 0;
+}
+
                               (long)proj.stride(0),
                               seg_slot.data_ptr<int>(), seg_row0.data_ptr<int>(), seg_nrows.data_ptr<int>(),
                               row_kvlen.data_ptr<int>(), (const int*)cptr(row_base),
@@ -434,6 +451,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemv", &gemv);
   m.def("gemm", &gemm);
   m.def("gemm_workspace_bytes", &gemm_workspace_bytes);
+  m.def("attn_decode_keys", &attn_decode_keys);
   m.def("attn_prep", &attn_prep);
   m.def("attn_decode", &attn_decode);
   m.def("attn_prefill", &attn_prefill);

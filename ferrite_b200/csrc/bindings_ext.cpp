@@ -710,7 +710,8 @@ void gqa_attn(Tensor out, Tensor o_part, Tensor ml_part, Tensor q, Tensor k_cach
       TORCH_CHECK(m && m->is_contiguous() && m->scalar_type() == q.scalar_type() && m->size(0) == k_cache.size(0) &&
                   m->size(1) == (kv_block + pool - 1) / pool && m->size(2) == kvh && m->size(3) == hd, "gqa_attn: means");
   if (!cuda_cores) {
-    const int rc = fb_attn_decode_keys(o_part.data_ptr<float>(), ml_part.data_ptr<float>(), q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
+    // (more pairs of row and head than a CTA of that kernel takes share their keys better on the other one)
+    const int rc = !pool && max_rows * (heads / kvh) > 16 ? -20 : fb_attn_decode_keys(o_part.data_ptr<float>(), ml_part.data_ptr<float>(), q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
                                        seg_slot.data_ptr<int>(), seg_row0.data_ptr<int>(), seg_nrows.data_ptr<int>(), row_kvlen.data_ptr<int>(),
                                        block_table.data_ptr<int>(), (int)block_table.size(1), (int)kv_block, (int)seg_slot.numel(), (int)max_rows,
                                        rows, heads, kvh, hd, (int)nsplit, (float)scale, kbp, pkp, (int)row_first, status.data_ptr<int>(), cur_stream());

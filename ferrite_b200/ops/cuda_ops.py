@@ -21,6 +21,9 @@ from .mixers import CudaMixers
 from .qweight import Exl3Weight, ExpertsFP4, GgufWeight, QWeight, StackWeight
 
 GEMV_MAX_ROWS = 8
+# CTAs per SM that the decode attention's key splits aim at, by head width (as many as are resident; four rows against 6000 keys each, 4 kv heads
+# of 256: 47 us, 97 with the splits of whole rows over one warp's keys)
+DECODE_KEYS_CTAS = {64: 4, 128: 2, 256: 1}
 MOE_PAIR_ROWS = 64     # up to this many rows (the largest graph-captured step) the experts run as per-pair GEMVs,
                        # beyond as grouped GEMMs, which read the per-expert row counts on the host
 
@@ -553,10 +556,21 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
             key = (n_slots, toks, nkv, hd)
             if self._kv_scratch is None or self._kv_scratch[0] != key:
                 # zeros: rows past the decoded ones are masked by causality but still multiplied (0 x value) by the
+        # the heads of a group for a row or two at a time, keys split over the warps of a CTA, and as many splits as fill the GPU. Rows of every
+        # count take this kernel, so that a verified row has the bits of a decoded one; trees (ancestor masks) and quantised caches do not.
+        G = nq // nkv
+        keys = (segs is not None and kv_scale is None and row_mask is None and self.attn_mma and G <= 16 and kv_block % 64 == 0
+                and hd in DECODE_KEYS_CTAS)
+        if keys:
+            ctas = segs[0].numel() * nkv * -(-segs[3] // (16 // G))
+            nsplit = max(1, min(nsplit, self.sm_count * DECODE_KEYS_CTAS[hd] // ctas))
                 # tensor-core kernel, so they must hold finite numbers
                 ks = torch.zeros(n_slots * max_blocks, kv_block, nkv, hd, dtype=self.dtype, device=self.device)
                 vs = torch.zeros_like(ks)
                 ident = torch.arange(n_slots * max_blocks, dtype=torch.int32, device=self.device).view(n_slots, max_blocks)
+        if keys and self.C.attn_decode_keys(out, o_part, ml_part, q, k_cache, v_cache, proj, *segs, row_kvlen, block_table, kv_block, nq, nkv, hd,
+                                            nsplit, gated, self.status_word) == 0:
+            return out
                 self._kv_scratch = (key, ks, vs, ident.contiguous())
             _, ks, vs, ident = self._kv_scratch
             self.launches += 1

@@ -700,3 +700,27 @@ def test_canary_padded_output_buffers_catch_a_stray_write(ops):
             ops.check_canaries()
     finally:
         ops.enable_canaries(False)
+
+
+@pytest.mark.parametrize("hd,nq,nkv", [(256, 24, 4), (256, 2, 2), (256, 32, 2), (128, 8, 2), (64, 4, 4)])
+@pytest.mark.parametrize("rows", [1, 2, 17])
+@pytest.mark.parametrize("nsplit", [1, 7, 64])
+def test_attention_keys_over_warps(ops, tops, hd, nq, nkv, rows, nsplit):
+    """Rows with the keys split over the warps: contexts of one key, around the 16 keys of a warp and the 64 of a tile, more splits than tiles,
+    rows in several groups, against 32-bit math; 16 heads to a group fill a CTA's pairs with one row."""
+    lens = [rows, 15 + rows, 63 + rows, 64 + rows, 129, 700]
+    kv_block, S, nb = 64, len(lens), 12
+    g = torch.Generator(device=DEV).manual_seed(hd + nq + rows)
+    bt = torch.randperm(S * nb, generator=g, device=DEV).to(torch.int32).view(S, nb)
+    kc, vc = (torch.randn(S * nb, kv_block, nkv, hd, generator=g, device=DEV).to(torch.bfloat16) for _ in "kv")
+    q = torch.randn(S * rows, nq, hd, generator=g, device=DEV).to(torch.bfloat16)
+    proj = torch.randn(S * rows, nq * hd * 2 + 2 * nkv * hd, generator=g, device=DEV).to(torch.bfloat16)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    slot = i32([s for s in range(S) for _ in range(rows)])
+    kvlen = i32([n - rows + 1 + r for n in lens for r in range(rows)])
+    segs = (i32(list(range(S))), i32([s * rows for s in range(S)]), i32([rows] * S), rows)
+    got = ops.attention(q, proj, kc, vc, slot, kvlen, bt, kv_block, nq, nkv, hd, True, nsplit=nsplit, segs=segs).float()
+    want = tops.attention(q, proj, kc, vc, slot, kvlen, bt, kv_block, nq, nkv, hd, True).float()
+    # weights of 16 bits and 32-bit sums under the rounding of the result, |o| <= 4.5
+    assert (got - want).abs().max().item() <= 2 ** -8 * max(1.0, want.abs().max().item()) + 2e-4
+    assert ops.status() == 0
