@@ -64,7 +64,7 @@ constexpr size_t RS_STAGING = 4 * 32 * GM_RS_COLS * 2;      // transpose buffers
 
 template <int COMM>
 int launch(const GemmPlan& p, const CUtensorMap& tmA, const CUtensorMap& tmB, cudaStream_t s) {
-  const size_t smem = p.smem + (COMM == 1 ? RS_STAGING : 0);
+  const size_t smem = p.smem + (COMM == 1 ? RS_STAGING - 4 * GM_EPI_BYTES : 0);      // (that epilogue has a staging of its own)
   constexpr size_t limit = 226 * 1024;                     // 227 KB per CTA minus the kernel's static shared memory
   if (smem > limit) return -23;
   static bool attr_done = false;

@@ -7,7 +7,7 @@
 //
 // Two orientations share the code, because both operands are K-major and UMMA N is a run-time field of the
 // instruction descriptor:
-//   normal (M > 64): A = 128 token rows, B = 256 output features (or 128 gate + 128 up rows for SwiGLU).
+//   normal (M > 64): A = 128 token rows, B = up to 256 output features (SwiGLU: half of them gate, half up rows).
 //   swapped (M <= 64, decode / verify rows): A = 128 output features, B = the token rows (N = 16..64), with
 //     deterministic split-K so the few weight tiles still cover every SM; partial tiles go to an fp32
 //     workspace and the last CTA of a tile sums them in split order.
@@ -95,6 +95,8 @@ struct GemmArgs {
   int tiles_a, tiles_b;     // tile counts along the A-row and B-row dimensions
   int acc_cols;             // TMEM columns per accumulator buffer (n_a * bn)
   int tmem_cols;            // allocated columns (power of two >= 2 * acc_cols)
+  // plain normal orientation: tiles from tail_first on (fewer than the CTAs) are cut along K into tail_split pieces of tail_kb k blocks
+  int tail_first, tail_tiles, tail_split, tail_kb;
 };
 
 __device__ __forceinline__ bool mbar_wait_or_flag(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
@@ -109,8 +111,10 @@ __device__ __forceinline__ bool mbar_wait_or_flag(uint64_t* bar, uint32_t parity
   return false;
 }
 
+constexpr int GM_KB_COST = 400, GM_TAIL_COST = 18, GM_PIECE_COST = 20, GM_TAIL_MAX = 4;      // see plan_gemm
 constexpr int GM_COPY_WARPS = 2;   // mode 2: warps 6 and 7 gather remote rows
 constexpr int GM_COPY_COLS = 512;  // columns of X per gather work item (two 16-byte loads per lane and row)
+constexpr int GM_EPI_BYTES = 32 * 32 * 4;   // an epilogue warp's piece of the output on its way
 constexpr int GM_RS_COLS = 128;   // mode 1: columns staged per warp before the coalesced peer stores
 constexpr int GM_COPY_ROWS = 8;    // rows per gather work item: 16 loads of 16 bytes in flight per lane
 
@@ -181,6 +185,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const int groups_second = (a.tiles_a - n_first + gs - 1) / gs;
     total_work = (groups_first + groups_second) * gs * a.tiles_b;      // padded: short groups leave invalid items
   }
+  if constexpr (COMM == 0) total_work += a.tail_tiles * (a.tail_split - 1);
   (void)parity;
 
   // work item -> (tile along A rows, tile along B rows, k split); A-row tiles vary fastest in the normal
@@ -221,9 +226,14 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
     ks = w % a.split_k;
     int t = w / a.split_k;
-    if (a.swap) { tb = t % a.tiles_b; ta = t / a.tiles_b; }
-    else { ta = t % a.tiles_a; tb = t / a.tiles_a; }
+    if (a.swap) { tb = t % a.tiles_b; ta = t / a.tiles_b; return true; }
+    if (w >= a.tail_first) { ks = (w - a.tail_first) / a.tail_tiles; t = a.tail_first + (w - a.tail_first) % a.tail_tiles; }
+    ta = t % a.tiles_a; tb = t / a.tiles_a;
     return true;
+  };
+  auto k_range = [&](int w, int ks, int& kb0, int& kb1) {
+    const int per = COMM == 0 && w >= a.tail_first ? a.tail_kb : kb_per_split;
+    kb0 = ks * per; kb1 = min(kblocks_total, kb0 + per);
   };
 
   if (warp == 0) {
@@ -237,7 +247,8 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x) {
         int ta, tb, ks;
         if (!decode_work(w, ta, tb, ks)) continue;
-        const int kb0 = ks * kb_per_split, kb1 = min(kblocks_total, kb0 + kb_per_split);
+        int kb0, kb1;
+        k_range(w, ks, kb0, kb1);
         if constexpr (COMM == 2) {
           // rows of this tile that live on other ranks must have arrived in the local full-X buffer
           const int trows = min(GM_BM, a.M - ta * GM_BM);
@@ -331,7 +342,8 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x) {
         int ta, tb, ks;
         if (!decode_work(w, ta, tb, ks)) continue;
-        const int kb0 = ks * kb_per_split, kb1 = min(kblocks_total, kb0 + kb_per_split);
+        int kb0, kb1;
+        k_range(w, ks, kb0, kb1);
         if (!mbar_wait_or_flag(&tempty_bar[buf], tphase[buf] ^ 1u, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d0 = tmem_base + (uint32_t)(buf * a.acc_cols);
@@ -515,64 +527,172 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         if (lane == 0) mbar_arrive(&tempty_bar[buf]);
         if (!ok) break;
       } else if (!a.swap) {
-        // lanes = token rows, columns = output features
-        const int m = (COMM == 3 ? g_row0 : ta * GM_BM) + etid;
+        // lanes = token rows, columns = output features. A warp takes 32 columns of its 32 rows at a time through shared memory (fp32, 16-byte
+        // pieces swizzled by row: free of bank conflicts both ways), so that residual and output move as whole 64- or 128-byte pieces of rows
+        // instead of 16 bytes in each of 32 rows, with the residual on its way before the accumulator is read. (Written from the accumulator's
+        // registers, with a dynamically indexed tail that kept them in local memory, 256 columns took 28 us, twice the products of
+        // K = 2048, and 2048 x 5120 x 2048 105 us; now 53.)
+        const int row_first = (COMM == 3 ? g_row0 : ta * GM_BM) + quad * 32;
+        const int m = row_first + lane;
         const int m_end = COMM == 3 ? g_row_end : a.M;
         const int ncols_out = a.dual ? a.bn / 2 : a.bn;
         const int n0 = tb * ncols_out;
-        for (int c = 0; c < ncols_out; c += 32) {
-          uint32_t r0[32], r1[32];
-          tmem_ld32(tbase + (uint32_t)c, r0);
-          if (a.dual) tmem_ld32(tbase + (uint32_t)(c + a.bn / 2), r1);
-          tmem_ld_wait();
-          if (m < m_end) {
-            const int n = n0 + c;
-            float v[32];
+        const float sm_row = a.scale_m && m < m_end ? a.scale_m[m] : 1.f;
+        const uint32_t stage_w = smem_u32(tiles + (size_t)a.stages * stage_bytes + (size_t)quad * GM_EPI_BYTES);
+        const int rr = lane >> 2, rc = (lane & 3) * 8;    // bf16 output: row of a group of 8, column of the 32
+        // A piece of a tile (tail of the tile list): 64 accumulator columns at a time go to the workspace as fp32, and the warp that brings a
+        // block's last piece sums the pieces in their order and finishes it. The pieces begin at different columns, which spreads the sums over
+        // the CTAs; nobody waits.
+        const bool piece_of = COMM == 0 && w >= a.tail_first;
+        const int steps = a.dual ? ncols_out / 32 : (ncols_out + 63) / 64, halves = a.dual ? 1 : 2;
+        float4* wsp = nullptr;
+        const size_t ws_piece = (size_t)(a.bn / 32) * 4 * 256;      // float4 of one piece: [bn / 32][4 warps][8][32 lanes]
+        if (piece_of) wsp = reinterpret_cast<float4*>(a.workspace) + (size_t)((w - a.tail_first) % a.tail_tiles) * a.tail_split * ws_piece + quad * 256 + lane;
+        for (int i = 0; i < steps * halves; ++i) {
+          int st = i / halves;
+          if (piece_of) st = (st + ks * steps / a.tail_split) % steps;
+          if (piece_of && i % halves == 0) {
+            for (int h = 0; h < 2; ++h) {
+              const int col = a.dual ? st * 32 + h * (a.bn / 2) : st * 64 + h * 32;
+              if (col >= a.bn || (!a.dual && n0 + col >= a.N)) break;
+              uint32_t r[32];
+              tmem_ld32(tbase + (uint32_t)col, r);
+              tmem_ld_wait();
+              float4* dst = wsp + ks * ws_piece + (size_t)(col / 32) * 1024;
 #pragma unroll
-            const float sm_row = a.scale_m ? a.scale_m[m] : 1.f;
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              float x = __uint_as_float(r0[j]) * sm_row;
-              float u = a.dual ? __uint_as_float(r1[j]) * sm_row : 0.f;
-              if (a.scale_n && n + j < a.N) {
-                x *= a.scale_n[n + j];
-                if (a.dual) u *= a.scale_n[a.N + n + j];
-              }
-              v[j] = a.dual ? glu_act(x, u, a.limit) : epilogue_act(x, a.act);
+              for (int q = 0; q < 8; ++q)
+                __stcg(dst + q * 32, make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]), __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3])));
             }
-            if (n + 32 <= a.N) {
+            __threadfence();
+            __syncwarp();
+            int* ctr = a.counters + (((w - a.tail_first) % a.tail_tiles) * 8 + st) * 4 + quad;
+            int last = 0;
+            if (lane == 0) {
+              last = atomicAdd(ctr, 1) == a.tail_split - 1;
+              if (last) *ctr = 0;                         // self-cleaning for the next launch
+            }
+            last = __shfl_sync(0xffffffffu, last, 0);
+            if (!last) { i += halves - 1; continue; }
+            __threadfence();
+          }
+          const int c = a.dual ? st * 32 : st * 64 + (i % halves) * 32;
+          if (c >= ncols_out || n0 + c >= a.N) continue;
+          const int n = n0 + c;
+          uint4 rv[4];
+          if (a.res)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const int row = row_first + q * 8 + rr;
+              rv[q] = row < m_end && n + rc + 8 <= a.N ? *reinterpret_cast<const uint4*>(a.res + (size_t)row * a.ldy + n + rc) : make_uint4(0, 0, 0, 0);
+            }
+          const float sn = a.scale_n && n + lane < a.N ? a.scale_n[n + lane] : 1.f, sn_up = a.dual && a.scale_n && n + lane < a.N ? a.scale_n[a.N + n + lane] : 1.f;
+          uint32_t r0[32], r1[32];
+          if (piece_of) {
+            auto sum = [&](int col, uint32_t (&r)[32]) {
+              float4 acc[8], o[8];
+              const float4* src = wsp + (size_t)(col / 32) * 1024;
+#pragma unroll
+              for (int q = 0; q < 8; ++q) acc[q] = __ldcg(src + q * 32);
+#pragma unroll 1
+              for (int p = 1; p < a.tail_split; ++p) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) o[q] = __ldcg(src + p * ws_piece + q * 32);
+#pragma unroll
+                for (int q = 0; q < 8; ++q) { acc[q].x += o[q].x; acc[q].y += o[q].y; acc[q].z += o[q].z; acc[q].w += o[q].w; }
+              }
+#pragma unroll
+              for (int q = 0; q < 8; ++q) {
+                r[4 * q] = __float_as_uint(acc[q].x); r[4 * q + 1] = __float_as_uint(acc[q].y);
+                r[4 * q + 2] = __float_as_uint(acc[q].z); r[4 * q + 3] = __float_as_uint(acc[q].w);
+              }
+            };
+            sum(c, r0);
+            if (a.dual) sum(c + a.bn / 2, r1);
+          } else {
+            tmem_ld32(tbase + (uint32_t)c, r0);
+            if (a.dual) tmem_ld32(tbase + (uint32_t)(c + a.bn / 2), r1);
+            tmem_ld_wait();
+          }
+          // (straight runs of 32 under one test each: a test per element made a lone warp's 32 columns cost 2.7 us)
+          float v[32];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r0[j]);
+          if (a.scale_m) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] *= sm_row;
+          }
+          if (a.scale_n) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] *= __shfl_sync(0xffffffffu, sn, j);
+          }
+          if (a.dual) {
+            float u[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) u[j] = __uint_as_float(r1[j]);
+            if (a.scale_m) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) u[j] *= sm_row;
+            }
+            if (a.scale_n) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) u[j] *= __shfl_sync(0xffffffffu, sn_up, j);
+            }
+            if (a.limit > 0.f) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = glu_act(v[j], u[j], a.limit);
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = glu_act(v[j], u[j], 0.f);
+            }
+          } else if (a.act) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = epilogue_act(v[j], a.act);
+          }
+          __syncwarp();                                   // the last 32 columns have been read
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(stage_w + (uint32_t)(lane * 128 + ((q ^ (lane & 7)) << 4))), "f"(v[4 * q]),
+                         "f"(v[4 * q + 1]), "f"(v[4 * q + 2]), "f"(v[4 * q + 3]) : "memory");
+          __syncwarp();
+          auto piece = [&](int row, int q) {
+            float4 f;
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f.x), "=f"(f.y), "=f"(f.z), "=f"(f.w)
+                         : "r"(stage_w + (uint32_t)(row * 128 + ((q ^ (row & 7)) << 4))));
+            return f;
+          };
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int row = q * 8 + rr, gm = row_first + row, nn = n + rc;
+            const float4 lo = piece(row, rc / 4), hi = piece(row, rc / 4 + 1);
+            float o[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+            if (gm >= m_end || nn >= a.N) continue;
+            const size_t at = (size_t)gm * a.ldy + nn;
+            if (nn + 8 <= a.N) {
               if (a.res) {
-                const uint4* rp = reinterpret_cast<const uint4*>(a.res + (size_t)m * a.ldy + n);
+                const uint32_t ru[4] = {rv[q].x, rv[q].y, rv[q].z, rv[q].w};
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                  uint4 rv = rp[q];
-                  uint32_t ru[4] = {rv.x, rv.y, rv.z, rv.w};
-#pragma unroll
-                  for (int j = 0; j < 4; ++j) { v[q * 8 + 2 * j] += bf_lo(ru[j]); v[q * 8 + 2 * j + 1] += bf_hi(ru[j]); }
-                }
+                for (int j = 0; j < 4; ++j) { o[2 * j] += bf_lo(ru[j]); o[2 * j + 1] += bf_hi(ru[j]); }
               }
               if (a.out_f32) {
-                float4* yf = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.Y) + (size_t)m * a.ldy + n);
-#pragma unroll
-                for (int q = 0; q < 8; ++q) yf[q] = make_float4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
+                float4* yf = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.Y) + at);
+                yf[0] = make_float4(o[0], o[1], o[2], o[3]);
+                yf[1] = make_float4(o[4], o[5], o[6], o[7]);
               } else {
-                uint4* yp = reinterpret_cast<uint4*>(Yb + (size_t)m * a.ldy + n);
+                *reinterpret_cast<uint4*>(Yb + at) = make_uint4(pack_bf2(o[0], o[1]), pack_bf2(o[2], o[3]), pack_bf2(o[4], o[5]), pack_bf2(o[6], o[7]));
+              }
+            } else {                                      // the ragged end of a row
 #pragma unroll
-                for (int q = 0; q < 4; ++q)
-                  yp[q] = make_uint4(pack_bf2(v[q * 8], v[q * 8 + 1]), pack_bf2(v[q * 8 + 2], v[q * 8 + 3]),
-                                     pack_bf2(v[q * 8 + 4], v[q * 8 + 5]), pack_bf2(v[q * 8 + 6], v[q * 8 + 7]));
-              }
-            } else {
-              for (int j = 0; j < 32 && n + j < a.N; ++j) {
-                float x = v[j];
-                if (a.res) x += bf2f(a.res[(size_t)m * a.ldy + n + j]);
-                if (a.out_f32) reinterpret_cast<float*>(a.Y)[(size_t)m * a.ldy + n + j] = x;
-                else Yb[(size_t)m * a.ldy + n + j] = f2bf(x);
-              }
+              for (int j = 0; j < 8; ++j)
+                if (nn + j < a.N) {
+                  const float x = a.res ? o[j] + bf2f(a.res[at + j]) : o[j];
+                  if (a.out_f32) reinterpret_cast<float*>(a.Y)[at + j] = x;
+                  else Yb[at + j] = f2bf(x);
+                }
             }
           }
         }
         tc_fence_before();
+        __syncwarp();
         if (lane == 0) mbar_arrive(&tempty_bar[buf]);
       } else {
         // lanes = output features, columns = token rows
@@ -737,7 +857,19 @@ static int round_up_pow2(int v) { int p = 32; while (p < v) p <<= 1; return p; }
 
 struct GemmPlan { GemmArgs a; int grid; size_t smem; };
 
-static int plan_gemm(GemmPlan& p, int M, int N, int K, int mode, int split_k, int sm_count, int fp8 = 0) {
+// bytes of workspace / ints of counters that the pieces of any tail fit: a CTA has one piece at most
+inline long gemm_tail_bytes(int sm_count) { return (long)(sm_count > 0 ? sm_count : 148) * GM_BM * 256 * (long)sizeof(float); }
+constexpr int GM_TAIL_CTRS = 148 * 32;
+
+// Normal orientation, tile width and tail (tail = 1: widths only; 2: the last tiles may be cut along K, workspace and counters are there). A k block
+// of a tile takes 0.26 us + 0.00066 us a column with every SM at work (L2 to shared memory, 50 to 56 bytes a clock and SM, and from 192 columns on
+// the tensor cores close to what the power limit sustains): cost bn + GM_KB_COST per k block and wave. What a fixed width of 256 lost is the last
+// wave: 2048 x 5120 x 17408 is 2.16 waves and took three. The rule takes the width with the cheapest sum of waves, and where the tiles of the
+// last, partial wave leave room it cuts them along K into pieces that the idle CTAs take; a piece's way through the workspace costs as much as
+// GM_TAIL_COST + GM_PIECE_COST x pieces k block units a column (3.3 us + 3.3 us a piece for 256 columns), so shallow products stay whole.
+// us, width 256 / best width / with pieces: 2048 x 5120 x 17408 348 / 319 / 288, 1111 rows of it 255 / 210 / 177, 300 rows 135 / 104 / 82, 140 rows
+// 128 / 100 / 66; 2048 x 5120 x 2048 53 / 47 / 55 (whole), 140 x 2048 x 4096 38 / 30 / 21. More than four pieces gained nothing.
+static int plan_gemm(GemmPlan& p, int M, int N, int K, int mode, int split_k, int sm_count, int fp8 = 0, int tail = 0) {
   GemmArgs& a = p.a;
   a.fp8 = fp8; a.scale_m = nullptr; a.scale_n = nullptr; a.out_f32 = 0; a.act = ACT_NONE; a.limit = 0.f;
   a.M = M; a.N = N; a.K = K;
@@ -753,11 +885,28 @@ static int plan_gemm(GemmPlan& p, int M, int N, int K, int mode, int split_k, in
     a.split_k = split_k < 1 ? 1 : split_k;
   } else {
     a.bn = (a.dual || N > 128) ? 256 : 128;
+    a.tail_split = 1;
+    if (tail) {
+      const int kb = (K + (fp8 ? 2 * GM_BK : GM_BK) - 1) / (fp8 ? 2 * GM_BK : GM_BK);
+      long best = -1;
+      for (int bn = 256; bn >= 64; bn -= a.dual ? 64 : 32) {
+        const int cols = a.dual ? bn / 2 : bn;
+        const long tiles = (long)((M + GM_BM - 1) / GM_BM) * ((N + cols - 1) / cols);
+        const int rest = (int)(tiles % sm_count);
+        const long full = tiles / sm_count * kb * (bn + GM_KB_COST);
+        for (int s = 1; s <= GM_TAIL_MAX; ++s) {
+          if (s > 1 && (tail < 2 || rest * s > sm_count || kb / s < 4)) break;
+          const int per = (kb + s - 1) / s;
+          const long cost = full + (rest ? (long)per * (bn + GM_KB_COST) + (s > 1 ? bn * (GM_TAIL_COST + s * GM_PIECE_COST) : 0) : 0);
+          if (best < 0 || cost < best) { best = cost; a.bn = bn; a.tail_split = (kb + per - 1) / per; a.tail_tiles = a.tail_split > 1 ? rest : 0; a.tail_kb = per; }
+        }
+      }
+    }
     a.n_a = 1;
     a.n_b = a.dual ? 2 : 1;
-    a.b_box_rows = a.dual ? 128 : a.bn;
+    a.b_box_rows = a.dual ? a.bn / 2 : a.bn;
     a.tiles_a = (M + GM_BM - 1) / GM_BM;
-    int ncols_out = a.dual ? 128 : a.bn;
+    int ncols_out = a.dual ? a.bn / 2 : a.bn;
     a.tiles_b = (N + ncols_out - 1) / ncols_out;
     a.split_k = 1;
   }
@@ -779,9 +928,12 @@ static int plan_gemm(GemmPlan& p, int M, int N, int K, int mode, int split_k, in
   if (a.stages > GM_MAX_STAGES) a.stages = GM_MAX_STAGES;
   if (a.stages < 2) return -5;
   // more than half the shared memory of an SM, so one CTA (and one TMEM allocation) per SM
-  p.smem = (size_t)a.stages * stage_bytes + 1024;
+  p.smem = (size_t)a.stages * stage_bytes + 1024 + (a.swap ? 0 : 4 * GM_EPI_BYTES);
   if (p.smem < 120 * 1024) p.smem = 120 * 1024;
   int total = a.tiles_a * a.tiles_b * a.split_k;
+  a.tail_first = total - a.tail_tiles;
+  if (a.tail_tiles == 0) { a.tail_first = 0x7fffffff; a.tail_split = 1; }
+  total += a.tail_tiles * (a.tail_split - 1);
   p.grid = total < sm_count ? total : sm_count;
   return 0;
 }

@@ -4,7 +4,8 @@
 using namespace fb;
 
 extern "C" long fb_gemm_workspace_bytes(int M, int N, int split_k) {
-  if (M > 64 || split_k <= 1) return 0;
+  if (M > 64) return gemm_tail_bytes(0);
+  if (split_k <= 1) return 0;
   int bn = ((M + 15) / 16) * 16;
   long tiles = (N + GM_BM - 1) / GM_BM;
   return tiles * split_k * 2L * bn * GM_BM * (long)sizeof(float);
@@ -20,7 +21,7 @@ extern "C" int fb_gemm_bf16_glu(void* Y, const void* X, const void* W, const voi
   if (K % 8 || ldx % 8 || (ldy % 8 && M > 64)) return -1;
   if (sm_count <= 0) sm_count = 148;
   GemmPlan p{};
-  int rc = plan_gemm(p, M, N, K, mode, split_k, sm_count);
+  int rc = plan_gemm(p, M, N, K, mode, split_k, sm_count, 0, workspace && counters && sm_count <= 148 ? 2 : 1);
   if (rc) return rc;
   GemmArgs& a = p.a;
   if (a.split_k > 1 && (!workspace || !counters)) return -6;
@@ -40,7 +41,7 @@ extern "C" int fb_gemm_bf16_glu(void* Y, const void* X, const void* W, const voi
   if (rc) return rc;
   static bool attr_done = false;
   if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
     if (e != cudaSuccess) return (int)e;
     attr_done = true;
   }
@@ -106,7 +107,7 @@ extern "C" int fb_gemm_fp8(void* Y, const void* Xq, const void* Wq, const float*
   if (K % 16 || (ldy % 8 && M > 64)) return -1;
   if (sm_count <= 0) sm_count = 148;
   GemmPlan p{};
-  int rc = plan_gemm(p, M, N, K, mode, split_k, sm_count, 1);
+  int rc = plan_gemm(p, M, N, K, mode, split_k, sm_count, 1, workspace && counters && sm_count <= 148 ? 2 : 1);
   if (rc) return rc;
   GemmArgs& a = p.a;
   if (a.split_k > 1 && (!workspace || !counters)) return -6;
@@ -126,7 +127,7 @@ extern "C" int fb_gemm_fp8(void* Y, const void* Xq, const void* Wq, const float*
   if (rc) return rc;
   static bool attr_done = false;
   if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
     if (e != cudaSuccess) return (int)e;
     attr_done = true;
   }

@@ -21,7 +21,7 @@ from .mixers import CudaMixers
 from .qweight import Exl3Weight, ExpertsFP4, GgufWeight, QWeight, StackWeight
 
 GEMV_MAX_ROWS = 8
-# CTAs per SM that the decode attention's key splits aim at, by head width (as many as are resident; four rows against 6000 keys each, 4 kv heads
+# CTAs per SM that the decode attention's key splits aim at, by head width (as many as are resident; four rows against 8000 keys each, 4 kv heads
 # of 256: 47 us, 97 with the splits of whole rows over one warp's keys)
 DECODE_KEYS_CTAS = {64: 4, 128: 2, 256: 1}
 MOE_PAIR_ROWS = 64     # up to this many rows (the largest graph-captured step) the experts run as per-pair GEMVs,
@@ -45,7 +45,9 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         self.sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
         self.status_word = torch.zeros(1, dtype=torch.int32, device=self.device)
         self._ws: Optional[torch.Tensor] = None
-        self._counters = torch.zeros(16384, dtype=torch.int32, device=self.device)
+        self._counters = torch.zeros(32768, dtype=torch.int32, device=self.device)
+        self._tail = None
+        self._tail_counters = torch.zeros(148 * 32, dtype=torch.int32, device=self.device)
         self.empty = torch.empty            # every output buffer of the ops comes from here (see enable_canaries)
         self._guarded = []
         self._dl_sync = torch.zeros(2, dtype=torch.int32, device=self.device)      # grid-barrier words of the persistent layer kernel
@@ -89,6 +91,16 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         """Debug aid (reference: canary-padded allocations, `crates/fe-cuda/src/lib.rs:299-343`): every output buffer the
         ops allocate gets 256 guard bytes in front and behind, filled with a pattern; `check_canaries()` verifies them, so
         a kernel that writes just past (or before) its output is caught at the step that did it. Eager steps only (the
+    def _gemm_scratch(self, M: int, N: int, split: int):
+        """Workspace and counters of a GEMM call: K splits of few rows, or (more than 64 rows) the last tiles' pieces. The latter have buffers of
+        their own, held by the first stream that asks; on any other stream such calls run without pieces."""
+        if M <= 64:
+            return (self._workspace(self.C.gemm_workspace_bytes(M, N, split)), self._counters) if split > 1 else (None, None)
+        stream = torch.cuda.current_stream(self.device).cuda_stream
+        if self._tail is None:
+            self._tail = (stream, torch.empty(self.C.gemm_workspace_bytes(M, N, 1) // 4, dtype=torch.float32, device=self.device))
+        return (self._tail[1], self._tail_counters) if self._tail[0] == stream else (None, None)
+
         guard zones of a captured graph are checked after replays as long as canaries stay enabled)."""
         self.empty = self._empty_guarded if on else torch.empty
         if not on:
@@ -257,11 +269,7 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         y = out if out is not None else self.empty(M, (N + 7) // 8 * 8, dtype=torch.float32 if out_f32 else self.dtype,
                                                     device=self.device)[:, :N]
         split = self._split_k(M, N, K) if M <= 64 else 1
-        ws = cnt = None
-        if split > 1:
-            nb = self.C.gemm_workspace_bytes(M, N, split)
-            ws = self._workspace(nb)
-            cnt = self._counters
+        ws, cnt = self._gemm_scratch(M, N, split)
         self.launches += 1
         self.C.gemm(y, x, w, res, (1 if swiglu else 0) | (2 if out_f32 else 0) | (4 if act else 0), split, ws, cnt, self.status_word)
         return y
@@ -285,10 +293,7 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         self.C.quant_fp8(xq, xs, x, norm_w, eps)
         y = self.empty(M, (N + 7) // 8 * 8, dtype=self.dtype, device=self.device)[:, :N]
         split = self._split_k(M, N, K // 2) if M <= 64 else 1
-        ws = cnt = None
-        if split > 1:
-            ws = self._workspace(self.C.gemm_workspace_bytes(M, N, split))
-            cnt = self._counters
+        ws, cnt = self._gemm_scratch(M, N, split)
         self.launches += 2
         self.C.gemm_fp8(y, xq, wq, xs, w_scale, res, 1 if swiglu else 0, split, ws, cnt, self.status_word)
         return y

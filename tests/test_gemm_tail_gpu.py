@@ -1,0 +1,71 @@
+"""Prompt-sized GEMMs whose tile width follows the shape and whose last tiles may be cut along K, against 64-bit sums."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.fixture(scope="module")
+def ops(ext):
+    from ferrite_b200.ops.cuda_ops import CudaOps
+    return CudaOps(DEV)
+
+
+def rnd(*shape, seed=0, scale=1.0):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    return (torch.randn(*shape, generator=g, device=DEV) * scale).to(torch.bfloat16)
+
+
+def plain(ops, x, w, mode, res=None):
+    """The same call without scratch: no pieces."""
+    N = w.shape[0] // 2 if mode & 1 else w.shape[0]
+    y = torch.empty(x.shape[0], (N + 7) // 8 * 8, dtype=torch.float32 if mode & 2 else torch.bfloat16, device=DEV)[:, :N]
+    ops.C.gemm(y, x, w, res, mode, 1, None, None, ops.status_word)
+    return y
+
+
+# widths that end in every part of a tile (one column, ragged 8s, multiples of 32 and 64), one tile, several waves; pieces: K deep enough for two
+# to four of them, also where the last piece is shorter (K = 4104: 65 k blocks)
+@pytest.mark.parametrize("M,N,K,pieces", [(65, 1, 64, False), (128, 100, 72, False), (129, 264, 1000, False), (1531, 5120, 264, False), (2048, 2500, 512, False),
+                                          (70, 1000, 8192, True), (140, 2048, 4104, True), (300, 1111, 8192, True), (1111, 5120, 8192, True)])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_widths_and_pieces(ops, M, N, K, pieces, swiglu):
+    x, w = rnd(M, K, seed=1), rnd((2 if swiglu else 1) * N, K, seed=2, scale=K ** -0.5)
+    want = x.double() @ w.double().t()
+    if swiglu:
+        want = torch.nn.functional.silu(want[:, :N]) * want[:, N:]
+    # 32-bit sums of products exact in 32 bits, outputs of size one; the oracle's size bounds what the activation passes on
+    bound = 2 ** -14 * max(1.0, want.abs().max().item())
+    y = ops.linear(x, w, swiglu=swiglu, out_f32=True)
+    assert (y.double() - want).abs().max().item() <= bound
+    assert torch.equal(y, ops.linear(x, w, swiglu=swiglu, out_f32=True))            # whichever piece comes last
+    whole = plain(ops, x, w, 3 if swiglu else 2)
+    assert (whole.double() - want).abs().max().item() <= bound
+    if pieces and not swiglu:
+        assert not torch.equal(y, whole)
+    if not swiglu:
+        res = rnd(M, N + 8 - N % 8, seed=3)[:, :N]                                  # the residual shares the output's leading dimension
+        y16 = torch.empty(M, N + 8 - N % 8, dtype=torch.bfloat16, device=DEV)[:, :N]
+        got = ops.linear(x, w, res=res, out=y16)
+        assert torch.equal(got, (y + res.float()).to(torch.bfloat16))
+        assert torch.equal(ops.linear(x, w, out_f32=True, act="relu2"), y.clamp_min(0).square())
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):                                                   # the scratch belongs to the first stream
+        assert torch.equal(ops.linear(x, w, swiglu=swiglu, out_f32=True), whole)
+    torch.cuda.synchronize()
+    assert ops.status() == 0 and int(ops._tail_counters.abs().sum()) == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 264, 1040), (140, 2048, 8208)])
+def test_scaled_fp8(ops, M, N, K):
+    x, w = rnd(M, K, seed=1), rnd(N, K, seed=2, scale=K ** -0.5)
+    wq, ws = ops.quantize_weight_fp8(w)
+    xq, xs = torch.empty(M, K, dtype=torch.uint8, device=DEV), torch.empty(M, device=DEV)
+    ops.C.quant_fp8(xq, xs, x, None, 1e-6)
+    f8 = lambda q: q.view(torch.float8_e4m3fn).double()
+    want = f8(xq) @ f8(wq).t() * xs.double()[:, None] * ws.double()
+    # tensor cores add e4m3 products in 32 bits or a little less; then one rounding to bf16
+    got = ops.linear_fp8(x, wq, ws).double()
+    assert ((got - want).abs() <= 2 ** -8 * want.abs() + 2 ** -9).all()
