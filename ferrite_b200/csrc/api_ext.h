@@ -136,7 +136,8 @@ long fb_ep_workspace_bytes(int n_experts, int hidden, long cap_rows);
 long fb_ep_recv_offset(int n_experts, int hidden, long cap_rows);
 long fb_ep_out_offset(int n_experts, int hidden, long cap_rows);
 int fb_ep_moe(void* out, int out_f32, float limit, const void* x, const int* ids, const float* wts, const void* w_gu, const void* w_down,
-              const void* shared, const float* shared_gate, long gate_ld, const void* res, void* act, int* plan, int rows, int top_k,
+              const void* sf_gu, const void* sf_down, float gs_gu, float gs_down, const void* shared, const float* shared_gate, long gate_ld,
+              const void* res, void* act, int* plan, int rows, int top_k,
               int n_experts, int hidden, int inter, long cap_rows, const void* const* peers, int rank, int world,
               uint32_t* ctr, int* status, unsigned spin_limit, int sm_count, cudaStream_t s);
 
@@ -144,6 +145,12 @@ int fb_ep_moe(void* out, int out_f32, float limit, const void* x, const int* ids
 int fb_gguf_dequant(void* out_bf16, const void* raw, int type, long n_values, cudaStream_t s);
 int fb_q8_1_quant(void* out, const void* x_bf16, long n_values, cudaStream_t s);
 int fb_gguf_gemv(void* y, const void* x, const void* raw, const void* res, int type, int M, int N, int K, long ldx,
+// ---- moe_stream.cu: experts of prompt-sized steps straight from their NVFP4 codes ----
+int fb_moe_stream_rows();
+int fb_moe_stream_fits(int N, int K, int experts);
+int fb_moe_stream(void* y, const void* x, const void* codes, const void* scales, float w_scale, const int* tile_start, const int* row_base, int experts,
+                  int cap_rows, int N, int K, long ldx, long ldy, int mode, float limit, int* status, int sm_count, cudaStream_t s);
+
                  long ldy, cudaStream_t s);
 
 // ---- exl3.cu: EXL3 trellis-quantised linears ----

@@ -360,13 +360,15 @@ int is_f32(const Tensor& t) {
 
 void ep_moe(const EpHandle& c, Tensor out, Tensor x, Tensor ids, Tensor wts, Tensor w_gu, Tensor w_down,
             c10::optional<Tensor> shared, c10::optional<Tensor> shared_gate, c10::optional<Tensor> res, Tensor act,
-            Tensor plan, double limit, bool add) {
-  int rows = (int)x.size(0), top_k = (int)ids.size(1), inter = (int)w_down.size(2);
+            Tensor plan, double limit, bool add, c10::optional<Tensor> sf_gu, c10::optional<Tensor> sf_down, double gs_gu, double gs_down) {
+  int rows = (int)x.size(0), top_k = (int)ids.size(1), inter = (int)w_down.size(2) * (sf_down ? 2 : 1);
+  TORCH_CHECK(w_gu.is_contiguous() && w_down.is_contiguous() && (!sf_gu || sf_gu->is_contiguous()) && (!sf_down || sf_down->is_contiguous()) &&
+              w_gu.size(1) == 2 * inter && w_down.size(1) == c.hidden && w_gu.size(2) * (sf_gu ? 2 : 1) == c.hidden, "ep_moe: expert stacks");
   TORCH_CHECK(plan.numel() >= (int64_t)rows * top_k + 3 * c.n_experts + 8, "ep_moe: plan scratch too small");
   TORCH_CHECK(act.numel() >= c.cap_rows * inter, "ep_moe: activation scratch too small");
   TORCH_CHECK(!shared_gate || (is_f32(*shared_gate) && shared_gate->dim() == 1 && shared_gate->size(0) == rows), "ep_moe: gates of the shared expert");
   check(fb_ep_moe(out.data_ptr(), is_f32(out) ? (add ? 1 : 2) : 0, (float)limit, x.data_ptr(), ids.data_ptr<int>(), wts.data_ptr<float>(), w_gu.data_ptr(),
-                  w_down.data_ptr(), cptr(shared), shared_gate.has_value() ? shared_gate->data_ptr<float>() : nullptr,
+                  w_down.data_ptr(), cptr(sf_gu), cptr(sf_down), (float)gs_gu, (float)gs_down, cptr(shared), shared_gate.has_value() ? shared_gate->data_ptr<float>() : nullptr,
                   shared_gate.has_value() ? (long)shared_gate->stride(0) : 0, cptr(res), act.data_ptr(), plan.data_ptr<int>(), rows, top_k, c.n_experts, c.hidden, inter, c.cap_rows,
                   c.peers.data(), c.rank, c.world, (uint32_t*)c.ctr.data_ptr(), c.status.data_ptr<int>(), c.spin_limit,
                   c.sm, cur_stream()), "ep_moe");
@@ -999,7 +1001,9 @@ void register_ext(pybind11::module_& m) {
   m.def("ep_workspace_bytes", [](int64_t e, int64_t h, int64_t cap) { return (int64_t)fb_ep_workspace_bytes((int)e, (int)h, cap); });
   m.def("ep_moe", &ep_moe, pybind11::arg("comm"), pybind11::arg("out"), pybind11::arg("x"), pybind11::arg("ids"), pybind11::arg("wts"), pybind11::arg("w_gu"),
         pybind11::arg("w_down"), pybind11::arg("shared"), pybind11::arg("shared_gate"), pybind11::arg("res"), pybind11::arg("act"), pybind11::arg("plan"),
-        pybind11::arg("limit") = 0.0, pybind11::arg("add") = true);
+        pybind11::arg("limit") = 0.0, pybind11::arg("add") = true, pybind11::arg("sf_gu") = pybind11::none(), pybind11::arg("sf_down") = pybind11::none(),
+        pybind11::arg("gs_gu") = 1.0, pybind11::arg("gs_down") = 1.0);
+  m.def("moe_stream_fits", &fb_moe_stream_fits);
   m.def("gemm_grouped", &gemm_grouped);
   m.def("gemm_batched", &gemm_batched);
   m.def("head_linear", &head_linear);

@@ -25,7 +25,7 @@
 // pair sort (`ggq_moe_sort_*`, `kernels/k-gguf/src/sort.rs`) and ownership masks (`fx_mask_own`,
 // `kernels/k-fnext/src/fast.rs:1718`). No TMA or bulk copy touches peer memory; every wait is bounded.
 #include "api_ext.h"
-#include "common.cuh"
+#include "stream_mma.cuh"
 
 namespace fb {
 
@@ -61,10 +61,11 @@ __device__ __forceinline__ __nv_bfloat16* ep_out(void* base, const EpComm& c) {
 
 // ---- 1. plan ---------------------------------------------------------------------------------------------------
 // pos[pair]: position of the pair inside its (this rank, expert) bucket; send_off[e]: first row of this rank's
-// bucket for expert e inside the owner's buffers; row_base / tile_start: prefix sums over the experts this rank owns.
+// bucket for expert e inside the owner's buffers; row_base / tile_start: prefix sums over the experts this rank owns, of rows and of what
+// multiplies them at once (tile_rows).
 __global__ void __launch_bounds__(1024) ep_plan_kernel(EpComm c, const int* __restrict__ ids, int n_pairs,
                                                        int* __restrict__ pos, int* __restrict__ send_off,
-                                                       int* __restrict__ row_base, int* __restrict__ tile_start) {
+                                                       int* __restrict__ row_base, int* __restrict__ tile_start, int tile_rows) {
   __shared__ int hist[EP_MAX_EXPERTS];
   __shared__ int rows_e[EP_MAX_EXPERTS];
   __shared__ int before_me[EP_MAX_EXPERTS];
@@ -111,7 +112,7 @@ __global__ void __launch_bounds__(1024) ep_plan_kernel(EpComm c, const int* __re
       send_off[e] = acc + before_me[e];
       if (tid == c.rank) { row_base[j] = acc; tile_start[j] = tiles; }
       acc += rows_e[e];
-      tiles += (rows_e[e] + 127) / 128;
+      tiles += (rows_e[e] + tile_rows - 1) / tile_rows;
     }
     if (tid == c.rank) {
       row_base[c.per_rank] = acc;
@@ -124,7 +125,7 @@ __global__ void __launch_bounds__(1024) ep_plan_kernel(EpComm c, const int* __re
 // ---- 2. dispatch -----------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) ep_dispatch_kernel(EpComm c, const __nv_bfloat16* __restrict__ x,
                                                           const int* __restrict__ ids, const int* __restrict__ pos,
-                                                          const int* __restrict__ send_off, int n_pairs, int top_k) {
+                                                          const int* __restrict__ send_off, int n_pairs, int top_k, int pieces) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int pair = blockIdx.x * 8 + warp;
   if (pair < n_pairs) {
@@ -133,7 +134,7 @@ __global__ void __launch_bounds__(256) ep_dispatch_kernel(EpComm c, const __nv_b
     if (row < c.cap_rows) {
       const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)(pair / top_k) * c.hidden);
       uint4* dst = reinterpret_cast<uint4*>(ep_recv(c.peer[o], c) + (size_t)row * c.hidden);
-      for (int i = lane; i < c.hidden / 8; i += 32) dst[i] = src[i];
+      for (int i = lane; i < c.hidden / 8; i += 32) dst[i] = pieces ? sm_piece(src[i]) : src[i];
     }
   }
   // the last CTA to finish tells every owner that this rank's rows are in place
@@ -258,13 +259,16 @@ extern "C" long fb_ep_out_offset(int n_experts, int hidden, long cap_rows) { ret
 
 // One expert-parallel MoE block over this rank's `rows` tokens. `act` is scratch [cap_rows][inter] bf16; `plan` is int
 // scratch of rows * top_k + 3 * n_experts + 8 entries. w_gu / w_down hold only the experts this rank owns. out_f32: `out` holds
-// fp32 rows, 1: to which the experts' sum is added, 2: which take it. limit: of clamped gated units (0: SwiGLU).
+// fp32 rows, 1: to which the experts' sum is added, 2: which take it. limit: of clamped gated units (0: SwiGLU). sf_gu, sf_down: the stacks are
+// e2m1 codes with these block scales and the tensor scales gs_gu, gs_down (moe_stream.cu; null: bf16, grouped tcgen05 GEMMs).
 extern "C" int fb_ep_moe(void* out, int out_f32, float limit, const void* x, const int* ids, const float* wts, const void* w_gu, const void* w_down,
-                         const void* shared, const float* shared_gate, long gate_ld, const void* res, void* act, int* plan, int rows,
+                         const void* sf_gu, const void* sf_down, float gs_gu, float gs_down, const void* shared, const float* shared_gate, long gate_ld, const void* res, void* act, int* plan, int rows,
                          int top_k, int n_experts, int hidden, int inter, long cap_rows, const void* const* peers, int rank,
                          int world, uint32_t* ctr, int* status, unsigned spin_limit, int sm_count, cudaStream_t s) {
   if (world < 1 || world > EP_MAX_RANKS || n_experts > EP_MAX_EXPERTS || n_experts % world || hidden % 8 || inter % 8)
     return -1;
+  const bool fp4 = sf_gu && sf_down;
+  if (fp4 && (!fb_moe_stream_fits(inter, hidden, n_experts / world) || !fb_moe_stream_fits(hidden, inter, n_experts / world))) return -1;
   EpLayout l = ep_layout(n_experts, hidden, cap_rows);
   EpComm c;
   for (int i = 0; i < EP_MAX_RANKS; ++i) c.peer[i] = i < world ? const_cast<void*>(peers[i]) : nullptr;
@@ -276,18 +280,27 @@ extern "C" int fb_ep_moe(void* out, int out_f32, float limit, const void* x, con
   int* send_off = pos + n_pairs;
   int* row_base = send_off + n_experts;
   int* tile_start = row_base + c.per_rank + 1;
-  ep_plan_kernel<<<1, 1024, 0, s>>>(c, ids, n_pairs, pos, send_off, row_base, tile_start);
+  ep_plan_kernel<<<1, 1024, 0, s>>>(c, ids, n_pairs, pos, send_off, row_base, tile_start, fp4 ? fb_moe_stream_rows() : 128);
   const int dgrid = n_pairs > 0 ? (n_pairs + 7) / 8 : 1;
-  ep_dispatch_kernel<<<dgrid, 256, 0, s>>>(c, (const __nv_bfloat16*)x, ids, pos, send_off, n_pairs, top_k);
+  ep_dispatch_kernel<<<dgrid, 256, 0, s>>>(c, (const __nv_bfloat16*)x, ids, pos, send_off, n_pairs, top_k, fp4 ? 1 : 0);
   ep_wait_kernel<<<1, 32, 0, s>>>(c);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   const char* local = reinterpret_cast<const char*>(peers[rank]);
-  int rc = fb_gemm_grouped(act, local + l.recv_off, w_gu, tile_start, row_base, c.per_rank, (int)cap_rows, inter, hidden,
-                           hidden, inter, 1, limit, status, sm_count, s);
-  if (rc) return rc;
-  rc = fb_gemm_grouped(const_cast<char*>(local) + l.out_off, act, w_down, tile_start, row_base, c.per_rank, (int)cap_rows,
-                       hidden, inter, inter, hidden, 0, 0.f, status, sm_count, s);
+  char* rows_out = const_cast<char*>(local) + l.out_off;
+  int rc;
+  if (fp4) {
+    rc = fb_moe_stream(act, local + l.recv_off, w_gu, sf_gu, gs_gu, tile_start, row_base, c.per_rank, (int)cap_rows, inter, hidden, hidden, inter, 1, limit,
+                       status, sm_count, s);
+    if (rc) return rc;
+    rc = fb_moe_stream(rows_out, act, w_down, sf_down, gs_down, tile_start, row_base, c.per_rank, (int)cap_rows, hidden, inter, inter, hidden, 0, 0.f,
+                       status, sm_count, s);
+  } else {
+    rc = fb_gemm_grouped(act, local + l.recv_off, w_gu, tile_start, row_base, c.per_rank, (int)cap_rows, inter, hidden, hidden, inter, 1, limit, status,
+                         sm_count, s);
+    if (rc) return rc;
+    rc = fb_gemm_grouped(rows_out, act, w_down, tile_start, row_base, c.per_rank, (int)cap_rows, hidden, inter, inter, hidden, 0, 0.f, status, sm_count, s);
+  }
   if (rc) return rc;
   ep_signal_kernel<<<1, 32, 0, s>>>(c);
   ep_combine_kernel<<<rows > 0 ? rows : 1, 256, 0, s>>>(c, (__nv_bfloat16*)out, out_f32 ? (float*)out : nullptr, ids, wts, pos, send_off,

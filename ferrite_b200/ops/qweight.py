@@ -82,7 +82,8 @@ def quantize_weight(w: torch.Tensor, kind: str = "nvfp4", keep_dense: bool = Tru
 class ExpertsFP4:
     """Stacked expert matrices [experts, rows, cols] in NVFP4: `packed` uint8 [E, rows, cols/2] (low nibble = even
     element), `scales` uint8 [E, rows, cols/16] holding e4m3 bits, one `global_scale` for the whole stack. Decode rows
-    stream this form (`csrc/moe_fp4.cu`); prompt-sized steps dequantise it into a bf16 scratch for the grouped GEMM."""
+    stream this form (`csrc/moe_fp4.cu`), prompt-sized steps too where experts get few rows each (`csrc/moe_stream.cu`); beyond, it is
+    dequantised into a bf16 scratch for the grouped GEMM."""
     packed: torch.Tensor
     scales: torch.Tensor
     global_scale: float

@@ -14,6 +14,8 @@ from typing import Optional
 import torch
 import torch.distributed as dist
 
+from ..ops.qweight import ExpertsFP4
+
 
 class ExpertParallel:
     def __init__(self, tp, device, n_experts: int, hidden: int, cap_rows: int, spin_limit: int = 0, status=None):
@@ -54,6 +56,18 @@ class ExpertParallel:
             raise RuntimeError(f"expert-parallel rank {self.rank}: status {int(self.status.item())} "
                                "(2 = a peer wait ran out, 5 = receive buffer capacity exceeded)")
 
+    CODE_ROWS = 96
+
+    def takes_codes(self, pairs: int, w_gu, w_down) -> bool:
+        """Whether NVFP4 stacks are multiplied as they are (`csrc/moe_stream.cu`) rather than as bf16 copies by the grouped tcgen05 GEMM: with
+        up to CODE_ROWS rows per expert. Unpacking again for every 32 rows costs 0.2 us per expert of 3 x 2048 x 512 there; the copies and
+        128-row tiles cost 4.2 us an expert however few rows it has, and tiles that are full win. One rank only: the order of the values in
+        the dispatched rows depends on the answer, which ranks with different row counts could give differently."""
+        e, rows, hidden = w_gu.shape
+        return (self.fused and self.world == 1 and w_down.shape[2] % 256 == 0 and bool(self.C.moe_stream_fits(rows // 2, hidden, self.n_experts))
+                and bool(self.C.moe_stream_fits(hidden, w_down.shape[2], self.n_experts))
+                and pairs <= self.CODE_ROWS * self.n_experts)
+
     def moe(self, ops, h, ids, wts, w_gu, w_down, shared=None, shared_gate=None, res=None, acc=None, add=True, limit=0.0):
         """out[t] = res[t] + shared[t] * sigmoid(shared_gate[t]) + sum_k wts[t, k] * expert_{ids[t, k]}(h[t]) for this
         rank's token rows; w_gu / w_down hold the experts this rank owns. `acc` (fp32 rows): the sum is added to it, or with `add` off
@@ -61,6 +75,13 @@ class ExpertParallel:
         self.calls += 1
         T, K = ids.shape
         inter = w_down.shape[2]
+        codes = {}
+        if isinstance(w_gu, ExpertsFP4):
+            if self.takes_codes(T * K, w_gu, w_down):
+                codes = dict(sf_gu=w_gu.scales, sf_down=w_down.scales, gs_gu=w_gu.global_scale, gs_down=w_down.global_scale)
+                w_gu, w_down = w_gu.packed, w_down.packed
+            else:
+                w_gu, w_down = ops.experts_dense(w_gu, 0), ops.experts_dense(w_down, 1)
         if self.fused:
             assert T * K <= self.cap_rows or self.world > 1, f"{T * K} (token, expert) pairs, room for {self.cap_rows}"
             if self._act is None or self._act.numel() < self.cap_rows * inter:
@@ -73,7 +94,7 @@ class ExpertParallel:
             if sg is not None and (sg.dim() != 1 or sg.dtype != torch.float32):
                 sg = sg.reshape(-1).float().contiguous()
             self.C.ep_moe(self.handle, out, h.contiguous(), ids.contiguous(), wts.contiguous(), w_gu, w_down, shared, sg,
-                          res, self._act, self._plan, limit, add)
+                          res, self._act, self._plan, limit, add, **codes)
             ops.launches += 7
             return out
         # process-group statement of the same block

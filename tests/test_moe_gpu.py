@@ -213,3 +213,46 @@ def test_moe_engine_nvfp4_experts(ext):
                                     reduction="batchmean").item()
     assert kl < 2e-2, kl
     eng.check()
+
+
+@pytest.mark.parametrize("E,K,H,I", [(16, 4, 512, 256), (6, 2, 256, 256), (40, 3, 768, 512)])
+@pytest.mark.parametrize("T", [1, 31, 65, 200])
+@pytest.mark.parametrize("limit", [0.0, 3.0])
+def test_prompt_experts_from_their_codes(ops, E, K, H, I, T, limit):
+    """Prompt-sized rows against NVFP4 stacks multiplied as they are (no bf16 copy): experts without rows, with one, around and over the 32
+    rows of a work item (all tokens on one expert's list), every code and scale; against math in 64 bits on the dequantised values."""
+    from ferrite_b200.ops.qweight import ExpertsFP4
+    from ferrite_b200.parallel.ep import ExpertParallel
+    g = torch.Generator(device=DEV).manual_seed(E * 7 + T)
+    def stack(rows, cols):
+        scales = torch.randint(0, 120, (E + 1, rows, cols // 16), generator=g, device=DEV, dtype=torch.uint8)
+        return ExpertsFP4(torch.randint(0, 256, (E + 1, rows, cols // 2), generator=g, device=DEV, dtype=torch.uint8), scales, 2.0 ** -13)
+    w_gu, w_dn = stack(2 * I, H), stack(H, I)
+    h = (torch.randn(T, H, generator=g, device=DEV) * 0.3).to(torch.bfloat16)
+    ids = torch.stack([torch.randperm(E - 1, generator=g, device=DEV)[:K] for _ in range(T)]).to(torch.int32)        # the last expert has no rows
+    ids[:, 0] = 0                                                                                                    # the first one all of them
+    ids[:, 1:] = torch.where(ids[:, 1:] == 0, torch.full_like(ids[:, 1:], E - 2), ids[:, 1:])
+    wts = torch.rand(T, K, generator=g, device=DEV)
+    ep = ExpertParallel(None, DEV, E, H, cap_rows=T * K)
+    assert T * K > ExpertParallel.CODE_ROWS * E or ep.takes_codes(T * K, w_gu, w_dn)
+    acc = torch.zeros(T, H, dtype=torch.float32, device=DEV)
+    launches = ops._expert_scratch.copy()
+    ep.moe(ops, h, ids, wts, w_gu, w_dn, acc=acc, limit=limit)
+    assert ops._expert_scratch.keys() == launches.keys()                                                             # no bf16 copies
+    gu, dn = w_gu.dequantize(torch.float64), w_dn.dequantize(torch.float64)
+    want, mag = torch.zeros(T, H, dtype=torch.float64, device=DEV), torch.zeros(T, H, dtype=torch.float64, device=DEV)
+    for t in range(T):
+        for k in range(K):
+            e = int(ids[t, k])
+            y = gu[e] @ h[t].double()
+            a, b = y[:I], y[I:]
+            if limit:
+                a = a.clamp(max=limit)
+                act = a * torch.sigmoid(1.702 * a) * (b.clamp(-limit, limit) + 1)
+            else:
+                act = a * torch.sigmoid(a) * b
+            want[t] += float(wts[t, k]) * (dn[e] @ act)
+            mag[t] += float(wts[t, k]) * (dn[e].abs() @ act.abs())
+    # roundings to bf16 of the activation and of an expert's row (2^-9 each), on top of 32-bit sums
+    assert bool(((acc.double() - want).abs() <= 2 ** -7 * mag + 1e-6).all())
+    ep.check()
