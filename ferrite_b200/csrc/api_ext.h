@@ -63,6 +63,10 @@ int fb_gemm_nvfp4_swiglu_q(void* q_codes, void* q_sf, float* q_row_scale, float 
                            const float* row_scale, const void* Wq, const void* w_sf, float w_scale, int M, int N, int K,
                            int* status, int sm_count, cudaStream_t s);
 
+// ---- gemv_stream.cu: products of up to 32 rows, bf16 or NVFP4 weights streamed through a TMA ring ----
+int fb_gemv_stream(void* y, const void* x, const void* w, const void* sf, float w_scale, const float* row_alpha, const void* norm_w, const void* res,
+                   int M, int N, int K, long ldx, long ldy, float eps, int mode, int out_f32, float* ws, long ws_floats, int* counters, int n_counters,
+                   int* status, int sm_count, cudaStream_t s);
 // ---- gemv_nvfp4_tc.cu: few-row NVFP4 linear on the block-scaled tensor cores, activations as residual NVFP4 terms ----
 long fb_gemv_nvfp4_tc_workspace_bytes(int M, int N, int K, int dual, int terms, int sm_count, int ctas_per_sm);
 int fb_gemv_nvfp4_tc_terms(int M, int N, int K, int dual, int terms);
@@ -141,16 +145,16 @@ int fb_ep_moe(void* out, int out_f32, float limit, const void* x, const int* ids
               int n_experts, int hidden, int inter, long cap_rows, const void* const* peers, int rank, int world,
               uint32_t* ctr, int* status, unsigned spin_limit, int sm_count, cudaStream_t s);
 
-// ---- gguf_quant.cu: GGUF block formats ----
-int fb_gguf_dequant(void* out_bf16, const void* raw, int type, long n_values, cudaStream_t s);
-int fb_q8_1_quant(void* out, const void* x_bf16, long n_values, cudaStream_t s);
-int fb_gguf_gemv(void* y, const void* x, const void* raw, const void* res, int type, int M, int N, int K, long ldx,
 // ---- moe_stream.cu: experts of prompt-sized steps straight from their NVFP4 codes ----
 int fb_moe_stream_rows();
 int fb_moe_stream_fits(int N, int K, int experts);
 int fb_moe_stream(void* y, const void* x, const void* codes, const void* scales, float w_scale, const int* tile_start, const int* row_base, int experts,
                   int cap_rows, int N, int K, long ldx, long ldy, int mode, float limit, int* status, int sm_count, cudaStream_t s);
 
+// ---- gguf_quant.cu: GGUF block formats ----
+int fb_gguf_dequant(void* out_bf16, const void* raw, int type, long n_values, cudaStream_t s);
+int fb_q8_1_quant(void* out, const void* x_bf16, long n_values, cudaStream_t s);
+int fb_gguf_gemv(void* y, const void* x, const void* raw, const void* res, int type, int M, int N, int K, long ldx,
                  long ldy, cudaStream_t s);
 
 // ---- exl3.cu: EXL3 trellis-quantised linears ----

@@ -84,17 +84,6 @@ void gemm(Tensor Y, Tensor X, Tensor W, c10::optional<Tensor> res, int64_t mode,
                      (int*)mptr(status), sm_count(), cur_stream()), "gemm");
 }
 
-void gemv_mma(Tensor Y, Tensor X, Tensor W, c10::optional<Tensor> norm_w, c10::optional<Tensor> res, double eps,
-              int64_t mode, c10::optional<Tensor> workspace, c10::optional<Tensor> counters) {
-  int M = (int)X.size(0), K = (int)X.size(1);
-  int N = (int)(mode == 1 ? W.size(0) / 2 : W.size(0));
-  long wsf = workspace.has_value() ? (long)(workspace->numel() * workspace->element_size() / 4) : 0;
-  int nc = counters.has_value() ? (int)counters->numel() : 0;
-  check(fb_gemv_mma(Y.data_ptr(), X.data_ptr(), W.data_ptr(), cptr(norm_w), cptr(res), M, N, K, (long)X.stride(0),
-                    (long)Y.stride(0), (float)eps, (int)mode, Y.scalar_type() == torch::kFloat32 ? 1 : 0,
-                    (float*)mptr(workspace), wsf, (int*)mptr(counters), nc, sm_count(), cur_stream()), "gemv_mma");
-}
-
 void quant_fp8(Tensor q, Tensor scale, Tensor x, c10::optional<Tensor> norm_w, double eps) {
   check(fb_quant_fp8(q.data_ptr(), scale.data_ptr<float>(), x.data_ptr(), cptr(norm_w), (int)x.size(0), (int)x.size(1),
                      (long)x.stride(0), (float)eps, cur_stream()), "quant_fp8");
@@ -230,6 +219,17 @@ int64_t attn_decode_mma(Tensor out, Tensor o_part, Tensor ml_part, Tensor q, Ten
                         c10::optional<Tensor> kv_scale) {
   int rc = fb_attn_decode_mma(out.data_ptr(), o_part.data_ptr<float>(), ml_part.data_ptr<float>(), q.data_ptr(),
                               k_cache.data_ptr(), v_cache.data_ptr(), (const float*)cptr(kv_scale), proj.data_ptr(),
+                              (long)proj.stride(0),
+                              seg_slot.data_ptr<int>(), seg_row0.data_ptr<int>(), seg_nrows.data_ptr<int>(),
+                              row_kvlen.data_ptr<int>(), (const int*)cptr(row_base),
+                              (const unsigned long long*)cptr(row_mask), block_table.data_ptr<int>(),
+                              (int)block_table.size(1), (int)kv_block, (int)seg_slot.numel(), (int)max_rows,
+                              (int)row_kvlen.numel(), (int)nq, (int)nkv, (int)hd, (int)nsplit, gated ? 1 : 0, 0.f, 0, nullptr, 0, cur_stream());
+  if (rc == -20) return rc;
+  check(rc, "attn_decode_mma");
+  return 0;
+}
+
 // The same without ancestor masks, keys split over the warps of a CTA.
 int64_t attn_decode_keys(Tensor out, Tensor o_part, Tensor ml_part, Tensor q, Tensor k_cache, Tensor v_cache, Tensor proj, Tensor seg_slot,
                          Tensor seg_row0, Tensor seg_nrows, int64_t max_rows, Tensor row_kvlen, Tensor block_table, int64_t kv_block, int64_t nq,
@@ -244,17 +244,6 @@ int64_t attn_decode_keys(Tensor out, Tensor o_part, Tensor ml_part, Tensor q, Te
   check(rc, "attn_decode_keys");
   check(fb_attn_combine(out.data_ptr(), o_part.data_ptr<float>(), ml_part.data_ptr<float>(), proj.data_ptr(), (long)proj.stride(0), rows, (int)nq, (int)hd,
                         (int)nsplit, gated ? 1 : 0, cur_stream()), "attn_combine");
-  return 0;
-}
-
-                              (long)proj.stride(0),
-                              seg_slot.data_ptr<int>(), seg_row0.data_ptr<int>(), seg_nrows.data_ptr<int>(),
-                              row_kvlen.data_ptr<int>(), (const int*)cptr(row_base),
-                              (const unsigned long long*)cptr(row_mask), block_table.data_ptr<int>(),
-                              (int)block_table.size(1), (int)kv_block, (int)seg_slot.numel(), (int)max_rows,
-                              (int)row_kvlen.numel(), (int)nq, (int)nkv, (int)hd, (int)nsplit, gated ? 1 : 0, 0.f, 0, nullptr, 0, cur_stream());
-  if (rc == -20) return rc;
-  check(rc, "attn_decode_mma");
   return 0;
 }
 
@@ -451,7 +440,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemv", &gemv);
   m.def("gemm", &gemm);
   m.def("gemm_workspace_bytes", &gemm_workspace_bytes);
-  m.def("attn_decode_keys", &attn_decode_keys);
   m.def("attn_prep", &attn_prep);
   m.def("attn_decode", &attn_decode);
   m.def("attn_prefill", &attn_prefill);
@@ -463,12 +451,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("vdim") = 0, py::arg("eps") = 0.0, py::arg("k_mean") = py::none(), py::arg("v_mean") = py::none(),
         py::arg("mean_start") = py::none(), py::arg("pool") = 0);
   m.def("attn_decode_mma", &attn_decode_mma);
+  m.def("attn_decode_keys", &attn_decode_keys);
   m.def("gdn_conv", &gdn_conv);
   m.def("gdn_rec", &gdn_rec);
   m.def("gdn_conv_tree", &gdn_conv_tree);
   m.def("gdn_rec_tree", &gdn_rec_tree);
   m.def("kv_dequant", &kv_dequant);
-  m.def("gemv_mma", &gemv_mma);
   m.def("gdn_step", &gdn_step);
   m.def("quant_fp8", &quant_fp8);
   m.def("gemm_fp8", &gemm_fp8);

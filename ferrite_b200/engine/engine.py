@@ -123,12 +123,14 @@ class Engine:
         else:
             from ..ops.torch_ops import TorchOps
             ops = TorchOps(self.device, self.dtype)
-        # "nvfp4": few-row steps multiply the packed weights on the block-scaled tensor cores with the activations expanded
-        #   into residual NVFP4 renderings (16-bit-activation accuracy); prompt-sized steps take the dequantised copy;
-        # "nvfp4-w4a4": weights and activations in NVFP4 for every row count (prompt rows: one rendering);
+        # "nvfp4": steps of up to 8 rows stream the codes and unpack them in registers against 16-bit activations, or, where one or two rows meet
+        #   large weights, multiply them on the block-scaled tensor cores with the activations as three residual NVFP4 renderings (16-bit
+        #   accuracy); prompt-sized steps take the dequantised copy;
+        # "nvfp4-w4a4": weights and activations in NVFP4 for every row count (few rows: up to three renderings, prompt rows: one);
         # "nvfp4-a16": NVFP4 weights against 16-bit activations on the SIMT GEMV for decode rows, dense copy for prompts
         if on_gpu:
-            ops.fp4_act = self.ecfg.weight_dtype in ("nvfp4", "nvfp4-w4a4")
+            ops.fp4_act = self.ecfg.weight_dtype == "nvfp4-w4a4"
+            ops.fp4_rows = self.ecfg.weight_dtype == "nvfp4" and world == 1
             ops.fp4_prompt = self.ecfg.weight_dtype == "nvfp4-w4a4"
             if world > 1:
                 # a rank's shard of a projection is too small for the tensor-core kernel's fixed cost to pay: few-row
@@ -138,7 +140,7 @@ class Engine:
         self.tp = tp
         if tp is not None and tp.world > 1 and self.ecfg.seq_parallel and tp.sp_max is None:
             tp.setup_big(self.ecfg.max_step_rows, cfg.hidden)
-        if on_gpu and ops.fp4_act and world == 1:
+        if on_gpu and (ops.fp4_act or ops.fp4_rows) and world == 1:
             # execution order of the NVFP4 linears, so that each few-row call can prefetch the next one's weights
             from ..ops.qweight import QWeight
             order = []

@@ -26,6 +26,11 @@ GEMV_MAX_ROWS = 8
 DECODE_KEYS_CTAS = {64: 4, 128: 2, 256: 1}
 MOE_PAIR_ROWS = 64     # up to this many rows (the largest graph-captured step) the experts run as per-pair GEMVs,
                        # beyond as grouped GEMMs, which read the per-expert row counts on the host
+# NVFP4 weights of so many 128 x 256 units and more against one or two rows run on the block-scaled tensor cores (activations as three residual
+# renderings), smaller ones on the row kernel that unpacks the codes: it starts faster and unpacks 1.6 us a unit and CTA. One row, us: 17408 x 2 x
+# 5120 (5440 units) 30.5 / 34.5, 151936 x 5120 (23740) 79 / 127, 14336 x 5120 (2240) 20.5 / 20.6, 8224 x 5120 (1300) 18.9 / 15.2,
+# 5120 x 2048 (320) 11.8 / 7.8.
+FP4_TC_UNITS = 2560
 
 
 class CudaOps(CudaLatent, CudaMixers, CudaExtras):
@@ -57,7 +62,7 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         self.force_gemv_chunks = False      # debug: run any row count through 8-row GEMV passes
         self.launches = 0                   # kernels launched (or recorded into a graph) through this object
         self.moe_pair_rows = MOE_PAIR_ROWS
-        self.mma_gemv_rows = (2, 32)        # row counts routed to the mma.sync weight-streaming kernel
+        self.mma_gemv_rows = (2, 32)        # row counts routed to the mma.sync weight-streaming kernel (`gemv_stream`)
         self.attn_mma = os.environ.get("FB_ATTN_MMA", "1") != "0"   # decode attention on mma.sync (0: SIMT kernel)
         self.attn_tc = os.environ.get("FB_ATTN_TC", "1") != "0"     # prompt attention on tcgen05 (0: mma.sync kernel)
         self._gdn_scratch = None
@@ -65,6 +70,8 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         self._expert_scratch = {}
         self._kv_scratch = None
         self.fp4_act = False                # NVFP4 weights: quantise activations too and use the tcgen05 GEMM
+        self.fp4_rows = False               # ... only where one or two rows meet large weights (FP4_TC_UNITS), and other few-row steps unpack
+                                            # the codes in registers (`gemv_stream`)
         self.fp4_prompt = False             # ... for prompt-sized steps too (one NVFP4 rendering per activation row)
         self.fp4_terms = 3                  # few-row NVFP4 steps: NVFP4 renderings per activation row (0 = older fused kernel,
                                             # -1 = the SIMT GEMV with 16-bit activations)
@@ -84,13 +91,6 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
             self._ws = self.empty(max(nbytes // 4, 16 << 20), dtype=torch.float32, device=self.device)   # 64 MB up front: graphs keep the pointer
         return self._ws
 
-    # ---- debug: canary-padded output buffers --------------------------------------------------------------
-    CANARY_BYTES, CANARY_BYTE = 256, 0xA5
-
-    def enable_canaries(self, on: bool = True) -> None:
-        """Debug aid (reference: canary-padded allocations, `crates/fe-cuda/src/lib.rs:299-343`): every output buffer the
-        ops allocate gets 256 guard bytes in front and behind, filled with a pattern; `check_canaries()` verifies them, so
-        a kernel that writes just past (or before) its output is caught at the step that did it. Eager steps only (the
     def _gemm_scratch(self, M: int, N: int, split: int):
         """Workspace and counters of a GEMM call: K splits of few rows, or (more than 64 rows) the last tiles' pieces. The latter have buffers of
         their own, held by the first stream that asks; on any other stream such calls run without pieces."""
@@ -101,6 +101,13 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
             self._tail = (stream, torch.empty(self.C.gemm_workspace_bytes(M, N, 1) // 4, dtype=torch.float32, device=self.device))
         return (self._tail[1], self._tail_counters) if self._tail[0] == stream else (None, None)
 
+    # ---- debug: canary-padded output buffers --------------------------------------------------------------
+    CANARY_BYTES, CANARY_BYTE = 256, 0xA5
+
+    def enable_canaries(self, on: bool = True) -> None:
+        """Debug aid (reference: canary-padded allocations, `crates/fe-cuda/src/lib.rs:299-343`): every output buffer the
+        ops allocate gets 256 guard bytes in front and behind, filled with a pattern; `check_canaries()` verifies them, so
+        a kernel that writes just past (or before) its output is caught at the step that did it. Eager steps only (the
         guard zones of a captured graph are checked after replays as long as canaries stay enabled)."""
         self.empty = self._empty_guarded if on else torch.empty
         if not on:
@@ -236,6 +243,13 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
                     and w.mma_scales is not None and w.cols % 256 == 0 and (not out_f32 or M <= 8)
                     and (not swiglu or N % 128 == 0) and (M <= 64 or N % 8 == 0)):
                 return self._linear_w4a4(x, w, norm_w, eps, res, swiglu, M, N, out_f32)
+            if self.fp4_rows and M <= GEMV_MAX_ROWS and out is None and w.mma_scales is not None and not self.force_gemv_chunks:
+                if (M <= 2 and w.cols % 256 == 0 and (not swiglu or N % 128 == 0)
+                        and (w.rows + 127) // 128 * (w.cols // 256) >= FP4_TC_UNITS):
+                    return self._linear_w4_tc(x, w, norm_w, eps, res, swiglu, M, N, out_f32)
+                y = self._stream(x, w.packed, w.mma_scales, w.global_scale, w.row_alpha, norm_w, eps, res, 1 if swiglu else 0, N, out_f32)
+                if y is not None:
+                    return y
             if M <= GEMV_MAX_ROWS and not self.force_gemv_chunks:
                 N = w.rows // 2 if swiglu else w.rows
                 y = self.empty(M, N, dtype=torch.float32 if out_f32 else self.dtype, device=self.device)
@@ -246,15 +260,11 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
             w = w.dense
         M, K = x.shape
         N = w.shape[0] // 2 if swiglu else w.shape[0]
-        # 2..8 rows always; 9..32 rows unless the matrix is very wide (lm_head), where the swapped tcgen05 GEMM with its
-        # TMA pipeline measured faster
-        if (self.mma_gemv_rows[0] <= M <= self.mma_gemv_rows[1] and K % 32 == 0 and not self.force_gemv_chunks
-                and w.stride(0) == K and (M <= 8 or N < 65536)):
+        if self.mma_gemv_rows[0] <= M <= self.mma_gemv_rows[1] and not self.force_gemv_chunks:
             # a few rows (concurrent decode streams, speculative verify): weights streamed once into mma.sync fragments
-            y = out if out is not None else self.empty(M, N, dtype=torch.float32 if out_f32 else self.dtype, device=self.device)
-            self.launches += 1
-            self.C.gemv_mma(y, x, w, norm_w, res, eps, 1 if swiglu else 2 if act else 0, self._workspace(8 << 20), self._counters)
-            return y
+            y = self._stream(x, w, None, 1.0, None, norm_w, eps, res, 1 if swiglu else 2 if act else 0, N, out_f32, out)
+            if y is not None:
+                return y
         if M <= GEMV_MAX_ROWS or self.force_gemv_chunks:
             y = out if out is not None else self.empty(M, N, dtype=torch.float32 if out_f32 else self.dtype, device=self.device)
             for r0 in range(0, M, GEMV_MAX_ROWS):
@@ -272,6 +282,19 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         ws, cnt = self._gemm_scratch(M, N, split)
         self.launches += 1
         self.C.gemm(y, x, w, res, (1 if swiglu else 0) | (2 if out_f32 else 0) | (4 if act else 0), split, ws, cnt, self.status_word)
+        return y
+
+    def _stream(self, x, w, sf, scale, row_alpha, norm_w, eps, res, mode, N, out_f32, out=None):
+        """Up to 32 rows: weights (bf16, or e2m1 codes with scale tiles `sf`) streamed through a TMA ring into mma.sync fragments. None where
+        the kernel does not take the shape (rows that are no multiple of 16 bytes, 4-bit rows that are no multiple of 256 values)."""
+        if not w.is_contiguous():
+            return None
+        if norm_w is not None and x.shape[0] > 8 and sf is None:
+            x, norm_w = self.rmsnorm(x, norm_w, eps, True)[0], None      # rows beyond one token tile come in by TMA as they are
+        y = out if out is not None else self.empty(x.shape[0], N, dtype=torch.float32 if out_f32 else self.dtype, device=self.device)
+        if self.C.gemv_stream(y, x, w, sf, scale, row_alpha, norm_w, res, eps, mode, self._workspace(8 << 20), self._counters, self.status_word) < 0:
+            return None
+        self.launches += 1
         return y
 
     # ---- FP8 (e4m3) weights and activations -----------------------------------------------------------
@@ -533,10 +556,21 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         segment) and a bf16 cache the tensor-core kernel runs: the rows of a segment share one pass over the K/V of
         each kv head (bf16 and e4m3 caches). The 4-bit cache and callers without segment tables take the SIMT kernel."""
         T = q.shape[0]
+        # the heads of a group for a row or two at a time, keys split over the warps of a CTA, and as many splits as fill the GPU. Rows of every
+        # count take this kernel, so that a verified row has the bits of a decoded one; trees (ancestor masks) and quantised caches do not.
+        G = nq // nkv
+        keys = (segs is not None and kv_scale is None and row_mask is None and self.attn_mma and G <= 16 and kv_block % 64 == 0
+                and hd in DECODE_KEYS_CTAS)
+        if keys:
+            ctas = segs[0].numel() * nkv * -(-segs[3] // (16 // G))
+            nsplit = max(1, min(nsplit, self.sm_count * DECODE_KEYS_CTAS[hd] // ctas))
         out = self.empty(T, nq * hd, dtype=self.dtype, device=self.device)
         o_part = self.empty(T, nq, nsplit, hd, dtype=torch.float32, device=self.device)
         ml_part = self.empty(T, nq, nsplit, 2, dtype=torch.float32, device=self.device)
         self.launches += 2
+        if keys and self.C.attn_decode_keys(out, o_part, ml_part, q, k_cache, v_cache, proj, *segs, row_kvlen, block_table, kv_block, nq, nkv, hd,
+                                            nsplit, gated, self.status_word) == 0:
+            return out
         fp8_cache = kv_scale is not None and k_cache.shape[-1] == hd           # (the 4-bit cache has hd / 2 bytes per row)
         if segs is not None and (kv_scale is None or fp8_cache) and self.attn_mma and nq // nkv <= 64:
             rc = self.C.attn_decode_mma(out, o_part, ml_part, q, k_cache, v_cache, proj, segs[0], segs[1], segs[2], segs[3],
@@ -561,21 +595,10 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
             key = (n_slots, toks, nkv, hd)
             if self._kv_scratch is None or self._kv_scratch[0] != key:
                 # zeros: rows past the decoded ones are masked by causality but still multiplied (0 x value) by the
-        # the heads of a group for a row or two at a time, keys split over the warps of a CTA, and as many splits as fill the GPU. Rows of every
-        # count take this kernel, so that a verified row has the bits of a decoded one; trees (ancestor masks) and quantised caches do not.
-        G = nq // nkv
-        keys = (segs is not None and kv_scale is None and row_mask is None and self.attn_mma and G <= 16 and kv_block % 64 == 0
-                and hd in DECODE_KEYS_CTAS)
-        if keys:
-            ctas = segs[0].numel() * nkv * -(-segs[3] // (16 // G))
-            nsplit = max(1, min(nsplit, self.sm_count * DECODE_KEYS_CTAS[hd] // ctas))
                 # tensor-core kernel, so they must hold finite numbers
                 ks = torch.zeros(n_slots * max_blocks, kv_block, nkv, hd, dtype=self.dtype, device=self.device)
                 vs = torch.zeros_like(ks)
                 ident = torch.arange(n_slots * max_blocks, dtype=torch.int32, device=self.device).view(n_slots, max_blocks)
-        if keys and self.C.attn_decode_keys(out, o_part, ml_part, q, k_cache, v_cache, proj, *segs, row_kvlen, block_table, kv_block, nq, nkv, hd,
-                                            nsplit, gated, self.status_word) == 0:
-            return out
                 self._kv_scratch = (key, ks, vs, ident.contiguous())
             _, ks, vs, ident = self._kv_scratch
             self.launches += 1

@@ -29,7 +29,7 @@ def cases(ops, dev):
     wk = rnd(2048, 17408, scale=0.02)
     xk = rnd(17, 17408)
     out["gemv 1 row"] = lambda: ops.linear(x1, w)
-    out["gemv_mma 4 rows (split k)"] = lambda: ops.linear(x4, w)
+    out["gemv_stream 4 rows (runs that share tiles)"] = lambda: ops.linear(x4, w)
     out["tcgen05 gemm 17 rows, K 17408 (split k)"] = lambda: ops.linear(xk, wk)
     out["tcgen05 gemm 17 rows fp32 out"] = lambda: ops.linear(x17, w, out_f32=True)
     q = quantize_weight(w)

@@ -1,0 +1,85 @@
+"""Few-row products that stream bf16 or NVFP4 weights through a TMA ring (`gemv_stream`) against 32-bit math on the same values."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.fixture(scope="module")
+def ops(ext):
+    from ferrite_b200.ops.cuda_ops import CudaOps
+    return CudaOps(DEV)
+
+
+def rnd(*shape, seed=0, scale=1.0):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    return (torch.randn(*shape, generator=g, device=DEV) * scale).to(torch.bfloat16)
+
+
+def reference(x, w, norm_w, eps, swiglu):
+    x = x.double()
+    if norm_w is not None:
+        x = x * torch.rsqrt(x.square().mean(-1, keepdim=True) + eps) * (1 + norm_w.double())
+    y = x @ w.double().t()
+    half = y.shape[1] // 2
+    return torch.nn.functional.silu(y[:, :half]) * y[:, half:] if swiglu else y
+
+
+# rows at the edges of the 8-token tiles; outputs and K around tiles (128, 64 for SwiGLU), units (64 / 256) and runs; K of one unit; a tile
+# shared by many runs and runs over many tiles
+@pytest.mark.parametrize("M", [1, 2, 4, 5, 8, 9, 17, 32])
+@pytest.mark.parametrize("N,K", [(1, 8), (129, 64), (127, 72), (640, 5000), (4112, 1024), (20000, 264)])
+@pytest.mark.parametrize("norm,swiglu", [(False, False), (True, False), (True, True)])
+def test_bf16_weights(ops, M, N, K, norm, swiglu):
+    x, w = rnd(M, K, seed=M), rnd((2 if swiglu else 1) * N, K, seed=2, scale=K ** -0.5)
+    nw = rnd(K, seed=3, scale=0.1) if norm else None
+    want = reference(x, w, nw, 1e-6, swiglu)
+    y = ops._stream(x, w, None, 1.0, None, nw, 1e-6, None, 1 if swiglu else 0, N, True)
+    # operands rounded to bf16 once (2^-9 each value, under the norm), 32-bit sums; outputs of size one
+    assert (y.double() - want).abs().max().item() <= (2 ** -6 if norm else 2 ** -14) * max(1.0, want.abs().max().item())
+    if not swiglu:
+        res = rnd(M, N, seed=4)
+        got = ops._stream(x, w, None, 1.0, None, nw, 1e-6, res, 0, N, False)
+        assert torch.equal(got, (y + res.float()).to(torch.bfloat16))
+        relu2 = ops._stream(x, w, None, 1.0, None, nw, 1e-6, None, 2, N, True)
+        assert torch.equal(relu2, y.clamp_min(0).square())
+    assert torch.equal(y, ops._stream(x, w, None, 1.0, None, nw, 1e-6, None, 1 if swiglu else 0, N, True))
+    assert ops.status() == 0 and int(ops._counters.abs().sum()) == 0
+
+
+@pytest.mark.parametrize("M", [1, 2, 4, 5, 8])
+@pytest.mark.parametrize("N,K,swiglu", [(1, 256, False), (130, 512, False), (8224, 1280, False), (128, 256, True), (1536, 2048, True)])
+@pytest.mark.parametrize("norm", [False, True])
+def test_nvfp4_weights(ops, M, N, K, swiglu, norm):
+    """Every code and scale: the unpacked weights are exact, so only x (1 + w) is rounded (not at all up to four rows)."""
+    from ferrite_b200.formats import nvfp4
+    rows = (2 if swiglu else 1) * N
+    g = torch.Generator(device=DEV).manual_seed(K + N)
+    packed = torch.randint(0, 256, (rows, K // 2), generator=g, device=DEV, dtype=torch.uint8)
+    scales = torch.randint(0, 127, (rows, K // 16), generator=g, device=DEV, dtype=torch.uint8)       # 0 .. 448, subnormal ones among them
+    t = nvfp4.NVFP4Tensor(packed, scales.view(torch.float8_e4m3fn), 2.0 ** -10, rows, K)
+    w = t.dequantize(torch.float64)
+    alpha = torch.rand(rows, generator=g, device=DEV) + 0.5
+    x, nw = rnd(M, K, seed=M), rnd(K, seed=3, scale=0.1) if norm else None
+    tiles = nvfp4.tile_scales_mma(t.scales).contiguous()
+    for ra in (None, alpha):
+        wr = w if ra is None else w / t.global_scale * ra.double()[:, None] * 2.0 ** -10
+        want = reference(x, wr, nw, 1e-6, swiglu)
+        y = ops._stream(x, packed, tiles, t.global_scale, None if ra is None else ra * 2.0 ** -10, nw, 1e-6, None, 1 if swiglu else 0, N, True)
+        mag = (x.double().abs() @ wr.abs().t()).max().item()
+        tol = 2 ** -19 if not norm or M <= 4 else 2 ** -10
+        if swiglu:
+            assert (y.double() - want).abs().max().item() <= 2 ** -6 * max(1.0, want.abs().max().item())
+        else:
+            assert (y.double() - want).abs().max().item() <= tol * mag * (1.5 if norm else 1.0)
+        assert torch.equal(y, ops._stream(x, packed, tiles, t.global_scale, None if ra is None else ra * 2.0 ** -10, nw, 1e-6, None, 1 if swiglu else 0, N, True))
+    assert ops.status() == 0 and int(ops._counters.abs().sum()) == 0
+
+
+def test_shapes_left_to_other_kernels(ops):
+    """Refused before anything is launched: rows that are no multiple of 16 bytes, 4-bit rows that are no multiple of a unit."""
+    assert ops._stream(rnd(2, 16), rnd(64, 16)[:, :16], None, 1.0, None, None, 1e-6, None, 0, 64, True) is not None
+    assert ops._stream(rnd(2, 12), rnd(64, 12), None, 1.0, None, None, 1e-6, None, 0, 64, True) is None
+    z = torch.zeros(64, 64, dtype=torch.uint8, device=DEV)
+    assert ops._stream(rnd(2, 128), z, z, 1.0, None, None, 1e-6, None, 0, 64, True) is None
