@@ -25,20 +25,53 @@ __global__ void attn_prep_kernel(__nv_bfloat16* __restrict__ q_out, void* __rest
                                  const int* __restrict__ row_slot, const int* __restrict__ row_pos,
                                  const int* __restrict__ row_cpos,
                                  const int* __restrict__ block_table, int max_blocks, int kv_block, int nq, int nkv,
-                                 int rot, int gated, float eps, int* status, int hrot) {
+                                 int rot, int gated, float eps, int* status, int hrot, int vec) {
   pdl_launch_dependents();
-  pdl_wait();
   constexpr int EPL = HD / 32;
   const int row = blockIdx.x;
+  // the row's angles once for all heads, while the projection is still being made (positions do not depend on it)
+  __shared__ float2 turn[HD];
+  const int pos = row_pos[row], half = rot / 2;
+  for (int i = threadIdx.x; i < min(half, HD); i += blockDim.x) {
+    float sn, cs;
+    sincosf((float)pos * inv_freq[i], &sn, &cs);
+    turn[i] = make_float2(cs, sn);
+  }
+  __syncthreads();
+  pdl_wait();
+  proj = after_wait(proj);
   // one warp per (q or kv) head; blockIdx.y carries the heads beyond the first 32
   const int warp = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (warp >= nq + nkv) return;
   const bool is_q = warp < nq;
   const int qw = gated ? 2 * HD : HD;
   const __nv_bfloat16* src = proj + (size_t)row * proj_stride + (is_q ? (size_t)warp * qw : (size_t)nq * qw + (size_t)(warp - nq) * HD);
+  // EPL neighbours of a lane at once where everything lies on 16 bytes
+  auto load = [&](const __nv_bfloat16* p, __nv_bfloat16 (&to)[EPL]) {
+    if (vec & 1) {
+      if constexpr (EPL == 8) *reinterpret_cast<uint4*>(to) = *reinterpret_cast<const uint4*>(p + lane * EPL);
+      else if constexpr (EPL == 4) *reinterpret_cast<uint2*>(to) = *reinterpret_cast<const uint2*>(p + lane * EPL);
+      else *reinterpret_cast<uint32_t*>(to) = *reinterpret_cast<const uint32_t*>(p + lane * EPL);
+    } else {
+#pragma unroll
+      for (int j = 0; j < EPL; ++j) to[j] = p[lane * EPL + j];
+    }
+  };
+  auto store = [&](__nv_bfloat16* p, const __nv_bfloat16 (&from)[EPL]) {
+    if (vec & 2) {
+      if constexpr (EPL == 8) *reinterpret_cast<uint4*>(p + lane * EPL) = *reinterpret_cast<const uint4*>(from);
+      else if constexpr (EPL == 4) *reinterpret_cast<uint2*>(p + lane * EPL) = *reinterpret_cast<const uint2*>(from);
+      else *reinterpret_cast<uint32_t*>(p + lane * EPL) = *reinterpret_cast<const uint32_t*>(from);
+    } else {
+#pragma unroll
+      for (int j = 0; j < EPL; ++j) p[lane * EPL + j] = from[j];
+    }
+  };
+  alignas(16) __nv_bfloat16 raw[EPL];
+  load(src, raw);
   float v[EPL];
 #pragma unroll
-  for (int j = 0; j < EPL; ++j) v[j] = bf2f(src[lane * EPL + j]);
+  for (int j = 0; j < EPL; ++j) v[j] = bf2f(raw[j]);
   float ss = 0.f;
 #pragma unroll
   for (int j = 0; j < EPL; ++j) ss += v[j] * v[j];
@@ -48,19 +81,14 @@ __global__ void attn_prep_kernel(__nv_bfloat16* __restrict__ q_out, void* __rest
 #pragma unroll
   for (int j = 0; j < EPL; ++j) v[j] = v[j] * r * (1.f + bf2f(nw[lane * EPL + j]));
   // partial RoPE, rotate-half pairing (i, i + rot/2) inside the first `rot` dims
-  const int pos = row_pos[row];
-  const int half = rot / 2;
   const int partner_lanes = half / EPL;                  // lane distance between the two halves of a pair
 #pragma unroll
   for (int j = 0; j < EPL; ++j) {
     float other = __shfl_xor_sync(0xffffffffu, v[j], partner_lanes);
     int d = lane * EPL + j;
     if (d < rot) {
-      int i = d < half ? d : d - half;
-      float ang = (float)pos * inv_freq[i];
-      float sn, cs;
-      sincosf(ang, &sn, &cs);
-      v[j] = d < half ? (v[j] * cs - other * sn) : (v[j] * cs + other * sn);
+      const float2 t = turn[d < half ? d : d - half];
+      v[j] = d < half ? (v[j] * t.x - other * t.y) : (v[j] * t.x + other * t.y);
     }
   }
   if (hrot) {
@@ -87,9 +115,9 @@ __global__ void attn_prep_kernel(__nv_bfloat16* __restrict__ q_out, void* __rest
     for (int j = 0; j < EPL; ++j) v[j] *= hs;
   }
   if (is_q) {
-    __nv_bfloat16* dst = q_out + ((size_t)row * nq + warp) * HD;
 #pragma unroll
-    for (int j = 0; j < EPL; ++j) dst[lane * EPL + j] = f2bf(v[j]);
+    for (int j = 0; j < EPL; ++j) raw[j] = f2bf(v[j]);
+    store(q_out + ((size_t)row * nq + warp) * HD, raw);
   } else {
     const int kvh = warp - nq;
     const int slot = row_slot[row];
@@ -186,9 +214,10 @@ __global__ void attn_prep_kernel(__nv_bfloat16* __restrict__ q_out, void* __rest
       __nv_bfloat16* k_cache = reinterpret_cast<__nv_bfloat16*>(k_cache_v);
       __nv_bfloat16* v_cache = reinterpret_cast<__nv_bfloat16*>(v_cache_v);
 #pragma unroll
-      for (int j = 0; j < EPL; ++j) k_cache[off + lane * EPL + j] = f2bf(v[j]);
-#pragma unroll
-      for (int j = 0; j < EPL; ++j) v_cache[off + lane * EPL + j] = vsrc[lane * EPL + j];
+      for (int j = 0; j < EPL; ++j) raw[j] = f2bf(v[j]);
+      store(k_cache + off, raw);
+      load(vsrc, raw);
+      store(v_cache + off, raw);
     }
   }
 }
@@ -535,11 +564,14 @@ static int attn_prep_impl(void* q_out, void* k_cache, void* v_cache, float* kv_s
   const int hgroups = (heads + 31) / 32;
   int epl = hd / 32;
   if (rot % 2 || (rot / 2) % epl || ((rot / 2 / epl) & (rot / 2 / epl - 1))) return -3;
+  // rows (bit 0) and what is written (bit 1) lie on 16 bytes
+  const int vec = ((((uintptr_t)proj | (uintptr_t)(proj_stride * 2)) & 15) ? 0 : 1) |
+                  ((((uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) ? 0 : 2);
 #define FB_PREP(HDV, K8)                                                                                          \
   launch_pdl(attn_prep_kernel<HDV, K8>, dim3(rows, hgroups), dim3(threads), (size_t)(0), s, (__nv_bfloat16*)q_out, k_cache, v_cache, \
       kv_scale, (const __nv_bfloat16*)proj, proj_stride, (const __nv_bfloat16*)q_norm,                            \
       (const __nv_bfloat16*)k_norm, inv_freq, row_slot, row_pos, row_cpos, block_table, max_blocks, kv_block, nq, nkv, rot, \
-      gated, eps, status, hrot)
+      gated, eps, status, hrot, vec)
   if (kv_scale && bits == 6) {
     if (hd == 256) FB_PREP(256, 3); else if (hd == 128) FB_PREP(128, 3); else if (hd == 64) FB_PREP(64, 3); else return -2;
   } else if (kv_scale && bits == 4) {
