@@ -243,6 +243,10 @@ class Executor:
         self._ring = [torch.zeros(5 * R + 4 * S, dtype=torch.int32, pin_memory=(dev.type == "cuda")) for _ in range(4)]
         self._ring_ev = [None] * 4
         self._ring_i = 0
+        # kept rows per segment of verify steps: a ring of its own (a plain copy would wait for the step's kernels before it returned)
+        self._kring = [torch.zeros(S, dtype=torch.int32, pin_memory=(dev.type == "cuda")) for _ in range(4)]
+        self._kring_ev = [None] * 4
+        self._kring_i = 0
         self.h2d_bytes = 0
         self._R, self._S = R, S
         self.graphs: "OrderedDict[tuple, tuple]" = OrderedDict()
@@ -1104,7 +1108,7 @@ class Executor:
         simply overwritten by later steps."""
         mv, max_seg_rows = self._last_meta
         c, w, ops = self.cfg, self.w, self.ops
-        mv["snrows"].copy_(torch.tensor(list(keep), dtype=torch.int32), non_blocking=False)
+        self._upload_kept(mv["snrows"], keep)
         mr = max(max(keep), 1)
         if (self._last_graph_key is not None and self.profile is None
                 and ((self._replay_fused(mr) and "gdn" in self.kinds) or {"cdelta", "ssm"} & set(self.kinds) or self.canon_at)):
@@ -1125,6 +1129,19 @@ class Executor:
             self.ops.launches += g[1]
             return
         self._replay_layers(mv, mr)
+
+    def _upload_kept(self, snrows, keep: Sequence[int]) -> None:
+        i = self._kring_i
+        self._kring_i = (i + 1) % len(self._kring)
+        if self._kring_ev[i] is not None:
+            self._kring_ev[i].synchronize()                  # the copy that last read this buffer
+        buf = self._kring[i][:len(keep)]
+        buf.copy_(torch.tensor(list(keep), dtype=torch.int32))
+        snrows.copy_(buf, non_blocking=True)
+        if self.device.type == "cuda":
+            ev = torch.cuda.Event()
+            ev.record()
+            self._kring_ev[i] = ev
 
     def _replay_layers(self, mv, mr: int) -> None:
         c, w, ops = self.cfg, self.w, self.ops
