@@ -540,6 +540,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         const float sm_row = a.scale_m && m < m_end ? a.scale_m[m] : 1.f;
         const uint32_t stage_w = smem_u32(tiles + (size_t)a.stages * stage_bytes + (size_t)quad * GM_EPI_BYTES);
         const int rr = lane >> 2, rc = (lane & 3) * 8;    // bf16 output: row of a group of 8, column of the 32
+        const bool wide = (((uintptr_t)a.Y | (uintptr_t)a.res) & 15) == 0;
         // A piece of a tile (tail of the tile list): 64 accumulator columns at a time go to the workspace as fp32, and the warp that brings a
         // block's last piece sums the pieces in their order and finishes it. The pieces begin at different columns, which spreads the sums over
         // the CTAs; nobody waits.
@@ -583,7 +584,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               const int row = row_first + q * 8 + rr;
-              rv[q] = row < m_end && n + rc + 8 <= a.N ? *reinterpret_cast<const uint4*>(a.res + (size_t)row * a.ldy + n + rc) : make_uint4(0, 0, 0, 0);
+              rv[q] = wide && row < m_end && n + rc + 8 <= a.N ? *reinterpret_cast<const uint4*>(a.res + (size_t)row * a.ldy + n + rc) : make_uint4(0, 0, 0, 0);
             }
           const float sn = a.scale_n && n + lane < a.N ? a.scale_n[n + lane] : 1.f, sn_up = a.dual && a.scale_n && n + lane < a.N ? a.scale_n[a.N + n + lane] : 1.f;
           uint32_t r0[32], r1[32];
@@ -667,7 +668,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             float o[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
             if (gm >= m_end || nn >= a.N) continue;
             const size_t at = (size_t)gm * a.ldy + nn;
-            if (nn + 8 <= a.N) {
+            if (wide && nn + 8 <= a.N) {
               if (a.res) {
                 const uint32_t ru[4] = {rv[q].x, rv[q].y, rv[q].z, rv[q].w};
 #pragma unroll
@@ -680,7 +681,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
               } else {
                 *reinterpret_cast<uint4*>(Yb + at) = make_uint4(pack_bf2(o[0], o[1]), pack_bf2(o[2], o[3]), pack_bf2(o[4], o[5]), pack_bf2(o[6], o[7]));
               }
-            } else {                                      // the ragged end of a row
+            } else {                                      // the ragged end of a row, or an output that lies on no 16 bytes
 #pragma unroll
               for (int j = 0; j < 8; ++j)
                 if (nn + j < a.N) {

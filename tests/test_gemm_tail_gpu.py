@@ -58,6 +58,15 @@ def test_widths_and_pieces(ops, M, N, K, pieces, swiglu):
     assert ops.status() == 0 and int(ops._tail_counters.abs().sum()) == 0
 
 
+@pytest.mark.parametrize("N", [24, 100])
+def test_output_on_no_16_bytes(ops, N):
+    M, K = 130, 256
+    x, w, res = rnd(M, K, seed=1), rnd(N, K, seed=2, scale=K ** -0.5), rnd(M, 104, seed=3)[:, :N]
+    want = ops.linear(x, w, res=res, out=torch.empty(M, 104, dtype=torch.bfloat16, device=DEV)[:, :N])
+    out = torch.zeros(M * 104 + 1, dtype=torch.bfloat16, device=DEV)[1:].view(M, 104)
+    assert torch.equal(ops.linear(x, w, res=res, out=out[:, :N]), want) and int(out[:, N:].count_nonzero()) == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(129, 264, 1040), (140, 2048, 8208)])
 def test_scaled_fp8(ops, M, N, K):
     x, w = rnd(M, K, seed=1), rnd(N, K, seed=2, scale=K ** -0.5)
