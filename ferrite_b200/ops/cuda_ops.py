@@ -26,6 +26,10 @@ GEMV_MAX_ROWS = 8
 DECODE_KEYS_CTAS = {64: 4, 128: 2, 256: 1}
 MOE_PAIR_ROWS = 64     # up to this many rows (the largest graph-captured step) the experts run as per-pair GEMVs,
                        # beyond as grouped GEMMs, which read the per-expert row counts on the host
+# 2..32 rows against bf16 weights of so many values and more stream them through a TMA ring (`gemv_stream`), less through registers (`gemv_mma`), which
+# starts 2 us sooner: 17 products of a model of width 1024 (1M to 6M values) take 35 us less a step, the
+# products of a 27B model (10M and more) 17 % less through the ring.
+STREAM_VALUES = 8 << 20
 # NVFP4 weights of so many 128 x 256 units and more against one or two rows run on the block-scaled tensor cores (activations as three residual
 # renderings), smaller ones on the row kernel that unpacks the codes: it starts faster and unpacks 1.6 us a unit and CTA. One row, us: 17408 x 2 x
 # 5120 (5440 units) 30.5 / 34.5, 151936 x 5120 (23740) 79 / 127, 14336 x 5120 (2240) 20.5 / 20.6, 8224 x 5120 (1300) 18.9 / 15.2,
@@ -62,7 +66,7 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         self.force_gemv_chunks = False      # debug: run any row count through 8-row GEMV passes
         self.launches = 0                   # kernels launched (or recorded into a graph) through this object
         self.moe_pair_rows = MOE_PAIR_ROWS
-        self.mma_gemv_rows = (2, 32)        # row counts routed to the mma.sync weight-streaming kernel (`gemv_stream`)
+        self.mma_gemv_rows = (2, 32)        # row counts routed to the mma.sync weight-streaming kernels
         self.attn_mma = os.environ.get("FB_ATTN_MMA", "1") != "0"   # decode attention on mma.sync (0: SIMT kernel)
         self.attn_tc = os.environ.get("FB_ATTN_TC", "1") != "0"     # prompt attention on tcgen05 (0: mma.sync kernel)
         self._gdn_scratch = None
@@ -262,6 +266,11 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         N = w.shape[0] // 2 if swiglu else w.shape[0]
         if self.mma_gemv_rows[0] <= M <= self.mma_gemv_rows[1] and not self.force_gemv_chunks:
             # a few rows (concurrent decode streams, speculative verify): weights streamed once into mma.sync fragments
+            if w.numel() < STREAM_VALUES and K % 32 == 0 and w.stride(0) == K:
+                y = out if out is not None else self.empty(M, N, dtype=torch.float32 if out_f32 else self.dtype, device=self.device)
+                self.launches += 1
+                self.C.gemv_mma(y, x, w, norm_w, res, eps, 1 if swiglu else 2 if act else 0, self._workspace(8 << 20), self._counters)
+                return y
             y = self._stream(x, w, None, 1.0, None, norm_w, eps, res, 1 if swiglu else 2 if act else 0, N, out_f32, out)
             if y is not None:
                 return y
