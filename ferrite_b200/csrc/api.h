@@ -52,7 +52,7 @@ int fb_bf16_to_f32(float* out, const void* in, long n, cudaStream_t s);
 
 // ---- gemv.cu ----
 int fb_gemv_bf16(void* Y, const void* X, const void* W, const void* norm_w, const void* res, int M, int N, int K,
-                 long ldx, long ldy, float eps, int centred, int out_f32, int mode, int sm_count, cudaStream_t s);
+                 long ldx, long ldy, float eps, int centred, int out_f32, int mode, int fresh_w, int sm_count, cudaStream_t s);
 
 // ---- gemm_tcgen05.cu ----
 // Y[M][N] = X[M][K] * W[N][K]^T (+ res), or SwiGLU over W = [gate rows | up rows] (2N rows). bf16 in/out,
@@ -66,7 +66,7 @@ long fb_gemm_workspace_bytes(int M, int N, int split_k);
 // 2..32 rows: weight-streaming linear on mma.sync with in-register A fragments (gemv_mma.cu)
 int fb_gemv_mma(void* y, const void* x, const void* w, const void* norm_w, const void* res, int M, int N, int K, long ldx,
                 long ldy, float eps, int mode, int out_f32, float* ws, long ws_floats, int* counters, int n_counters,
-                int sm_count, cudaStream_t s);
+                int fresh_w, int sm_count, cudaStream_t s);
 // FP8 (e4m3) GEMM with per-row / per-feature scales, and the activation quantiser (gemm_tcgen05.cu)
 int fb_quant_fp8(void* q, float* scale, const void* x, const void* norm_w, int rows, int K, long ldx, float eps,
                  cudaStream_t s);

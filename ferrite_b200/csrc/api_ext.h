@@ -66,7 +66,7 @@ int fb_gemm_nvfp4_swiglu_q(void* q_codes, void* q_sf, float* q_row_scale, float 
 // ---- gemv_stream.cu: products of up to 32 rows, bf16 or NVFP4 weights streamed through a TMA ring ----
 int fb_gemv_stream(void* y, const void* x, const void* w, const void* sf, float w_scale, const float* row_alpha, const void* norm_w, const void* res,
                    int M, int N, int K, long ldx, long ldy, float eps, int mode, int out_f32, float* ws, long ws_floats, int* counters, int n_counters,
-                   int* status, int sm_count, cudaStream_t s);
+                   int fresh_w, int* status, int sm_count, cudaStream_t s);
 // ---- gemv_nvfp4_tc.cu: few-row NVFP4 linear on the block-scaled tensor cores, activations as residual NVFP4 terms ----
 long fb_gemv_nvfp4_tc_workspace_bytes(int M, int N, int K, int dual, int terms, int sm_count, int ctas_per_sm);
 int fb_gemv_nvfp4_tc_terms(int M, int N, int K, int dual, int terms);

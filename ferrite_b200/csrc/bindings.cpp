@@ -63,12 +63,12 @@ void add_bf16(Tensor x, Tensor y) { check(fb_add_bf16(x.data_ptr(), y.data_ptr()
 
 // Y[M][N] (+)= X W^T, small M. mode 0 plain / 1 swiglu.
 void gemv(Tensor Y, Tensor X, Tensor W, c10::optional<Tensor> norm_w, c10::optional<Tensor> res, double eps,
-          bool centred, int64_t mode) {
+          bool centred, int64_t mode, bool fresh_w) {
   int M = (int)X.size(0), K = (int)X.size(1);
   int N = (int)(mode == 1 ? W.size(0) / 2 : W.size(0));
   check(fb_gemv_bf16(Y.data_ptr(), X.data_ptr(), W.data_ptr(), cptr(norm_w), cptr(res), M, N, K, (long)X.stride(0),
                      (long)Y.stride(0), (float)eps, centred ? 1 : 0, Y.scalar_type() == torch::kFloat32 ? 1 : 0,
-                     (int)mode, sm_count(), cur_stream()), "gemv");
+                     (int)mode, fresh_w ? 1 : 0, sm_count(), cur_stream()), "gemv");
 }
 
 int64_t gemm_workspace_bytes(int64_t M, int64_t N, int64_t split_k) {
@@ -85,14 +85,14 @@ void gemm(Tensor Y, Tensor X, Tensor W, c10::optional<Tensor> res, int64_t mode,
 }
 
 void gemv_mma(Tensor Y, Tensor X, Tensor W, c10::optional<Tensor> norm_w, c10::optional<Tensor> res, double eps,
-              int64_t mode, c10::optional<Tensor> workspace, c10::optional<Tensor> counters) {
+              int64_t mode, c10::optional<Tensor> workspace, c10::optional<Tensor> counters, bool fresh_w) {
   int M = (int)X.size(0), K = (int)X.size(1);
   int N = (int)(mode == 1 ? W.size(0) / 2 : W.size(0));
   long wsf = workspace.has_value() ? (long)(workspace->numel() * workspace->element_size() / 4) : 0;
   int nc = counters.has_value() ? (int)counters->numel() : 0;
   check(fb_gemv_mma(Y.data_ptr(), X.data_ptr(), W.data_ptr(), cptr(norm_w), cptr(res), M, N, K, (long)X.stride(0),
                     (long)Y.stride(0), (float)eps, (int)mode, Y.scalar_type() == torch::kFloat32 ? 1 : 0,
-                    (float*)mptr(workspace), wsf, (int*)mptr(counters), nc, sm_count(), cur_stream()), "gemv_mma");
+                    (float*)mptr(workspace), wsf, (int*)mptr(counters), nc, fresh_w ? 1 : 0, sm_count(), cur_stream()), "gemv_mma");
 }
 
 void quant_fp8(Tensor q, Tensor scale, Tensor x, c10::optional<Tensor> norm_w, double eps) {
@@ -448,9 +448,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gated_norm", &gated_norm);
   m.def("gather_rows", &gather_rows);
   m.def("add_bf16", &add_bf16);
-  m.def("gemv", &gemv);
+  m.def("gemv", &gemv, py::arg("Y"), py::arg("X"), py::arg("W"), py::arg("norm_w"), py::arg("res"), py::arg("eps"), py::arg("centred"), py::arg("mode"),
+        py::arg("fresh_w") = false);
   m.def("gemm", &gemm);
-  m.def("gemv_mma", &gemv_mma);
+  m.def("gemv_mma", &gemv_mma, py::arg("Y"), py::arg("X"), py::arg("W"), py::arg("norm_w"), py::arg("res"), py::arg("eps"), py::arg("mode"),
+        py::arg("workspace"), py::arg("counters"), py::arg("fresh_w") = false);
   m.def("gemm_workspace_bytes", &gemm_workspace_bytes);
   m.def("attn_prep", &attn_prep);
   m.def("attn_decode", &attn_decode);

@@ -448,18 +448,24 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 
 // Host helper: launch with programmatic stream serialization, so the grid may be scheduled while its
 // predecessor drains. Every kernel launched this way executes griddepcontrol.wait before it touches anything
-// the predecessor wrote.
+// the predecessor wrote. Kernels that load their weights ahead of that wait take `overlap` false where those were written on the
+// same stream just before (a scratch that packed weights were decoded into): they then start behind it like any launch.
 template <typename... KArgs, typename... Args>
-static inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                                     Args&&... args) {
+static inline cudaError_t launch_pdl_if(bool overlap, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                        Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   static const bool no_pdl = [] { const char* e = getenv("FB_NO_PDL"); return e && e[0] == '1'; }();   // debugging aid
-  cfg.attrs = attr; cfg.numAttrs = no_pdl ? 0 : 1;
+  cfg.attrs = attr; cfg.numAttrs = no_pdl || !overlap ? 0 : 1;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+static inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                     Args&&... args) {
+  return launch_pdl_if(true, kern, grid, block, smem, s, static_cast<Args&&>(args)...);
 }
 
 #define FB_CUDA_CHECK(expr)                                                                      \

@@ -4,7 +4,7 @@
 //
 // Launched with programmatic stream serialization: the grid may become resident while the previous kernel of
 // the stream drains; it issues its first batch of weight loads (weights never depend on the previous kernel)
-// and only then executes griddepcontrol.wait before touching X. The reference overlaps the same way
+// and only then executes griddepcontrol.wait before touching X (weights that were written on the stream just before: `fresh_w`). The reference overlaps the same way
 // ("L2 prefetch before griddepcontrol.wait", `crates/fe-exl3/src/gpu/pdl.rs`).
 #include "api.h"
 #include "gemv_core.cuh"
@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, (M <= 2 ? 4 : (M <= 4 ? 3 : 2)))
 }
 
 template <int M, int R, bool SWIGLU>
-static int launch_gemv(GemvArgs a, int sm_count, cudaStream_t s) {
+static int launch_gemv(GemvArgs a, int fresh_w, int sm_count, cudaStream_t s) {
   a.kc = gemv_chunk_len(M, a.K);
   int nchunks = (a.K + a.kc - 1) / a.kc;
   constexpr int RW = SWIGLU ? 1 : R;
@@ -63,22 +63,17 @@ static int launch_gemv(GemvArgs a, int sm_count, cudaStream_t s) {
     if (e != cudaSuccess) return (int)e;
     attr_done = true;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(GEMV_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, kern, a);
+  return (int)launch_pdl_if(!fresh_w, kern, dim3(grid), dim3(GEMV_THREADS), smem, s, a);
 }
 
 }  // namespace fb
 
 using namespace fb;
 
-// mode: 0 = plain (optional residual), 1 = SwiGLU (W has 2N rows: gate rows then up rows), 2 = squared relu
+// mode: 0 = plain (optional residual), 1 = SwiGLU (W has 2N rows: gate rows then up rows), 2 = squared relu. fresh_w: W was written on this
+// stream just before, so its loads wait like those of X
 extern "C" int fb_gemv_bf16(void* Y, const void* X, const void* W, const void* norm_w, const void* res, int M, int N,
-                            int K, long ldx, long ldy, float eps, int centred, int out_f32, int mode, int sm_count,
+                            int K, long ldx, long ldy, float eps, int centred, int out_f32, int mode, int fresh_w, int sm_count,
                             cudaStream_t s) {
   if (M <= 0 || N <= 0) return 0;
   if (M > 8 || (K % 8) != 0 || (ldx % 8) != 0) return -1;
@@ -89,13 +84,13 @@ extern "C" int fb_gemv_bf16(void* Y, const void* X, const void* W, const void* n
   a.act = mode == 2 ? ACT_RELU2 : ACT_NONE;
   if (sm_count <= 0) sm_count = 148;
   if (mode == 1) {
-    if (M == 1) return launch_gemv<1, 2, true>(a, sm_count, s);
-    if (M == 2) return launch_gemv<2, 2, true>(a, sm_count, s);
-    if (M <= 4) return launch_gemv<4, 2, true>(a, sm_count, s);
-    return launch_gemv<8, 2, true>(a, sm_count, s);
+    if (M == 1) return launch_gemv<1, 2, true>(a, fresh_w, sm_count, s);
+    if (M == 2) return launch_gemv<2, 2, true>(a, fresh_w, sm_count, s);
+    if (M <= 4) return launch_gemv<4, 2, true>(a, fresh_w, sm_count, s);
+    return launch_gemv<8, 2, true>(a, fresh_w, sm_count, s);
   }
-  if (M == 1) return launch_gemv<1, 2, false>(a, sm_count, s);
-  if (M == 2) return launch_gemv<2, 2, false>(a, sm_count, s);
-  if (M <= 4) return launch_gemv<4, 2, false>(a, sm_count, s);
-  return launch_gemv<8, 2, false>(a, sm_count, s);
+  if (M == 1) return launch_gemv<1, 2, false>(a, fresh_w, sm_count, s);
+  if (M == 2) return launch_gemv<2, 2, false>(a, fresh_w, sm_count, s);
+  if (M <= 4) return launch_gemv<4, 2, false>(a, fresh_w, sm_count, s);
+  return launch_gemv<8, 2, false>(a, fresh_w, sm_count, s);
 }

@@ -31,6 +31,7 @@ struct GemvMmaArgs {
   float eps;
   int out_f32;
   int act;                        // epilogue activation of the plain form
+  int fresh_w;                    // host: W was written on this stream just before (no loads of it ahead of the wait)
   // split-K over blockIdx.y: partial tiles (and partial sums of squares) go to `ws`, the last CTA of a tile to arrive
   // adds them up in split order (deterministic) and runs the epilogue; counters clean themselves
   int split, klen;                // klen = k values per split (multiple of 32)
@@ -275,7 +276,7 @@ static int launch_g2(GemvMmaArgs a, int split, float* ws, long ws_floats, int* c
   a.split = split;
   a.klen = ((a.K / 32 + split - 1) / split) * 32;
   a.ws = ws; a.counters = counters;
-  return (int)launch_pdl(gemv_mma_kernel<MT, RT, DUAL>, dim3(tiles, split), dim3(GM2_WARPS * 32), Gm2<MT>::SMEM, s, a);
+  return (int)launch_pdl_if(!a.fresh_w, gemv_mma_kernel<MT, RT, DUAL>, dim3(tiles, split), dim3(GM2_WARPS * 32), Gm2<MT>::SMEM, s, a);
 }
 
 // Row tiles per CTA (RT x 16 weight rows) and k split. Two CTAs are resident per SM; a CTA first stages its k range of
@@ -317,10 +318,11 @@ static int pick_rt(const GemvMmaArgs& a, int sm_count, float* ws, long ws_floats
 
 using namespace fb;
 
-// mode 1: SwiGLU (W = [gate rows | up rows], 2N rows), mode 2: squared relu. M <= 32, K % 32 == 0, ldx % 8 == 0.
+// mode 1: SwiGLU (W = [gate rows | up rows], 2N rows), mode 2: squared relu. M <= 32, K % 32 == 0, ldx % 8 == 0. fresh_w: W was written on
+// this stream just before.
 extern "C" int fb_gemv_mma(void* y, const void* x, const void* w, const void* norm_w, const void* res, int M, int N, int K,
                            long ldx, long ldy, float eps, int mode, int out_f32, float* ws, long ws_floats, int* counters,
-                           int n_counters, int sm_count, cudaStream_t s) {
+                           int n_counters, int fresh_w, int sm_count, cudaStream_t s) {
   if (M <= 0 || N <= 0) return 0;
   if (M > 32 || K % 32 || ldx % 8) return -1;
   if (sm_count <= 0) sm_count = 148;
@@ -328,7 +330,7 @@ extern "C" int fb_gemv_mma(void* y, const void* x, const void* w, const void* no
   a.y = y; a.x = (const __nv_bfloat16*)x; a.w = (const __nv_bfloat16*)w; a.norm_w = (const __nv_bfloat16*)norm_w;
   a.res = (const __nv_bfloat16*)res; a.M = M; a.N = N; a.K = K; a.ldx = ldx; a.ldy = ldy; a.eps = eps; a.out_f32 = out_f32;
   a.act = mode == 2 ? ACT_RELU2 : ACT_NONE;
-  a.split = 1; a.klen = K; a.ws = nullptr; a.counters = nullptr;
+  a.split = 1; a.klen = K; a.ws = nullptr; a.counters = nullptr; a.fresh_w = fresh_w;
   const int mt = (M + 7) / 8;
 #define FB_G2(MTT, D) return pick_rt<MTT, D>(a, sm_count, ws, ws_floats, counters, n_counters, s)
   if (mode == 1) {

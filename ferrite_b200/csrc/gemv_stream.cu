@@ -4,7 +4,8 @@
 // What bounds such a product is how many bytes of weights are in flight, and what every launch costs before its first and after its last
 // byte. So:
 //   * one thread keeps a ring of 16 KB TMA loads full (about 200 KB in flight per SM in two CTAs), from before the previous kernel has ended:
-//     weights do not depend on it. Loads held in registers (the form this replaced) kept 64 KB in flight.
+//     weights do not depend on it (where they do, `fresh_w`, the launch starts behind it). Loads held in registers (the form this replaced) kept
+//     64 KB in flight.
 //   * the units of work (128 rows x 128 bytes of K, stream_mma.cuh) of all row tiles form one list that is cut into equal runs, one per CTA,
 //     whatever N and K are.
 //   * three warps bring the rows of x beside each unit, in turn, scaled by (1 + w) of the norm, and sum their squares on the way; the norm's
@@ -354,7 +355,7 @@ static GsPlan gs_plan(int M, int N, int K, bool fp4, bool dual, int sm_count) {
 }
 
 template <int MT, bool FP4, bool DUAL, bool XT>
-static int launch_gs(GsArgs a, const GsPlan& p, const CUtensorMap& tw, const CUtensorMap& tx, cudaStream_t s) {
+static int launch_gs(GsArgs a, const GsPlan& p, const CUtensorMap& tw, const CUtensorMap& tx, bool fresh_w, cudaStream_t s) {
   using C = Gs<MT, FP4, DUAL, XT>;
   static const cudaError_t attr =
       cudaFuncSetAttribute(gemv_stream_kernel<MT, FP4, DUAL, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_SMEM);
@@ -362,7 +363,7 @@ static int launch_gs(GsArgs a, const GsPlan& p, const CUtensorMap& tw, const CUt
   int stages = (int)((GS_SMEM - 1024) / C::STAGE);
   if (stages > GS_MAX_STAGES) stages = GS_MAX_STAGES;
   a.stages = stages;
-  return (int)launch_pdl(gemv_stream_kernel<MT, FP4, DUAL, XT>, dim3(p.grid), dim3(C::THREADS), (size_t)stages * C::STAGE + 1024, s, tw, tx, a);
+  return (int)launch_pdl_if(!fresh_w, gemv_stream_kernel<MT, FP4, DUAL, XT>, dim3(p.grid), dim3(C::THREADS), (size_t)stages * C::STAGE + 1024, s, tw, tx, a);
 }
 
 }  // namespace fb
@@ -370,10 +371,11 @@ static int launch_gs(GsArgs a, const GsPlan& p, const CUtensorMap& tw, const CUt
 using namespace fb;
 
 // Weights bf16 [N or 2N][K] (sf null; K % 8 == 0; M <= 32, with norm_w M <= 8) or e2m1 codes [..][K / 2] with scale tiles sf (K % 256 == 0,
-// SwiGLU: N % 128 == 0; M <= 8). mode 1: SwiGLU over [gate rows | up rows], 2: squared relu.
+// SwiGLU: N % 128 == 0; M <= 8). mode 1: SwiGLU over [gate rows | up rows], 2: squared relu. fresh_w: the weights were written on this stream
+// just before.
 extern "C" int fb_gemv_stream(void* y, const void* x, const void* w, const void* sf, float w_scale, const float* row_alpha, const void* norm_w,
                               const void* res, int M, int N, int K, long ldx, long ldy, float eps, int mode, int out_f32, float* ws,
-                              long ws_floats, int* counters, int n_counters, int* status, int sm_count, cudaStream_t s) {
+                              long ws_floats, int* counters, int n_counters, int fresh_w, int* status, int sm_count, cudaStream_t s) {
   if (M <= 0 || N <= 0) return 0;
   const bool fp4 = sf != nullptr, dual = mode == 1;
   if (sm_count <= 0) sm_count = 148;
@@ -391,11 +393,11 @@ extern "C" int fb_gemv_stream(void* y, const void* x, const void* w, const void*
   CUtensorMap tw, tx;
   if (!sm_map(&tw, w, fp4, fp4 ? K / 2 : K, dual ? 2L * N : N, fp4 ? K / 2 : 2L * K, fp4 ? 128 : 64, 64)) return -12;
   if (fp4 || norm_w) {
-    if (fp4) return dual ? launch_gs<1, true, true, false>(a, p, tw, tw, s) : launch_gs<1, true, false, false>(a, p, tw, tw, s);
-    return dual ? launch_gs<1, false, true, false>(a, p, tw, tw, s) : launch_gs<1, false, false, false>(a, p, tw, tw, s);
+    if (fp4) return dual ? launch_gs<1, true, true, false>(a, p, tw, tw, fresh_w, s) : launch_gs<1, true, false, false>(a, p, tw, tw, fresh_w, s);
+    return dual ? launch_gs<1, false, true, false>(a, p, tw, tw, fresh_w, s) : launch_gs<1, false, false, false>(a, p, tw, tw, fresh_w, s);
   }
   if (!sm_map(&tx, x, false, K, M, 2L * ldx, 64, 8 * mt)) return -12;
-#define FB_GS(MT) return dual ? launch_gs<MT, false, true, true>(a, p, tw, tx, s) : launch_gs<MT, false, false, true>(a, p, tw, tx, s)
+#define FB_GS(MT) return dual ? launch_gs<MT, false, true, true>(a, p, tw, tx, fresh_w, s) : launch_gs<MT, false, false, true>(a, p, tw, tx, fresh_w, s)
   switch (mt) {
     case 1: FB_GS(1);
     case 2: FB_GS(2);

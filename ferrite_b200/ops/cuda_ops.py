@@ -189,8 +189,10 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         self.C.relu2(y, x)
         return y
 
-    def linear(self, x, w, norm_w=None, eps=1e-6, res=None, swiglu=False, out_f32=False, out=None, act=None):
-        """`act`: activation of the epilogue ("relu2": squared relu), not together with SwiGLU."""
+    def linear(self, x, w, norm_w=None, eps=1e-6, res=None, swiglu=False, out_f32=False, out=None, act=None, fresh_w=False):
+        """`act`: activation of the epilogue ("relu2": squared relu), not together with SwiGLU. `fresh_w`: a dense `w` that the call before
+        wrote on this stream (a scratch that packed weights were decoded into): the few-row kernels, which else ask for weights before the
+        launch ahead of them has ended, start behind it."""
         if self.dtype == torch.float32:
             assert norm_w is None and res is None, "fp32 linears have an activation epilogue only"
             return self.silu_mul_f32(self.linear_f32(x, w), out) if swiglu else self.linear_f32(x, w, act, out)
@@ -211,7 +213,7 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
                     dense = self.scratch("gguf_dense", w.rows * w.cols).view(w.rows, w.cols)
                     self.launches += 1
                     self.C.gguf_dequant(dense, w.raw, w.type_id)
-                    y = self.linear(x, dense, res=None if swiglu else res)
+                    y = self.linear(x, dense, res=None if swiglu else res, fresh_w=True)
             else:
                 y = torch.cat([self.linear(x, p) for p in w.parts], 1)
                 self.launches += 1
@@ -269,9 +271,9 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
             if w.numel() < STREAM_VALUES and K % 32 == 0 and w.stride(0) == K:
                 y = out if out is not None else self.empty(M, N, dtype=torch.float32 if out_f32 else self.dtype, device=self.device)
                 self.launches += 1
-                self.C.gemv_mma(y, x, w, norm_w, res, eps, 1 if swiglu else 2 if act else 0, self._workspace(8 << 20), self._counters)
+                self.C.gemv_mma(y, x, w, norm_w, res, eps, 1 if swiglu else 2 if act else 0, self._workspace(8 << 20), self._counters, fresh_w)
                 return y
-            y = self._stream(x, w, None, 1.0, None, norm_w, eps, res, 1 if swiglu else 2 if act else 0, N, out_f32, out)
+            y = self._stream(x, w, None, 1.0, None, norm_w, eps, res, 1 if swiglu else 2 if act else 0, N, out_f32, out, fresh_w)
             if y is not None:
                 return y
         if M <= GEMV_MAX_ROWS or self.force_gemv_chunks:
@@ -280,7 +282,7 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
                 r1 = min(M, r0 + GEMV_MAX_ROWS)
                 self.launches += 1
                 self.C.gemv(y[r0:r1], x[r0:r1], w, norm_w, None if res is None else res[r0:r1], eps, True,
-                            1 if swiglu else 2 if act else 0)
+                            1 if swiglu else 2 if act else 0, fresh_w)
             return y
         if norm_w is not None:
             x, _ = self.rmsnorm(x, norm_w, eps, True)
@@ -293,7 +295,7 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         self.C.gemm(y, x, w, res, (1 if swiglu else 0) | (2 if out_f32 else 0) | (4 if act else 0), split, ws, cnt, self.status_word)
         return y
 
-    def _stream(self, x, w, sf, scale, row_alpha, norm_w, eps, res, mode, N, out_f32, out=None):
+    def _stream(self, x, w, sf, scale, row_alpha, norm_w, eps, res, mode, N, out_f32, out=None, fresh_w=False):
         """Up to 32 rows: weights (bf16, or e2m1 codes with scale tiles `sf`) streamed through a TMA ring into mma.sync fragments. None where
         the kernel does not take the shape (rows that are no multiple of 16 bytes, 4-bit rows that are no multiple of 256 values)."""
         if not w.is_contiguous():
@@ -301,7 +303,8 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         if norm_w is not None and x.shape[0] > 8 and sf is None:
             x, norm_w = self.rmsnorm(x, norm_w, eps, True)[0], None      # rows beyond one token tile come in by TMA as they are
         y = out if out is not None else self.empty(x.shape[0], N, dtype=torch.float32 if out_f32 else self.dtype, device=self.device)
-        if self.C.gemv_stream(y, x, w, sf, scale, row_alpha, norm_w, res, eps, mode, self._workspace(8 << 20), self._counters, self.status_word) < 0:
+        if self.C.gemv_stream(y, x, w, sf, scale, row_alpha, norm_w, res, eps, mode, self._workspace(8 << 20), self._counters, self.status_word,
+                              fresh_w) < 0:
             return None
         self.launches += 1
         return y

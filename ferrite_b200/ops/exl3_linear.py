@@ -41,7 +41,7 @@ class Exl3Linear:
         C.exl3_had(xh, x.contiguous(), self.suh, None, None, HAD)
         w_hat_t = ops.scratch("exl3_w_hat", self.n * self.k).view(self.n, self.k)
         C.exl3_decode(w_hat_t, self.trellis, self.bits)
-        z = ops.linear(xh, w_hat_t)
+        z = ops.linear(xh, w_hat_t, fresh_w=True)
         C.exl3_had(y, z, None, self.svh, res, HAD)
         ops.launches += 3
         return y

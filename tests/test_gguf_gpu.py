@@ -78,6 +78,22 @@ def test_gemv_matches_dequantised_matmul(ops, name, M):
     assert (got - want).abs().max().item() < 2e-2 * max(1.0, want.abs().max().item())
 
 
+@pytest.mark.parametrize("M", [1, 2, 9, 32])
+@pytest.mark.parametrize("N", [96, 1300])
+def test_two_weights_through_one_scratch(ops, M, N):
+    """Wide blocks, or more rows than the GEMV on the blocks takes: decoded into a scratch that the next weight overwrites, and multiplied by
+    kernels that ask for weights early. Each product is that of its own weight."""
+    from ferrite_b200.ops.qweight import GgufWeight
+    K, tid = 6656, TYPE_ID["Q8_0"]
+    raws = [torch.from_numpy(random_blocks("Q8_0", N * K // 32, seed=s)).to(DEV) for s in (1, 2)]
+    ws = [GgufWeight(r, tid, N, K) for r in raws]
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).to(DEV)
+    want = [ops.linear(x, ops.gguf_dequant(r, tid, (N, K)), fresh_w=True) for r in raws]
+    assert not torch.equal(*want)
+    for i in range(16):
+        assert torch.equal(ops.linear(x, ws[i % 2]), want[i % 2]), i
+
+
 def test_q8_1_quant(ops):
     x = torch.randn(64 * 32, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16)
     out = ops.q8_1_quant(x.to(DEV)).cpu().numpy().reshape(-1, 36)
