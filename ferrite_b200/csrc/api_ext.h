@@ -64,6 +64,9 @@ int fb_gemm_nvfp4_swiglu_q(void* q_codes, void* q_sf, float* q_row_scale, float 
                            int* status, int sm_count, cudaStream_t s);
 
 // ---- gemv_stream.cu: products of up to 32 rows, bf16 or NVFP4 weights streamed through a TMA ring ----
+int fb_gemv_stream_fits(const void* x, const void* w, const void* sf, const void* norm_w, int M, int N, int K, long ldx, int mode);
+long fb_gemv_stream_ws_floats(int sm_count);
+int fb_gemv_stream_counters(int sm_count);
 int fb_gemv_stream(void* y, const void* x, const void* w, const void* sf, float w_scale, const float* row_alpha, const void* norm_w, const void* res,
                    int M, int N, int K, long ldx, long ldy, float eps, int mode, int out_f32, float* ws, long ws_floats, int* counters, int n_counters,
                    int fresh_w, int* status, int sm_count, cudaStream_t s);

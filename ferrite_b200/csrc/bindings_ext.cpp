@@ -216,20 +216,26 @@ void gemm_nvfp4_fused(Tensor Y, Tensor X, c10::optional<Tensor> norm_w, double e
         "gemm_nvfp4_fused");
 }
 
-// Y = act(X (optionally RMSNorm(1 + w)) W^T) (+ res) for up to 32 rows; W bf16, or e2m1 codes with scale tiles `sf`. Returns the code of an
-// unsupported shape (negative) instead of raising: the caller has other kernels.
-int64_t gemv_stream(Tensor Y, Tensor X, Tensor W, c10::optional<Tensor> sf, double w_scale, c10::optional<Tensor> row_alpha,
-                    c10::optional<Tensor> norm_w, c10::optional<Tensor> res, double eps, int64_t mode, Tensor workspace, Tensor counters, Tensor status,
-                    bool fresh_w) {
+// Whether `gemv_stream` takes the call (made: the rows are still to be written, contiguous, as a norm leaves them).
+bool gemv_stream_fits(Tensor X, Tensor W, c10::optional<Tensor> sf, c10::optional<Tensor> norm_w, int64_t mode, bool made) {
+  const int M = (int)X.size(0), K = (int)X.size(1), N = (int)(mode == 1 ? W.size(0) / 2 : W.size(0));
+  return W.is_contiguous() &&
+         fb_gemv_stream_fits(made ? nullptr : X.data_ptr(), W.data_ptr(), cptr(sf), made ? nullptr : cptr(norm_w), M, N, K,
+                             made ? (long)K : (long)X.stride(0), (int)mode) != 0;
+}
+
+// Y = act(X (optionally RMSNorm(1 + w)) W^T) (+ res) for up to 32 rows; W bf16, or e2m1 codes with scale tiles `sf`. Calls that
+// `gemv_stream_fits` says no to raise.
+void gemv_stream(Tensor Y, Tensor X, Tensor W, c10::optional<Tensor> sf, double w_scale, c10::optional<Tensor> row_alpha,
+                 c10::optional<Tensor> norm_w, c10::optional<Tensor> res, double eps, int64_t mode, Tensor workspace, Tensor counters, Tensor status,
+                 bool fresh_w) {
   const int M = (int)X.size(0), K = (int)X.size(1), N = (int)(mode == 1 ? W.size(0) / 2 : W.size(0));
   TORCH_CHECK(X.stride(1) == 1 && Y.stride(1) == 1 && W.is_contiguous() && W.size(1) == (sf.has_value() ? K / 2 : K), "gemv_stream: layouts");
   TORCH_CHECK(!res.has_value() || res->stride(0) == Y.stride(0) || M == 1, "gemv_stream: residual rows lie apart as the output's do");
-  const int rc = fb_gemv_stream(Y.data_ptr(), X.data_ptr(), W.data_ptr(), cptr(sf), (float)w_scale, (const float*)cptr(row_alpha), cptr(norm_w), cptr(res),
-                                M, N, K, (long)X.stride(0), (long)Y.stride(0), (float)eps, (int)mode, Y.scalar_type() == torch::kFloat32 ? 1 : 0,
-                                workspace.data_ptr<float>(), (long)workspace.numel(), counters.data_ptr<int>(), (int)counters.numel(), fresh_w ? 1 : 0,
-                                status.data_ptr<int>(), at::cuda::getCurrentDeviceProperties()->multiProcessorCount, cur_stream());
-  if (rc > 0) check(rc, "gemv_stream");
-  return rc;
+  check(fb_gemv_stream(Y.data_ptr(), X.data_ptr(), W.data_ptr(), cptr(sf), (float)w_scale, (const float*)cptr(row_alpha), cptr(norm_w), cptr(res),
+                       M, N, K, (long)X.stride(0), (long)Y.stride(0), (float)eps, (int)mode, Y.scalar_type() == torch::kFloat32 ? 1 : 0,
+                       workspace.data_ptr<float>(), (long)workspace.numel(), counters.data_ptr<int>(), (int)counters.numel(), fresh_w ? 1 : 0,
+                       status.data_ptr<int>(), at::cuda::getCurrentDeviceProperties()->multiProcessorCount, cur_stream()), "gemv_stream");
 }
 
 int64_t gemv_nvfp4_tc_workspace_bytes(int64_t M, int64_t N, int64_t K, bool dual, int64_t terms, int64_t ctas_per_sm) {
@@ -1072,6 +1078,9 @@ void register_ext(pybind11::module_& m) {
   m.def("gemm_nvfp4", &gemm_nvfp4);
   m.def("gemm_nvfp4_fused", &gemm_nvfp4_fused);
   m.def("gemm_nvfp4_swiglu_q", &gemm_nvfp4_swiglu_q);
+  m.def("gemv_stream_fits", &gemv_stream_fits);
+  m.def("gemv_stream_ws_floats", &fb_gemv_stream_ws_floats);
+  m.def("gemv_stream_counters", &fb_gemv_stream_counters);
   m.def("gemv_stream", &gemv_stream, pybind11::arg("Y"), pybind11::arg("X"), pybind11::arg("W"), pybind11::arg("sf"), pybind11::arg("w_scale"),
         pybind11::arg("row_alpha"), pybind11::arg("norm_w"), pybind11::arg("res"), pybind11::arg("eps"), pybind11::arg("mode"), pybind11::arg("workspace"),
         pybind11::arg("counters"), pybind11::arg("status"), pybind11::arg("fresh_w") = false);

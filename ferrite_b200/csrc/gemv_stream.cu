@@ -37,13 +37,15 @@ struct GsArgs {
   const uint8_t* sf;              // NVFP4: scale tiles [row tile][K / 64][512]
   const float* row_alpha;         // NVFP4: tensor scale per weight row (null: w_scale)
   float w_scale, eps;
-  float* ws;                      // records [item][slot][warp]: sums of the lanes, sums of squares
-  int* counters;                  // [item][warp], left zero
+  // What a CTA leaves of a tile that it does not do alone. A run meets at most two such tiles: one that began in a run before it and one that
+  // begins in it and goes on, so records and counters follow the grid and not the number of outputs.
+  float* ws;                      // records [CTA][begun before, begins here][warp]: sums of the lanes, sums of squares
+  int* counters;                  // [CTA in which the tile begins][warp], left zero
   int* status;
   int M, N, K;
   long ldx, ldy;
   int act, out_f32;
-  int kblocks, items, stages, max_slots;
+  int kblocks, items, stages;
   int lo_rows;                    // token columns from here on hold what bf16 rounds off x (1 + w); 0: none
 };
 
@@ -235,8 +237,9 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       if (kb0 != 0 || kb1 != a.kblocks) {
         const long long ui0 = (long long)item * a.kblocks;
         const int c_first = (int)(((ui0 + 1) * gridDim.x - 1) / U), c_last = (int)(((ui0 + a.kblocks) * gridDim.x - 1) / U);
-        float* rec0 = a.ws + (size_t)item * a.max_slots * GS_MATH * C::REC;
-        float* rec = rec0 + (size_t)(((int)blockIdx.x - c_first) * GS_MATH + warp) * C::REC;
+        auto record = [&](int cta) { return a.ws + (size_t)((cta * 2 + (cta == c_first ? 1 : 0)) * GS_MATH + warp) * C::REC; };
+        float* rec = record((int)blockIdx.x);
+        int* counter = a.counters + c_first * GS_MATH + warp;
 #pragma unroll
         for (int i = 0; i < MT; ++i) {
           __stcg(reinterpret_cast<float4*>(rec) + i * 32 + lane, make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]));
@@ -245,7 +248,7 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         __threadfence();
         __syncwarp();
         int old = 0;
-        if (lane == 0) old = atomicAdd(&a.counters[item * GS_MATH + warp], kb1 - kb0);
+        if (lane == 0) old = atomicAdd(counter, kb1 - kb0);
         finish = __shfl_sync(0xffffffffu, old, 0) + (kb1 - kb0) == a.kblocks;
         if (finish) {
           __threadfence();
@@ -258,7 +261,7 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
             float2 q[B][MT];
 #pragma unroll
             for (int j = 0; j < B; ++j) {
-              const float* r = rec0 + (size_t)(min(s0 + j, ns - 1) * GS_MATH + warp) * C::REC;
+              const float* r = record(c_first + min(s0 + j, ns - 1));
 #pragma unroll
               for (int i = 0; i < MT; ++i) {
                 p[j][i] = __ldcg(reinterpret_cast<const float4*>(r) + i * 32 + lane);
@@ -274,7 +277,7 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                   if (!XT) { sq[i][0] += q[j][i].x; sq[i][1] += q[j][i].y; }
                 }
           }
-          if (lane == 0) a.counters[item * GS_MATH + warp] = 0;
+          if (lane == 0) *counter = 0;
         }
       }
       if (!finish) continue;
@@ -323,7 +326,7 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       for (uint32_t p = 0; p < 2; ++p) (void)mbar_wait(&full_bar[i], p, 1u << 12);
 }
 
-struct GsPlan { int grid, items, kblocks, max_slots; long rec_floats; };
+struct GsPlan { int grid, items, kblocks; long rec_floats; };
 
 // How many runs the units are cut into. A run costs its share of the ring's first turn and, where it ends inside a tile, a record that another
 // one reads: short runs lose. Measured (us a call in a row of calls, one row, N x K):
@@ -344,13 +347,7 @@ static GsPlan gs_plan(int M, int N, int K, bool fp4, bool dual, int sm_count) {
   // nearly as many tiles as CTAs: a whole tile each has nothing to merge
   if (p.items <= grid && (long long)p.items * 8 >= grid * 7) grid = p.items;
   p.grid = (int)grid;
-  const long long per_lo = U / grid;
-  long long slots = p.kblocks / (per_lo > 0 ? per_lo : 1) + 2;
-  if (slots > p.kblocks) slots = p.kblocks;
-  if (slots > grid) slots = grid;
-  p.max_slots = (int)slots;
-  const int mt = (M + 7) / 8;
-  p.rec_floats = (long)p.items * p.max_slots * GS_MATH * (136 * mt);
+  p.rec_floats = (long)p.grid * 2 * GS_MATH * (136 * ((M + 7) / 8));
   return p;
 }
 
@@ -370,6 +367,19 @@ static int launch_gs(GsArgs a, const GsPlan& p, const CUtensorMap& tw, const CUt
 
 using namespace fb;
 
+// Whether the kernel takes a call: 0 leaves it to other kernels (rows that lie on no 16 bytes or over one another, more rows than its token tiles,
+// 4-bit rows that are no whole units). x may be null (rows that are still to be made, ldx apart).
+extern "C" int fb_gemv_stream_fits(const void* x, const void* w, const void* sf, const void* norm_w, int M, int N, int K, long ldx, int mode) {
+  const bool fp4 = sf != nullptr;
+  if (M > (fp4 || norm_w ? 8 : 32) || K <= 0 || K % 8 || (fp4 && (K % 256 || (mode == 1 && N % 128)))) return 0;
+  if (ldx % 8 || (!fp4 && !norm_w && M > 1 && ldx < K)) return 0;
+  return (((uintptr_t)x | (uintptr_t)w | (uintptr_t)sf | (uintptr_t)norm_w) & 15) == 0;
+}
+
+// Floats of workspace and ints of counters that any call of up to 32 rows fits, whatever its sizes.
+extern "C" long fb_gemv_stream_ws_floats(int sm_count) { return 2L * sm_count * 2 * GS_MATH * 136 * 4; }
+extern "C" int fb_gemv_stream_counters(int sm_count) { return 2 * sm_count * GS_MATH; }
+
 // Weights bf16 [N or 2N][K] (sf null; K % 8 == 0; M <= 32, with norm_w M <= 8) or e2m1 codes [..][K / 2] with scale tiles sf (K % 256 == 0,
 // SwiGLU: N % 128 == 0; M <= 8). mode 1: SwiGLU over [gate rows | up rows], 2: squared relu. fresh_w: the weights were written on this stream
 // just before.
@@ -379,15 +389,14 @@ extern "C" int fb_gemv_stream(void* y, const void* x, const void* w, const void*
   if (M <= 0 || N <= 0) return 0;
   const bool fp4 = sf != nullptr, dual = mode == 1;
   if (sm_count <= 0) sm_count = 148;
-  if (M > (fp4 || norm_w ? 8 : 32) || K <= 0 || K % 8 || (fp4 && (K % 256 || (dual && N % 128))) || ldx % 8) return -1;
-  if (((uintptr_t)x | (uintptr_t)w | (uintptr_t)sf | (uintptr_t)norm_w) & 15) return -1;
+  if (!x || !w || !fb_gemv_stream_fits(x, w, sf, norm_w, M, N, K, ldx, mode)) return -1;
   const GsPlan p = gs_plan(M, N, K, fp4, dual, sm_count);
-  if (!ws || !counters || p.rec_floats > ws_floats || p.items > n_counters / GS_MATH) return -6;
+  if (!ws || !counters || p.rec_floats > ws_floats || p.grid > n_counters / GS_MATH) return -6;
   GsArgs a;
   a.y = y; a.res = (const __nv_bfloat16*)res; a.x = (const __nv_bfloat16*)x; a.norm_w = (const __nv_bfloat16*)norm_w; a.sf = (const uint8_t*)sf;
   a.row_alpha = row_alpha; a.w_scale = w_scale; a.eps = eps; a.ws = ws; a.counters = counters; a.status = status; a.M = M; a.N = N; a.K = K;
   a.ldx = ldx; a.ldy = ldy; a.act = mode == 2 ? ACT_RELU2 : ACT_NONE; a.out_f32 = out_f32; a.kblocks = p.kblocks; a.items = p.items;
-  a.max_slots = p.max_slots; a.stages = 0;
+  a.stages = 0;
   a.lo_rows = norm_w && M <= 4 ? 4 : 0;
   const int mt = (M + 7) / 8;
   CUtensorMap tw, tx;
@@ -396,7 +405,7 @@ extern "C" int fb_gemv_stream(void* y, const void* x, const void* w, const void*
     if (fp4) return dual ? launch_gs<1, true, true, false>(a, p, tw, tw, fresh_w, s) : launch_gs<1, true, false, false>(a, p, tw, tw, fresh_w, s);
     return dual ? launch_gs<1, false, true, false>(a, p, tw, tw, fresh_w, s) : launch_gs<1, false, false, false>(a, p, tw, tw, fresh_w, s);
   }
-  if (!sm_map(&tx, x, false, K, M, 2L * ldx, 64, 8 * mt)) return -12;
+  if (!sm_map(&tx, x, false, K, M, 2L * (M > 1 ? ldx : K), 64, 8 * mt)) return -12;
 #define FB_GS(MT) return dual ? launch_gs<MT, false, true, true>(a, p, tw, tx, fresh_w, s) : launch_gs<MT, false, false, true>(a, p, tw, tx, fresh_w, s)
   switch (mt) {
     case 1: FB_GS(1);

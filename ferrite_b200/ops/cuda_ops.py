@@ -54,7 +54,8 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         self.sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
         self.status_word = torch.zeros(1, dtype=torch.int32, device=self.device)
         self._ws: Optional[torch.Tensor] = None
-        self._counters = torch.zeros(32768, dtype=torch.int32, device=self.device)
+        self._counters = torch.zeros(max(32768, self.C.gemv_stream_counters(self.sm_count)), dtype=torch.int32, device=self.device)
+        self._stream_bytes = 4 * self.C.gemv_stream_ws_floats(self.sm_count)       # of the workspace, whatever the sizes of the product
         self._tail = None
         self._tail_counters = torch.zeros(148 * 32, dtype=torch.int32, device=self.device)
         self.empty = torch.empty            # every output buffer of the ops comes from here (see enable_canaries)
@@ -296,17 +297,18 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         return y
 
     def _stream(self, x, w, sf, scale, row_alpha, norm_w, eps, res, mode, N, out_f32, out=None, fresh_w=False):
-        """Up to 32 rows: weights (bf16, or e2m1 codes with scale tiles `sf`) streamed through a TMA ring into mma.sync fragments. None where
-        the kernel does not take the shape (rows that are no multiple of 16 bytes, 4-bit rows that are no multiple of 256 values)."""
-        if not w.is_contiguous():
+        """Up to 32 rows: weights (bf16, or e2m1 codes with scale tiles `sf`) streamed through a TMA ring into mma.sync fragments. None, before
+        anything is launched, where the kernel does not take the call (rows that are no multiple of 16 bytes or lie on none, 4-bit rows that are
+        no multiple of 256 values)."""
+        apart = norm_w is not None and x.shape[0] > 8 and sf is None     # rows beyond one token tile come in by TMA as they are
+        if not self.C.gemv_stream_fits(x, w, sf, norm_w, mode, apart):
             return None
-        if norm_w is not None and x.shape[0] > 8 and sf is None:
-            x, norm_w = self.rmsnorm(x, norm_w, eps, True)[0], None      # rows beyond one token tile come in by TMA as they are
+        if apart:
+            x, norm_w = self.rmsnorm(x, norm_w, eps, True)[0], None
         y = out if out is not None else self.empty(x.shape[0], N, dtype=torch.float32 if out_f32 else self.dtype, device=self.device)
-        if self.C.gemv_stream(y, x, w, sf, scale, row_alpha, norm_w, res, eps, mode, self._workspace(8 << 20), self._counters, self.status_word,
-                              fresh_w) < 0:
-            return None
         self.launches += 1
+        self.C.gemv_stream(y, x, w, sf, scale, row_alpha, norm_w, res, eps, mode, self._workspace(self._stream_bytes), self._counters, self.status_word,
+                           fresh_w)
         return y
 
     # ---- FP8 (e4m3) weights and activations -----------------------------------------------------------

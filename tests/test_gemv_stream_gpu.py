@@ -83,3 +83,25 @@ def test_shapes_left_to_other_kernels(ops):
     assert ops._stream(rnd(2, 12), rnd(64, 12), None, 1.0, None, None, 1e-6, None, 0, 64, True) is None
     z = torch.zeros(64, 64, dtype=torch.uint8, device=DEV)
     assert ops._stream(rnd(2, 128), z, z, 1.0, None, None, 1e-6, None, 0, 64, True) is None
+    n0 = ops.launches
+    assert ops._stream(rnd(9, 12), rnd(64, 12), None, 1.0, None, rnd(12), 1e-6, None, 0, 64, True) is None            # nor the norm of more rows
+    odd = rnd(64 * 64 + 1)[1:].view(64, 64)                                                                          # weights on no 16 bytes
+    assert ops._stream(rnd(9, 64), odd, None, 1.0, None, rnd(64), 1e-6, None, 0, 64, True) is None
+    assert ops._stream(rnd(1, 64).expand(3, 64), rnd(64, 64), None, 1.0, None, None, 1e-6, None, 0, 64, True) is None   # one row three times
+    assert ops.launches == n0
+    with pytest.raises(RuntimeError):
+        ops.C.gemv_stream(torch.empty(2, 64, device=DEV), rnd(2, 12), rnd(64, 12), None, 1.0, None, None, None, 1e-6, 0, ops._workspace(1),
+                          ops._counters, ops.status_word)
+
+
+def test_records_follow_the_grid_and_not_the_outputs(ops):
+    """As many rows against as wide a head as there is: what the runs leave behind fits, and the call is not left to another kernel."""
+    M, N, K = 32, 262144, 512
+    x, w = rnd(M, K, seed=1), rnd(N, K, seed=2, scale=K ** -0.5)
+    y = ops._stream(x, w, None, 1.0, None, None, 1e-6, None, 0, N, True)
+    assert y is not None
+    for n in range(0, N, 65536):
+        want = x.double() @ w[n:n + 65536].double().t()
+        # 32-bit sums of products exact in 32 bits
+        assert (y[:, n:n + 65536].double() - want).abs().max().item() <= 2 ** -14 * max(1.0, want.abs().max().item())
+    assert ops.status() == 0 and int(ops._counters.abs().sum()) == 0
