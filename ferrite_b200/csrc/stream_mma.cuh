@@ -66,11 +66,16 @@ __device__ __forceinline__ uint32_t sm_mul_bf2(uint32_t a, uint32_t b) {
 // e2m1 to bf16 by bit placement: sign to bit 15, the three bits of exponent and fraction to bits 8..6, so that a code's value comes out times
 // 2^-126 (0.5 as a subnormal). The e4m3 block scale is placed the same way (its seven bits to 10..4: times 2^-120) and brought to 2^118 by
 // two exact products; code x scale, six significant bits, is exact in bf16 and holds the weight times 2^-8, which the caller makes up for.
+// e4m3 has one NaN and no infinity: its bits would be 480, the next step after the largest value, 448. A factor of 1.1 x 2^112 (at a scale times
+// 2^7) overflows for the one and not for the other, and adding 0 x that product turns only it into NaN. (Beside the ~40 instructions that unpack
+// a scale's 16 codes these two, of the multiplier pipe, are not seen.)
 constexpr float SM_FP4_FACTOR = 256.f;
 __device__ __forceinline__ uint2 sm_scales(uint32_t two) {                       // two neighbouring block scales -> each in both halves
   uint32_t v = ((two & 0xffu) << 4) | ((two & 0xff00u) << 12);
   v = sm_mul_bf2(v, 0x7f007f00u);                                               // 2^127
+  const uint32_t top = sm_mul_bf2(v, 0x778d778du);                              // 1.1 x 2^112
   v = sm_mul_bf2(v, 0x77007700u);                                               // 2^111
+  asm("fma.rn.bf16x2 %0, %1, %2, %0;" : "+r"(v) : "r"(top), "r"(0u));
   return make_uint2(__byte_perm(v, v, 0x1010), __byte_perm(v, v, 0x3232));
 }
 // Nibbles j and j + 4 of a word, j = 0 .. 3, times their scale. The product with 2^12 + 2^6 (nibble at bit 0; 2^8 + 2^2 at bit 4) writes the

@@ -77,6 +77,27 @@ def test_nvfp4_weights(ops, M, N, K, swiglu, norm):
     assert ops.status() == 0 and int(ops._counters.abs().sum()) == 0
 
 
+@pytest.mark.parametrize("M", [1, 8])
+def test_nan_scales_of_4_bit_weights(ops, M):
+    """e4m3's NaN (0x7f) as a block scale makes its row's outputs NaN and no other; the largest scale (0x7e, 448) stays what it is."""
+    from ferrite_b200.formats import nvfp4
+    N, K = 130, 512
+    g = torch.Generator(device=DEV).manual_seed(M)
+    packed = torch.randint(0, 256, (N, K // 2), generator=g, device=DEV, dtype=torch.uint8)
+    scales = torch.full((N, K // 16), 0x7e, device=DEV, dtype=torch.uint8)
+    bad = [0, 15, 77, 129]
+    for i, r in enumerate(bad):
+        scales[r, i * 9] = 0x7f
+    t = nvfp4.NVFP4Tensor(packed, scales.view(torch.float8_e4m3fn), 1.0, N, K)
+    x = rnd(M, K, seed=M)
+    y = ops._stream(x, packed, nvfp4.tile_scales_mma(t.scales).contiguous(), 1.0, None, None, 1e-6, None, 0, N, True)
+    nan = torch.zeros(N, dtype=torch.bool, device=DEV)
+    nan[bad] = True
+    assert torch.equal(y.isnan(), nan.expand(M, N))
+    w = t.dequantize(torch.float64)[~nan]
+    assert ((y[:, ~nan].double() - x.double() @ w.t()).abs() <= 2 ** -19 * (x.double().abs() @ w.abs().t())).all()
+
+
 def test_shapes_left_to_other_kernels(ops):
     """Refused before anything is launched: rows that are no multiple of 16 bytes, 4-bit rows that are no multiple of a unit."""
     assert ops._stream(rnd(2, 16), rnd(64, 16)[:, :16], None, 1.0, None, None, 1e-6, None, 0, 64, True) is not None

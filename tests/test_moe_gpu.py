@@ -256,3 +256,25 @@ def test_prompt_experts_from_their_codes(ops, E, K, H, I, T, limit):
     # roundings to bf16 of the activation and of an expert's row (2^-9 each), on top of 32-bit sums
     assert bool(((acc.double() - want).abs() <= 2 ** -7 * mag + 1e-6).all())
     ep.check()
+
+
+def test_prompt_experts_with_a_nan_scale(ops):
+    """A NaN scale in one expert's down projection reaches the rows that picked this expert, in one column, and no others."""
+    from ferrite_b200.ops.qweight import ExpertsFP4
+    from ferrite_b200.parallel.ep import ExpertParallel
+    E, K, H, I, T = 8, 2, 256, 256, 40
+    g = torch.Generator(device=DEV).manual_seed(1)
+    stack = lambda rows, cols: ExpertsFP4(torch.randint(0, 256, (E, rows, cols // 2), generator=g, device=DEV, dtype=torch.uint8),
+                                          torch.randint(0, 127, (E, rows, cols // 16), generator=g, device=DEV, dtype=torch.uint8), 2.0 ** -13)
+    w_gu, w_dn = stack(2 * I, H), stack(H, I)
+    w_dn.scales[5, 33, 7] = 0x7f
+    h = (torch.randn(T, H, generator=g, device=DEV) * 0.3).to(torch.bfloat16)
+    ids = torch.stack([torch.randperm(E, generator=g, device=DEV)[:K] for _ in range(T)]).to(torch.int32)
+    ep = ExpertParallel(None, DEV, E, H, cap_rows=T * K)
+    assert ep.takes_codes(T * K, w_gu, w_dn)
+    acc = torch.zeros(T, H, dtype=torch.float32, device=DEV)
+    ep.moe(ops, h, ids, torch.rand(T, K, generator=g, device=DEV), w_gu, w_dn, acc=acc)
+    want = torch.zeros(T, H, dtype=torch.bool, device=DEV)
+    want[(ids == 5).any(1), 33] = True
+    assert torch.equal(acc.isnan(), want) and want.any()
+    ep.check()
