@@ -56,12 +56,15 @@ int fb_gemv_bf16(void* Y, const void* X, const void* W, const void* norm_w, cons
 
 // ---- gemm_tcgen05.cu ----
 // Y[M][N] = X[M][K] * W[N][K]^T (+ res), or SwiGLU over W = [gate rows | up rows] (2N rows). bf16 in/out,
-// fp32 accumulation in TMEM. workspace/counters are needed only when split_k > 1.
+// fp32 accumulation in TMEM. workspace / counters (fb_gemm_workspace_bytes, fb_gemm_counters, with the sizes that are there): needed when
+// split_k > 1; with more than 64 rows, the last tiles are cut along K where they are given and large enough.
 int fb_gemm_bf16_glu(void* Y, const void* X, const void* W, const void* res, int M, int N, int K, long ldx, long ldy,
-                     int mode, float limit, int split_k, float* workspace, int* counters, int* status, int sm_count, cudaStream_t s);
+                     int mode, float limit, int split_k, float* workspace, long ws_bytes, int* counters, int n_counters, int* status, int sm_count,
+                     cudaStream_t s);
 int fb_gemm_bf16(void* Y, const void* X, const void* W, const void* res, int M, int N, int K, long ldx, long ldy,
-                 int mode, int split_k, float* workspace, int* counters, int* status, int sm_count, cudaStream_t s);
+                 int mode, int split_k, float* workspace, long ws_bytes, int* counters, int n_counters, int* status, int sm_count, cudaStream_t s);
 long fb_gemm_workspace_bytes(int M, int N, int split_k);
+int fb_gemm_counters(int M, int N, int split_k);
 
 // 2..32 rows: weight-streaming linear on mma.sync with in-register A fragments (gemv_mma.cu)
 int fb_gemv_mma(void* y, const void* x, const void* w, const void* norm_w, const void* res, int M, int N, int K, long ldx,
@@ -77,8 +80,8 @@ int fb_quant_fp8_block(void* q, float* scale, const void* x, int rows, int K, lo
 int fb_gemm_fp8_block(void* Y, const void* Xq, const float* sx, const void* Wq, const float* sw, const void* res, int M,
                       int N, int K, long ldy, int* status, cudaStream_t s);
 int fb_gemm_fp8(void* Y, const void* Xq, const void* Wq, const float* scale_m, const float* scale_n, const void* res, int M,
-                int N, int K, long ldy, int mode, int split_k, float* workspace, int* counters, int* status, int sm_count,
-                cudaStream_t s);
+                int N, int K, long ldy, int mode, int split_k, float* workspace, long ws_bytes, int* counters, int n_counters, int* status,
+                int sm_count, cudaStream_t s);
 
 // ---- attn.cu ----
 int fb_attn_prep(void* q_out, void* k_cache, void* v_cache, const void* proj, long proj_stride, const void* q_norm,

@@ -74,14 +74,17 @@ void gemv(Tensor Y, Tensor X, Tensor W, c10::optional<Tensor> norm_w, c10::optio
 int64_t gemm_workspace_bytes(int64_t M, int64_t N, int64_t split_k) {
   return fb_gemm_workspace_bytes((int)M, (int)N, (int)split_k);
 }
+int64_t gemm_counters(int64_t M, int64_t N, int64_t split_k) { return fb_gemm_counters((int)M, (int)N, (int)split_k); }
+long bytes_of(const c10::optional<Tensor>& t) { return t.has_value() ? (long)(t->numel() * t->element_size()) : 0; }
+int ints_of(const c10::optional<Tensor>& t) { return t.has_value() ? (int)t->numel() : 0; }
 
 void gemm(Tensor Y, Tensor X, Tensor W, c10::optional<Tensor> res, int64_t mode, int64_t split_k,
           c10::optional<Tensor> workspace, c10::optional<Tensor> counters, c10::optional<Tensor> status) {
   int M = (int)X.size(0), K = (int)X.size(1);
   int N = (int)((mode & 1) ? W.size(0) / 2 : W.size(0));
   check(fb_gemm_bf16(Y.data_ptr(), X.data_ptr(), W.data_ptr(), cptr(res), M, N, K, (long)X.stride(0),
-                     (long)Y.stride(0), (int)mode, (int)split_k, (float*)mptr(workspace), (int*)mptr(counters),
-                     (int*)mptr(status), sm_count(), cur_stream()), "gemm");
+                     (long)Y.stride(0), (int)mode, (int)split_k, (float*)mptr(workspace), bytes_of(workspace), (int*)mptr(counters),
+                     ints_of(counters), (int*)mptr(status), sm_count(), cur_stream()), "gemm");
 }
 
 void gemv_mma(Tensor Y, Tensor X, Tensor W, c10::optional<Tensor> norm_w, c10::optional<Tensor> res, double eps,
@@ -123,7 +126,7 @@ void gemm_fp8(Tensor Y, Tensor Xq, Tensor Wq, c10::optional<Tensor> scale_m, c10
   int N = (int)(mode == 1 ? Wq.size(0) / 2 : Wq.size(0));
   check(fb_gemm_fp8(Y.data_ptr(), Xq.data_ptr(), Wq.data_ptr(), (const float*)cptr(scale_m), (const float*)cptr(scale_n),
                     cptr(res), M, N, K, (long)Y.stride(0), (int)mode, (int)split_k, (float*)mptr(workspace),
-                    (int*)mptr(counters), (int*)mptr(status), sm_count(), cur_stream()), "gemm_fp8");
+                    bytes_of(workspace), (int*)mptr(counters), ints_of(counters), (int*)mptr(status), sm_count(), cur_stream()), "gemm_fp8");
 }
 
 void attn_prep(Tensor q_out, Tensor k_cache, Tensor v_cache, Tensor proj, Tensor q_norm, Tensor k_norm,
@@ -454,6 +457,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemv_mma", &gemv_mma, py::arg("Y"), py::arg("X"), py::arg("W"), py::arg("norm_w"), py::arg("res"), py::arg("eps"), py::arg("mode"),
         py::arg("workspace"), py::arg("counters"), py::arg("fresh_w") = false);
   m.def("gemm_workspace_bytes", &gemm_workspace_bytes);
+  m.def("gemm_counters", &gemm_counters);
   m.def("attn_prep", &attn_prep);
   m.def("attn_decode", &attn_decode);
   m.def("attn_prefill", &attn_prefill);

@@ -184,7 +184,8 @@ void gemm_glu(Tensor Y, Tensor X, Tensor W, double limit, int64_t split_k, OptTe
   const int M = (int)X.size(0), K = (int)X.size(1), N = (int)W.size(0) / 2;
   TORCH_CHECK(!f32(X) && X.stride(1) == 1 && W.is_contiguous() && Y.size(0) == M && Y.size(1) == N && Y.stride(1) == 1 && W.size(1) == K, "gemm_glu: layouts");
   check(fb_gemm_bf16_glu(Y.data_ptr(), X.data_ptr(), W.data_ptr(), nullptr, M, N, K, (long)X.stride(0), (long)Y.stride(0), 1, (float)limit,
-                         (int)split_k, ptr<float>(workspace), ptr<int>(counters), status.data_ptr<int>(),
+                         (int)split_k, ptr<float>(workspace), workspace ? (long)(workspace->numel() * 4) : 0, ptr<int>(counters),
+                         counters ? (int)counters->numel() : 0, status.data_ptr<int>(),
                          at::cuda::getCurrentDeviceProperties()->multiProcessorCount, cur_stream()), "gemm_glu");
 }
 

@@ -112,6 +112,7 @@ __device__ __forceinline__ bool mbar_wait_or_flag(uint64_t* bar, uint32_t parity
 }
 
 constexpr int GM_KB_COST = 400, GM_TAIL_COST = 18, GM_PIECE_COST = 20, GM_TAIL_MAX = 4;      // see plan_gemm
+constexpr int GM_TILE_CTRS = 32;     // counters of a tile that is cut along K: up to 8 column steps x 4 epilogue warps
 constexpr int GM_COPY_WARPS = 2;   // mode 2: warps 6 and 7 gather remote rows
 constexpr int GM_COPY_COLS = 512;  // columns of X per gather work item (two 16-byte loads per lane and row)
 constexpr int GM_EPI_BYTES = 32 * 32 * 4;   // an epilogue warp's piece of the output on its way
@@ -566,7 +567,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             }
             __threadfence();
             __syncwarp();
-            int* ctr = a.counters + (((w - a.tail_first) % a.tail_tiles) * 8 + st) * 4 + quad;
+            int* ctr = a.counters + ((w - a.tail_first) % a.tail_tiles) * GM_TILE_CTRS + st * 4 + quad;
             int last = 0;
             if (lane == 0) {
               last = atomicAdd(ctr, 1) == a.tail_split - 1;
@@ -858,9 +859,10 @@ static int round_up_pow2(int v) { int p = 32; while (p < v) p <<= 1; return p; }
 
 struct GemmPlan { GemmArgs a; int grid; size_t smem; };
 
-// bytes of workspace / ints of counters that the pieces of any tail fit: a CTA has one piece at most
-inline long gemm_tail_bytes(int sm_count) { return (long)(sm_count > 0 ? sm_count : 148) * GM_BM * 256 * (long)sizeof(float); }
-constexpr int GM_TAIL_CTRS = 148 * 32;
+// bytes of workspace / ints of counters that the pieces of any tail fit on 148 SMs (a CTA has one piece at most), and what those of a plan take
+constexpr long GM_TAIL_BYTES = 148L * GM_BM * 256 * (long)sizeof(float);
+constexpr int GM_TAIL_CTRS = 148 * GM_TILE_CTRS;
+inline long gemm_tail_need(const GemmArgs& a) { return (long)a.tail_tiles * a.tail_split * GM_BM * a.bn * (long)sizeof(float); }
 
 // Normal orientation, tile width and tail (tail = 1: widths only; 2: the last tiles may be cut along K, workspace and counters are there). A k block
 // of a tile takes 0.26 us + 0.00066 us a column with every SM at work (L2 to shared memory, 50 to 56 bytes a clock and SM, and from 192 columns on

@@ -4,27 +4,45 @@
 using namespace fb;
 
 extern "C" long fb_gemm_workspace_bytes(int M, int N, int split_k) {
-  if (M > 64) return gemm_tail_bytes(0);
+  if (M > 64) return GM_TAIL_BYTES;
   if (split_k <= 1) return 0;
   int bn = ((M + 15) / 16) * 16;
   long tiles = (N + GM_BM - 1) / GM_BM;
   return tiles * split_k * 2L * bn * GM_BM * (long)sizeof(float);
 }
 
+// Zeroed ints beside that workspace; every call leaves them zero.
+extern "C" int fb_gemm_counters(int M, int N, int split_k) {
+  if (M > 64) return GM_TAIL_CTRS;
+  return split_k > 1 ? (N + GM_BM - 1) / GM_BM : 0;
+}
+
+// A plan whose K splits and pieces fit the scratch: pieces need not be taken, splits that do not fit are an error of the caller.
+static int plan_in(GemmPlan& p, int M, int N, int K, int mode, int split_k, int sm_count, int fp8, const float* ws, long ws_bytes, const int* counters,
+                   int n_counters) {
+  if (!ws || !counters) ws_bytes = n_counters = 0;
+  int rc = plan_gemm(p, M, N, K, mode, split_k, sm_count, fp8, ws_bytes > 0 && n_counters > 0 ? 2 : 1);
+  if (!rc && (gemm_tail_need(p.a) > ws_bytes || p.a.tail_tiles * GM_TILE_CTRS > n_counters)) {
+    p = GemmPlan{};
+    rc = plan_gemm(p, M, N, K, mode, split_k, sm_count, fp8, 1);
+  }
+  if (!rc && p.a.split_k > 1 && (fb_gemm_workspace_bytes(M, N, p.a.split_k) > ws_bytes || p.a.tiles_a * p.a.tiles_b > n_counters)) return -6;
+  return rc;
+}
+
 // mode bit 0: SwiGLU over gate|up rows (with a limit, clamped gated units); bit 2: squared relu; bit 1: Y is fp32 (residual stays bf16 with the same leading dimension)
 extern "C" int fb_gemm_bf16_glu(void* Y, const void* X, const void* W, const void* res, int M, int N, int K, long ldx,
-                                long ldy, int mode, float limit, int split_k, float* workspace, int* counters, int* status,
-                                int sm_count, cudaStream_t s) {
+                                long ldy, int mode, float limit, int split_k, float* workspace, long ws_bytes, int* counters, int n_counters,
+                                int* status, int sm_count, cudaStream_t s) {
   if (M <= 0 || N <= 0) return 0;
   const int out_f32 = (mode >> 1) & 1, act = (mode & 4) ? ACT_RELU2 : ACT_NONE;
   mode &= 1;
   if (K % 8 || ldx % 8 || (ldy % 8 && M > 64)) return -1;
   if (sm_count <= 0) sm_count = 148;
   GemmPlan p{};
-  int rc = plan_gemm(p, M, N, K, mode, split_k, sm_count, 0, workspace && counters && sm_count <= 148 ? 2 : 1);
+  int rc = plan_in(p, M, N, K, mode, split_k, sm_count, 0, workspace, ws_bytes, counters, n_counters);
   if (rc) return rc;
   GemmArgs& a = p.a;
-  if (a.split_k > 1 && (!workspace || !counters)) return -6;
   a.Y = Y; a.res = (const __nv_bfloat16*)res; a.workspace = workspace; a.counters = counters; a.status = status;
   a.ldy = ldy; a.out_f32 = out_f32; a.act = act; a.limit = limit;
   const int w_rows = a.dual ? 2 * N : N;
@@ -50,9 +68,9 @@ extern "C" int fb_gemm_bf16_glu(void* Y, const void* X, const void* W, const voi
 }
 
 extern "C" int fb_gemm_bf16(void* Y, const void* X, const void* W, const void* res, int M, int N, int K, long ldx,
-                            long ldy, int mode, int split_k, float* workspace, int* counters, int* status,
+                            long ldy, int mode, int split_k, float* workspace, long ws_bytes, int* counters, int n_counters, int* status,
                             int sm_count, cudaStream_t s) {
-  return fb_gemm_bf16_glu(Y, X, W, res, M, N, K, ldx, ldy, mode, 0.f, split_k, workspace, counters, status, sm_count, s);
+  return fb_gemm_bf16_glu(Y, X, W, res, M, N, K, ldx, ldy, mode, 0.f, split_k, workspace, ws_bytes, counters, n_counters, status, sm_count, s);
 }
 
 // ---- FP8 (e4m3) operands ----------------------------------------------------------------------------------
@@ -102,15 +120,14 @@ extern "C" int fb_quant_fp8(void* q, float* scale, const void* x, const void* no
 
 extern "C" int fb_gemm_fp8(void* Y, const void* Xq, const void* Wq, const float* scale_m, const float* scale_n,
                            const void* res, int M, int N, int K, long ldy, int mode, int split_k, float* workspace,
-                           int* counters, int* status, int sm_count, cudaStream_t s) {
+                           long ws_bytes, int* counters, int n_counters, int* status, int sm_count, cudaStream_t s) {
   if (M <= 0 || N <= 0) return 0;
   if (K % 16 || (ldy % 8 && M > 64)) return -1;
   if (sm_count <= 0) sm_count = 148;
   GemmPlan p{};
-  int rc = plan_gemm(p, M, N, K, mode, split_k, sm_count, 1, workspace && counters && sm_count <= 148 ? 2 : 1);
+  int rc = plan_in(p, M, N, K, mode, split_k, sm_count, 1, workspace, ws_bytes, counters, n_counters);
   if (rc) return rc;
   GemmArgs& a = p.a;
-  if (a.split_k > 1 && (!workspace || !counters)) return -6;
   a.Y = Y; a.res = (const __nv_bfloat16*)res; a.workspace = workspace; a.counters = counters; a.status = status;
   a.ldy = ldy; a.scale_m = scale_m; a.scale_n = scale_n;
   const int w_rows = a.dual ? 2 * N : N;

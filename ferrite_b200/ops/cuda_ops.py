@@ -57,7 +57,7 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         self._counters = torch.zeros(max(32768, self.C.gemv_stream_counters(self.sm_count)), dtype=torch.int32, device=self.device)
         self._stream_bytes = 4 * self.C.gemv_stream_ws_floats(self.sm_count)       # of the workspace, whatever the sizes of the product
         self._tail = None
-        self._tail_counters = torch.zeros(148 * 32, dtype=torch.int32, device=self.device)
+        self._tail_counters = torch.zeros(self.C.gemm_counters(65, 1, 1), dtype=torch.int32, device=self.device)
         self.empty = torch.empty            # every output buffer of the ops comes from here (see enable_canaries)
         self._guarded = []
         self._dl_sync = torch.zeros(2, dtype=torch.int32, device=self.device)      # grid-barrier words of the persistent layer kernel

@@ -58,6 +58,24 @@ def test_widths_and_pieces(ops, M, N, K, pieces, swiglu):
     assert ops.status() == 0 and int(ops._tail_counters.abs().sum()) == 0
 
 
+def test_scratch_that_is_too_small_takes_no_pieces(ops):
+    """Scratch of any size may come with a call: pieces are taken where they fit it, and nothing past its end is written."""
+    M, N, K = 300, 1111, 8192
+    x, w = rnd(M, K, seed=1), rnd(N, K, seed=2, scale=K ** -0.5)
+    whole, pieces = plain(ops, x, w, 2), ops.linear(x, w, out_f32=True)
+    assert not torch.equal(whole, pieces)
+    room, ctrs = ops.C.gemm_workspace_bytes(M, N, 1) // 4, ops.C.gemm_counters(M, N, 1)
+    for n_ws, n_ctr, want in [(room, ctrs, pieces), (1024, ctrs, whole), (room, 32, whole), (1024, 1, whole)]:
+        ws, cnt = torch.full((n_ws + 4096,), 7.0, device=DEV), torch.zeros(n_ctr + 4096, dtype=torch.int32, device=DEV)
+        y = torch.empty(M, 1112, device=DEV)[:, :N]
+        ops.C.gemm(y, x, w, None, 2, 1, ws[:n_ws], cnt[:n_ctr], ops.status_word)
+        assert torch.equal(y, want) and bool((ws[n_ws:] == 7).all()) and int(cnt.abs().sum()) == 0
+    with pytest.raises(RuntimeError):                                                # the K splits of few rows need theirs
+        ops.C.gemm(torch.empty(48, N, device=DEV), x[:48], w, None, 2, 8, torch.empty(16, device=DEV), torch.zeros(64, dtype=torch.int32, device=DEV),
+                   ops.status_word)
+    assert ops.status() == 0
+
+
 @pytest.mark.parametrize("N", [24, 100])
 def test_output_on_no_16_bytes(ops, N):
     M, K = 130, 256
