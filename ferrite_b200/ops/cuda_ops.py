@@ -30,6 +30,7 @@ MOE_PAIR_ROWS = 64     # up to this many rows (the largest graph-captured step) 
 # starts 2 us sooner: 17 products of a model of width 1024 (1M to 6M values) take 35 us less a step, the
 # products of a 27B model (10M and more) 17 % less through the ring.
 STREAM_VALUES = 8 << 20
+TAIL_STREAMS = 4       # streams that keep the scratch of a prompt GEMM's last tiles
 # NVFP4 weights of so many 128 x 256 units and more against one or two rows run on the block-scaled tensor cores (activations as three residual
 # renderings), smaller ones on the row kernel that unpacks the codes: it starts faster and unpacks 1.6 us a unit and CTA. One row, us: 17408 x 2 x
 # 5120 (5440 units) 30.5 / 34.5, 151936 x 5120 (23740) 79 / 127, 14336 x 5120 (2240) 20.5 / 20.6, 8224 x 5120 (1300) 18.9 / 15.2,
@@ -56,8 +57,7 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         self._ws: Optional[torch.Tensor] = None
         self._counters = torch.zeros(max(32768, self.C.gemv_stream_counters(self.sm_count)), dtype=torch.int32, device=self.device)
         self._stream_bytes = 4 * self.C.gemv_stream_ws_floats(self.sm_count)       # of the workspace, whatever the sizes of the product
-        self._tail = None
-        self._tail_counters = torch.zeros(self.C.gemm_counters(65, 1, 1), dtype=torch.int32, device=self.device)
+        self._tails = {}                    # stream -> workspace and counters of prompt GEMMs, see _gemm_scratch
         self.empty = torch.empty            # every output buffer of the ops comes from here (see enable_canaries)
         self._guarded = []
         self._dl_sync = torch.zeros(2, dtype=torch.int32, device=self.device)      # grid-barrier words of the persistent layer kernel
@@ -97,14 +97,22 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         return self._ws
 
     def _gemm_scratch(self, M: int, N: int, split: int):
-        """Workspace and counters of a GEMM call: K splits of few rows, or (more than 64 rows) the last tiles' pieces. The latter have buffers of
-        their own, held by the first stream that asks; on any other stream such calls run without pieces."""
+        """Workspace and counters of a GEMM call: K splits of few rows, or (more than 64 rows) the last tiles' pieces. The latter belong to the
+        current stream, so that a call has the same bits on every one; up to TAIL_STREAMS of them keep theirs (20 MB each: the one that asked
+        first gives its own back to the allocator, in whose order of that stream it is used again). A capture takes buffers of its own."""
         if M <= 64:
             return (self._workspace(self.C.gemm_workspace_bytes(M, N, split)), self._counters) if split > 1 else (None, None)
+        make = lambda: (torch.empty(self.C.gemm_workspace_bytes(M, N, 1) // 4, dtype=torch.float32, device=self.device),
+                        torch.zeros(self.C.gemm_counters(M, N, 1), dtype=torch.int32, device=self.device))
+        if torch.cuda.is_current_stream_capturing():
+            return make()
         stream = torch.cuda.current_stream(self.device).cuda_stream
-        if self._tail is None:
-            self._tail = (stream, torch.empty(self.C.gemm_workspace_bytes(M, N, 1) // 4, dtype=torch.float32, device=self.device))
-        return (self._tail[1], self._tail_counters) if self._tail[0] == stream else (None, None)
+        held = self._tails.get(stream)
+        if held is None:
+            for oldest in list(self._tails)[:max(0, len(self._tails) + 1 - TAIL_STREAMS)]:
+                self._tails.pop(oldest, None)
+            held = self._tails[stream] = make()
+        return held
 
     # ---- debug: canary-padded output buffers --------------------------------------------------------------
     CANARY_BYTES, CANARY_BYTE = 256, 0xA5
