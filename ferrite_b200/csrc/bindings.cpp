@@ -244,16 +244,16 @@ int64_t attn_decode_mma(Tensor out, Tensor o_part, Tensor ml_part, Tensor q, Ten
   return 0;
 }
 
-// The same without ancestor masks, keys split over the warps of a CTA.
+// The same without ancestor masks, keys split over the warps of a CTA. by_context: splits of a row by its context alone, nsplit has room for them.
 int64_t attn_decode_keys(Tensor out, Tensor o_part, Tensor ml_part, Tensor q, Tensor k_cache, Tensor v_cache, Tensor proj, Tensor seg_slot,
                          Tensor seg_row0, Tensor seg_nrows, int64_t max_rows, Tensor row_kvlen, Tensor block_table, int64_t kv_block, int64_t nq,
-                         int64_t nkv, int64_t hd, int64_t nsplit, bool gated, Tensor status) {
+                         int64_t nkv, int64_t hd, int64_t nsplit, bool gated, Tensor status, bool by_context) {
   const int rows = (int)row_kvlen.numel();
   TORCH_CHECK(o_part.numel() >= (int64_t)rows * nq * nsplit * hd && ml_part.numel() >= (int64_t)rows * nq * nsplit * 2, "attn_decode_keys: scratch");
   int rc = fb_attn_decode_keys(o_part.data_ptr<float>(), ml_part.data_ptr<float>(), q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
                                seg_slot.data_ptr<int>(), seg_row0.data_ptr<int>(), seg_nrows.data_ptr<int>(), row_kvlen.data_ptr<int>(),
                                block_table.data_ptr<int>(), (int)block_table.size(1), (int)kv_block, (int)seg_slot.numel(), (int)max_rows, rows, (int)nq,
-                               (int)nkv, (int)hd, (int)nsplit, 1.f / sqrtf((float)hd), nullptr, nullptr, 0, status.data_ptr<int>(), cur_stream());
+                               (int)nkv, (int)hd, (int)nsplit, by_context ? 1 : 0, 1.f / sqrtf((float)hd), nullptr, nullptr, 0, status.data_ptr<int>(), cur_stream());
   if (rc == -20) return rc;
   check(rc, "attn_decode_keys");
   check(fb_attn_combine(out.data_ptr(), o_part.data_ptr<float>(), ml_part.data_ptr<float>(), proj.data_ptr(), (long)proj.stride(0), rows, (int)nq, (int)hd,
@@ -469,7 +469,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("vdim") = 0, py::arg("eps") = 0.0, py::arg("k_mean") = py::none(), py::arg("v_mean") = py::none(),
         py::arg("mean_start") = py::none(), py::arg("pool") = 0);
   m.def("attn_decode_mma", &attn_decode_mma);
-  m.def("attn_decode_keys", &attn_decode_keys);
+  m.def("attn_decode_keys", &attn_decode_keys, py::arg("out"), py::arg("o_part"), py::arg("ml_part"), py::arg("q"), py::arg("k_cache"), py::arg("v_cache"),
+        py::arg("proj"), py::arg("seg_slot"), py::arg("seg_row0"), py::arg("seg_nrows"), py::arg("max_rows"), py::arg("row_kvlen"), py::arg("block_table"),
+        py::arg("kv_block"), py::arg("nq"), py::arg("nkv"), py::arg("hd"), py::arg("nsplit"), py::arg("gated"), py::arg("status"),
+        py::arg("by_context") = false);
   m.def("gdn_conv", &gdn_conv);
   m.def("gdn_rec", &gdn_rec);
   m.def("gdn_conv_tree", &gdn_conv_tree);

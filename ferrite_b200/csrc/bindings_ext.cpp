@@ -738,7 +738,7 @@ void gqa_attn(Tensor out, Tensor o_part, Tensor ml_part, Tensor q, Tensor k_cach
     const int rc = !pool && max_rows * (heads / kvh) > 16 ? -20 : fb_attn_decode_keys(o_part.data_ptr<float>(), ml_part.data_ptr<float>(), q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
                                        seg_slot.data_ptr<int>(), seg_row0.data_ptr<int>(), seg_nrows.data_ptr<int>(), row_kvlen.data_ptr<int>(),
                                        block_table.data_ptr<int>(), (int)block_table.size(1), (int)kv_block, (int)seg_slot.numel(), (int)max_rows,
-                                       rows, heads, kvh, hd, (int)nsplit, (float)scale, kbp, pkp, (int)row_first, status.data_ptr<int>(), cur_stream());
+                                       rows, heads, kvh, hd, (int)nsplit, 0, (float)scale, kbp, pkp, (int)row_first, status.data_ptr<int>(), cur_stream());
     TORCH_CHECK(rc != -20 || !pool, "gqa_attn: means outside the tensor-core kernel's shapes");
     if (rc != -20) check(rc, "attn_decode_keys");
     else check(fb_attn_decode_mma(nullptr, o_part.data_ptr<float>(), ml_part.data_ptr<float>(), q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),

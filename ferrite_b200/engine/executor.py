@@ -1012,7 +1012,8 @@ class Executor:
                 else:
                     o = ops.attention(q, proj, self.k_cache[i], self.v_cache[i], mv["slot"], mv["kvlen"],
                                       self.block_table, self.ecfg.kv_block, c.n_q, c.n_kv, c.head_dim, c.attn_gate,
-                                      nsplit=nsplit, segs=(mv["sslot"], mv["srow0"], mv["snrows"], max_seg_rows), **kvs)
+                                      nsplit=nsplit, segs=(mv["sslot"], mv["srow0"], mv["snrows"], max_seg_rows),
+                                      picked=self.ecfg.attn_splits <= 0, **kvs)
                 if fuse:                             # the rest of this layer opens the next run
                     run.append({"o": o, **tail(p)})
                     run_idx.append(i)

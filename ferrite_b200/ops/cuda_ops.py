@@ -21,9 +21,6 @@ from .mixers import CudaMixers
 from .qweight import Exl3Weight, ExpertsFP4, GgufWeight, QWeight, StackWeight
 
 GEMV_MAX_ROWS = 8
-# CTAs per SM that the decode attention's key splits aim at, by head width (as many as are resident; four rows against 8000 keys each, 4 kv heads
-# of 256: 47 us, 97 with the splits of whole rows over one warp's keys)
-DECODE_KEYS_CTAS = {64: 4, 128: 2, 256: 1}
 MOE_PAIR_ROWS = 64     # up to this many rows (the largest graph-captured step) the experts run as per-pair GEMVs,
                        # beyond as grouped GEMMs, which read the per-expert row counts on the host
 # 2..32 rows against bf16 weights of so many values and more stream them through a TMA ring (`gemv_stream`), less through registers (`gemv_mma`), which
@@ -573,25 +570,25 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         return q
 
     def attention(self, q, proj, k_cache, v_cache, row_slot, row_kvlen, block_table, kv_block, nq, nkv, hd, gated,
-                  row_base=None, row_mask=None, nsplit=1, kv_scale=None, segs=None):
-        """Split-KV decode / verify / tree attention. With `segs` = (seg_slot, seg_row0, seg_nrows, max rows per
+                  row_base=None, row_mask=None, nsplit=1, kv_scale=None, segs=None, picked=False):
+        """Split-KV decode / verify / tree attention over `nsplit` key splits; `picked`: that number was picked from the longest context of the
+        step (a split per 64 keys, rounded up to a power of two, 64 at most) and not asked for, so a kernel may split otherwise. With `segs` = (seg_slot, seg_row0, seg_nrows, max rows per
         segment) and a bf16 cache the tensor-core kernel runs: the rows of a segment share one pass over the K/V of
         each kv head (bf16 and e4m3 caches). The 4-bit cache and callers without segment tables take the SIMT kernel."""
         T = q.shape[0]
-        # the heads of a group for a row or two at a time, keys split over the warps of a CTA, and as many splits as fill the GPU. Rows of every
-        # count take this kernel, so that a verified row has the bits of a decoded one; trees (ancestor masks) and quantised caches do not.
-        G = nq // nkv
-        keys = (segs is not None and kv_scale is None and row_mask is None and self.attn_mma and G <= 16 and kv_block % 64 == 0
-                and hd in DECODE_KEYS_CTAS)
-        if keys:
-            ctas = segs[0].numel() * nkv * -(-segs[3] // (16 // G))
-            nsplit = max(1, min(nsplit, self.sm_count * DECODE_KEYS_CTAS[hd] // ctas))
+        # bf16 caches without trees (ancestor masks): one or two groups of 16 (row, head) pairs at a time, keys split over the warps of a CTA. Rows
+        # of every count take this kernel, and a row's splits follow its own context (dk_split_keys in attn_decode_keys.cu, which needs half the
+        # splits that are picked for the others beyond 8), so that it has the same bits decoded, verified and among other streams.
+        keys = (segs is not None and kv_scale is None and row_mask is None and self.attn_mma and nq // nkv <= 16 and kv_block % 64 == 0
+                and hd in (64, 128, 256))
+        if keys and picked and nsplit > 8:
+            nsplit //= 2
         out = self.empty(T, nq * hd, dtype=self.dtype, device=self.device)
         o_part = self.empty(T, nq, nsplit, hd, dtype=torch.float32, device=self.device)
         ml_part = self.empty(T, nq, nsplit, 2, dtype=torch.float32, device=self.device)
         self.launches += 2
         if keys and self.C.attn_decode_keys(out, o_part, ml_part, q, k_cache, v_cache, proj, *segs, row_kvlen, block_table, kv_block, nq, nkv, hd,
-                                            nsplit, gated, self.status_word) == 0:
+                                            nsplit, gated, self.status_word, picked) == 0:
             return out
         fp8_cache = kv_scale is not None and k_cache.shape[-1] == hd           # (the 4-bit cache has hd / 2 bytes per row)
         if segs is not None and (kv_scale is None or fp8_cache) and self.attn_mma and nq // nkv <= 64:

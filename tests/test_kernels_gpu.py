@@ -724,3 +724,41 @@ def test_attention_keys_over_warps(ops, tops, hd, nq, nkv, rows, nsplit):
     # weights of 16 bits and 32-bit sums under the rounding of the result, |o| <= 4.5
     assert (got - want).abs().max().item() <= 2 ** -8 * max(1.0, want.abs().max().item()) + 2e-4
     assert ops.status() == 0
+
+
+@pytest.mark.parametrize("hd,nq,nkv", [(256, 24, 4), (256, 16, 1), (128, 8, 2), (64, 6, 2)])
+@pytest.mark.parametrize("first", [30, 490, 500, 1015, 2040, 4090, 6130])
+def test_a_row_has_its_bits_in_every_step(ops, tops, hd, nq, nkv, first):
+    """The engine's split counts: a row alone, as one of a verified segment (in two groups of pairs, and in one), and beside other streams, whose
+    longer contexts raise the number of splits. The segment's contexts cross the places where a context's splits become longer (512 keys, multiples
+    of 2048 beyond 4096) and where the engine picks more of them (1024, 2048)."""
+    from ferrite_b200.engine.executor import Executor
+    from types import SimpleNamespace
+    splits = lambda n: Executor.attn_splits(SimpleNamespace(ecfg=SimpleNamespace(attn_splits=0)), n)
+    kvb, rows, lens = 64, 17, [first + 17, 700, 5000]
+    g = torch.Generator(device=DEV).manual_seed(hd + nq + first)
+    nb = (max(lens) + kvb - 1) // kvb
+    bt = torch.randperm(3 * nb, generator=g, device=DEV).to(torch.int32).view(3, nb)
+    kc, vc = (torch.randn(3 * nb, kvb, nkv, hd, generator=g, device=DEV).to(torch.bfloat16) for _ in "kv")
+    q = torch.randn(rows + 2, nq, hd, generator=g, device=DEV).to(torch.bfloat16)
+    proj = torch.randn(rows + 2, nq * hd * 2 + 2 * nkv * hd, generator=g, device=DEV).to(torch.bfloat16)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+
+    def step(parts):                                         # (stream, first row, rows) of each segment
+        at = [r for _, r, n in parts for r in range(r, r + n)]
+        own = [(lens[s] - rows + 1 + (r - a) + a if s == 0 else lens[s]) for s, a, n in parts for r in range(a, a + n)]
+        slot, row0 = [s for s, _, n in parts for _ in range(n)], [sum(n for _, _, n in parts[:i]) for i in range(len(parts))]
+        segs = (i32([s for s, _, _ in parts]), i32(row0), i32([n for _, _, n in parts]), max(n for _, _, n in parts))
+        return ops.attention(q[at], proj[at], kc, vc, i32(slot), i32(own), bt, kvb, nq, nkv, hd, True, nsplit=splits(max(own)), segs=segs, picked=True)
+
+    whole = step([(0, 0, rows)])
+    want = tops.attention(q[:rows], proj[:rows], kc, vc, i32([0] * rows), i32([first + 1 + r for r in range(rows)]), bt, kvb, nq, nkv, hd, True).float()
+    # weights of 16 bits and 32-bit sums under the rounding of the result, |o| <= 4.5
+    assert (whole.float() - want).abs().max().item() <= 2 ** -8 * max(1.0, want.abs().max().item()) + 2e-4
+    for r in range(rows):
+        assert torch.equal(step([(0, r, 1)])[0], whole[r]), r
+    assert torch.equal(step([(0, 3, 2)]), whole[3:5])
+    beside = step([(1, rows, 1), (0, 0, rows), (2, rows + 1, 1)])
+    assert torch.equal(beside[1:1 + rows], whole)
+    assert torch.equal(step([(1, rows, 1)])[0], beside[0]) and torch.equal(step([(2, rows + 1, 1)])[0], beside[-1])
+    assert ops.status() == 0
