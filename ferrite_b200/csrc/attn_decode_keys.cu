@@ -7,7 +7,7 @@
 // Segments of more pairs (drafted rows) bring two groups of 16 to a CTA, four warps each over the same tiles: what a row's warps do, and with it
 // its bits, is the same in both forms.
 //
-// A row's key splits are those of its own context (dk_split_keys; `by_context`: whatever the number of splits of the launch), and rows of a CTA
+// A row's key splits are those of its own context (context_split_keys; `by_context`: whatever the number of splits of the launch), and rows of a CTA
 // whose splits end elsewhere go in passes of their own. So a row has the same bits alone, among other rows and among other streams. (Windows and
 // chunks begin with the first row's earliest key, and their callers pick splits by the step: they make no such promise.)
 //
@@ -44,16 +44,10 @@ __device__ __forceinline__ void dk_mma(float (&c)[4], const uint32_t (&a)[4], ui
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// Keys of a split of a context: what shares it evenly over the launch's splits, or (by_context) at least 64 keys up to 512, 128 up to 4096 and a
-// 32nd beyond. One decoded row wants many short splits, twenty streams few long ones, and a row must not know which of the two it is in.
-// us, 24 heads over 4 of 256 columns, streams x keys, splits of 64 keys (at most 64 of them) / of this rule / as few as fill the GPU:
+// The split rule (context_split_keys): one decoded row wants many short splits, twenty streams few long ones, and a row must not know which of
+// the two it is in. us, 24 heads over 4 of 256 columns, streams x keys, splits of 64 keys (at most 64 of them) / of this rule / as few as fill the GPU:
 // 1 x 2048 15.0 / 13.5 / 14.3, 1 x 12000 30.7 / 22.9 / 24.1, 4 x 8000 57 / 45 / 39, 8 x 3000 60 / 39 / 34, 24 x 1500 78 / 53 / 55,
 // 32 x 1000 68 / 50 / 40 (attn_decode_mma.cu, splits of 64 keys: 18.4, 34.8, 66, 61, 77, 64).
-__host__ __device__ __forceinline__ int dk_split_keys(int len, int nsplit, int by_context) {
-  const int even = ((len + nsplit - 1) / nsplit + DK_KEYS - 1) / DK_KEYS * DK_KEYS;
-  return !by_context ? even : max(even, len <= 512 ? DK_KEYS : max(2 * DK_KEYS, ((len + 31) / 32 + DK_KEYS - 1) / DK_KEYS * DK_KEYS));
-}
-
 template <int HD, bool POOL, int MG>            // MG: groups of pairs
 __global__ void __launch_bounds__(MG * DK_WARPS * 32)
 attn_decode_keys_kernel(float* __restrict__ o_part, float* __restrict__ ml_part, const __nv_bfloat16* __restrict__ q,
@@ -81,9 +75,9 @@ attn_decode_keys_kernel(float* __restrict__ o_part, float* __restrict__ ml_part,
   const int* bt = block_table + (size_t)seg_slot[seg] * max_blocks;
   for (int ra = 0, rb = rows_here; ra < rows_here; ra = rb, rb = rows_here) {
     if (!POOL && !window && !chunk) {           // [ra, rb): rows whose splits end at the same keys (contexts grow from row to row)
-      const int keys = dk_split_keys(row_kvlen[row0 + ra], nsplit, by_context);
-      if (dk_split_keys(row_kvlen[row0 + rb - 1], nsplit, by_context) != keys)
-        for (rb = ra + 1; dk_split_keys(row_kvlen[row0 + rb], nsplit, by_context) == keys;) ++rb;
+      const int keys = context_split_keys(row_kvlen[row0 + ra], nsplit, by_context);
+      if (context_split_keys(row_kvlen[row0 + rb - 1], nsplit, by_context) != keys)
+        for (rb = ra + 1; context_split_keys(row_kvlen[row0 + rb], nsplit, by_context) == keys;) ++rb;
     }
     // rows of a segment follow one another: the last one sees the latest key, the first one the earliest
     const int kv_end = row_kvlen[row0 + rb - 1];
@@ -91,7 +85,7 @@ attn_decode_keys_kernel(float* __restrict__ o_part, float* __restrict__ ml_part,
     // list of keys: place u < shift is mean u (those of the last row's blocks), the others are token u - shift + kv_lo
     const int nb = POOL ? first_key(kv_end - 1, window, 0) / pool : 0, shift = POOL ? (nb + DK_KEYS - 1) / DK_KEYS * DK_KEYS : 0;
     const int at0 = POOL ? 0 : kv_lo, list_end = POOL ? shift + kv_end - kv_lo : kv_end;
-    const int per = dk_split_keys(list_end - at0, nsplit, by_context);
+    const int per = context_split_keys(list_end - at0, nsplit, by_context);
     const int lo = at0 + split * per, hi = min(list_end, lo + per);
     // (row, head) pair m of this CTA: whether its row is of this pass, and its record
     auto mine = [&](int m) { return m >= ra * G && m < rb * G; };
@@ -274,7 +268,7 @@ using namespace fb;
 
 // Records of key splits as fb_attn_decode_mma leaves them (o_part [rows][nq][nsplit][hd], ml_part two floats each); scale of the scores; kb:
 // window, chunk and softcap, or null; pool: means of the blocks before the window, or null. Returns -20 for shapes it does not take: heads of 64,
-// 128 or (without means) 256 columns, nq / nkv <= 16, pages of a multiple of 64 keys. by_context: dk_split_keys; no bounds then.
+// 128 or (without means) 256 columns, nq / nkv <= 16, pages of a multiple of 64 keys. by_context: context_split_keys; no bounds then.
 extern "C" int fb_attn_decode_keys(float* o_part, float* ml_part, const void* q, const void* k_cache, const void* v_cache, const int* seg_slot,
                                    const int* seg_row0, const int* seg_nrows, const int* row_kvlen, const int* block_table, int max_blocks,
                                    int kv_block, int nseg, int max_rows, int rows, int nq, int nkv, int hd, int nsplit, int by_context, float scale,

@@ -47,6 +47,13 @@ __host__ __device__ __forceinline__ int first_key(int pos, int window, int chunk
   if (window > 0) return pos >= window ? pos - window + 1 : 0;
   return chunk > 0 ? pos - pos % chunk : 0;
 }
+// Keys of a split of a context, in tiles of 64: what shares it evenly over the launch's splits, or (by_context) at least 64 keys up to 512, 128 up to
+// 4096 and a 32nd beyond, whatever that number is. A split count of a power of two with 64 keys a split up to 8, and half of that beyond (32 at
+// most), has room for it.
+__host__ __device__ __forceinline__ int context_split_keys(int len, int nsplit, int by_context) {
+  const int even = ((len + nsplit - 1) / nsplit + 63) / 64 * 64, own = len <= 512 ? 64 : len <= 4096 ? 128 : ((len + 31) / 32 + 63) / 64 * 64;
+  return by_context && own > even ? own : even;
+}
 // tanh(x) = 1 - 2 / (e^2x + 1); off by a few 2^-23 of one
 __device__ __forceinline__ float tanh_exp(float x) {
   float e;

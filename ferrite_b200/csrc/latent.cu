@@ -625,7 +625,9 @@ __global__ void __launch_bounds__(256) head_mix_kernel(T* __restrict__ out, long
 // tiles and 64 queries do not fit.
 // It also serves the multi-head latent attention of the MLA models (512 + 64 columns, 128 heads), whose CUDA-core kernel (mla.cu) has
 // every head read the latents for itself: 6 streams of 1.6K to 4K tokens took 441 us there and 62 us in the merge of its 64 key splits;
-// here the splits are what fills the GPU (6) and the two take 53 and 9 us.
+// here the two take about 70 us. There (`apart`) a tile holds heads of one row, and its splits may follow its own context (context_split_keys), so
+// that a row has the same bits alone, among the rows of its segment and among other streams. us, streams x keys, splits that fill the GPU / this
+// rule: 1 x 4000 18.2 / 17.9, 1 x 16000 40 / 44, 6 x 4000 60 / 68, 8 x 2000 48 / 51.
 constexpr int LM_KEYS = 64, LM_THREADS = 256, LM_LDP = LM_KEYS + 8;
 
 __device__ __forceinline__ void lm_cp16(void* smem, const void* gmem, bool valid) {
@@ -659,7 +661,7 @@ latent_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ o_part, f
                   const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache, const int* __restrict__ seg_slot,
                   const int* __restrict__ seg_row0, const int* __restrict__ seg_nrows, const int* __restrict__ row_kvlen,
                   const int* __restrict__ block_table, int max_blocks, int kv_block, int heads, int row_base, int tiles_per_seg,
-                  int nsplit, float scale_log2, int window, int* status) {
+                  int nsplit, int apart, float scale_log2, int window, int* status) {
   constexpr int LAT = Lm<NJ>::LAT, LD = Lm<NJ>::LD, CPR = LAT / 8, LM_M = Lm<NJ>::LM_M, MT = LM_M / 16, VL = VJ * 64;
   extern __shared__ __align__(16) unsigned char lm_smem[];
   __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(lm_smem);           // [M][LD]
@@ -671,15 +673,15 @@ latent_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ o_part, f
   pdl_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int seg = blockIdx.x / tiles_per_seg, tile_m = blockIdx.x % tiles_per_seg, split = blockIdx.y;
-  const int n = seg_nrows[seg], m_all = n * heads, m0 = tile_m * LM_M;
-  if (m0 >= m_all) return;
-  const int valid_m = min(LM_M, m_all - m0);
+  const int row_tiles = (heads + LM_M - 1) / LM_M;
+  const int n = seg_nrows[seg], m0 = apart ? tile_m / row_tiles * heads + tile_m % row_tiles * LM_M : tile_m * LM_M;
+  if (m0 >= n * heads) return;
+  const int valid_m = min(LM_M, (apart ? (tile_m / row_tiles + 1) * heads : n * heads) - m0);
   const int row0 = seg_row0[seg];
   const int* bt = block_table + (size_t)seg_slot[seg] * max_blocks;
   const int kv_end = row_kvlen[row0 + (m0 + valid_m - 1) / heads - row_base];          // rows of a segment see ever more keys
   const int kv_lo = first_key(row_kvlen[row0 + m0 / heads - row_base] - 1, window, 0) / LM_KEYS * LM_KEYS;
-  int per = (kv_end - kv_lo + nsplit - 1) / nsplit;
-  per = (per + LM_KEYS - 1) / LM_KEYS * LM_KEYS;
+  const int per = context_split_keys(kv_end - kv_lo, nsplit, apart == 2);
   const int lo = kv_lo + split * per, hi = min(kv_end, lo + per);
   // (row, head) flat index of an M row in q / out, which start at row row_base of the step
   const size_t flat0 = (size_t)(row0 - row_base) * heads + m0;
@@ -1145,15 +1147,17 @@ extern "C" int fb_head_mix(void* out, long ldo, const float* in, const float* la
 
 // The same on tensor cores for bf16, lat <= 512 with vl = lat, or 576 with vl = 512, and pages of a multiple of 64 keys (-20 otherwise). Rows come in
 // segments (consecutive rows of one slot); seg_row0 counts the rows of the step, of which q / out / row_kvlen hold those from row_base on.
+// apart: rows share no tile (2: and a row's splits follow its own context); without a window.
 extern "C" int fb_latent_mma(void* out, float* o_part, float* ml_part, const void* q, const void* cache, const int* seg_slot,
                              const int* seg_row0, const int* seg_nrows, int nseg, int max_rows, const int* row_kvlen,
                              const int* block_table, int max_blocks, int kv_block, int rows, int row_base, int heads, int lat,
-                             int vl, int window, int nsplit, float scale, int* status, cudaStream_t s) {
+                             int vl, int window, int nsplit, int apart, float scale, int* status, cudaStream_t s) {
   if (rows <= 0 || nseg <= 0) return 0;
   const bool key_part = vl == lat - 64 && (lat == 128 || lat == 192 || lat == 576);
   if (lat % 64 || lat > 576 || (!key_part && (lat > 512 || vl != lat)) || kv_block % LM_KEYS) return -20;
-  if (nsplit < 1 || nsplit > 4096 || window < 0) return -1;
-  const int m_tile = lat <= 512 ? 64 : 32, tps = (max_rows * heads + m_tile - 1) / m_tile;
+  if (nsplit < 1 || nsplit > 4096 || window < 0 || (apart && window)) return -1;
+  const int m_tile = lat <= 512 ? 64 : 32;
+  const int tps = apart ? max_rows * ((heads + m_tile - 1) / m_tile) : (max_rows * heads + m_tile - 1) / m_tile;
   const dim3 grid(nseg * tps, nsplit);
   const float sl = scale * 1.4426950408889634f;
   int rc = 0;
@@ -1164,7 +1168,7 @@ extern "C" int fb_latent_mma(void* out, float* o_part, float* ml_part, const voi
     if (e != cudaSuccess) return (int)e;                                                                                       \
     rc = (int)launch_pdl(kern, grid, dim3(LM_THREADS), Lm<NJ>::SMEM, s, (bf16*)out, o_part, ml_part, (const bf16*)q,           \
                          (const bf16*)cache, seg_slot, seg_row0, seg_nrows, row_kvlen, block_table, max_blocks, kv_block, heads, \
-                         row_base, tps, nsplit, sl, window, status);                                                           \
+                         row_base, tps, nsplit, apart, sl, window, status);                                                           \
     break;                                                                                                                     \
   }
   switch (lat / 64 * 16 + vl / 64) {

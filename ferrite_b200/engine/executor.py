@@ -987,7 +987,8 @@ class Executor:
                                            self.block_table, self.ecfg.kv_block, c.n_q, L, R,
                                            1.0 / math.sqrt(c.nope_head_dim + R),
                                            nsplit=nsplit if max_seg_rows <= FLASH_MIN_ROWS else 1,
-                                           segs=(mv["sslot"], mv["srow0"], mv["snrows"], max_seg_rows))
+                                           segs=(mv["sslot"], mv["srow0"], mv["snrows"], max_seg_rows),
+                                           picked=self.ecfg.attn_splits <= 0)
                     o = ops.mla_out(ol, w_uv)
                 x = row(o, w[p + "out_proj"], x)
             else:

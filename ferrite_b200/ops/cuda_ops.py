@@ -577,7 +577,7 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         each kv head (bf16 and e4m3 caches). The 4-bit cache and callers without segment tables take the SIMT kernel."""
         T = q.shape[0]
         # bf16 caches without trees (ancestor masks): one or two groups of 16 (row, head) pairs at a time, keys split over the warps of a CTA. Rows
-        # of every count take this kernel, and a row's splits follow its own context (dk_split_keys in attn_decode_keys.cu, which needs half the
+        # of every count take this kernel, and a row's splits follow its own context (context_split_keys in common.cuh, which needs half the
         # splits that are picked for the others beyond 8), so that it has the same bits decoded, verified and among other streams.
         keys = (segs is not None and kv_scale is None and row_mask is None and self.attn_mma and nq // nkv <= 16 and kv_block % 64 == 0
                 and hd in (64, 128, 256))
@@ -766,14 +766,29 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
                                    nq, nq, HP, False, max(n for _, _, n in segs))
         return o.view(T, nq, HP)[:, :, :dv].contiguous().view(T, nq * dv)
 
-    def mla_attention(self, qabs, cache, row_slot, row_kvlen, block_table, kv_block, nq, L, R, scale, nsplit=1, segs=None):
+    def mla_attention(self, qabs, cache, row_slot, row_kvlen, block_table, kv_block, nq, L, R, scale, nsplit=1, segs=None, picked=False):
         """Every head attends the cached latents. With `segs` = (seg_slot, seg_row0, seg_nrows, max rows per segment) and pages of whole
-        64-key tiles the tensor-core kernel of the listed models runs: heads and rows of a segment share every pass over the latents, and the
-        key splits are what fills the GPU. Callers without segment tables and other page sizes take the CUDA-core kernel."""
+        64-key tiles the tensor-core kernel of the listed models runs, heads of a row sharing every pass over the latents. Rows of segments of
+        up to 32 rows share nothing and, with `picked` splits (see `attention`), are split by their own context: a row has the same bits
+        decoded, verified and among other streams. Callers without segment tables and other page sizes take the CUDA-core kernel."""
         T = qabs.shape[0]
         if segs is not None and kv_block % 64 == 0 and R == 64 and L in (64, 128, 512):
-            return self.latent_attention(qabs, cache.view(-1, kv_block, L + R), SegGroup(0, segs[0].numel(), 0, T, segs[3]), row_slot, row_kvlen,
-                                         segs[:3], block_table, kv_block, scale, nsplit, vlat=L)
+            if qabs.dtype != torch.bfloat16:
+                return self.latent_attention(qabs, cache.view(-1, kv_block, L + R), SegGroup(0, segs[0].numel(), 0, T, segs[3]), row_slot, row_kvlen,
+                                             segs[:3], block_table, kv_block, scale, nsplit, vlat=L)
+            apart = 0 if segs[3] > 32 else 2 if picked else 1
+            if apart == 2 and nsplit > 8:
+                nsplit //= 2                                  # what context_split_keys (common.cuh) needs
+            out = self.empty(T, nq, L, dtype=self.dtype, device=self.device)
+            o_part = ml_part = None
+            if nsplit > 1:
+                o_part = self.empty(T * nq * nsplit * L, dtype=torch.float32, device=self.device)
+                ml_part = self.empty(T * nq * nsplit * 2, dtype=torch.float32, device=self.device)
+            rc = self.C.latent_mma(out, o_part, ml_part, qabs, cache.view(-1, kv_block, L + R), *segs, row_kvlen, block_table, kv_block, 0, nsplit, scale,
+                                   self.status_word, 0, apart)
+            assert rc == 0, "mla_attention: shape outside the tensor-core kernel"
+            self.launches += 1 if nsplit == 1 else 2
+            return out
         out = self.empty(T, nq, L, dtype=self.dtype, device=self.device)
         o_part = self.empty(T * nq * nsplit * L, dtype=torch.float32, device=self.device)
         ml_part = self.empty(T * nq * nsplit * 2, dtype=torch.float32, device=self.device)

@@ -292,7 +292,7 @@ class TorchOps(TorchLatent, TorchMixers, TorchExtras):
         qn = torch.einsum("thd,hld->thl", q3[..., :dn], w_uk_t.float())
         return torch.cat([qn, qr], -1).to(self.dtype)
 
-    def mla_attention(self, qabs, cache, row_slot, row_kvlen, block_table, kv_block, nq, L, R, scale, nsplit=1, segs=None):
+    def mla_attention(self, qabs, cache, row_slot, row_kvlen, block_table, kv_block, nq, L, R, scale, nsplit=1, segs=None, picked=False):
         T = qabs.shape[0]
         out = torch.zeros(T, nq, L, dtype=torch.float32, device=qabs.device)
         for t in range(T):

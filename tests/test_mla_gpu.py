@@ -71,6 +71,38 @@ def test_mla_attention_of_segments(ops, L, R, nq, lens, rows, nsplit):
     assert ops.status() == 0
 
 
+@pytest.mark.parametrize("L,nq", [(512, 128), (512, 16), (128, 5), (64, 70)])
+@pytest.mark.parametrize("first", [30, 490, 2040, 4090])
+def test_mla_row_has_its_bits_in_every_step(ops, L, nq, first):
+    """The engine's split counts: a row alone, in a verified segment and beside other streams, at contexts where splits become longer (512 keys,
+    beyond 4096) or more (2048)."""
+    from ferrite_b200.engine.executor import Executor
+    from types import SimpleNamespace
+    splits = lambda n: Executor.attn_splits(SimpleNamespace(ecfg=SimpleNamespace(attn_splits=0)), n)
+    R, kvb, rows, lens = 64, 64, 17, [first + 17, 60, 5000]
+    g = torch.Generator(device=DEV).manual_seed(L + nq + first)
+    nb = (max(lens) + kvb - 1) // kvb
+    cache = torch.randn(3 * nb, kvb, L + R, generator=g, device=DEV).to(torch.bfloat16)
+    bt = torch.randperm(3 * nb, generator=g, device=DEV).to(torch.int32).view(3, nb)
+    q = torch.randn(rows + 2, nq, L + R, generator=g, device=DEV).to(torch.bfloat16)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+
+    def step(parts):                                         # (stream, first row, rows) of each segment
+        at = [r for _, r, n in parts for r in range(r, r + n)]
+        own = [first + 1 + r if s == 0 else lens[s] for s, a, n in parts for r in range(a, a + n)]
+        slot, row0 = [s for s, _, n in parts for _ in range(n)], [sum(n for _, _, n in parts[:i]) for i in range(len(parts))]
+        segs = (i32([s for s, _, _ in parts]), i32(row0), i32([n for _, _, n in parts]), max(n for _, _, n in parts))
+        return ops.mla_attention(q[at], cache, i32(slot), i32(own), bt, kvb, nq, L, R, (L + R) ** -0.5, nsplit=splits(max(own)), segs=segs, picked=True)
+
+    whole = step([(0, 0, rows)])
+    for r in range(rows):
+        assert torch.equal(step([(0, r, 1)])[0], whole[r]), r
+    beside = step([(1, rows, 1), (0, 0, rows), (2, rows + 1, 1)])
+    assert torch.equal(beside[1:1 + rows], whole)
+    assert torch.equal(step([(1, rows, 1)])[0], beside[0]) and torch.equal(step([(2, rows + 1, 1)])[0], beside[-1])
+    assert ops.status() == 0
+
+
 @pytest.mark.parametrize("T", [1, 6, 8, 19, 300])
 @pytest.mark.parametrize("nh,N,K", [(16, 512, 128), (16, 128, 512), (4, 64, 32), (3, 40, 64)])
 def test_head_linear_row_kernel_and_batched_gemm(ops, T, nh, N, K):
