@@ -201,7 +201,7 @@ int fb_latent_attn(void* out, float* o_part, float* ml_part, const void* q, cons
 int fb_latent_mma(void* out, float* o_part, float* ml_part, const void* q, const void* cache, const int* seg_slot,
                   const int* seg_row0, const int* seg_nrows, int nseg, int max_rows, const int* row_kvlen, const int* block_table,
                   int max_blocks, int kv_block, int rows, int row_base, int heads, int lat, int vl, int window, int nsplit, int apart,
-                  float scale, int* status, cudaStream_t s);
+                  int exact_p, float scale, int* status, cudaStream_t s);
 int fb_gqa_attn(void* out, float* o_part, float* ml_part, const void* q, const void* k_cache, const void* v_cache, const float* sink,
                 const int* row_slot, const int* row_kvlen, const int* block_table, int max_blocks, int kv_block, int rows, int heads,
                 int kv_heads, int hd, int nsplit, float scale, const KeyBounds* kb, const PoolKeys* pool, long ldo, int f32, int* status,

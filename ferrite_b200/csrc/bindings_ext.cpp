@@ -880,14 +880,14 @@ void latent_attn(Tensor out, c10::optional<Tensor> o_part, c10::optional<Tensor>
 
 int64_t latent_mma(Tensor out, c10::optional<Tensor> o_part, c10::optional<Tensor> ml_part, Tensor q, Tensor cache, Tensor seg_slot,
                    Tensor seg_row0, Tensor seg_nrows, int64_t max_rows, Tensor row_kvlen, Tensor block_table, int64_t kv_block,
-                   int64_t row_base, int64_t nsplit, double scale, Tensor status, int64_t window, int64_t apart) {
+                   int64_t row_base, int64_t nsplit, double scale, Tensor status, int64_t window, int64_t apart, bool exact_p) {
   TORCH_CHECK(q.dim() == 3 && q.is_contiguous() && out.is_contiguous() && cache.is_contiguous() && cache.size(-1) == q.size(2) &&
               !is_f32(q) && (nsplit == 1 || (o_part && ml_part)), "latent_mma: layouts");
   const int rc = fb_latent_mma(out.data_ptr(), (float*)optr(o_part), (float*)optr(ml_part), q.data_ptr(), cache.data_ptr(),
                                seg_slot.data_ptr<int>(), seg_row0.data_ptr<int>(), seg_nrows.data_ptr<int>(), (int)seg_slot.numel(),
                                (int)max_rows, row_kvlen.data_ptr<int>(), block_table.data_ptr<int>(), (int)block_table.size(1),
                                (int)kv_block, (int)q.size(0), (int)row_base, (int)q.size(1), (int)q.size(2), (int)out.size(2),
-                               (int)window, (int)nsplit, (int)apart, (float)scale, status.data_ptr<int>(), cur_stream());
+                               (int)window, (int)nsplit, (int)apart, exact_p ? 1 : 0, (float)scale, status.data_ptr<int>(), cur_stream());
   if (rc == -20) return rc;                     // shape outside this kernel: the caller takes the CUDA-core kernel
   check(rc, "latent_mma");
   return 0;
@@ -989,7 +989,7 @@ void register_ext(pybind11::module_& m) {
   m.def("latent_mma", &latent_mma, pybind11::arg("out"), pybind11::arg("o_part"), pybind11::arg("ml_part"), pybind11::arg("q"), pybind11::arg("cache"),
         pybind11::arg("seg_slot"), pybind11::arg("seg_row0"), pybind11::arg("seg_nrows"), pybind11::arg("max_rows"), pybind11::arg("row_kvlen"),
         pybind11::arg("block_table"), pybind11::arg("kv_block"), pybind11::arg("row_base"), pybind11::arg("nsplit"), pybind11::arg("scale"),
-        pybind11::arg("status"), pybind11::arg("window") = 0, pybind11::arg("apart") = 0);
+        pybind11::arg("status"), pybind11::arg("window") = 0, pybind11::arg("apart") = 0, pybind11::arg("exact_p") = false);
   m.def("gemm_f32", &gemm_f32);
   m.def("silu_mul_f32", &silu_mul_f32);
   m.def("gqa_prep", &gqa_prep);

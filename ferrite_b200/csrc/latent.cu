@@ -619,15 +619,15 @@ __global__ void __launch_bounds__(256) head_mix_kernel(T* __restrict__ out, long
 // serves 64 of them. grid (segments x M tiles, splits), 8 warps. Scores: warp = 16 M rows x 32 of the tile's 64 keys over the
 // whole latent (16 keys when at most 32 M rows are in use, so that no warp idles). Values are the same shared-memory tile read
 // transposed: warp = all 64 M rows x lat / 8 columns. The softmax weights go through shared memory as a bf16 value plus its bf16
-// remainder, two products each, so they keep 16 bits of mantissa instead of 8; scores, maxima, exponentials and row sums are
-// 32-bit.
+// remainder, two products each, so they keep 16 bits of mantissa instead of 8, or (PARTS 3: the MLA models, whose CUDA-core kernel multiplies
+// 32-bit weights) with the remainder's remainder all 24; scores, maxima, exponentials and row sums are 32-bit.
 // A cache row has 64 NJ columns; values are its first 64 VJ (the rest is a key part). M is 64, or 32 where rows are so wide that two key
 // tiles and 64 queries do not fit.
 // It also serves the multi-head latent attention of the MLA models (512 + 64 columns, 128 heads), whose CUDA-core kernel (mla.cu) has
 // every head read the latents for itself: 6 streams of 1.6K to 4K tokens took 441 us there and 62 us in the merge of its 64 key splits;
 // here the two take about 70 us. There (`apart`) a tile holds heads of one row, and its splits may follow its own context (context_split_keys), so
 // that a row has the same bits alone, among the rows of its segment and among other streams. us, streams x keys, splits that fill the GPU / this
-// rule: 1 x 4000 18.2 / 17.9, 1 x 16000 40 / 44, 6 x 4000 60 / 68, 8 x 2000 48 / 51.
+// rule / with all bits of the weights: 1 x 4000 18.5 / 18.2 / 19.6, 1 x 16000 41 / 44 / 49, 6 x 4000 61 / 65 / 71, 8 x 2000 48 / 51 / 55.
 constexpr int LM_KEYS = 64, LM_THREADS = 256, LM_LDP = LM_KEYS + 8;
 
 __device__ __forceinline__ void lm_cp16(void* smem, const void* gmem, bool valid) {
@@ -648,26 +648,27 @@ __device__ __forceinline__ void lm_mma(float (&c)[4], const uint32_t (&a)[4], ui
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-template <int NJ>
+template <int NJ, int PARTS>
 struct Lm {
   static constexpr int LM_M = NJ <= 8 ? 64 : 32;
   static constexpr int LAT = NJ * 64, LD = LAT + 8;
-  static constexpr size_t SMEM = (size_t)(LM_M + 2 * LM_KEYS) * LD * 2 + (size_t)2 * LM_M * LM_LDP * 2 + 6 * LM_M * 4;
+  static constexpr size_t SMEM = (size_t)(LM_M + 2 * LM_KEYS) * LD * 2 + (size_t)PARTS * LM_M * LM_LDP * 2 + 6 * LM_M * 4;
 };
 
-template <int NJ, int VJ>
+template <int NJ, int VJ, int PARTS>
 __global__ void __launch_bounds__(LM_THREADS, 1)
 latent_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ o_part, float* __restrict__ ml_part,
                   const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache, const int* __restrict__ seg_slot,
                   const int* __restrict__ seg_row0, const int* __restrict__ seg_nrows, const int* __restrict__ row_kvlen,
                   const int* __restrict__ block_table, int max_blocks, int kv_block, int heads, int row_base, int tiles_per_seg,
                   int nsplit, int apart, float scale_log2, int window, int* status) {
-  constexpr int LAT = Lm<NJ>::LAT, LD = Lm<NJ>::LD, CPR = LAT / 8, LM_M = Lm<NJ>::LM_M, MT = LM_M / 16, VL = VJ * 64;
+  using L = Lm<NJ, PARTS>;
+  constexpr int LAT = L::LAT, LD = L::LD, CPR = LAT / 8, LM_M = L::LM_M, MT = LM_M / 16, VL = VJ * 64;
   extern __shared__ __align__(16) unsigned char lm_smem[];
   __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(lm_smem);           // [M][LD]
   __nv_bfloat16* sK = sQ + LM_M * LD;                                      // [2][KEYS][LD]
-  __nv_bfloat16* sP = sK + 2 * LM_KEYS * LD;                               // [value | remainder][M][LDP]
-  float* smx = reinterpret_cast<float*>(sP + 2 * LM_M * LM_LDP);           // [4][M] maxima of the key groups, then sums
+  __nv_bfloat16* sP = sK + 2 * LM_KEYS * LD;                               // [value | remainder ..][M][LDP]
+  float* smx = reinterpret_cast<float*>(sP + PARTS * LM_M * LM_LDP);           // [4][M] maxima of the key groups, then sums
   float* sfac = smx + 4 * LM_M;                                            // [M] rescale factor of the tile
   float* sinv = sfac + LM_M;                                               // [M] 1 / row sum
   pdl_wait();
@@ -803,7 +804,10 @@ latent_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ o_part, f
           const uint32_t v = pack_bf2(p0, p1);
           const int at = r * LM_LDP + key0 + nt * 8 + (lane & 3) * 2;
           *reinterpret_cast<uint32_t*>(sP + at) = v;
-          *reinterpret_cast<uint32_t*>(sP + LM_M * LM_LDP + at) = pack_bf2(p0 - bf_lo(v), p1 - bf_hi(v));
+          const float d0 = p0 - bf_lo(v), d1 = p1 - bf_hi(v);
+          const uint32_t x = pack_bf2(d0, d1);
+          *reinterpret_cast<uint32_t*>(sP + LM_M * LM_LDP + at) = x;
+          if (PARTS == 3) *reinterpret_cast<uint32_t*>(sP + 2 * LM_M * LM_LDP + at) = pack_bf2(d0 - bf_lo(x), d1 - bf_hi(x));
         }
         lrow[h] = lrow[h] * f + ls;
         if (nw == 0 && (lane & 3) == 0) sfac[r] = f;
@@ -829,7 +833,7 @@ latent_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ o_part, f
 #pragma unroll
         for (int k2 = 0; k2 < 2; ++k2) {
 #pragma unroll
-          for (int part = 0; part < 2; ++part) {
+          for (int part = 0; part < PARTS; ++part) {
             uint32_t a[4];
             lm_ldsm(a, sP + (part * LM_M + mt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LM_LDP + (kp * 2 + k2) * 16 + (lane >> 4) * 8);
 #pragma unroll
@@ -1147,32 +1151,35 @@ extern "C" int fb_head_mix(void* out, long ldo, const float* in, const float* la
 
 // The same on tensor cores for bf16, lat <= 512 with vl = lat, or 576 with vl = 512, and pages of a multiple of 64 keys (-20 otherwise). Rows come in
 // segments (consecutive rows of one slot); seg_row0 counts the rows of the step, of which q / out / row_kvlen hold those from row_base on.
-// apart: rows share no tile (2: and a row's splits follow its own context); without a window.
+// apart: rows share no tile (2: and a row's splits follow its own context); without a window. exact_p: all 24 bits of the softmax weights, for
+// rows with a key part.
 extern "C" int fb_latent_mma(void* out, float* o_part, float* ml_part, const void* q, const void* cache, const int* seg_slot,
                              const int* seg_row0, const int* seg_nrows, int nseg, int max_rows, const int* row_kvlen,
                              const int* block_table, int max_blocks, int kv_block, int rows, int row_base, int heads, int lat,
-                             int vl, int window, int nsplit, int apart, float scale, int* status, cudaStream_t s) {
+                             int vl, int window, int nsplit, int apart, int exact_p, float scale, int* status, cudaStream_t s) {
   if (rows <= 0 || nseg <= 0) return 0;
   const bool key_part = vl == lat - 64 && (lat == 128 || lat == 192 || lat == 576);
-  if (lat % 64 || lat > 576 || (!key_part && (lat > 512 || vl != lat)) || kv_block % LM_KEYS) return -20;
+  if (lat % 64 || lat > 576 || (!key_part && (lat > 512 || vl != lat)) || kv_block % LM_KEYS || (exact_p && !key_part)) return -20;
   if (nsplit < 1 || nsplit > 4096 || window < 0 || (apart && window)) return -1;
   const int m_tile = lat <= 512 ? 64 : 32;
   const int tps = apart ? max_rows * ((heads + m_tile - 1) / m_tile) : (max_rows * heads + m_tile - 1) / m_tile;
   const dim3 grid(nseg * tps, nsplit);
   const float sl = scale * 1.4426950408889634f;
   int rc = 0;
-#define FB_LM(NJ, VJ)                                                                                                          \
-  case NJ * 16 + VJ: {                                                                                                         \
-    auto kern = latent_mma_kernel<NJ, VJ>;                                                                                     \
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lm<NJ>::SMEM);                \
+#define FB_LM(NJ, VJ, PARTS)                                                                                                   \
+  case (NJ * 16 + VJ) * 4 + PARTS: {                                                                                           \
+    auto kern = latent_mma_kernel<NJ, VJ, PARTS>;                                                                              \
+    constexpr size_t smem = Lm<NJ, PARTS>::SMEM;                                                                               \
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                        \
     if (e != cudaSuccess) return (int)e;                                                                                       \
-    rc = (int)launch_pdl(kern, grid, dim3(LM_THREADS), Lm<NJ>::SMEM, s, (bf16*)out, o_part, ml_part, (const bf16*)q,           \
+    rc = (int)launch_pdl(kern, grid, dim3(LM_THREADS), smem, s, (bf16*)out, o_part, ml_part, (const bf16*)q,                   \
                          (const bf16*)cache, seg_slot, seg_row0, seg_nrows, row_kvlen, block_table, max_blocks, kv_block, heads, \
-                         row_base, tps, nsplit, apart, sl, window, status);                                                           \
+                         row_base, tps, nsplit, apart, sl, window, status);                                                    \
     break;                                                                                                                     \
   }
-  switch (lat / 64 * 16 + vl / 64) {
-    FB_LM(1, 1) FB_LM(2, 2) FB_LM(3, 3) FB_LM(4, 4) FB_LM(5, 5) FB_LM(6, 6) FB_LM(7, 7) FB_LM(8, 8) FB_LM(2, 1) FB_LM(3, 2) FB_LM(9, 8)
+  switch ((lat / 64 * 16 + vl / 64) * 4 + (exact_p ? 3 : 2)) {
+    FB_LM(1, 1, 2) FB_LM(2, 2, 2) FB_LM(3, 3, 2) FB_LM(4, 4, 2) FB_LM(5, 5, 2) FB_LM(6, 6, 2) FB_LM(7, 7, 2) FB_LM(8, 8, 2)
+    FB_LM(2, 1, 2) FB_LM(3, 2, 2) FB_LM(9, 8, 2) FB_LM(2, 1, 3) FB_LM(3, 2, 3) FB_LM(9, 8, 3)
   }
 #undef FB_LM
   if (rc || nsplit == 1) return rc;

@@ -785,7 +785,7 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
                 o_part = self.empty(T * nq * nsplit * L, dtype=torch.float32, device=self.device)
                 ml_part = self.empty(T * nq * nsplit * 2, dtype=torch.float32, device=self.device)
             rc = self.C.latent_mma(out, o_part, ml_part, qabs, cache.view(-1, kv_block, L + R), *segs, row_kvlen, block_table, kv_block, 0, nsplit, scale,
-                                   self.status_word, 0, apart)
+                                   self.status_word, 0, apart, True)
             assert rc == 0, "mla_attention: shape outside the tensor-core kernel"
             self.launches += 1 if nsplit == 1 else 2
             return out

@@ -71,6 +71,38 @@ def test_mla_attention_of_segments(ops, L, R, nq, lens, rows, nsplit):
     assert ops.status() == 0
 
 
+@pytest.mark.parametrize("L,nq", [(512, 128), (128, 6), (64, 8)])
+@pytest.mark.parametrize("ctx,nsplit", [(1, 2), (70, 2), (100, 2), (2000, 16)])
+def test_mla_softmax_weights_keep_32_bits(ops, L, nq, ctx, nsplit):
+    """The 32-bit records of the key splits, merged here in 64 bits, against the plain statement in 64 bits. With few keys, weights cut to 16 bits
+    are what such sums are off by; all their bits bring them at least twice as close. (With many keys the weights' errors cancel and the tensor
+    cores' sums, cut and not rounded at each step, are the larger part.)"""
+    R, kvb = 64, 64
+    g = torch.Generator(device=DEV).manual_seed(L + ctx)
+    nb = (ctx + kvb - 1) // kvb
+    cache = torch.randn(nb, kvb, L + R, generator=g, device=DEV).to(torch.bfloat16)
+    q = torch.randn(1, nq, L + R, generator=g, device=DEV).to(torch.bfloat16)
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    bt, scale = torch.arange(nb, dtype=torch.int32, device=DEV).view(1, nb), (L + R) ** -0.5
+    keys = cache.view(-1, L + R)[:ctx].double()
+    want = torch.softmax(q[0].double() @ keys.t() * scale, -1) @ keys[:, :L]
+
+    def off(run):
+        o, ml = torch.empty(nq, nsplit, L, device=DEV), torch.empty(nq, nsplit, 2, device=DEV)
+        run(torch.empty(1, nq, L, dtype=torch.bfloat16, device=DEV), o, ml)
+        f = torch.exp2(ml[..., 0].double() - ml[..., 0].amax(1, keepdim=True).double())
+        merged = (torch.where(f[..., None] > 0, o.double(), 0.0) * f[..., None]).sum(1) / (ml[..., 1].double() * f).sum(1)[:, None]
+        return ((merged - want).norm() / want.norm()).item()
+
+    mma = lambda exact: lambda out, o, ml: ops.C.latent_mma(out, o, ml, q, cache, i32(0), i32(0), i32(1), 1, i32(ctx), bt, kvb, 0, nsplit, scale,
+                                                            ops.status_word, 0, 1, exact)
+    three, two = off(mma(True)), off(mma(False))
+    # scores of up to 4, summed over (L + R) / 16 steps that each cut up to 2^-23 of them; the exponential passes that on
+    assert three <= (L + R) / 16 * 4 * 2 ** -23, (three, two)
+    assert ctx == 1 or two > (2 if ctx <= 100 else 1) * three, (three, two)
+    assert ops.status() == 0
+
+
 @pytest.mark.parametrize("L,nq", [(512, 128), (512, 16), (128, 5), (64, 70)])
 @pytest.mark.parametrize("first", [30, 490, 2040, 4090])
 def test_mla_row_has_its_bits_in_every_step(ops, L, nq, first):
