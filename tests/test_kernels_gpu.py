@@ -683,6 +683,27 @@ def test_determinism_over_cross_cta_hand_offs(capsys):
     assert rc == 0, out
 
 
+def test_determinism_cases_reach_the_kernels_they_name(ext, monkeypatch):
+    from ferrite_b200.ops.cuda_ops import CudaOps
+    from ferrite_b200.utils.detcheck import cases
+
+    class Seen:
+        calls = []
+
+        def __getattr__(self, name):
+            Seen.calls.append(name)
+            return getattr(ext, name)
+
+    monkeypatch.setattr("ferrite_b200._ext.load", lambda *a: Seen())
+    ops = CudaOps(DEV)
+    ops.C = Seen()
+    for name, fn in cases(ops, DEV).items():
+        Seen.calls.clear()
+        fn()
+        assert name.split(":")[0] in Seen.calls, (name, Seen.calls)
+    assert ops.status() == 0
+
+
 def test_canary_padded_output_buffers_catch_a_stray_write(ops):
     """Debug allocator: guard bytes around every output buffer; a decode-sized forward leaves them intact, a write one
     element past a buffer is reported at the next check."""
