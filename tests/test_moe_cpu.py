@@ -130,3 +130,13 @@ def test_expert_heat_counters(tmp_path, monkeypatch):
     assert json.loads(path.read_text())["layers"][str(moe_layers[0])] == heat[moe_layers[0]]
     monkeypatch.delenv("FE_EXPERT_HEAT")
     assert Engine(cfg, None, EngineConfig(n_slots=1, max_ctx=64), device="cpu").expert_heat() == {}
+
+
+def test_experts_with_many_rows_are_not_multiplied_from_their_codes():
+    """Up to 80 rows per expert on average, however they are spread: beyond, unpacking every 32 rows anew costs more than a bf16 copy."""
+    from types import SimpleNamespace
+    from ferrite_b200.parallel.ep import ExpertParallel
+    ep = SimpleNamespace(fused=True, world=1, n_experts=64, CODE_ROWS=ExpertParallel.CODE_ROWS, C=SimpleNamespace(moe_stream_fits=lambda n, k, e: True))
+    w_gu, w_down = SimpleNamespace(shape=(64, 1024, 2048)), SimpleNamespace(shape=(64, 2048, 512))
+    for pairs, codes in [(1, True), (29 * 64, True), (80 * 64, True), (80 * 64 + 1, False), (96 * 64, False)]:
+        assert ExpertParallel.takes_codes(ep, pairs, w_gu, w_down) is codes
