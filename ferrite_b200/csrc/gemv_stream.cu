@@ -17,9 +17,10 @@
 // token columns to spare the rounding of x (1 + w) to bf16 goes into columns of its own.
 // SwiGLU: a tile is 64 gate and 64 up rows, a fragment's rows 0..7 the gate's and 8..15 the up's, so both meet in one thread.
 //
-// The tensor path is mma.sync because tcgen05 takes its weights from shared memory only: 4-bit ones would have to be written back there in
-// 16 bits (82 of the 128 bytes a clock that shared memory has, and as many to read them), and for bf16 the products are a tenth of the time
-// either way.
+// The tensor path is mma.sync: for bf16 the products are a tenth of the time, and fragments come out of the ring as they are. For 4-bit weights it
+// is part of the bound (issue slots 72 % busy, unpacking and products in the same slots). tcgen05 could take the unpacked weights as its A operand
+// from tensor memory, as the prompt attention does with its softmax weights (attn_prefill_tc.cu), and leave those slots to the unpacking: not
+// built.
 #include "api_ext.h"
 #include "stream_mma.cuh"
 

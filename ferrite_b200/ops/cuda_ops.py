@@ -41,8 +41,10 @@ def through_registers(rows: int, values: int, K: int, norm: bool) -> bool:
 TAIL_STREAMS = 4       # streams that keep the scratch of a prompt GEMM's last tiles
 # NVFP4 weights of so many 128 x 256 units and more against one or two rows run on the block-scaled tensor cores (activations as three residual
 # renderings), smaller ones on the row kernel that unpacks the codes: it starts faster and unpacks 1.6 us a unit and CTA. One row, us: 17408 x 2 x
-# 5120 (5440 units) 30.5 / 34.5, 151936 x 5120 (23740) 79 / 127, 14336 x 5120 (2240) 20.5 / 20.6, 8224 x 5120 (1300) 18.9 / 15.2,
-# 5120 x 2048 (320) 11.8 / 7.8.
+# 5120 (5440 units) 28.7 / 33.0, 151936 x 5120 (23740) 78 / 127, 14336 x 5120 (2240) 19.4 / 19.4, 8224 x 5120 (1300) 17.6 / 14.4,
+# 5120 x 2048 (320) 11.7 / 7.8. Three to eight rows always unpack: the block-scaled kernel has room for two renderings of three or four rows (0.9 %
+# off) and for one of more (9 %), and only the head is slower for it. 3 rows (8): 34816 x 5120 36.5 / 35.1 (56 / 39), 5120 x 17408 32.4 / 21.7
+# (55 / 23), 8224 x 5120 27.1 / 15.5 (50 / 17), 151936 x 5120 91 / 134 (123 / 150).
 FP4_TC_UNITS = 2560
 
 
