@@ -620,14 +620,16 @@ __global__ void __launch_bounds__(256) head_mix_kernel(T* __restrict__ out, long
 // whole latent (16 keys when at most 32 M rows are in use, so that no warp idles). Values are the same shared-memory tile read
 // transposed: warp = all 64 M rows x lat / 8 columns. The softmax weights go through shared memory as a bf16 value plus its bf16
 // remainder, two products each, so they keep 16 bits of mantissa instead of 8, or (PARTS 3: the MLA models, whose CUDA-core kernel multiplies
-// 32-bit weights) with the remainder's remainder all 24; scores, maxima, exponentials and row sums are 32-bit.
+// 32-bit weights) with the remainder's remainder all 24; scores, maxima, exponentials and row sums are 32-bit. The tensor cores cut a running sum
+// at every step instead of rounding it, which over a split's steps adds up to 1e-6 of it: PARTS 3 lets them sum 64 columns of a score, or 32 keys of
+// a value, and adds those sums with rounding.
 // A cache row has 64 NJ columns; values are its first 64 VJ (the rest is a key part). M is 64, or 32 where rows are so wide that two key
 // tiles and 64 queries do not fit.
 // It also serves the multi-head latent attention of the MLA models (512 + 64 columns, 128 heads), whose CUDA-core kernel (mla.cu) has
 // every head read the latents for itself: 6 streams of 1.6K to 4K tokens took 441 us there and 62 us in the merge of its 64 key splits;
-// here the two take about 70 us. There (`apart`) a tile holds heads of one row, and its splits may follow its own context (context_split_keys), so
+// here the two take about 73 us. There (`apart`) a tile holds heads of one row, and its splits may follow its own context (context_split_keys), so
 // that a row has the same bits alone, among the rows of its segment and among other streams. us, streams x keys, splits that fill the GPU / this
-// rule / with all bits of the weights: 1 x 4000 18.5 / 18.2 / 19.6, 1 x 16000 41 / 44 / 49, 6 x 4000 61 / 65 / 71, 8 x 2000 48 / 51 / 55.
+// rule / with PARTS 3: 1 x 4000 18.5 / 18.1 / 20.2, 1 x 16000 40 / 44 / 51, 6 x 4000 61 / 65 / 73, 8 x 2000 48 / 51 / 57.
 constexpr int LM_KEYS = 64, LM_THREADS = 256, LM_LDP = LM_KEYS + 8;
 
 __device__ __forceinline__ void lm_cp16(void* smem, const void* gmem, bool valid) {
@@ -741,9 +743,13 @@ latent_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ o_part, f
     __syncthreads();                                         // the tile has landed; everyone is done with the other buffer
     if (tile + 1 < ntiles) load_tile(lo + (tile + 1) * LM_KEYS, stage ^ 1);
     const __nv_bfloat16* K = sK + stage * LM_KEYS * LD;
-    float s[4][4];
+    float s[4][4], step[4][4];                               // step (PARTS 3): sums of 64 columns
+    float (&acc)[4][4] = PARTS == 3 ? step : s;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) { s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f; }
+    for (int i = 0; i < 4; ++i) {
+      s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
+      step[i][0] = step[i][1] = step[i][2] = step[i][3] = 0.f;
+    }
     float mx[2] = {-INFINITY, -INFINITY};
     if (score_on) {
       // fragments are loaded one k step ahead of the products
@@ -761,11 +767,17 @@ latent_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ o_part, f
           lm_ldsm(b[cur ^ 1][0], pb + (ks + 1) * 16);
           if (!few) lm_ldsm(b[cur ^ 1][1], pb + 16 * LD + (ks + 1) * 16);
         }
-        lm_mma(s[0], a[cur], b[cur][0][0], b[cur][0][1]);
-        lm_mma(s[1], a[cur], b[cur][0][2], b[cur][0][3]);
+        lm_mma(acc[0], a[cur], b[cur][0][0], b[cur][0][1]);
+        lm_mma(acc[1], a[cur], b[cur][0][2], b[cur][0][3]);
         if (!few) {
-          lm_mma(s[2], a[cur], b[cur][1][0], b[cur][1][1]);
-          lm_mma(s[3], a[cur], b[cur][1][2], b[cur][1][3]);
+          lm_mma(acc[2], a[cur], b[cur][1][0], b[cur][1][1]);
+          lm_mma(acc[3], a[cur], b[cur][1][2], b[cur][1][3]);
+        }
+        if (PARTS == 3 && (ks & 3) == 3) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { s[i][e] += step[i][e]; step[i][e] = 0.f; }
         }
       }
       const int kbase = lo + tile * LM_KEYS + key0 + (lane & 3) * 2;
@@ -830,6 +842,10 @@ latent_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ o_part, f
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
         if (mt * 16 >= valid_m) break;
+        float po[VJ][4];                                     // (PARTS 3): sums of 32 keys
+        float (&to)[VJ][4] = PARTS == 3 ? po : o[mt];
+#pragma unroll
+        for (int j = 0; j < VJ; ++j) po[j][0] = po[j][1] = po[j][2] = po[j][3] = 0.f;
 #pragma unroll
         for (int k2 = 0; k2 < 2; ++k2) {
 #pragma unroll
@@ -837,8 +853,12 @@ latent_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ o_part, f
             uint32_t a[4];
             lm_ldsm(a, sP + (part * LM_M + mt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LM_LDP + (kp * 2 + k2) * 16 + (lane >> 4) * 8);
 #pragma unroll
-            for (int j = 0; j < VJ; ++j) lm_mma(o[mt][j], a, b[j][2 * k2], b[j][2 * k2 + 1]);
+            for (int j = 0; j < VJ; ++j) lm_mma(to[j], a, b[j][2 * k2], b[j][2 * k2 + 1]);
           }
+        }
+        if (PARTS == 3) {
+#pragma unroll
+          for (int j = 0; j < VJ; ++j) { o[mt][j][0] += po[j][0]; o[mt][j][1] += po[j][1]; o[mt][j][2] += po[j][2]; o[mt][j][3] += po[j][3]; }
         }
       }
     }

@@ -72,11 +72,10 @@ def test_mla_attention_of_segments(ops, L, R, nq, lens, rows, nsplit):
 
 
 @pytest.mark.parametrize("L,nq", [(512, 128), (128, 6), (64, 8)])
-@pytest.mark.parametrize("ctx,nsplit", [(1, 2), (70, 2), (100, 2), (2000, 16)])
+@pytest.mark.parametrize("ctx,nsplit", [(1, 2), (70, 2), (2000, 16), (4000, 32), (2000, 2)])
 def test_mla_softmax_weights_keep_32_bits(ops, L, nq, ctx, nsplit):
-    """The 32-bit records of the key splits, merged here in 64 bits, against the plain statement in 64 bits. With few keys, weights cut to 16 bits
-    are what such sums are off by; all their bits bring them at least twice as close. (With many keys the weights' errors cancel and the tensor
-    cores' sums, cut and not rounded at each step, are the larger part.)"""
+    """The 32-bit records of the key splits, merged here in 64 bits, against the plain statement in 64 bits: off by a few 2^-24, as the kernel that
+    multiplies 32-bit weights on the CUDA cores is, where weights of 16 bits and sums cut at every step are several times as far off."""
     R, kvb = 64, 64
     g = torch.Generator(device=DEV).manual_seed(L + ctx)
     nb = (ctx + kvb - 1) // kvb
@@ -97,9 +96,10 @@ def test_mla_softmax_weights_keep_32_bits(ops, L, nq, ctx, nsplit):
     mma = lambda exact: lambda out, o, ml: ops.C.latent_mma(out, o, ml, q, cache, i32(0), i32(0), i32(1), 1, i32(ctx), bt, kvb, 0, nsplit, scale,
                                                             ops.status_word, 0, 1, exact)
     three, two = off(mma(True)), off(mma(False))
-    # scores of up to 4, summed over (L + R) / 16 steps that each cut up to 2^-23 of them; the exponential passes that on
-    assert three <= (L + R) / 16 * 4 * 2 ** -23, (three, two)
-    assert ctx == 1 or two > (2 if ctx <= 100 else 1) * three, (three, two)
+    plain = off(lambda out, o, ml: ops.C.mla_attn(out, o, ml, q, cache, i32(0), i32(ctx), bt, kvb, nq, L, R, nsplit, scale))
+    # four cut steps to a sum of a score's columns and six to one of a value's keys (2^-24 of it on average each), then rounded sums
+    assert max(three, plain) <= 10 * 2 ** -24, (three, two, plain)
+    assert ctx == 1 or two > 3 * three, (three, two, plain)
     assert ops.status() == 0
 
 
