@@ -10,7 +10,7 @@
 // warp order, so results do not depend on scheduling. Epilogues: residual add, SwiGLU over gate|up rows, fp32 output;
 // prologue: RMSNorm(1 + w) of the rows (scales computed in-kernel).
 //
-// This is the path of 2..32 rows against small weights (up to 8M values, with short rows up to 20M): a few microseconds each, where a launch
+// This is the path of 2..32 rows against small weights (up to 8M values): a few microseconds each, where a launch
 // without a ring of shared memory starts sooner and the norm rides along (a model of width 1024, 2 / 4 / 8 streams: 126 / 129 / 135 us a step,
 // with the ring of gemv_stream.cu 160 / 165 / 173); larger weights stream through that ring (0.55 to 0.7 of the copy rate here, 0.85 there). The
 // tensor path is mma.sync, whose fragments are what a warp loads from global memory; 33..64 rows take tcgen05 with the weights as its 128-row

@@ -25,19 +25,11 @@ MOE_PAIR_ROWS = 64     # up to this many rows (the largest graph-captured step) 
                        # beyond as grouped GEMMs, which read the per-expert row counts on the host
 # 2..32 rows against bf16 weights of so many values and more stream them through a TMA ring (`gemv_stream`), less through registers (`gemv_mma`), which
 # starts 2 us sooner: 17 products of a model of width 1024 (1M to 6M values) take 35 us less a step, the products of a 27B model (10M and more) 17 %
-# less through the ring. Short rows of weights cut the ring's runs short, so there registers win up to more values, the more so the fewer token rows
-# they have to stage. us, registers / ring, 4 rows (17): 4096 x 1024 4.5 / 6.4 (7.9 / 8.9), 9216 x 1024 6.8 / 9.3 (10.6 / 13.2), 16384 x 1024
-# 9.3 / 11.5 (14.2 / 16.1), 24576 x 1024 15.5 / 13.4 (24: 26 / 16), 8192 x 2048 10.3 / 11.6 (17.8 / 16.1), 12352 x 2048 14.4 / 14.3, 4096 x 3072
-# 10.0 / 10.8 (16: 15.4 / 13.5), 4096 x 4096 12.4 / 12.0 (21 / 17), 2048 x 5120 11.0 / 10.7 (19 / 15.5), 1024 x 16384 11.2 / 10.9. Up to four rows
-# under a norm stay on the ring there: it multiplies what bf16 rounds off x (1 + w) too, registers do not.
-STREAM_VALUES, STREAM_VALUES_SHORT = 8 << 20, 20 << 20
-
-
-def through_registers(rows: int, values: int, K: int, norm: bool) -> bool:
-    return values < STREAM_VALUES or (values < STREAM_VALUES_SHORT and not (norm and rows <= 4)
-                                      and K <= (3072 if rows <= 8 else 1024 if rows <= 24 else 0))
-
-
+# less through the ring. Alone, weights of short rows are faster through registers up to 20M values (us, registers / ring, 4 rows: 9216 x 1024 6.8 /
+# 9.3, 16384 x 1024 9.3 / 11.5, 24576 x 1024 15.5 / 13.4, 4608 x 2048 7.8 / 9.6, 8192 x 2048 10.3 / 11.6, 4096 x 3072 10.0 / 10.8, 4096 x 4096 12.4 /
+# 12.0), but between other kernels the ring fills while the one before it ends: with 5120 x 2048 through registers, four streams of the 27B model
+# took 794 us a step of four layers instead of 777.
+STREAM_VALUES = 8 << 20
 TAIL_STREAMS = 4       # streams that keep the scratch of a prompt GEMM's last tiles
 # NVFP4 weights of so many 128 x 256 units and more against one or two rows run on the block-scaled tensor cores (activations as three residual
 # renderings), smaller ones on the row kernel that unpacks the codes: it starts faster and unpacks 1.6 us a unit and CTA. One row, us: 17408 x 2 x
@@ -287,7 +279,7 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         N = w.shape[0] // 2 if swiglu else w.shape[0]
         if self.mma_gemv_rows[0] <= M <= self.mma_gemv_rows[1] and not self.force_gemv_chunks:
             # a few rows (concurrent decode streams, speculative verify): weights streamed once into mma.sync fragments
-            if through_registers(M, w.numel(), K, norm_w is not None) and K % 32 == 0 and w.stride(0) == K:
+            if w.numel() < STREAM_VALUES and K % 32 == 0 and w.stride(0) == K:
                 y = out if out is not None else self.empty(M, N, dtype=torch.float32 if out_f32 else self.dtype, device=self.device)
                 self.launches += 1
                 self.C.gemv_mma(y, x, w, norm_w, res, eps, 1 if swiglu else 2 if act else 0, self._workspace(8 << 20), self._counters, fresh_w)

@@ -42,18 +42,3 @@ def test_scratch_copies_are_told_apart(rows, n, kernel):
     ops.C.calls.clear()
     ops.linear(x, torch.zeros(n, K, dtype=torch.bfloat16))
     assert ops.C.calls[0][0] == kernel and ops.C.calls[0][1][-1] is False
-
-
-# on both sides of the lines: values, length of the weights' rows, token rows
-@pytest.mark.parametrize("n,K,up_to", [(4096, 1024, 32), (1024, 8160, 32), (1024, 8192, 1), (9216, 1024, 24), (20448, 1024, 24), (20480, 1024, 1),
-                                       (8192, 2048, 8), (4096, 3072, 8), (4096, 3104, 1)])
-def test_short_rows_of_weights_go_through_registers(n, K, up_to):
-    ops, w = recording_ops(), torch.empty(n, K, dtype=torch.bfloat16)
-    for rows in (2, 8, 9, 24, 25, 32):
-        ops.C.calls.clear()
-        ops.linear(torch.empty(rows, K, dtype=torch.bfloat16), w)
-        assert ops.C.calls[0][0] == ("gemv_mma" if rows <= up_to else "gemv_stream"), rows
-    for rows in (4, 5):                                      # up to four rows under a norm: the kernel that multiplies their rounding too
-        ops.C.calls.clear()
-        ops.linear(torch.empty(rows, K, dtype=torch.bfloat16), w, norm_w=torch.empty(K, dtype=torch.bfloat16))
-        assert ops.C.calls[0][0] == ("gemv_mma" if n * K < 8 << 20 or 5 <= rows <= up_to else "gemv_stream"), rows
