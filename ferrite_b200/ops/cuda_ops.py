@@ -577,9 +577,9 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
     def attention(self, q, proj, k_cache, v_cache, row_slot, row_kvlen, block_table, kv_block, nq, nkv, hd, gated,
                   row_base=None, row_mask=None, nsplit=1, kv_scale=None, segs=None, picked=False):
         """Split-KV decode / verify / tree attention over `nsplit` key splits; `picked`: that number was picked from the longest context of the
-        step (a split per 64 keys, rounded up to a power of two, 64 at most) and not asked for, so a kernel may split otherwise. With `segs` = (seg_slot, seg_row0, seg_nrows, max rows per
-        segment) and a bf16 cache the tensor-core kernel runs: the rows of a segment share one pass over the K/V of
-        each kv head (bf16 and e4m3 caches). The 4-bit cache and callers without segment tables take the SIMT kernel."""
+        step (a split per 64 keys, rounded up to a power of two, 64 at most) and not asked for, so a kernel may split otherwise.
+        With `segs` = (seg_slot, seg_row0, seg_nrows, max rows per segment) and a bf16 or e4m3 cache the tensor-core kernels run: rows of a
+        segment share passes over the K/V of each kv head. The 4-bit cache and callers without segment tables take the SIMT kernel."""
         T = q.shape[0]
         # bf16 caches without trees (ancestor masks): one or two groups of 16 (row, head) pairs at a time, keys split over the warps of a CTA. Rows
         # of every count take this kernel, and a row's splits follow its own context (context_split_keys in common.cuh, which needs half the
