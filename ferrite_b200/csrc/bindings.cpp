@@ -379,7 +379,8 @@ void gdn_step(Tensor out, Tensor rec_state, Tensor conv_state, Tensor proj, Tens
   check(fb_gdn_step(out.data_ptr(), rec_state.data_ptr<float>(), conv_state.data_ptr(), proj.data_ptr(),
                     (long)proj.stride(0), conv_w.data_ptr(), A_log.data_ptr<float>(), dt_bias.data_ptr<float>(),
                     gnorm_w.data_ptr(), seg_slot.data_ptr<int>(), seg_row0.data_ptr<int>(), seg_nrows.data_ptr<int>(),
-                    (int)seg_slot.numel(), (int)nk, (int)nv, (int)dk, (int)dv, (float)eps, commit ? 1 : 0, cur_stream()),
+                    (int)seg_slot.numel(), (int)proj.size(0), (int)nk, (int)nv, (int)dk, (int)dv, (float)eps, commit ? 1 : 0,
+                    cur_stream()),
         "gdn_step");
 }
 

@@ -61,6 +61,7 @@ __device__ __forceinline__ float tanh_exp(float x) {
   return 1.f - __fdividef(2.f, e + 1.f);
 }
 // Two fp32 lanes in one register pair (sm_100: one instruction for both)
+__device__ __forceinline__ float2 bf2f2(uint32_t v) { return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
 __device__ __forceinline__ uint64_t f2_pack(float a, float b) {
   uint64_t v;
   asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
@@ -458,21 +459,40 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // the predecessor wrote. Kernels that load their weights ahead of that wait take `overlap` false where those were written on the
 // same stream just before (a scratch that packed weights were decoded into): they then start behind it like any launch.
 template <typename... KArgs, typename... Args>
-static inline cudaError_t launch_pdl_if(bool overlap, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                                        Args&&... args) {
+static inline cudaError_t launch_pdl_attrs(bool overlap, int cluster, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                           cudaStream_t s, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
+  cfg.attrs = attr; cfg.numAttrs = 0;
   static const bool no_pdl = [] { const char* e = getenv("FB_NO_PDL"); return e && e[0] == '1'; }();   // debugging aid
-  cfg.attrs = attr; cfg.numAttrs = no_pdl || !overlap ? 0 : 1;
+  if (cluster > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = cluster; attr[cfg.numAttrs].val.clusterDim.y = 1; attr[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+  }
+  if (overlap && !no_pdl) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
+  }
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+static inline cudaError_t launch_pdl_if(bool overlap, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                        Args&&... args) {
+  return launch_pdl_attrs(overlap, 1, kern, grid, block, smem, s, static_cast<Args&&>(args)...);
 }
 template <typename... KArgs, typename... Args>
 static inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                                      Args&&... args) {
-  return launch_pdl_if(true, kern, grid, block, smem, s, static_cast<Args&&>(args)...);
+  return launch_pdl_attrs(true, 1, kern, grid, block, smem, s, static_cast<Args&&>(args)...);
+}
+// the same in clusters of `cluster` CTAs along x (the grid's width is a multiple of it)
+template <typename... KArgs, typename... Args>
+static inline cudaError_t launch_pdl_cluster(int cluster, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                             Args&&... args) {
+  return launch_pdl_attrs(true, cluster, kern, grid, block, smem, s, static_cast<Args&&>(args)...);
 }
 
 #define FB_CUDA_CHECK(expr)                                                                      \

@@ -218,11 +218,11 @@ __global__ void __launch_bounds__(DL_THREADS, 1) decode_layer_kernel(const __gri
       if (pair < a.nv * a.M) {
         const int h = pair % a.nv, seg = pair / a.nv;
         if (a.dk == 128)
-          gdn_step_body<128, 128, 4>(L.o, L.rec_state, L.conv_state, reinterpret_cast<const __nv_bfloat16*>(L.g_in.Y),
+          gdn_step_body<128, 128, 4, false>(L.o, L.rec_state, L.conv_state, reinterpret_cast<const __nv_bfloat16*>(L.g_in.Y),
                                      L.g_in.ldy, L.conv_w, L.A_log, L.dt_bias, L.gnorm_w, 1, seg, a.seg_slot[seg], h, a.nk,
                                      a.nv, a.eps, 1);
         else
-          gdn_step_body<64, 64, 8>(L.o, L.rec_state, L.conv_state, reinterpret_cast<const __nv_bfloat16*>(L.g_in.Y),
+          gdn_step_body<64, 64, 8, false>(L.o, L.rec_state, L.conv_state, reinterpret_cast<const __nv_bfloat16*>(L.g_in.Y),
                                    L.g_in.ldy, L.conv_w, L.A_log, L.dt_bias, L.gnorm_w, 1, seg, a.seg_slot[seg], h, a.nk,
                                    a.nv, a.eps, 1);
       }

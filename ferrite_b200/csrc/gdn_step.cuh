@@ -5,12 +5,17 @@
 
 namespace fb {
 
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
 // Decode-row fusion of the three kernels above: causal conv + SiLU of this head's q / k / v channels, the delta-rule
 // recurrence, and the gated per-head RMSNorm (y * rsqrt(mean y^2 + eps) * w * silu(z)) in one pass.
 // Same arithmetic as the separate kernels (the conv output is rounded to bf16 as it would be when stored), so both
 // paths agree to fp32 rounding of the norm's sum. blockDim = DV * 8 as in gdn_rec_kernel.
 // Called by all DV * PARTS threads of a CTA for head h and the segment (n rows from row0, state slot `slot`).
-template <int DK, int DV, int PARTS>
+// The heads that share a key head read the same conv tails, which the first of them rewrites. CLUSTER: they are the CTAs of one cluster, and
+// the rewriting waits until all of them have read; without it (the persistent kernel) they start in step behind a barrier over the grid.
+template <int DK, int DV, int PARTS, bool CLUSTER>
 __device__ __forceinline__ void gdn_step_body(__nv_bfloat16* __restrict__ out, float* __restrict__ rec_state,
                                               __nv_bfloat16* __restrict__ conv_state, const __nv_bfloat16* __restrict__ proj,
                                               long proj_stride, const __nv_bfloat16* __restrict__ conv_w,
@@ -50,6 +55,7 @@ __device__ __forceinline__ void gdn_step_body(__nv_bfloat16* __restrict__ out, f
     for (int j = 0; j < CK - 1; ++j) cwin[j] = bf2f(st[(size_t)j * conv_dim + cch]);
   }
   const float gw = bf2f(gnorm_w[col]);
+  if (CLUSTER) cluster_arrive();
 
   // The rows of a segment are sequential, so a row's inputs are fetched while the row before it is computed: without
   // this every row paid a full global-memory round trip before its first FMA (3.2 us per row on B200, 55 us for a
@@ -135,12 +141,15 @@ __device__ __forceinline__ void gdn_step_body(__nv_bfloat16* __restrict__ out, f
   if (commit) {
 #pragma unroll
     for (int i = 0; i < RP; ++i) Sg[(size_t)(part * RP + i) * DV + col] = S[i];
+    if (CLUSTER) cluster_wait();
     // conv tail = the windows after the last row (q / k channels: first head of the group writes them)
     const bool own_qk = (h % (nv / nk)) == 0;
     if (crole == 2 || (crole >= 0 && own_qk)) {
 #pragma unroll
       for (int j = 0; j < CK - 1; ++j) st[(size_t)j * conv_dim + cch] = f2bf(cwin[j]);
     }
+  } else if (CLUSTER) {
+    cluster_wait();
   }
 }
 

@@ -195,6 +195,40 @@ def test_gdn_conv_and_recurrence(ops, tops, nk, nv, dk, dv):
     close(oa, ob)
 
 
+@pytest.mark.parametrize("nk,nv,d,streams,T,wide", [
+    (16, 16, 128, 1, 2, 0), (4, 4, 128, 3, 17, 0), (2, 4, 128, 2, 32, 0), (2, 4, 128, 1, 33, 0), (2, 8, 128, 2, 5, 0), (1, 8, 128, 1, 70, 0),
+    (4, 4, 64, 2, 9, 0), (2, 8, 64, 2, 33, 0), (1, 9, 64, 1, 3, 0), (16, 16, 128, 2, 1, 0), (16, 16, 128, 10, 1, 0), (2, 8, 128, 24, 1, 0),
+    (4, 4, 128, 2, 6, 3), (4, 4, 64, 1, 4, 1)])          # rows at an odd place or stride: the kernel for single rows takes them
+def test_gdn_step_rows_in_blocks_and_slices(ops, nk, nv, d, streams, T, wide):
+    """Segments of several rows (blocks of 32, heads cut over the CTAs of a cluster) carry the bits of the same rows one at a time, for every
+    number of heads that share a key head, and leave the same states behind; one stream keeps no row."""
+    conv_dim = 2 * nk * d + nv * d
+    width = conv_dim + nv * d + 2 * nv
+    proj = rnd(streams * T, width + wide, seed=1)[:, wide:]
+    conv_w = rnd(conv_dim, 4, scale=0.5, seed=2)
+    A_log = rnd(nv, scale=0.3, seed=3, dtype=torch.float32)
+    dtb = rnd(nv, scale=0.3, seed=4, dtype=torch.float32)
+    gw = (rnd(d, scale=0.1, seed=5).float() + 1).to(torch.bfloat16)
+    i32 = lambda v: torch.tensor(list(v), device=DEV, dtype=torch.int32)
+    rec = [rnd(streams + 1, nv, d, d, scale=0.2, seed=6, dtype=torch.float32) for _ in range(2)]
+    conv = [rnd(streams + 1, 3, conv_dim, seed=7) for _ in range(2)]
+    slots, row0 = [streams - s for s in range(streams)], [s * T for s in range(streams)]
+    step = lambda p, side, sl, r0, n, commit: ops.gdn_step(p, conv_w, rec[side], conv[side], A_log, dtb, gw, i32(sl), i32(r0), i32(n), nk, nv, d, d,
+                                                           1e-6, commit=commit)
+    before = [rec[0].clone(), conv[0].clone()]
+    dry = step(proj, 0, slots, row0, [T] * streams, False)
+    assert torch.equal(rec[0], before[0]) and torch.equal(conv[0], before[1])
+    keep = [T] * (streams - 1) + [0] if streams > 2 else [T] * streams
+    got = step(proj, 0, slots, row0, keep, True)
+    for s in range(streams):
+        for r in range(T):
+            one = step(proj[s * T + r:s * T + r + 1], 1, [slots[s]], [0], [1], keep[s] > 0)
+            if keep[s]:
+                assert torch.equal(dry[s * T + r], one[0]) and torch.equal(got[s * T + r], one[0])
+    assert torch.equal(rec[0], rec[1]) and torch.equal(conv[0], conv[1])
+    assert ops.status() == 0
+
+
 def test_verify_rows_carry_the_bits_of_decode_rows(ops):
     """A row computed inside a multi-row (verify) segment equals, bit for bit, the same row computed as a one-row decode
     step after its predecessors were committed: the Gated DeltaNet step kernel (conv window, delta rule and gated norm
