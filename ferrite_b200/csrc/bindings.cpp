@@ -393,6 +393,7 @@ void gdn_chunk(Tensor y, Tensor rec_state, Tensor conv_state, Tensor scratch, Te
                int64_t nv, int64_t dk, int64_t dv, double eps, bool commit) {
   TORCH_CHECK((int64_t)(scratch.numel() * scratch.element_size()) >=
                   gdn_chunk_scratch_bytes(qkv.size(0), seg_slot.numel(), nv, dk), "gdn_chunk: scratch too small");
+  if (reinterpret_cast<uintptr_t>(qkv.data_ptr()) & 15) qkv = qkv.clone();      // its rows are read 16 bytes at a time
   check(fb_gdn_chunk(y.data_ptr<float>(), rec_state.data_ptr<float>(), conv_state.data_ptr(), (float*)scratch.data_ptr(),
                      qkv.data_ptr(), proj.data_ptr(), (long)proj.stride(0), A_log.data_ptr<float>(),
                      dt_bias.data_ptr<float>(), seg_slot.data_ptr<int>(), seg_row0.data_ptr<int>(),

@@ -195,6 +195,51 @@ def test_gdn_conv_and_recurrence(ops, tops, nk, nv, dk, dv):
     close(oa, ob)
 
 
+@pytest.mark.parametrize("nk,nv,dv,ns,decay", [
+    (2, 2, 128, [1, 63, 64, 65], 1.0), (2, 4, 128, [129, 0, 17], 1.0), (1, 3, 48, [200], 0.1), (16, 32, 128, [70, 130], 6.0),
+    (4, 4, 144, [300], 1.0)])              # slices of 16 and of 32 columns; slow and steep decays
+@pytest.mark.parametrize("commit", [False, True])
+def test_gdn_chunked_scan_against_64_bits(ops, nk, nv, dv, ns, decay, commit):
+    """Chunks of every length, segments beside each other with rows that are NaN behind them, unlike key and value widths. The products carry 32 bits, as
+    does the row by row form in float64's place: y and the state within 5e-6 of their size (ten times what 64 rows of such sums show)."""
+    dk = 128
+    conv_dim, T = 2 * nk * dk + nv * dv, sum(ns) + 3
+    qkv = torch.nn.functional.silu(rnd(T, conv_dim, seed=1).float()).to(torch.bfloat16)
+    proj = rnd(T, conv_dim + nv * dv + 2 * nv, seed=2)
+    qkv[sum(ns):], proj[sum(ns):] = float("nan"), float("nan")
+    A_log = rnd(nv, scale=0.3, seed=3, dtype=torch.float32) + math.log(decay)
+    dtb = rnd(nv, scale=0.3, seed=4, dtype=torch.float32)
+    slots = list(range(len(ns), 0, -1))
+    row0 = [sum(ns[:i]) for i in range(len(ns))]
+    rec, conv = rnd(len(ns) + 1, nv, dk, dv, scale=0.2, seed=6, dtype=torch.float32), rnd(len(ns) + 1, 3, conv_dim, seed=7)
+    want_rec, want_conv = rec.double(), conv.clone()
+    i32 = lambda v: torch.tensor(v, device=DEV, dtype=torch.int32)
+    y = ops.gdn_rec(qkv, proj, rec, conv, A_log, dtb, i32(slots), i32(row0), i32(ns), nk, nv, dk, dv, 1e-6, commit=commit, chunked=True,
+                    max_rows=max(ns))
+    for s, n in enumerate(ns):
+        x, p = qkv[row0[s]:row0[s] + n].double(), proj[row0[s]:row0[s] + n].double()
+        q, k, v = x.split([nk * dk, nk * dk, nv * dv], 1)
+        unit = lambda t: (t.view(n, nk, dk) * torch.rsqrt(t.view(n, nk, dk).square().sum(-1, keepdim=True) + 1e-6)).repeat_interleave(nv // nk, 1)
+        q, k, v = unit(q) * dk ** -0.5, unit(k), v.view(n, nv, dv)
+        beta = torch.sigmoid(p[:, conv_dim + nv * dv:conv_dim + nv * dv + nv])
+        g = torch.exp(-A_log.double().exp() * torch.nn.functional.softplus(p[:, conv_dim + nv * dv + nv:] + dtb.double()))
+        S = want_rec[slots[s]].clone()
+        out = torch.empty(n, nv, dv, dtype=torch.float64, device=DEV)
+        for t in range(n):
+            S = S * g[t][:, None, None]
+            d = (v[t] - torch.einsum("hkv,hk->hv", S, k[t])) * beta[t][:, None]
+            S = S + k[t][:, :, None] * d[:, None]
+            out[t] = torch.einsum("hkv,hk->hv", S, q[t])
+        if n:
+            assert (y[row0[s]:row0[s] + n].double() - out.view(n, -1)).norm() <= 5e-6 * out.norm()
+        if commit:
+            want_rec[slots[s]] = S
+            tail = torch.cat([want_conv[slots[s]], proj[row0[s]:row0[s] + n, :conv_dim]])
+            want_conv[slots[s]] = tail[tail.shape[0] - 3:]
+    assert (rec.double() - want_rec).norm() <= 5e-6 * want_rec.norm()
+    assert torch.equal(conv, want_conv)
+
+
 @pytest.mark.parametrize("nk,nv,d,streams,T,wide", [
     (16, 16, 128, 1, 2, 0), (4, 4, 128, 3, 17, 0), (2, 4, 128, 2, 32, 0), (2, 4, 128, 1, 33, 0), (2, 8, 128, 2, 5, 0), (1, 8, 128, 1, 70, 0),
     (4, 4, 64, 2, 9, 0), (2, 8, 64, 2, 33, 0), (1, 9, 64, 1, 3, 0), (16, 16, 128, 2, 1, 0), (16, 16, 128, 10, 1, 0), (2, 8, 128, 24, 1, 0),
