@@ -749,20 +749,29 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           if (last_flag_s) {
             __threadfence();
             const float* wt = a.workspace + ((size_t)(tile_id * a.split_k) * cols) * GM_BM;
-            for (int c = 0; c < a.bn; ++c) {
-              const int m = m0 + c;
-              if (m >= a.M) break;
-              float g = 0.f, u = 0.f;
+            // eight columns at a time, their loads all under way: one after another the 64 x 3 of them took 70 us
+            for (int c = 0; c < a.bn && m0 + c < a.M; c += 8) {
+              float g[8], u[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) g[j] = u[j] = 0.f;
+#pragma unroll 2
               for (int s2 = 0; s2 < a.split_k; ++s2) {
-                const float* p = wt + ((size_t)s2 * cols) * GM_BM;
-                g += __ldcg(p + (size_t)c * GM_BM + etid);
-                if (a.dual) u += __ldcg(p + (size_t)(a.bn + c) * GM_BM + etid);
+                const float* p = wt + ((size_t)s2 * cols + c) * GM_BM + etid;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) g[j] += __ldcg(p + j * GM_BM);
+                if (a.dual) {
+#pragma unroll
+                  for (int j = 0; j < 8; ++j) u[j] += __ldcg(p + (a.bn + j) * GM_BM);
+                }
               }
-              if (n_ok) {
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                const int m = m0 + c + j;
+                if (!n_ok || m >= a.M) continue;
                 const float sc = (a.scale_m ? a.scale_m[m] : 1.f);
-                g *= sc * (a.scale_n ? a.scale_n[n] : 1.f);
-                if (a.dual) u *= sc * (a.scale_n ? a.scale_n[a.N + n] : 1.f);
-                float x = a.dual ? glu_act(g, u, a.limit) : epilogue_act(g, a.act);
+                float x = g[j] * (sc * (a.scale_n ? a.scale_n[n] : 1.f));
+                if (a.dual) x = glu_act(x, u[j] * (sc * (a.scale_n ? a.scale_n[a.N + n] : 1.f)), a.limit);
+                else x = epilogue_act(x, a.act);
                 if (a.res) x += bf2f(a.res[(size_t)m * a.ldy + n]);
                 if (a.out_f32) reinterpret_cast<float*>(a.Y)[(size_t)m * a.ldy + n] = x;
                 else Yb[(size_t)m * a.ldy + n] = f2bf(x);
@@ -872,12 +881,14 @@ inline long gemm_tail_need(const GemmArgs& a) { return (long)a.tail_tiles * a.ta
 // GM_TAIL_COST + GM_PIECE_COST x pieces k block units a column (3.3 us + 3.3 us a piece for 256 columns), so shallow products stay whole.
 // us, width 256 / best width / with pieces: 2048 x 5120 x 17408 348 / 319 / 288, 1111 rows of it 255 / 210 / 177, 300 rows 135 / 104 / 82, 140 rows
 // 128 / 100 / 66; 2048 x 5120 x 2048 53 / 47 / 55 (whole), 140 x 2048 x 4096 38 / 30 / 21. More than four pieces gained nothing.
+// Up to 64 rows are the narrow side of the product (weights on the tensor cores' 128 lanes) and K is cut into split_k, unless split_k < 0 asks for the
+// orientation of more rows.
 static int plan_gemm(GemmPlan& p, int M, int N, int K, int mode, int split_k, int sm_count, int fp8 = 0, int tail = 0) {
   GemmArgs& a = p.a;
   a.fp8 = fp8; a.scale_m = nullptr; a.scale_n = nullptr; a.out_f32 = 0; a.act = ACT_NONE; a.limit = 0.f;
   a.M = M; a.N = N; a.K = K;
   a.dual = mode == 1;
-  a.swap = M <= 64;
+  a.swap = M <= 64 && split_k >= 0;
   if (a.swap) {
     a.bn = ((M + 15) / 16) * 16;
     a.n_a = a.dual ? 2 : 1;

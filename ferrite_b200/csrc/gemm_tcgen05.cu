@@ -37,7 +37,7 @@ extern "C" int fb_gemm_bf16_glu(void* Y, const void* X, const void* W, const voi
   if (M <= 0 || N <= 0) return 0;
   const int out_f32 = (mode >> 1) & 1, act = (mode & 4) ? ACT_RELU2 : ACT_NONE;
   mode &= 1;
-  if (K % 8 || ldx % 8 || (ldy % 8 && M > 64)) return -1;
+  if (K % 8 || ldx % 8 || (ldy % 8 && (M > 64 || split_k < 0))) return -1;
   if (sm_count <= 0) sm_count = 148;
   GemmPlan p{};
   int rc = plan_in(p, M, N, K, mode, split_k, sm_count, 0, workspace, ws_bytes, counters, n_counters);
@@ -122,7 +122,7 @@ extern "C" int fb_gemm_fp8(void* Y, const void* Xq, const void* Wq, const float*
                            const void* res, int M, int N, int K, long ldy, int mode, int split_k, float* workspace,
                            long ws_bytes, int* counters, int n_counters, int* status, int sm_count, cudaStream_t s) {
   if (M <= 0 || N <= 0) return 0;
-  if (K % 16 || (ldy % 8 && M > 64)) return -1;
+  if (K % 16 || (ldy % 8 && (M > 64 || split_k < 0))) return -1;
   if (sm_count <= 0) sm_count = 148;
   GemmPlan p{};
   int rc = plan_in(p, M, N, K, mode, split_k, sm_count, 1, workspace, ws_bytes, counters, n_counters);

@@ -2,7 +2,7 @@
 
 Same signatures as `torch_ops.TorchOps`. Row counts pick the kernel: up to `GEMV_MAX_ROWS` rows stream the
 weights through the SIMT GEMV (fused norm / SwiGLU / residual), more rows go to the tcgen05 GEMM (swapped
-orientation with split-K up to 64 rows, normal orientation beyond). There is no PyTorch fallback here: a
+orientation with split-K up to `GEMM_SWAP_ROWS` rows, normal orientation beyond). There is no PyTorch fallback here: a
 missing extension raises.
 """
 from __future__ import annotations
@@ -30,6 +30,11 @@ MOE_PAIR_ROWS = 64     # up to this many rows (the largest graph-captured step) 
 # 12.0), but between other kernels the ring fills while the one before it ends: with 5120 x 2048 through registers, four streams of the 27B model
 # took 794 us a step of four layers instead of 777.
 STREAM_VALUES = 8 << 20
+# Rows of a tcgen05 GEMM up to which they are the narrow side of the product, K cut into splits; beyond, they fill what they can of tiles of 128 rows,
+# whose last ones are cut along K. 33, 48, 64 rows against n x k, us, narrow side / tiles: 8224 x 5120 46, 53, 64 / 31; 5120 x 17408 65, 70, 79 / 49;
+# 17408 x 5120 53, 59, 69 / 52; 5120 x 2048 38, 43, 53 / 22; 2048 x 4096 43, 52, 67 / 19. (The other kernels take up to 32 rows; odd widths, whose
+# rows of y lie on no 16 bytes, keep the narrow side up to 64.)
+GEMM_SWAP_ROWS = 32
 TAIL_STREAMS = 4       # streams that keep the scratch of a prompt GEMM's last tiles
 # NVFP4 weights of so many 128 x 256 units and more against one or two rows run on the block-scaled tensor cores (activations as three residual
 # renderings), smaller ones on the row kernel that unpacks the codes: it starts faster and unpacks 1.6 us a unit and CTA. One row, us: 17408 x 2 x
@@ -99,11 +104,12 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         return self._ws
 
     def _gemm_scratch(self, M: int, N: int, split: int):
-        """Workspace and counters of a GEMM call: K splits of few rows, or (more than 64 rows) the last tiles' pieces. The latter belong to the
+        """Workspace and counters of a GEMM call: K splits of few rows, or (split < 0: normal orientation) the last tiles' pieces. The latter belong to the
         current stream, so that a call has the same bits on every one; up to TAIL_STREAMS of them keep theirs (20 MB each: the one that asked
         first gives its own back to the allocator, in whose order of that stream it is used again). A capture takes buffers of its own."""
-        if M <= 64:
+        if split >= 0:
             return (self._workspace(self.C.gemm_workspace_bytes(M, N, split)), self._counters) if split > 1 else (None, None)
+        M = max(M, 65)
         make = lambda: (torch.empty(self.C.gemm_workspace_bytes(M, N, 1) // 4, dtype=torch.float32, device=self.device),
                         torch.zeros(self.C.gemm_counters(M, N, 1), dtype=torch.int32, device=self.device))
         if torch.cuda.is_current_stream_capturing():
@@ -300,7 +306,7 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         # the wide-M epilogue stores 16-byte row pieces: give odd widths a padded leading dimension
         y = out if out is not None else self.empty(M, (N + 7) // 8 * 8, dtype=torch.float32 if out_f32 else self.dtype,
                                                     device=self.device)[:, :N]
-        split = self._split_k(M, N, K) if M <= 64 else 1
+        split = self._split_k(M, N, K) if M <= (64 if y.stride(0) % 8 else GEMM_SWAP_ROWS) else -1
         ws, cnt = self._gemm_scratch(M, N, split)
         self.launches += 1
         self.C.gemm(y, x, w, res, (1 if swiglu else 0) | (2 if out_f32 else 0) | (4 if act else 0), split, ws, cnt, self.status_word)
@@ -339,7 +345,7 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         xs = self.empty(M, dtype=torch.float32, device=self.device)
         self.C.quant_fp8(xq, xs, x, norm_w, eps)
         y = self.empty(M, (N + 7) // 8 * 8, dtype=self.dtype, device=self.device)[:, :N]
-        split = self._split_k(M, N, K // 2) if M <= 64 else 1
+        split = self._split_k(M, N, K // 2) if M <= (64 if y.stride(0) % 8 else GEMM_SWAP_ROWS) else -1
         ws, cnt = self._gemm_scratch(M, N, split)
         self.launches += 2
         self.C.gemm_fp8(y, xq, wq, xs, w_scale, res, 1 if swiglu else 0, split, ws, cnt, self.status_word)

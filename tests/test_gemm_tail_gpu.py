@@ -58,6 +58,29 @@ def test_widths_and_pieces(ops, M, N, K, pieces, swiglu):
     assert ops.status() == 0 and all(int(c.abs().sum()) == 0 for _, c in ops._tails.values())
 
 
+@pytest.mark.parametrize("M", [33, 40, 64])
+@pytest.mark.parametrize("N,K,width", [(1, 64, 8), (264, 1000, 264), (2500, 4104, 2504), (1111, 4104, 1111), (2048, 512, 2051)])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_33_to_64_rows_on_either_side(ops, M, N, K, width, swiglu):
+    """Rows that leave most of a 128-row tile empty, and (outputs `width` columns apart that are no multiple of 8) rows on the narrow side of the
+    product with K splits; rows of another width next to them stay as they are."""
+    x, w = rnd(M, K, seed=1), rnd((2 if swiglu else 1) * N, K, seed=2, scale=K ** -0.5)
+    want = x.double() @ w.double().t()
+    if swiglu:
+        want = torch.nn.functional.silu(want[:, :N]) * want[:, N:]
+    buf = torch.full((M, width + 8), 7.0, dtype=torch.float32, device=DEV)
+    flat = buf.view(-1)[:M * width].view(M, width)
+    y = ops.linear(x, w, swiglu=swiglu, out_f32=True, out=flat[:, :N])
+    bound = 2 ** -14 * max(1.0, want.abs().max().item())                             # as above
+    assert (y.double() - want).abs().max().item() <= bound
+    assert bool((flat[:, N:] == 7).all()) and bool((buf.view(-1)[M * width:] == 7).all())
+    if not swiglu:
+        res = rnd(M, width, seed=3)[:, :N]
+        got = ops.linear(x, w, res=res, out=torch.empty(M, width, dtype=torch.bfloat16, device=DEV)[:, :N])
+        assert torch.equal(got, (y + res.float()).to(torch.bfloat16))
+    assert ops.status() == 0
+
+
 def test_scratch_that_is_too_small_takes_no_pieces(ops):
     """Scratch of any size may come with a call: pieces are taken where they fit it, and nothing past its end is written."""
     M, N, K = 300, 1111, 8192
