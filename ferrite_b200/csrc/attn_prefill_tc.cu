@@ -215,49 +215,48 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ---- MMA issuer ---------------------------------------------------------------------------------------
-      constexpr uint32_t idesc_s = umma_idesc(1, 1, FT_BQ, FT_BKV);
-      constexpr uint32_t idesc_pv = umma_idesc(1, 1, FT_BQ, HV) | (1u << 16);     // B read MN-major
-      const uint32_t aQ = smem_u32(sQ), aK = smem_u32(sK), aV = smem_u32(sV);
-      bool ok = mbar_wait_or_flag(q_full, 0, abort_flag);
-      auto issue_s = [&](int j) -> bool {
-        const int s = j & 1, st = j % KS;
-        if (!mbar_wait_or_flag(&k_full[st], (j / KS) & 1, abort_flag)) return false;
-        if (j >= 2 && !mbar_wait_or_flag(PAIR ? &p_empty[s] : &s_empty[s], ((j >> 1) - 1) & 1, abort_flag)) return false;
-        tc_fence_after();
+    // ---- MMA issuer: the whole warp, one lane of it by predicate (tc_mma_f16_ts_if says why) ------------------------------
+    constexpr uint32_t idesc_s = umma_idesc(1, 1, FT_BQ, FT_BKV);
+    constexpr uint32_t idesc_pv = umma_idesc(1, 1, FT_BQ, HV) | (1u << 16);       // B read MN-major
+    const uint32_t aQ = smem_u32(sQ), aK = smem_u32(sK), aV = smem_u32(sV);
+    const bool issue = elect_one();
+    auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_or_flag(bar, parity, abort_flag)); };
+    bool ok = wait(q_full, 0);
+    auto issue_s = [&](int j) -> bool {
+      const int s = j & 1, st = j % KS;
+      if (!wait(&k_full[st], (j / KS) & 1)) return false;
+      if (j >= 2 && !wait(PAIR ? &p_empty[s] : &s_empty[s], ((j >> 1) - 1) & 1)) return false;
+      tc_fence_after();
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t off = (uint32_t)(kk & 3) * 32u;
-          tc_mma_f16(tmem + COL_S + s * FT_BKV, umma_desc_k128(aQ + (kk >> 2) * Q_CH + off),
-                     umma_desc_k128(aK + st * K_BYTES + (kk >> 2) * KV_CH + off), idesc_s, kk > 0 ? 1u : 0u);
-        }
-        tc_commit(&s_full[s]);
-        tc_commit(&k_empty[st]);
-        return true;
-      };
-      if (ok) ok = issue_s(0);
-      for (int j = 0; ok && j < nt; ++j) {
-        const int s = j & 1, st = j % VS;
-        if (j + 1 < nt && !issue_s(j + 1)) { ok = false; break; }
-        if (!mbar_wait_or_flag(&p_full[s], (j >> 1) & 1, abort_flag) ||
-            !mbar_wait_or_flag(&v_full[st], (j / VS) & 1, abort_flag)) { ok = false; break; }
-        tc_fence_after();
+      for (int kk = 0; kk < HD / 16; ++kk) {
+        const uint32_t off = (uint32_t)(kk & 3) * 32u;
+        tc_mma_f16_if(issue, tmem + COL_S + s * FT_BKV, umma_desc_k128(aQ + (kk >> 2) * Q_CH + off),
+                      umma_desc_k128(aK + st * K_BYTES + (kk >> 2) * KV_CH + off), idesc_s, kk > 0 ? 1u : 0u);
+      }
+      tc_commit_if(issue, &s_full[s]);
+      tc_commit_if(issue, &k_empty[st]);
+      return true;
+    };
+    if (ok) ok = issue_s(0);
+    for (int j = 0; ok && j < nt; ++j) {
+      const int s = j & 1, st = j % VS;
+      if (j + 1 < nt && !issue_s(j + 1)) { ok = false; break; }
+      if (!wait(&p_full[s], (j >> 1) & 1) || !wait(&v_full[st], (j / VS) & 1)) { ok = false; break; }
+      tc_fence_after();
+#pragma unroll
+      for (int kk = 0; kk < FT_BKV / 16; ++kk)
+        tc_mma_f16_ts_if(issue, tmem + COL_O, tmem + COL_P + s * P_STEP + kk * 8,
+                         umma_desc_mn128(aV + st * V_BYTES + kk * 16 * 128, KV_CH, 1024), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
+      if (PX) {
 #pragma unroll
         for (int kk = 0; kk < FT_BKV / 16; ++kk)
-          tc_mma_f16_ts(tmem + COL_O, tmem + COL_P + s * P_STEP + kk * 8,
-                        umma_desc_mn128(aV + st * V_BYTES + kk * 16 * 128, KV_CH, 1024), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
-        if (PX) {
-#pragma unroll
-          for (int kk = 0; kk < FT_BKV / 16; ++kk)
-            tc_mma_f16_ts(tmem + COL_O, tmem + COL_P + REM + s * P_STEP + kk * 8,
-                          umma_desc_mn128(aV + st * V_BYTES + kk * 16 * 128, KV_CH, 1024), idesc_pv, 1u);
-        }
-        tc_commit(&v_empty[st]);
-        tc_commit(&p_empty[s]);
+          tc_mma_f16_ts_if(issue, tmem + COL_O, tmem + COL_P + REM + s * P_STEP + kk * 8,
+                           umma_desc_mn128(aV + st * V_BYTES + kk * 16 * 128, KV_CH, 1024), idesc_pv, 1u);
       }
-      if (!ok) { set_status(status, ST_MBAR_TIMEOUT); *abort_p = 1; }
+      tc_commit_if(issue, &v_empty[st]);
+      tc_commit_if(issue, &p_empty[s]);
     }
+    if (!ok) { set_status(status, ST_MBAR_TIMEOUT); *abort_p = 1; }
   } else {
     // ---- softmax + epilogue: two threads per query row (warps 2..5 take keys 0..31 of a tile, warps 6..9 keys 32..63;
     // a row's two threads sit in the same TMEM lane quadrant) -----------------------------------------------------
