@@ -104,6 +104,79 @@ __global__ void __launch_bounds__(256, 2) head_linear_kernel(__nv_bfloat16* __re
   }
 }
 
+// Heads of up to 512 columns, a multiple of 32, on the tensor cores: m16n8k16 with outputs as M and the tile's rows (8) as N. A dot product does not
+// care about the order of k, so lane t of the four that share a fragment row takes whole 16-byte chunks, of the weights straight from global memory:
+// chunk 4 b + t of block b (32 columns) holds the lane's operands of two products. Sums of 128 columns are added in 32 bits rounded (the tensor
+// cores cut). A row's bits depend on no other row. grid (groups of WARPS * tiles outputs x 16, heads, tiles of 8 rows).
+// The kernel above needs four shuffles an output and row and takes 3.5 us a row at 128 heads of 512 x 128 (17 MB of weights, 2.6 us). us, it / this,
+// at 1, 2, 4, 6, 8 rows: 6.8, 8.8, 14.6, 23.7, 30.2 / 3.5, 3.5, 3.6, 3.5, 3.7; 128 x 512: 7.3, 9.2, 12.5, 21.3, 27.4 / 4.6, 4.7, 4.7, 5.0, 5.1.
+constexpr int HM_WARPS = 4;
+
+template <int SLABS>
+__global__ void __launch_bounds__(HM_WARPS * 32) head_mma_kernel(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* x, const __nv_bfloat16* W, int T, int N,
+                                                                 int K, long x_rs, long x_hs, long y_rs, long y_hs, int tiles) {
+  const int h = blockIdx.y, t0 = blockIdx.z * 8, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int n0 = (blockIdx.x * HM_WARPS + warp) * tiles * 16, n1 = min(N, n0 + tiles * 16);
+  pdl_launch_dependents();
+  {                                                   // (only L2 is asked: the kernel ahead may have written the weights)
+    const char* mine = reinterpret_cast<const char*>(W + ((size_t)h * N + n0) * K);
+    for (long i = lane * 128l; i < 2l * K * (n1 - n0); i += 32 * 128) prefetch_l2(mine + i);
+  }
+  pdl_wait();
+  x = after_wait(x);
+  W = after_wait(W);
+  if (n0 >= N) return;
+  const __nv_bfloat16* Wh = W + (size_t)h * N * K + t * 8;
+  auto load = [&](uint4 (&a)[4][2], int n, int slab) {
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int k = slab * 128 + b * 32;
+        a[b][i] = k < K && n < n1 ? ldg_stream(reinterpret_cast<const uint4*>(Wh + (size_t)min(n + g + i * 8, N - 1) * K + k)) : make_uint4(0, 0, 0, 0);
+      }
+  };
+  uint4 a[2][4][2];
+  load(a[0], n0, 0);
+  uint4 xr[SLABS * 4];
+#pragma unroll
+  for (int b = 0; b < SLABS * 4; ++b)
+    xr[b] = b * 32 < K && t0 + g < T ? *reinterpret_cast<const uint4*>(x + (size_t)(t0 + g) * x_rs + (size_t)h * x_hs + b * 32 + t * 8) : make_uint4(0, 0, 0, 0);
+  auto mma = [](float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  };
+  // two tiles at a time where a tile is one slab, so that the buffers' turns are known
+  for (int n = n0; n < n1; n += SLABS == 1 ? 32 : 16) {
+#pragma unroll
+    for (int half = 0; half < (SLABS == 1 ? 2 : 1); ++half) {
+      const int nn = n + half * 16;
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int s = 0; s < SLABS; ++s) {
+        constexpr bool one = SLABS == 1;
+        const int cur = one ? half : s & 1;
+        if (s + 1 < SLABS) load(a[cur ^ 1], nn, s + 1);
+        else load(a[cur ^ 1], nn + 16, 0);
+        float c[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const uint4 lo = a[cur][b][0], hi = a[cur][b][1], v = xr[s * 4 + b];
+          mma(c[0], lo.x, hi.x, lo.y, hi.y, v.x, v.y);
+          mma(c[1], lo.z, hi.z, lo.w, hi.w, v.z, v.w);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sum[e] += c[0][e] + c[1][e];
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int row = t0 + 2 * t + (e & 1), o = nn + g + (e >> 1) * 8;
+        if (row < T && o < n1) y[(size_t)row * y_rs + (size_t)h * y_hs + o] = __float2bfloat16(sum[e]);
+      }
+    }
+  }
+}
+
 }  // namespace fb
 
 using namespace fb;
@@ -115,6 +188,15 @@ extern "C" int fb_head_linear(void* y, const void* x, const void* W, int T, int 
   if (T <= 0 || heads <= 0) return 0;
   if (K < 8 || K > HL_MAX_K || K % 8 || x_rs % 8 || x_hs % 8 || heads > 65535) return -1;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(W)) & 15) return -1;
+  if (K % 32 == 0 && K <= 512) {
+    const int slabs = K <= 128 ? 1 : K <= 256 ? 2 : 4, z = (T + 7) / 8;
+    // tiles a warp: as many as leave every SM two CTAs
+    int tiles = slabs == 1 ? 2 : 1;
+    while (tiles < 8 && (long)heads * z * ((N + 2 * tiles * HM_WARPS * 16 - 1) / (2 * tiles * HM_WARPS * 16)) >= 2 * 148) tiles *= 2;
+    const auto kern = slabs == 1 ? head_mma_kernel<1> : slabs == 2 ? head_mma_kernel<2> : head_mma_kernel<4>;
+    return (int)launch_pdl(kern, dim3((N + tiles * HM_WARPS * 16 - 1) / (tiles * HM_WARPS * 16), heads, z), dim3(HM_WARPS * 32), (size_t)0, s,
+                           (__nv_bfloat16*)y, (const __nv_bfloat16*)x, (const __nv_bfloat16*)W, T, N, K, x_rs, x_hs, y_rs, y_hs, tiles);
+  }
   const int rows = T >= 8 ? 8 : T > 2 ? 4 : T;        // rows per tile: 1, 2, 4 or 8
   dim3 grid((N + HL_OUT - 1) / HL_OUT, heads, (T + rows - 1) / rows);
   const int chunks = K / 8, cpl = chunks <= 32 ? 1 : chunks <= 64 ? 2 : 4;

@@ -460,15 +460,25 @@ __global__ void __launch_bounds__(128 * LG_GROUPS) latent_merge_kernel(T* __rest
   const size_t rh = (size_t)blockIdx.x * heads + blockIdx.y, pbase = rh * nsplit;
   const int tid = threadIdx.x, grp = tid / 128, col = (tid % 128) * 4;
   float M = -INFINITY, Ls = 0.f;
-  for (int s = tid; s < nsplit; s += blockDim.x) M = fmaxf(M, ml_part[(pbase + s) * 2]);
-  M = block_max(M, red);
-  for (int s = tid; s < nsplit; s += blockDim.x) {
-    const float ms = ml_part[(pbase + s) * 2];
-    const float f = ms == -INFINITY ? 0.f : exp2f(ms - M);          // an empty split wrote no rows
-    sf[s] = f;
-    Ls += f == 0.f ? 0.f : ml_part[(pbase + s) * 2 + 1] * f;
+  if (nsplit <= 32) {                                      // every warp for itself: one trip to memory, one barrier
+    const int lane = tid & 31;
+    const float2 ml = lane < nsplit ? *reinterpret_cast<const float2*>(ml_part + (pbase + lane) * 2) : make_float2(-INFINITY, 0.f);
+    M = warp_max(ml.x);
+    const float f = ml.x == -INFINITY ? 0.f : exp2f(ml.x - M);      // an empty split wrote no rows
+    Ls = warp_sum(f == 0.f ? 0.f : ml.y * f);
+    if (tid < nsplit) sf[tid] = f;
+    __syncthreads();
+  } else {
+    for (int s = tid; s < nsplit; s += blockDim.x) M = fmaxf(M, ml_part[(pbase + s) * 2]);
+    M = block_max(M, red);
+    for (int s = tid; s < nsplit; s += blockDim.x) {
+      const float ms = ml_part[(pbase + s) * 2];
+      const float f = ms == -INFINITY ? 0.f : exp2f(ms - M);
+      sf[s] = f;
+      Ls += f == 0.f ? 0.f : ml_part[(pbase + s) * 2 + 1] * f;
+    }
+    Ls = block_sum(Ls, red);                               // (its barriers publish the factors)
   }
-  Ls = block_sum(Ls, red);                                 // (its barriers publish the factors)
   if (sink) Ls += exp2f(sink[blockIdx.y] * LOG2E - M);
   const float inv = Ls > 0.f ? 1.f / Ls : 0.f;
   float* sums = sf + nsplit;

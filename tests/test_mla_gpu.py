@@ -156,6 +156,26 @@ def test_head_linear_row_kernel_and_batched_gemm(ops, T, nh, N, K):
     assert ops.status() == 0
 
 
+@pytest.mark.parametrize("nh,N,K", [(128, 512, 128), (2, 16, 32), (3, 1, 96), (5, 100, 160), (128, 136, 256), (7, 129, 512), (2, 64, 544), (2, 64, 40)])
+def test_head_linear_rows_and_ragged_widths(ops, nh, N, K):
+    """Outputs that fill no tile of 16, columns that fill no slab of 128 (and too many, or no multiple of 32: the other row kernel): against 64 bits, within
+    the result's rounding to bf16 and 32-bit sums; a row alone has the bits that it has among others."""
+    g = torch.Generator(device=DEV).manual_seed(N + K)
+    W = (torch.randn(nh, N, K, generator=g, device=DEV) * K ** -0.5).to(torch.bfloat16)
+    x = torch.randn(8, nh, K, generator=g, device=DEV).to(torch.bfloat16)
+    want = torch.einsum("thk,hnk->thn", x.double(), W.double())
+    mag = torch.einsum("thk,hnk->thn", x.double().abs(), W.double().abs())
+    for T in (1, 2, 3, 5, 8):
+        y = torch.full((T, nh, N + 3), 7.0, device=DEV, dtype=torch.bfloat16)
+        ops.C.head_linear(y[:, :, :N], x[:T], W)
+        assert bool(((y[:, :, :N].double() - want[:T]).abs() <= want[:T].abs() * 2 ** -8 + mag[:T] * K * 2 ** -24).all())
+        assert bool((y[:, :, N:] == 7).all())
+        if T > 1:
+            assert torch.equal(y[:1], first)
+        first = y[:1].clone()
+    assert ops.status() == 0
+
+
 @pytest.mark.parametrize("nq,L,R,dn,dv", [(16, 512, 64, 128, 128), (4, 64, 64, 32, 32)])
 def test_mla_expanded_prefill_matches_absorbed(ops, nq, L, R, dn, dv):
     """Prompt segments through the expanded form (kv_b GEMM over the context's latent rows, padded per-head K / V, tcgen05
