@@ -22,21 +22,25 @@ __global__ void embed_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat1
 
 // out = bf16( x' * rsqrt(mean(x'^2) + eps) * (centred ? 1 + w : w) ), x' = x (+ res). When res != null the sum
 // x' is also written back to x_out (the residual stream), so a block's output add costs no extra pass.
+// PIECES: pieces of 8 values a thread keeps in registers (0: all of them in shared memory, rows of any length). A thread's eight neighbours
+// make shared memory eight ways conflicting: 2048 rows of 5120 took 12.5 us that way and take 8.0, 1500 of 2048
+// 5.0 and 3.3.
+template <int PIECES>
 __global__ void rmsnorm_kernel(__nv_bfloat16* __restrict__ out, __nv_bfloat16* __restrict__ x_out,
                                const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
                                const __nv_bfloat16* __restrict__ w, int hidden, float eps, int centred) {
   pdl_launch_dependents();
   pdl_wait();
-  extern __shared__ float xs[];          // hidden floats
+  extern __shared__ float xs[];          // PIECES == 0: hidden floats
   __shared__ float scratch[32];
   int row = blockIdx.x;
   const uint4* xp = reinterpret_cast<const uint4*>(x + (size_t)row * hidden);
   const uint4* rp = res ? reinterpret_cast<const uint4*>(res + (size_t)row * hidden) : nullptr;
+  float keep[PIECES > 0 ? PIECES : 1][8];
   float ss = 0.f;
-  for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x) {
+  auto piece = [&](int i, float (&v)[8]) {
     uint4 a = xp[i];
     uint32_t u[4] = {a.x, a.y, a.z, a.w};
-    float v[8];
 #pragma unroll
     for (int j = 0; j < 4; ++j) { v[2 * j] = bf_lo(u[j]); v[2 * j + 1] = bf_hi(u[j]); }
     if (rp) {
@@ -53,12 +57,23 @@ __global__ void rmsnorm_kernel(__nv_bfloat16* __restrict__ out, __nv_bfloat16* _
       reinterpret_cast<uint4*>(x_out + (size_t)row * hidden)[i] = o;
     }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) { xs[i * 8 + j] = v[j]; ss += v[j] * v[j]; }
+    for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
+  };
+  if constexpr (PIECES > 0) {
+#pragma unroll
+    for (int p = 0; p < PIECES; ++p)
+      if (threadIdx.x + p * blockDim.x < hidden / 8) piece(threadIdx.x + p * blockDim.x, keep[p]);
+  } else {
+    for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x) {
+      piece(i, keep[0]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) xs[i * 8 + j] = keep[0][j];
+    }
   }
   float tot = block_sum(ss, scratch);
   float r = rsqrtf(tot / (float)hidden + eps);
   const uint4* wp = reinterpret_cast<const uint4*>(w);
-  for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x) {
+  auto scaled = [&](int i, const float* v) {
     uint4 a = __ldg(wp + i);
     uint32_t u[4] = {a.x, a.y, a.z, a.w};
     float o[8];
@@ -66,12 +81,19 @@ __global__ void rmsnorm_kernel(__nv_bfloat16* __restrict__ out, __nv_bfloat16* _
     for (int j = 0; j < 4; ++j) {
       float w0 = bf_lo(u[j]), w1 = bf_hi(u[j]);
       if (centred) { w0 += 1.f; w1 += 1.f; }
-      o[2 * j] = xs[i * 8 + 2 * j] * r * w0;
-      o[2 * j + 1] = xs[i * 8 + 2 * j + 1] * r * w1;
+      o[2 * j] = v[2 * j] * r * w0;
+      o[2 * j + 1] = v[2 * j + 1] * r * w1;
     }
     uint4 ov;
     ov.x = pack_bf2(o[0], o[1]); ov.y = pack_bf2(o[2], o[3]); ov.z = pack_bf2(o[4], o[5]); ov.w = pack_bf2(o[6], o[7]);
     reinterpret_cast<uint4*>(out + (size_t)row * hidden)[i] = ov;
+  };
+  if constexpr (PIECES > 0) {
+#pragma unroll
+    for (int p = 0; p < PIECES; ++p)
+      if (threadIdx.x + p * blockDim.x < hidden / 8) scaled(threadIdx.x + p * blockDim.x, keep[p]);
+  } else {
+    for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x) scaled(i, xs + i * 8);
   }
 }
 
@@ -108,7 +130,9 @@ __global__ void silu_mul_kernel(__nv_bfloat16* __restrict__ out, const __nv_bflo
 // Gated per-head RMSNorm of the GDN output: out[r][h][d] = bf16( y * rsqrt(mean_d y^2 + eps) * w[d] * silu(z) ).
 // y is fp32 [rows][heads][dv]; z is a column block of the fused projection (row stride z_stride). SIG: gated by sigmoid(z) instead.
 // Output rows are ldo wide, zeros beyond the heads.
-template <typename T, typename Z, bool SIG>
+// PER: heads of 32 PER columns, all of a head's loads under way together (0: heads of any width). us, 0 / 4: 2048 rows of 16
+// heads of 128 14.0 / 8.0, 1500 of 32 19.5 / 11.5.
+template <typename T, typename Z, bool SIG, int PER>
 __global__ void gated_norm_kernel(T* __restrict__ out, int ldo, const float* __restrict__ y, const Z* __restrict__ z, long z_stride,
                                   const Z* __restrict__ w, int heads, int dv, float eps) {
   pdl_launch_dependents();
@@ -116,17 +140,35 @@ __global__ void gated_norm_kernel(T* __restrict__ out, int ldo, const float* __r
   int row = blockIdx.x;
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int nw = blockDim.x >> 5;
-  for (int h = warp; h < heads; h += nw) {
-    const float* yp = y + ((size_t)row * heads + h) * dv;
-    float ss = 0.f;
-    for (int d = lane; d < dv; d += 32) { float v = yp[d]; ss += v * v; }
-    ss = warp_sum(ss);
-    float r = rsqrtf(ss / (float)dv + eps);
-    const Z* zp = z + (size_t)row * z_stride + (size_t)h * dv;
-    for (int d = lane; d < dv; d += 32) {
-      const float zv = Elem<Z>::to(zp[d]);
-      const float v = yp[d] * r * Elem<Z>::to(w[d]) * (SIG ? 1.f / (1.f + expf(-zv)) : siluf_(zv));
-      out[(size_t)row * ldo + h * dv + d] = Elem<T>::from(v);
+  auto gated = [&](float v, float r, float wv, float zv) { return v * r * wv * (SIG ? 1.f / (1.f + expf(-zv)) : siluf_(zv)); };
+  if constexpr (PER > 0) {
+    float wv[PER];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) wv[j] = Elem<Z>::to(w[j * 32 + lane]);
+#pragma unroll 2
+    for (int h = warp; h < heads; h += nw) {
+      const float* yp = y + ((size_t)row * heads + h) * dv;
+      const Z* zp = z + (size_t)row * z_stride + (size_t)h * dv;
+      float v[PER], ss = 0.f;
+      Z zv[PER];
+#pragma unroll
+      for (int j = 0; j < PER; ++j) { v[j] = yp[j * 32 + lane]; zv[j] = zp[j * 32 + lane]; }
+#pragma unroll
+      for (int j = 0; j < PER; ++j) ss += v[j] * v[j];
+      ss = warp_sum(ss);
+      const float r = rsqrtf(ss / (float)dv + eps);
+#pragma unroll
+      for (int j = 0; j < PER; ++j) out[(size_t)row * ldo + h * dv + j * 32 + lane] = Elem<T>::from(gated(v[j], r, wv[j], Elem<Z>::to(zv[j])));
+    }
+  } else {
+    for (int h = warp; h < heads; h += nw) {
+      const float* yp = y + ((size_t)row * heads + h) * dv;
+      float ss = 0.f;
+      for (int d = lane; d < dv; d += 32) { float v = yp[d]; ss += v * v; }
+      ss = warp_sum(ss);
+      float r = rsqrtf(ss / (float)dv + eps);
+      const Z* zp = z + (size_t)row * z_stride + (size_t)h * dv;
+      for (int d = lane; d < dv; d += 32) out[(size_t)row * ldo + h * dv + d] = Elem<T>::from(gated(yp[d], r, Elem<Z>::to(w[d]), Elem<Z>::to(zp[d])));
     }
   }
   for (int c = heads * dv + threadIdx.x; c < ldo; c += blockDim.x) out[(size_t)row * ldo + c] = Elem<T>::from(0.f);
@@ -170,10 +212,11 @@ extern "C" int fb_rmsnorm(void* out, void* x_out, const void* x, const void* res
                           float eps, int centred, cudaStream_t s) {
   if (rows <= 0) return 0;
   if (hidden % 8) return -1;
-  size_t smem = (size_t)hidden * sizeof(float);
-  if (smem > 48 * 1024) cudaFuncSetAttribute(rmsnorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int threads = hidden >= 4096 ? 512 : 256;
-  launch_pdl(rmsnorm_kernel, dim3(rows), dim3(threads), (size_t)(smem), s, (__nv_bfloat16*)out, (__nv_bfloat16*)x_out, (const __nv_bfloat16*)x,
+  const int pieces = (hidden / 8 + threads - 1) / threads;
+  const size_t smem = pieces <= 2 ? 0 : (size_t)hidden * sizeof(float);
+  if (smem > 48 * 1024) cudaFuncSetAttribute(rmsnorm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  launch_pdl(pieces == 1 ? rmsnorm_kernel<1> : pieces == 2 ? rmsnorm_kernel<2> : rmsnorm_kernel<0>, dim3(rows), dim3(threads), (size_t)(smem), s, (__nv_bfloat16*)out, (__nv_bfloat16*)x_out, (const __nv_bfloat16*)x,
                                              (const __nv_bfloat16*)res, (const __nv_bfloat16*)w, hidden, eps, centred);
   return (int)cudaGetLastError();
 }
@@ -197,7 +240,7 @@ extern "C" int fb_gated_norm(void* out, const float* y, const void* z, long z_st
                              int heads, int dv, float eps, cudaStream_t s) {
   if (rows <= 0) return 0;
   int threads = heads >= 8 ? 256 : 32 * heads;
-  launch_pdl(gated_norm_kernel<__nv_bfloat16, __nv_bfloat16, false>, dim3(rows), dim3(threads), (size_t)(0), s, (__nv_bfloat16*)out,
+  launch_pdl(dv == 128 ? gated_norm_kernel<__nv_bfloat16, __nv_bfloat16, false, 4> : gated_norm_kernel<__nv_bfloat16, __nv_bfloat16, false, 0>, dim3(rows), dim3(threads), (size_t)(0), s, (__nv_bfloat16*)out,
              heads * dv, y, (const __nv_bfloat16*)z, z_stride, (const __nv_bfloat16*)w, heads, dv, eps);
   return (int)cudaGetLastError();
 }
@@ -209,9 +252,9 @@ extern "C" int fb_gated_norm_sigmoid(void* out, int ldo, const float* y, const f
   if (ldo < heads * dv) return -1;
   const dim3 b(heads >= 8 ? 256 : 32 * heads);
   if (f32)
-    return (int)launch_pdl(gated_norm_kernel<float, float, true>, dim3(rows), b, (size_t)0, s, (float*)out, ldo, y, z, z_stride, w, heads, dv,
+    return (int)launch_pdl(gated_norm_kernel<float, float, true, 0>, dim3(rows), b, (size_t)0, s, (float*)out, ldo, y, z, z_stride, w, heads, dv,
                            eps);
-  return (int)launch_pdl(gated_norm_kernel<__nv_bfloat16, float, true>, dim3(rows), b, (size_t)0, s, (__nv_bfloat16*)out, ldo, y, z, z_stride,
+  return (int)launch_pdl(gated_norm_kernel<__nv_bfloat16, float, true, 0>, dim3(rows), b, (size_t)0, s, (__nv_bfloat16*)out, ldo, y, z, z_stride,
                          w, heads, dv, eps);
 }
 
