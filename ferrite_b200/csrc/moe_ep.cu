@@ -10,7 +10,7 @@
 //                   inside an expert) and, for the experts it owns, the row / tile prefix sums of the grouped GEMM.
 //   2. ep_dispatch  one warp per pair: the token's hidden row is stored into the owner's receive buffer (16-byte peer
 //                   stores); the last CTA to finish releases one "rows are in" flag per owner.
-//   3. ep_wait      one CTA: bounded wait for the W dispatch flags.
+//   3. ep_wait      one CTA: bounded wait for the W dispatch flags. (One rank alone has the order of its stream: no flags, no 3, no 5.)
 //   4. two grouped tcgen05 GEMMs (gate|up + SwiGLU, down) over the expert-sorted rows (gemm_comm.cu), the second
 //      writing into the symmetric result buffer; 5. ep_signal: "results are ready" flag to every rank.
 //   6. ep_combine   one CTA per local token: bounded wait for the owners' flags, then the K result rows are PULLED from
@@ -20,6 +20,9 @@
 // Buffer reuse is safe by data flow: a rank dispatches call n+1 only after its combine n saw every owner's
 // "results ready" (so every owner is done reading its receive buffer), and an owner overwrites its result buffer
 // only after every source dispatched call n+1, i.e. after that source's combine n pulled its rows.
+//
+// One rank, 1500 tokens of ten picks among 512 experts, us: plan 25.4 -> 7.4 (one thread summed up the experts), dispatch 28.8 -> 11.6 (a system-wide
+// fence a CTA), wait and signal 4.7 -> 0, combine 25.9 -> 23.3 (each pick's row looked up behind the last one's sum).
 //
 // Replaces the reference's expert dispatch by peer copies (`layer_zc`, `crates/fe-dsc/src/engine.rs:2409-2496`), its
 // pair sort (`ggq_moe_sort_*`, `kernels/k-gguf/src/sort.rs`) and ownership masks (`fx_mask_own`,
@@ -31,6 +34,7 @@ namespace fb {
 
 constexpr int EP_MAX_RANKS = 8;
 constexpr int EP_MAX_EXPERTS = 1024;
+constexpr int EP_MAX_PICKS = 32;             // of a token whose rows are looked up ahead of the sum
 
 struct EpComm {
   void* peer[EP_MAX_RANKS];    // base of the symmetric EP workspace on each rank
@@ -103,21 +107,31 @@ __global__ void __launch_bounds__(1024) ep_plan_kernel(EpComm c, const int* __re
   }
   if (fail) set_status(c.status, ST_PEER_TIMEOUT);
   __syncthreads();
-  // prefix over the experts of each owner (per_rank <= 128 entries per owner: one thread per owner is plenty)
-  if (tid < c.world) {
-    int acc = 0, tiles = 0;
-    const int e0 = tid * c.per_rank;
-    for (int j = 0; j < c.per_rank; ++j) {
-      const int e = e0 + j;
-      send_off[e] = acc + before_me[e];
-      if (tid == c.rank) { row_base[j] = acc; tile_start[j] = tiles; }
-      acc += rows_e[e];
-      tiles += (rows_e[e] + tile_rows - 1) / tile_rows;
-    }
-    if (tid == c.rank) {
-      row_base[c.per_rank] = acc;
-      tile_start[c.per_rank] = tiles;
-      if (acc > c.cap_rows) set_status(c.status, ST_CAPACITY);
+  // prefix sums over the experts, a thread each (EP_MAX_EXPERTS threads), restarting at every owner's first: rows in the low half, tiles in the high
+  __shared__ unsigned long long warp_s[32], first_s[EP_MAX_RANKS];
+  unsigned long long mine = 0, upto;
+  if (tid < E) mine = (unsigned)rows_e[tid] | (unsigned long long)((rows_e[tid] + tile_rows - 1) / tile_rows) << 32;
+  upto = mine;
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long below = __shfl_up_sync(0xffffffffu, upto, o);
+    if ((tid & 31) >= o) upto += below;
+  }
+  if ((tid & 31) == 31) warp_s[tid >> 5] = upto;
+  __syncthreads();
+  for (int w = 0; w < (tid >> 5); ++w) upto += warp_s[w];
+  if (tid < E && tid % c.per_rank == 0) first_s[tid / c.per_rank] = upto - mine;
+  __syncthreads();
+  if (tid < E) {
+    upto -= first_s[tid / c.per_rank];
+    const unsigned long long before = upto - mine;
+    send_off[tid] = (int)(unsigned)before + before_me[tid];
+    if (tid / c.per_rank == c.rank) {
+      const int j = tid % c.per_rank;
+      row_base[j] = (int)(unsigned)before; tile_start[j] = (int)(before >> 32);
+      if (j == c.per_rank - 1) {
+        row_base[c.per_rank] = (int)(unsigned)upto; tile_start[c.per_rank] = (int)(upto >> 32);
+        if ((int)(unsigned)upto > c.cap_rows) set_status(c.status, ST_CAPACITY);
+      }
     }
   }
 }
@@ -137,6 +151,7 @@ __global__ void __launch_bounds__(256) ep_dispatch_kernel(EpComm c, const __nv_b
       for (int i = lane; i < c.hidden / 8; i += 32) dst[i] = pieces ? sm_piece(src[i]) : src[i];
     }
   }
+  if (c.world == 1) return;                // (what follows on the stream finds the rows)
   // the last CTA to finish tells every owner that this rank's rows are in place
   __threadfence_system();
   __syncthreads();
@@ -181,24 +196,40 @@ __global__ void __launch_bounds__(256) ep_combine_kernel(EpComm c, __nv_bfloat16
   const uint32_t epoch = c.ctr[0] + 1;
   if (threadIdx.x == 0) fail_s = 0;
   __syncthreads();
-  if (threadIdx.x < c.world)
+  if (threadIdx.x < c.world && c.world > 1)
     if (!wait_flag_ge(ep_flag(c.peer[c.rank], c, 1, threadIdx.x), epoch, c.spin_limit)) { fail_s = 1; set_status(c.status, ST_PEER_TIMEOUT); }
+  // where the token's result rows lie, and their weights (0 rows past the buffers' end)
+  __shared__ const __nv_bfloat16* row_s[EP_MAX_PICKS];
+  __shared__ float w_s[EP_MAX_PICKS];
+  for (int k = threadIdx.x; t < rows && k < min(top_k, EP_MAX_PICKS); k += blockDim.x) {
+    const int pair = t * top_k + k, e = ids[pair], row = send_off[e] + pos[pair];
+    row_s[k] = row < c.cap_rows ? ep_out(c.peer[e / c.per_rank], c) + (size_t)row * c.hidden : nullptr;
+    w_s[k] = wts[pair];
+  }
   __syncthreads();
   const int H = c.hidden;
   if (!fail_s && t < rows) {
     const float g = shared ? (shared_gate ? sigmoidf_(shared_gate[t * gate_ld]) : 1.f) : 0.f;
     for (int i = threadIdx.x; i < H / 8; i += blockDim.x) {
       float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      for (int k = 0; k < top_k; ++k) {
-        const int pair = t * top_k + k;
-        const int e = ids[pair], o = e / c.per_rank;
-        const int row = send_off[e] + pos[pair];
-        if (row >= c.cap_rows) continue;
-        const float w = wts[pair];
-        const uint4 raw = __ldcg(reinterpret_cast<const uint4*>(ep_out(c.peer[o], c) + (size_t)row * H) + i);
+      auto add_row = [&](float w, uint4 raw) {
         const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) { acc[2 * j] = fmaf(w, bf_lo(u[j]), acc[2 * j]); acc[2 * j + 1] = fmaf(w, bf_hi(u[j]), acc[2 * j + 1]); }
+      };
+      constexpr int AHEAD = 5;             // rows under way together, summed in pick order
+      for (int k = 0; k < min(top_k, EP_MAX_PICKS); k += AHEAD) {
+        uint4 raw[AHEAD];
+#pragma unroll
+        for (int j = 0; j < AHEAD; ++j)
+          if (k + j < top_k && k + j < EP_MAX_PICKS && row_s[k + j]) raw[j] = __ldcg(reinterpret_cast<const uint4*>(row_s[k + j]) + i);
+#pragma unroll
+        for (int j = 0; j < AHEAD; ++j)
+          if (k + j < top_k && k + j < EP_MAX_PICKS && row_s[k + j]) add_row(w_s[k + j], raw[j]);
+      }
+      for (int k = EP_MAX_PICKS; k < top_k; ++k) {
+        const int pair = t * top_k + k, e = ids[pair], row = send_off[e] + pos[pair];
+        if (row < c.cap_rows) add_row(wts[pair], __ldcg(reinterpret_cast<const uint4*>(ep_out(c.peer[e / c.per_rank], c) + (size_t)row * H) + i));
       }
       if (shared) {
         const uint4 raw = reinterpret_cast<const uint4*>(shared + (size_t)t * H)[i];
@@ -283,7 +314,7 @@ extern "C" int fb_ep_moe(void* out, int out_f32, float limit, const void* x, con
   ep_plan_kernel<<<1, 1024, 0, s>>>(c, ids, n_pairs, pos, send_off, row_base, tile_start, fp4 ? fb_moe_stream_rows() : 128);
   const int dgrid = n_pairs > 0 ? (n_pairs + 7) / 8 : 1;
   ep_dispatch_kernel<<<dgrid, 256, 0, s>>>(c, (const __nv_bfloat16*)x, ids, pos, send_off, n_pairs, top_k, fp4 ? 1 : 0);
-  ep_wait_kernel<<<1, 32, 0, s>>>(c);
+  if (world > 1) ep_wait_kernel<<<1, 32, 0, s>>>(c);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   const char* local = reinterpret_cast<const char*>(peers[rank]);
@@ -302,7 +333,7 @@ extern "C" int fb_ep_moe(void* out, int out_f32, float limit, const void* x, con
     rc = fb_gemm_grouped(rows_out, act, w_down, tile_start, row_base, c.per_rank, (int)cap_rows, hidden, inter, inter, hidden, 0, 0.f, status, sm_count, s);
   }
   if (rc) return rc;
-  ep_signal_kernel<<<1, 32, 0, s>>>(c);
+  if (world > 1) ep_signal_kernel<<<1, 32, 0, s>>>(c);
   ep_combine_kernel<<<rows > 0 ? rows : 1, 256, 0, s>>>(c, (__nv_bfloat16*)out, out_f32 ? (float*)out : nullptr, ids, wts, pos, send_off,
                                                         (const __nv_bfloat16*)shared, shared_gate, gate_ld, out_f32 == 1,
                                                         (const __nv_bfloat16*)res, rows, top_k);
