@@ -15,7 +15,7 @@
 // Bound by issue slots (0.8 of them taken): unpacking a unit is some 640 of its 1,300 cycles a scheduler, waits, scales, epilogue and the issue of the
 // products the rest. What it hung on before: products issued behind a branch for one lane (95 cycles each instead of 16, see tc_mma_f16_ts_if),
 // unrolled code that fell out of the instruction cache, two unpacking warps a scheduler instead of four.
-// 1500 rows, 512 experts, ten each, 2048 x 512, us: gate and up 174, down 105, the whole block 338; in mma.sync fragments, 32 rows an item, 367, 216,
+// 1500 rows, 512 experts, ten each, 2048 x 512, us: gate and up 174, down 105, the whole block 299; in mma.sync fragments, 32 rows an item, 367, 216,
 // 624; the grouped GEMM took 670 for each after 410 for the bf16 copy of each stack.
 #include "api_ext.h"
 #include "stream_mma.cuh"

@@ -62,9 +62,10 @@ class ExpertParallel:
         """Whether NVFP4 stacks are multiplied as they are (`csrc/moe_stream.cu`) rather than as bf16 copies by the grouped tcgen05 GEMM: with
         up to CODE_ROWS rows per expert. Every 64 rows of an expert of 3 x 2048 x 512 cost 0.5 us there, so at most pairs / 64 + experts times that,
         however the rows are spread; the copies and 128-row tiles cost about 3 us an expert whatever its rows. The whole block, us, codes /
-        copies, 512 experts, 29, 64, 80, 96, 128 rows each: 338 / 1476, 551 / 1543, 676 / 1576, 734 / 1606, 936 / 1811; all rows on 20 of
-        them, 750 and 2048 each: 233 / 1041, 512 / 1278. (The line was drawn when codes cost twice as much; they stay ahead up to some 600 rows.) One rank only: the order of the values in
-        the dispatched rows depends on the answer, which ranks with different row counts could give differently."""
+        copies, 512 experts, 29, 64, 80, 96, 128 rows each: 299 / 1436, 501 / 1488, 627 / 1524, 681 / 1544, 874 / 1733; all rows on 20 of
+        them, 750 and 2048 each: 193 / 1011, 454 / 1219. (The line was drawn when codes cost more than twice as much; they stay ahead beyond it.)
+        One rank only: the order of the values in the dispatched rows depends on the answer, which ranks with different row counts could give
+        differently."""
         e, rows, hidden = w_gu.shape
         return (self.fused and self.world == 1 and w_down.shape[2] % 256 == 0 and bool(self.C.moe_stream_fits(rows // 2, hidden, self.n_experts))
                 and bool(self.C.moe_stream_fits(hidden, w_down.shape[2], self.n_experts))
