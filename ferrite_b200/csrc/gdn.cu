@@ -284,6 +284,7 @@ gdn_rows_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ rec_state, 
   const int n = after_wait(seg_nrows)[seg], row0 = after_wait(seg_row0)[seg], slot = after_wait(seg_slot)[seg];
   proj = after_wait(proj);
   if (n <= 0) return;                      // (every CTA of the cluster)
+  cluster_arrive();                        // met ahead of the first store into another CTA's shared memory: by then that CTA has to run
   const __nv_bfloat16* prow = proj + (size_t)row0 * proj_stride;
   __nv_bfloat16* st = conv_state + (size_t)slot * (CK - 1) * conv_dim;
   const bool rec = warp < G::REC_WARPS;
@@ -380,6 +381,7 @@ gdn_rows_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ rec_state, 
     }
     __syncthreads();
     // gated norm over all of the head's columns
+    if (b0 == 0) cluster_wait();
     float* sn = ssn + ((b0 / rb) & 1) * rb * NG;
     for (int i = warp; i < m * VG; i += G::WARPS) {
       const int r = i / VG, g = i % VG;
