@@ -253,7 +253,7 @@ __device__ __forceinline__ void step_cp16(void* smem, const void* gmem) {
 }
 
 // grid (nv * SPLIT, segments); a cluster holds the slices of all heads of a key head, so that the conv tail, which all of them read, is
-// rewritten behind a barrier. `proj` lies on 16 bytes and so do its rows.
+// rewritten behind a barrier. `proj`, its rows, `conv_w` and `conv_state` lie on 16 bytes (elsewhere the kernel for single rows takes over).
 template <int DK, int DV, int PARTS, int SPLIT>
 __global__ void __launch_bounds__(GdnRows<DK, DV, PARTS, SPLIT>::THREADS)
 gdn_rows_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ rec_state, __nv_bfloat16* __restrict__ conv_state,
@@ -530,7 +530,8 @@ static int launch_step(void* out, float* rec_state, void* conv_state, const void
                 eps, commit, s);
   };
   const bool sliced = rb > 1 || (nv * split >= 64 && nv * split * nseg <= STEP_CTAS);
-  if (sliced && share <= 8 && proj_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(proj) & 15) == 0) {
+  const uintptr_t places = reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(conv_w) | reinterpret_cast<uintptr_t>(conv_state);
+  if (sliced && share <= 8 && proj_stride % 8 == 0 && (places & 15) == 0) {
     if constexpr (D == 128)
       if (split == 4) return go(launch_rows<D, D, PARTS, 4>);
     return split == 2 ? go(launch_rows<D, D, PARTS, 2>) : go(launch_rows<D, D, PARTS, 1>);

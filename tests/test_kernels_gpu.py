@@ -274,6 +274,29 @@ def test_gdn_step_rows_in_blocks_and_slices(ops, nk, nv, d, streams, T, wide):
     assert ops.status() == 0
 
 
+@pytest.mark.parametrize("what", ["conv_w", "conv_state"])
+@pytest.mark.parametrize("T", [1, 6])
+def test_gdn_step_operands_at_odd_places(ops, what, T):
+    """Convolution weights and tails that lie on no 16 bytes (a view into a larger buffer) give the bits of those that do, in the outputs and in
+    what is left behind."""
+    nk, nv, d, streams = 8, 16, 128, 2
+    conv_dim = 2 * nk * d + nv * d
+    proj = rnd(streams * T, conv_dim + nv * d + 2 * nv, seed=1)
+    A_log, dtb = rnd(nv, scale=0.3, seed=2, dtype=torch.float32), rnd(nv, scale=0.3, seed=3, dtype=torch.float32)
+    gw = (rnd(d, scale=0.1, seed=4).float() + 1).to(torch.bfloat16)
+    i32 = lambda *v: torch.tensor(list(v), device=DEV, dtype=torch.int32)
+    outs = []
+    for odd in (False, True):
+        place = lambda t, name: torch.cat([t.new_zeros(4), t.reshape(-1)])[4:].view(t.shape) if odd and name == what else t
+        conv_w, conv = place(rnd(conv_dim, 4, scale=0.5, seed=5), "conv_w"), place(rnd(streams, 3, conv_dim, seed=6), "conv_state")
+        assert {"conv_w": conv_w, "conv_state": conv}[what].data_ptr() % 16 == (8 if odd else 0)
+        rec = rnd(streams, nv, d, d, scale=0.2, seed=7, dtype=torch.float32)
+        y = ops.gdn_step(proj, conv_w, rec, conv, A_log, dtb, gw, i32(1, 0), i32(0, T), i32(T, T), nk, nv, d, d, 1e-6)
+        outs.append((y, rec, conv))
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
+    assert ops.status() == 0
+
+
 def test_verify_rows_carry_the_bits_of_decode_rows(ops):
     """A row computed inside a multi-row (verify) segment equals, bit for bit, the same row computed as a one-row decode
     step after its predecessors were committed: the Gated DeltaNet step kernel (conv window, delta rule and gated norm
