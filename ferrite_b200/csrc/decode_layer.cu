@@ -212,8 +212,7 @@ __global__ void __launch_bounds__(DL_THREADS, 1) decode_layer_kernel(const __gri
       dl_stamp(st, 1);
       bar.sync();
       dl_stamp(st, 2);
-      // every (head, sequence) pair has a CTA of its own (the host checks nv * M <= grid): the heads of a key group
-      // read the conv tail their first head rewrites at the end
+      // every (head, sequence) pair has a CTA of its own (the host checks nv * M <= grid)
       const int pair = blockIdx.x;
       if (pair < a.nv * a.M) {
         const int h = pair % a.nv, seg = pair / a.nv;
@@ -228,6 +227,14 @@ __global__ void __launch_bounds__(DL_THREADS, 1) decode_layer_kernel(const __gri
       }
       dl_stamp(st, 3);
       dl_gemv_reduce<M>(L.g_out, a.cb, epoch, 2u * li, xs, tile, rscale, scratch, at_barrier, st, 4);
+      // heads that share a key head have read its conv tail on the other side of that product's barrier: the first of them rewrites it
+      if (const int share = a.nv / a.nk; share > 1 && pair < a.nv * a.M && pair % a.nv % share == 0) {
+        const int kh = pair % a.nv / share, seg = pair / a.nv, conv_dim = 2 * a.nk * a.dk + a.nv * a.dk;
+        for (int i = threadIdx.x; i < 2 * a.dk; i += blockDim.x)
+          gdn_qk_tail(L.conv_state + (size_t)a.seg_slot[seg] * 3 * conv_dim,
+                      reinterpret_cast<const __nv_bfloat16*>(L.g_in.Y) + (size_t)seg * L.g_in.ldy, L.g_in.ldy, 1, conv_dim,
+                      (i < a.dk ? 0 : a.nk * a.dk) + kh * a.dk + i % a.dk);
+      }
     } else {
       dl_gemv_reduce<M>(L.g_out, a.cb, epoch, 2u * li, xs, tile, rscale, scratch, enter, st, 4);
       if (st != nullptr && threadIdx.x == 0) st[13] = st[4];

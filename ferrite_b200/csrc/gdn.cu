@@ -421,6 +421,18 @@ gdn_rows_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ rec_state, 
   }
 }
 
+// q / k tails of the heads that share a key head and are no cluster, behind the kernel in which all of them read the old ones.
+// grid ((2 nk dk + 255) / 256, segments)
+__global__ void __launch_bounds__(256) gdn_qk_tail_kernel(__nv_bfloat16* conv_state, const __nv_bfloat16* proj, long proj_stride, const int* seg_slot,
+                                                          const int* seg_row0, const int* seg_nrows, int qk, int conv_dim) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int c = blockIdx.x * 256 + threadIdx.x, n = after_wait(seg_nrows)[blockIdx.y];
+  if (c >= qk || n <= 0) return;
+  gdn_qk_tail(conv_state + (size_t)after_wait(seg_slot)[blockIdx.y] * 3 * conv_dim,
+              after_wait(proj) + (size_t)after_wait(seg_row0)[blockIdx.y] * proj_stride, proj_stride, n, conv_dim, c);
+}
+
 }  // namespace fb
 
 using namespace fb;
@@ -536,14 +548,18 @@ static int launch_step(void* out, float* rec_state, void* conv_state, const void
       if (split == 4) return go(launch_rows<D, D, PARTS, 4>);
     return split == 2 ? go(launch_rows<D, D, PARTS, 2>) : go(launch_rows<D, D, PARTS, 1>);
   }
-  // One row each. (Heads that share a key head in more than eights get no cluster.)
+  // One row each. (Heads that share a key head in more than eights get no cluster; their q / k tail is rewritten by a launch of its own.)
   const bool cluster = share > 1 && share <= 8;
   const auto one = cluster ? gdn_step_kernel<D, D, PARTS, true, 1> : gdn_step_kernel<D, D, PARTS, false, 1>;
   const auto two = cluster ? gdn_step_kernel<D, D, PARTS, true, 2> : gdn_step_kernel<D, D, PARTS, false, 2>;
-  return (int)launch_pdl_cluster(cluster ? share : 1, nv * nseg > STEP_CTAS ? two : one, dim3(nv, nseg), dim3(D * PARTS), (size_t)0, s,
-                                 (__nv_bfloat16*)out, rec_state, (__nv_bfloat16*)conv_state, (const __nv_bfloat16*)proj, proj_stride,
-                                 (const __nv_bfloat16*)conv_w, A_log, dt_bias, (const __nv_bfloat16*)gnorm_w, seg_slot, seg_row0, seg_nrows,
-                                 nk, nv, eps, commit);
+  const cudaError_t e = launch_pdl_cluster(cluster ? share : 1, nv * nseg > STEP_CTAS ? two : one, dim3(nv, nseg), dim3(D * PARTS), (size_t)0, s,
+                                           (__nv_bfloat16*)out, rec_state, (__nv_bfloat16*)conv_state, (const __nv_bfloat16*)proj, proj_stride,
+                                           (const __nv_bfloat16*)conv_w, A_log, dt_bias, (const __nv_bfloat16*)gnorm_w, seg_slot, seg_row0,
+                                           seg_nrows, nk, nv, eps, commit);
+  if (e != cudaSuccess || share <= 8 || !commit) return (int)e;
+  const int qk = 2 * nk * D;
+  return (int)launch_pdl(gdn_qk_tail_kernel, dim3((qk + 255) / 256, nseg), dim3(256), (size_t)0, s, (__nv_bfloat16*)conv_state,
+                         (const __nv_bfloat16*)proj, proj_stride, seg_slot, seg_row0, seg_nrows, qk, qk + nv * D);
 }
 
 // `rows`: rows of the step.

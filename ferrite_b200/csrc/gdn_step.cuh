@@ -13,8 +13,9 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // Same arithmetic as the separate kernels (the conv output is rounded to bf16 as it would be when stored), so both
 // paths agree to fp32 rounding of the norm's sum. blockDim = DV * 8 as in gdn_rec_kernel.
 // Called by all DV * PARTS threads of a CTA for head h and the segment (n rows from row0, state slot `slot`).
-// The heads that share a key head read the same conv tails, which the first of them rewrites. CLUSTER: they are the CTAs of one cluster, and
-// the rewriting waits until all of them have read; without it (the persistent kernel) they start in step behind a barrier over the grid.
+// The heads that share a key head read the same conv tails, which one of them may rewrite once all have read. CLUSTER: they are the CTAs of one
+// cluster, and the first rewrites behind a barrier of it. Without it, heads that share leave the q / k tail alone: the caller rewrites it
+// (gdn_qk_tail) where it knows that all of them are through.
 template <int DK, int DV, int PARTS, bool CLUSTER>
 __device__ __forceinline__ void gdn_step_body(__nv_bfloat16* __restrict__ out, float* __restrict__ rec_state,
                                               __nv_bfloat16* __restrict__ conv_state, const __nv_bfloat16* __restrict__ proj,
@@ -143,7 +144,7 @@ __device__ __forceinline__ void gdn_step_body(__nv_bfloat16* __restrict__ out, f
     for (int i = 0; i < RP; ++i) Sg[(size_t)(part * RP + i) * DV + col] = S[i];
     if (CLUSTER) cluster_wait();
     // conv tail = the windows after the last row (q / k channels: first head of the group writes them)
-    const bool own_qk = (h % (nv / nk)) == 0;
+    const bool own_qk = CLUSTER ? (h % (nv / nk)) == 0 : nv == nk;
     if (crole == 2 || (crole >= 0 && own_qk)) {
 #pragma unroll
       for (int j = 0; j < CK - 1; ++j) st[(size_t)j * conv_dim + cch] = f2bf(cwin[j]);
@@ -151,6 +152,14 @@ __device__ __forceinline__ void gdn_step_body(__nv_bfloat16* __restrict__ out, f
   } else if (CLUSTER) {
     cluster_wait();
   }
+}
+
+// The q / k channel c (of 2 nk DK) of a slot's conv tail `st` behind the n > 0 rows at `prow`.
+__device__ __forceinline__ void gdn_qk_tail(__nv_bfloat16* st, const __nv_bfloat16* prow, long proj_stride, int n, int conv_dim, int c) {
+  constexpr int K = 3;
+#pragma unroll
+  for (int j = 0; j < K; ++j)
+    st[(size_t)j * conv_dim + c] = n + j < K ? st[(size_t)(n + j) * conv_dim + c] : prow[(size_t)(n + j - K) * proj_stride + c];
 }
 
 }  // namespace fb

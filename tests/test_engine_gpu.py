@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from ferrite_b200.config import EngineConfig, hybrid_27b, scaled, tiny_hybrid
+from ferrite_b200.config import EngineConfig, ModelConfig, hybrid_27b, scaled, tiny_hybrid
 from ferrite_b200.engine.engine import Engine
 from ferrite_b200.engine.executor import Segment
 from ferrite_b200.models.ref import RefModel
@@ -379,6 +379,31 @@ def test_persistent_decode_layer_matches_the_separate_kernels(ext, streams):
         assert err < 0.05 * outs[0][0].abs().max().item() + 1e-3, (i, err)
         if streams == 1:
             assert torch.equal(outs[0][1], outs[1][1]), i
+    assert engs[1].ops.launches < engs[0].ops.launches
+    for e in engs:
+        e.check()
+
+
+@pytest.mark.parametrize("nk,nv", [(2, 32), (4, 12)])
+def test_persistent_decode_layer_moves_shared_conv_tails_on_by_one_row(ext, nk, nv):
+    """Heads that share a key head, in fours and more, read one conv tail that is rewritten in the same launch: every step moves it on by exactly one
+    row, and the row is the one that the separate kernels bring in."""
+    cfg = ModelConfig(name="shared", hidden=512, inter=1024, n_layers=4, head_dim=128, n_q=4, n_kv=2, rotary_dim=32, rope_theta=1e6, lin_k_heads=nk,
+                      lin_v_heads=nv, lin_dk=128, lin_dv=128, vocab=512, tie_embeddings=False)
+    engs = [Engine(cfg, None, EngineConfig(n_slots=4, max_ctx=256, fused_layers=f), device="cuda", seed=3) for f in (False, True)]
+    prompts = [_prompt(cfg, 9 + 5 * s, seed=10 + s) for s in range(4)]
+    for e in engs:
+        for s, p in enumerate(prompts):
+            e.prefill(s, p)
+    for i in range(5):
+        before = [{k: v.clone() for k, v in e.ex.conv_state.items()} for e in engs]
+        for e in engs:
+            e.forward([Segment(s, len(p) + i, [7 * i + s], "last") for s, p in enumerate(prompts)], commit=True, greedy=True)
+        for e, b in zip(engs, before):
+            assert all(torch.equal(v[:, :2], b[k][:, 1:]) for k, v in e.ex.conv_state.items())
+        for k, v in engs[0].ex.conv_state.items():
+            a, b = v[:, 2].float(), engs[1].ex.conv_state[k][:, 2].float()
+            assert (a - b).abs().max() <= 0.05 * a.abs().max()         # (the products' sums run in another order)
     assert engs[1].ops.launches < engs[0].ops.launches
     for e in engs:
         e.check()

@@ -297,6 +297,36 @@ def test_gdn_step_operands_at_odd_places(ops, what, T):
     assert ops.status() == 0
 
 
+@pytest.mark.parametrize("nk,nv,d", [(2, 18, 128), (2, 32, 64), (1, 40, 64)])
+@pytest.mark.parametrize("T", [1, 2, 5])
+def test_gdn_step_with_many_heads_to_a_key_head(ops, nk, nv, d, T):
+    """More than eight heads to a key head and several times as many CTAs as SMs: all of them read the conv tail before it moves on. Outputs, states and
+    tails have the bits of one stream and one row at a time; a segment without rows leaves its own alone."""
+    streams, conv_dim = 40, 2 * nk * d + nv * d
+    proj = rnd(streams * T, conv_dim + nv * d + 2 * nv, seed=1)
+    conv_w = rnd(conv_dim, 4, scale=0.5, seed=2)
+    A_log, dtb = rnd(nv, scale=0.3, seed=3, dtype=torch.float32), rnd(nv, scale=0.3, seed=4, dtype=torch.float32)
+    gw = (rnd(d, scale=0.1, seed=5).float() + 1).to(torch.bfloat16)
+    i32 = lambda v: torch.tensor(list(v), device=DEV, dtype=torch.int32)
+    rec = [rnd(streams, nv, d, d, scale=0.2, seed=6, dtype=torch.float32) for _ in range(2)]
+    conv = [rnd(streams, 3, conv_dim, seed=7) for _ in range(2)]
+    step = lambda p, side, sl, r0, n, commit=True: ops.gdn_step(p, conv_w, rec[side], conv[side], A_log, dtb, gw, i32(sl), i32(r0), i32(n), nk, nv, d, d,
+                                                                1e-6, commit=commit)
+    rows = [T] * (streams - 1) + [0]
+    dry = step(proj, 0, range(streams), range(0, streams * T, T), rows, False)
+    assert torch.equal(conv[0], conv[1]) and torch.equal(rec[0], rec[1])
+    got = step(proj, 0, range(streams), range(0, streams * T, T), rows)
+    live = (streams - 1) * T
+    assert torch.equal(got[:live], dry[:live])
+    for s in range(streams - 1):
+        for r in range(s * T, s * T + T):
+            assert torch.equal(got[r], step(proj[r:r + 1], 1, [s], [0], [1])[0])
+    assert torch.equal(rec[0], rec[1]) and torch.equal(conv[0], conv[1])
+    want = torch.cat([rnd(streams, 3, conv_dim, seed=7), proj.view(streams, T, -1)[:, :, :conv_dim]], 1)
+    assert torch.equal(conv[0][:-1], want[:-1, T:])
+    assert ops.status() == 0
+
+
 def test_verify_rows_carry_the_bits_of_decode_rows(ops):
     """A row computed inside a multi-row (verify) segment equals, bit for bit, the same row computed as a one-row decode
     step after its predecessors were committed: the Gated DeltaNet step kernel (conv window, delta rule and gated norm
