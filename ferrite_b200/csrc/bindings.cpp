@@ -375,12 +375,12 @@ void gdn_rec_tree(Tensor y, Tensor rec_state, Tensor qkv, Tensor proj, Tensor A_
 
 void gdn_step(Tensor out, Tensor rec_state, Tensor conv_state, Tensor proj, Tensor conv_w, Tensor A_log, Tensor dt_bias,
               Tensor gnorm_w, Tensor seg_slot, Tensor seg_row0, Tensor seg_nrows, int64_t nk, int64_t nv, int64_t dk,
-              int64_t dv, double eps, bool commit) {
+              int64_t dv, double eps, bool commit, int64_t max_rows) {
   check(fb_gdn_step(out.data_ptr(), rec_state.data_ptr<float>(), conv_state.data_ptr(), proj.data_ptr(),
                     (long)proj.stride(0), conv_w.data_ptr(), A_log.data_ptr<float>(), dt_bias.data_ptr<float>(),
                     gnorm_w.data_ptr(), seg_slot.data_ptr<int>(), seg_row0.data_ptr<int>(), seg_nrows.data_ptr<int>(),
-                    (int)seg_slot.numel(), (int)proj.size(0), (int)nk, (int)nv, (int)dk, (int)dv, (float)eps, commit ? 1 : 0,
-                    cur_stream()),
+                    (int)seg_slot.numel(), (int)proj.size(0), (int)max_rows, (int)nk, (int)nv, (int)dk, (int)dv, (float)eps,
+                    commit ? 1 : 0, cur_stream()),
         "gdn_step");
 }
 
@@ -481,6 +481,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gdn_rec_tree", &gdn_rec_tree);
   m.def("kv_dequant", &kv_dequant);
   m.def("gdn_step", &gdn_step);
+  m.def("gdn_step_sliced", [](int64_t nseg, int64_t rows, int64_t max_rows, int64_t nk, int64_t nv, int64_t d) {
+    TORCH_CHECK(nseg > 0 && nk > 0 && nv % nk == 0, "gdn_step_sliced: sizes");
+    return fb_gdn_step_sliced((int)nseg, (int)rows, (int)max_rows, (int)nk, (int)nv, (int)d) != 0;
+  });
   m.def("quant_fp8", &quant_fp8);
   m.def("gemm_fp8", &gemm_fp8);
   m.def("quant_fp8_block", &quant_fp8_block);

@@ -522,54 +522,74 @@ static int launch_rows(void* out, float* rec_state, void* conv_state, const void
                                  nk, nv, eps, commit, rb, cluster);
 }
 
+// A head in as many slices as a cluster of four holds beside the heads that share a key head (clusters of eight wait for SMs of one GPC: 17
+// rows of 32 heads on 16 took 30 us instead of 13).
+static int step_slices(int nk, int nv, int d) {
+  const int share = nv / nk;
+  return share == 1 && d == 128 ? 4 : (share <= 2 ? 2 : 1);
+}
+
+// Whether a step goes to the kernel of several rows, with heads in slices.
+static bool step_sliced(int nseg, int rows, int max_rows, int nk, int nv, int d) {
+  const int share = nv / nk, split = step_slices(nk, nv, d);
+  if (share > 8) return false;             // (no cluster holds them)
+  // The kernel of several rows pays less for a row and more for a CTA, of which it has `split` times as many, one an SM. us of a wave of CTAs: 4.5 and
+  // 0.35 a row (two slices 0.5, whole heads 5.9 and 0.8), against 2.8 + 1.8 a row of the kernel for single rows; heads of 64: 4.4 + 0.27 (whole 3.9 +
+  // 0.45), 1.9 + 1.2. Clusters of more than four find fewer SMs. A launch is its waves over segments of the mean length and what the longest has
+  // beyond it. One launch in a row of them, us, kernel for single rows / this one, 16 heads: 2 rows 6.4 / 4.8, 17 rows 33.4 / 10.7, 32 rows 60.4 / 15.8,
+  // four times 17 33.6 / 21.0; 8 segments of 2, 5, 17 rows 7.1 / 18.7, 12.6 / 23.5, 34.8 / 41.6, seven of 1 and one of 17 34.1 / 23.8; 24 of 2 22.7 / 58.5.
+  // Single rows whose slices fill a wave and no more: in a row 4.6 / 4.9, 32 heads on 16 4.9 / 5.3; between the other kernels of a step, where the states
+  // come from DRAM, this one is the faster all the same: 771.1 / 770.0 us a step of three such layers of 16 heads, 200.8 / 198.7 of one of 32, two streams.
+  const float mean = (float)rows / nseg, rest = max(0.f, (max_rows > 0 ? min(max_rows, rows - nseg + 1) : ceilf(mean)) - mean);
+  const float fix_new = d == 64 ? (split == 2 ? 4.4f : 3.9f) : split == 1 ? 5.9f : 4.5f, row_old = d == 64 ? 1.2f : 1.8f;
+  const float row_new = d == 64 ? (split == 2 ? 0.27f : 0.45f) : split == 4 ? 0.35f : split == 2 ? 0.5f : 0.8f;
+  const int slots = share * split <= 4 ? STEP_CTAS : 96;
+  const float waves_new = (nv * split * nseg + slots - 1) / slots, waves_old = max(1.f, (float)(nv * nseg) / STEP_CTAS);
+  return (rows == nseg && nv * split >= 64 && nv * split * nseg <= STEP_CTAS) ||
+         waves_new * (fix_new + row_new * mean) + row_new * rest < waves_old * ((d == 64 ? 1.9f : 2.8f) + row_old * mean) + row_old * rest;
+}
+
 template <int D, int PARTS>
 static int launch_step(void* out, float* rec_state, void* conv_state, const void* proj, long proj_stride, const void* conv_w,
                        const float* A_log, const float* dt_bias, const void* gnorm_w, const int* seg_slot, const int* seg_row0,
-                       const int* seg_nrows, int nseg, int rows, int nk, int nv, float eps, int commit, cudaStream_t s) {
+                       const int* seg_nrows, int nseg, int rows, int max_rows, int nk, int nv, float eps, int commit, cudaStream_t s) {
   const int share = nv / nk;
-  // A head in as many slices as a cluster of four holds beside the heads that share a key head (clusters of eight wait for SMs of one GPC: 17
-  // rows of 32 heads on 16 took 30 us instead of 13). Segments of several rows go this way, and single rows whose slices fill a wave of CTAs but no
-  // more. One launch in a row of them, us, kernel for single rows / this one:
-  //   16 heads: 1 row 4.7 / 4.25, 2 rows 6.5 / 4.5, 17 rows 33.5 / 10.2, 32 rows 60.4 / 15.4, four times 17 rows 33.9 / 20.0;
-  //             4 streams of one row 4.7 / 4.8, 24 13.1 (11.3 with two CTAs an SM) / 44
-  //   32 heads on 16: 1 row 4.9 / 5.1 (4.9 without a cluster, whose lack let a head read the conv tail that another had rewritten), 17 rows
-  //             33.7 / 12.8, 4 streams of one row 5.5 / -, 24 28.5 (21.3 with two CTAs an SM) / -
-  // In a model's step the single row of 16 heads saves 4 us a layer (its state comes from DRAM, four times as many CTAs ask for it); the one of 8
-  // heads, whose state is in L2, loses 0.7 to the kernels that start early beside it, and stays.
-  const int split = share == 1 && D == 128 ? 4 : (share <= 2 ? 2 : 1), rb = max(1, min(STEP_ROWS, rows - nseg + 1));
+  const int split = step_slices(nk, nv, D), rb = max(1, min(STEP_ROWS, rows - nseg + 1));
   auto go = [&](auto kern) {
     return kern(out, rec_state, conv_state, proj, proj_stride, conv_w, A_log, dt_bias, gnorm_w, seg_slot, seg_row0, seg_nrows, nseg, rb, nk, nv,
                 eps, commit, s);
   };
-  const bool sliced = rb > 1 || (nv * split >= 64 && nv * split * nseg <= STEP_CTAS);
   const uintptr_t places = reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(conv_w) | reinterpret_cast<uintptr_t>(conv_state);
-  if (sliced && share <= 8 && proj_stride % 8 == 0 && (places & 15) == 0) {
+  if (step_sliced(nseg, rows, max_rows, nk, nv, D) && proj_stride % 8 == 0 && (places & 15) == 0) {
     if constexpr (D == 128)
       if (split == 4) return go(launch_rows<D, D, PARTS, 4>);
     return split == 2 ? go(launch_rows<D, D, PARTS, 2>) : go(launch_rows<D, D, PARTS, 1>);
   }
-  // One row each. (Heads that share a key head in more than eights get no cluster; their q / k tail is rewritten by a launch of its own.)
-  const bool cluster = share > 1 && share <= 8;
+  // One row each. Heads that share a key head are a cluster (0.4 us) while clusters of their size find room at once; their q / k tail is rewritten by a
+  // launch of its own (1.3 us) otherwise: 16 heads on 2, 8 streams, 9.3 as clusters, 6.5 so; 24 streams of 12 heads of 64 on 2 7.2, 5.7.
+  const bool cluster = share > 1 && (share <= 4 || (share <= 8 && nv * nseg <= 96));
   const auto one = cluster ? gdn_step_kernel<D, D, PARTS, true, 1> : gdn_step_kernel<D, D, PARTS, false, 1>;
   const auto two = cluster ? gdn_step_kernel<D, D, PARTS, true, 2> : gdn_step_kernel<D, D, PARTS, false, 2>;
   const cudaError_t e = launch_pdl_cluster(cluster ? share : 1, nv * nseg > STEP_CTAS ? two : one, dim3(nv, nseg), dim3(D * PARTS), (size_t)0, s,
                                            (__nv_bfloat16*)out, rec_state, (__nv_bfloat16*)conv_state, (const __nv_bfloat16*)proj, proj_stride,
                                            (const __nv_bfloat16*)conv_w, A_log, dt_bias, (const __nv_bfloat16*)gnorm_w, seg_slot, seg_row0,
                                            seg_nrows, nk, nv, eps, commit);
-  if (e != cudaSuccess || share <= 8 || !commit) return (int)e;
+  if (e != cudaSuccess || share == 1 || cluster || !commit) return (int)e;
   const int qk = 2 * nk * D;
   return (int)launch_pdl(gdn_qk_tail_kernel, dim3((qk + 255) / 256, nseg), dim3(256), (size_t)0, s, (__nv_bfloat16*)conv_state,
                          (const __nv_bfloat16*)proj, proj_stride, seg_slot, seg_row0, seg_nrows, qk, qk + nv * D);
 }
 
-// `rows`: rows of the step.
+extern "C" int fb_gdn_step_sliced(int nseg, int rows, int max_rows, int nk, int nv, int d) { return step_sliced(nseg, rows, max_rows, nk, nv, d); }
+
+// `rows`: rows of the step; `max_rows`: of its longest segment, 0 where that is not known (it decides on the kernel only).
 extern "C" int fb_gdn_step(void* out, float* rec_state, void* conv_state, const void* proj, long proj_stride,
                            const void* conv_w, const float* A_log, const float* dt_bias, const void* gnorm_w,
-                           const int* seg_slot, const int* seg_row0, const int* seg_nrows, int nseg, int rows, int nk, int nv, int dk,
-                           int dv, float eps, int commit, cudaStream_t s) {
+                           const int* seg_slot, const int* seg_row0, const int* seg_nrows, int nseg, int rows, int max_rows, int nk, int nv,
+                           int dk, int dv, float eps, int commit, cudaStream_t s) {
   if (nseg <= 0) return 0;
   if (nv % nk) return -1;
   if (dk != dv || (dk != 128 && dk != 64)) return -2;
   return (dk == 128 ? launch_step<128, 4> : launch_step<64, 8>)(out, rec_state, conv_state, proj, proj_stride, conv_w, A_log, dt_bias, gnorm_w,
-                                                                 seg_slot, seg_row0, seg_nrows, nseg, rows, nk, nv, eps, commit, s);
+                                                                 seg_slot, seg_row0, seg_nrows, nseg, rows, max_rows, nk, nv, eps, commit, s);
 }

@@ -941,7 +941,7 @@ class Executor:
                         self.verify_proj[i] = proj
                     o = ops.gdn_step(proj, w[p + "conv_w"], self.rec_state[i], self.conv_state[i], w[p + "A_log"],
                                      w[p + "dt_bias"], w[p + "gnorm_w"], mv["sslot"], mv["srow0"], mv["snrows"],
-                                     c.lin_k_heads, c.lin_v_heads, c.lin_dk, c.lin_dv, eps, commit=commit)
+                                     c.lin_k_heads, c.lin_v_heads, c.lin_dk, c.lin_dv, eps, commit=commit, max_rows=max_seg_rows)
                     x = row(o, w[p + "out_proj"], x)
                     if c.is_moe(i):
                         x = self._moe_ffn_sp(x, i, col, row) if sp else self._moe_ffn(x, i)
@@ -1164,7 +1164,7 @@ class Executor:
                 # one launch per layer: the fused step kernel re-runs the kept rows and commits (its outputs are dropped)
                 ops.gdn_step(proj, w[p + "conv_w"], self.rec_state[i], self.conv_state[i], w[p + "A_log"],
                              w[p + "dt_bias"], w[p + "gnorm_w"], mv["sslot"], mv["srow0"], mv["snrows"],
-                             c.lin_k_heads, c.lin_v_heads, c.lin_dk, c.lin_dv, c.eps, commit=True)
+                             c.lin_k_heads, c.lin_v_heads, c.lin_dk, c.lin_dv, c.eps, commit=True, max_rows=self._last_meta[1])
                 continue
             qkv = ops.gdn_conv(proj, w[p + "conv_w"], self.conv_state[i], mv["sslot"], mv["srow0"], mv["snrows"],
                                c.conv_dim, **({"max_rows": mr} if ops.name == "cuda" else {}))
@@ -1212,7 +1212,7 @@ class Executor:
                 if self._replay_fused(mr):
                     ops.gdn_step(proj, w[p + "conv_w"], self.rec_state[i], self.conv_state[i], w[p + "A_log"],
                                  w[p + "dt_bias"], w[p + "gnorm_w"], sslot, srow0, snrows, c.lin_k_heads, c.lin_v_heads,
-                                 c.lin_dk, c.lin_dv, c.eps, commit=True)
+                                 c.lin_dk, c.lin_dv, c.eps, commit=True, max_rows=mr)
                     continue
                 qkv = ops.gdn_conv(proj, w[p + "conv_w"], self.conv_state[i], sslot, srow0, snrows, c.conv_dim,
                                    **({"max_rows": mr} if ops.name == "cuda" else {}))

@@ -708,12 +708,13 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         return cols["x_out"]
 
     def gdn_step(self, proj, conv_w, rec_state, conv_state, A_log, dt_bias, gnorm_w, seg_slot, seg_row0, seg_nrows, nk, nv,
-                 dk, dv, eps, commit=True):
-        """Decode rows: conv + recurrence + gated norm in one launch; returns bf16 [rows, nv * dv]."""
+                 dk, dv, eps, commit=True, max_rows=None):
+        """Decode rows: conv + recurrence + gated norm in one launch; returns bf16 [rows, nv * dv]. `max_rows`: rows of the longest segment, where
+        the caller knows (of two kernels with the same bits the faster one is picked)."""
         out = self.empty(proj.shape[0], nv * dv, dtype=self.dtype, device=self.device)
         self.launches += 1
         self.C.gdn_step(out, rec_state, conv_state, proj, conv_w, A_log, dt_bias, gnorm_w, seg_slot, seg_row0, seg_nrows, nk,
-                        nv, dk, dv, eps, commit)
+                        nv, dk, dv, eps, commit, max_rows or 0)
         return out
 
     def gdn_rec(self, qkv, proj, rec_state, conv_state, A_log, dt_bias, seg_slot, seg_row0, seg_nrows, nk, nv, dk, dv,
