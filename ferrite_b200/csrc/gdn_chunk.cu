@@ -68,30 +68,34 @@ constexpr int GC_VEC = 3 * GC + 4;
 __host__ __device__ constexpr long gc_rec_floats() { return 2l * GC * GC + GC_VEC; }
 
 // ---- prep ------------------------------------------------------------------------------------------------
-// T = (I + A)^{-1} of blocks of 2 w rows from that of their halves: T21 = -T22 (A21 T11). Zeros lie above T11's and T22's diagonals.
+// T = (I + A)^{-1} of blocks of 2 w rows from that of their halves: T21 = -T22 (A21 T11). Zeros lie above T11's and T22's diagonals; above T22's
+// nothing is added, so that a row which is no number reaches no row ahead of it.
 template <int w, int LDA>
 __device__ __forceinline__ void gc_merge(const float* Am, float* Tm, float* Xm) {
   constexpr int PER = w * w / (GC_PREP_THREADS / (GC / 2 / w));         // elements a thread, neighbours in a row: 2 or 4
   constexpr int EACH = w * w / PER;
   const int blk = threadIdx.x / EACH, u = threadIdx.x % EACH, r0 = blk * 2 * w, r = u * PER / w, c = u * PER % w;
   using V = typename std::conditional<PER == 4, float4, float2>::type;
-  auto dot = [&](const float* a, const float* b, float (&acc)[PER]) {
+  // (terms from the last-th on are not added)
+  auto dot = [&](const float* a, const float* b, int last, float (&acc)[PER]) {
 #pragma unroll
     for (int e = 0; e < PER; ++e) acc[e] = 0.f;
-#pragma unroll 8
-    for (int i = 0; i < w; ++i) {
-      const V v = *reinterpret_cast<const V*>(b + i * LDA);
-      const float x = a[i];
+#pragma unroll 1
+    for (int i0 = 0; i0 < last; i0 += 8)
 #pragma unroll
-      for (int e = 0; e < PER; ++e) acc[e] = fmaf(x, reinterpret_cast<const float*>(&v)[e], acc[e]);
-    }
+      for (int i = i0; i < i0 + 8; ++i) {
+        const V v = *reinterpret_cast<const V*>(b + i * LDA);
+        const float x = a[i];
+#pragma unroll
+        for (int e = 0; e < PER; ++e) acc[e] = i < last ? fmaf(x, reinterpret_cast<const float*>(&v)[e], acc[e]) : acc[e];
+      }
   };
   float acc[PER];
-  dot(Am + (r0 + w + r) * LDA + r0, Tm + r0 * LDA + r0 + c, acc);
+  dot(Am + (r0 + w + r) * LDA + r0, Tm + r0 * LDA + r0 + c, w, acc);
 #pragma unroll
   for (int e = 0; e < PER; ++e) Xm[(blk * w + r) * LDA + c + e] = acc[e];
   __syncthreads();
-  dot(Tm + (r0 + w + r) * LDA + r0 + w, Xm + blk * w * LDA + c, acc);
+  dot(Tm + (r0 + w + r) * LDA + r0 + w, Xm + blk * w * LDA + c, r + 1, acc);
 #pragma unroll
   for (int e = 0; e < PER; ++e) Tm[(r0 + w + r) * LDA + r0 + c + e] = -acc[e];
   __syncthreads();
@@ -278,7 +282,8 @@ gdn_chunk_prep_kernel(float* __restrict__ scratch, const __nv_bfloat16* qkv, con
     const int t = i / (GC / 4), c = i % (GC / 4) * 4;
     if (c > (t | 15)) continue;
     const float4 v = *reinterpret_cast<const float4*>(Tm + t * LDA + c);
-    *reinterpret_cast<float4*>(gT + t * GC + c) = make_float4(v.x * bs[c], v.y * bs[c + 1], v.z * bs[c + 2], v.w * bs[c + 3]);
+    *reinterpret_cast<float4*>(gT + t * GC + c) = make_float4(c <= t ? v.x * bs[c] : 0.f, c + 1 <= t ? v.y * bs[c + 1] : 0.f,
+                                                              c + 2 <= t ? v.z * bs[c + 2] : 0.f, c + 3 <= t ? v.w * bs[c + 3] : 0.f);
   }
 }
 
@@ -325,7 +330,9 @@ __device__ __forceinline__ void gc_rows(float (&x)[3][MT][2][4], const __nv_bflo
 }
 
 // out = A M^T for the warp's two tiles of 8 rows of M (32-bit, lower triangular, [GC][LDT]; first w, then 7 - w). A: three terms of [16 MT][LDB]. The
-// later tile needs 16-wide steps 0 .. 2 and for w < 2 also 3, the first 0 and for w >= 2 also 1: four fixed steps and a fifth, without branches.
+// later tile needs 16-wide steps 0 .. 2 and for w < 2 also 3, the first 0 and for w >= 2 also 1: four fixed steps and a fifth, without branches. A tile on
+// an even place ends in the middle of its last step; A's other half is zero there, since M's zeros would let no numbers through (the first row's padding of
+// A holds these zeros). That takes 4 of 124 us of 1500 rows of 32 heads; multiplying 8 wide instead 26.
 template <int MT, int LDT, int LDB>
 __device__ __forceinline__ void gc_triangle(float (&out)[MT][2][4], const __nv_bfloat16* A, const float* M, int w) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
@@ -348,22 +355,30 @@ __device__ __forceinline__ void gc_triangle(float (&out)[MT][2][4], const __nv_b
       gc_mma(acc[2][m], a[m][2], b0[0], b1[0]);
     }
   };
-  auto load = [&](uint32_t (&a)[MT][3][4], int ks) {
+  auto load = [&](uint32_t (&a)[MT][3][4], int ks, bool half) {
+    const bool zero = half && lane >= 16;  // (the lanes that say where the other half's rows lie)
+    const __nv_bfloat16* p = zero ? A + GC : A + (lane & 15) * LDB + ks * 16 + (lane >> 4) * 8;
+    const int next = zero ? 0 : 16 * LDB;
 #pragma unroll
     for (int m = 0; m < MT; ++m)
 #pragma unroll
-      for (int i = 0; i < 3; ++i) gc_ldsm(a[m][i], A + ((i * MT + m) * 16 + (lane & 15)) * LDB + ks * 16 + (lane >> 4) * 8);
+      for (int i = 0; i < 3; ++i) gc_ldsm(a[m][i], p + (i * MT + m) * next);
   };
   const bool late = w < 2;
 #pragma unroll
   for (int ks = 0; ks < 3; ++ks) {
     uint32_t a[MT][3][4];
-    load(a, ks);
+    load(a, ks, ks == 2 && w == 3);
     step(x[1], a, 7 - w, ks);
-    if (ks == 0) step(x[0], a, w, 0);
+    if (ks > 0) continue;
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int i = 0; i < 3; ++i) { a[m][i][2] = w ? a[m][i][2] : 0u; a[m][i][3] = w ? a[m][i][3] : 0u; }
+    step(x[0], a, w, 0);
   }
   uint32_t a[MT][3][4];
-  load(a, late ? 3 : 1);
+  load(a, late ? 3 : 1, w == 1 || w == 2);
   step(x[2], a, late ? 7 - w : w, late ? 3 : 1);
 #pragma unroll
   for (int m = 0; m < MT; ++m)
@@ -401,6 +416,7 @@ gdn_chunk_scan_kernel(float* __restrict__ y, float* __restrict__ rec_state, __nv
   const int q_off = kh * DK, k_off = nk * DK + kh * DK, v_off = 2 * nk * DK + h * dv + slice * W;
   float* Sg = rec_state + (((size_t)slot * nv + h) * DK) * dv + slice * W;
   const int nchunks = (n + GC - 1) / GC;
+  if (tid < 2) *reinterpret_cast<uint4*>((tid ? Ds : Bs) + GC) = make_uint4(0u, 0u, 0u, 0u);      // see gc_triangle
 
   if (role == 2) {                         // loads, a chunk ahead
     const int u = tid & 127;

@@ -240,6 +240,28 @@ def test_gdn_chunked_scan_against_64_bits(ops, nk, nv, dv, ns, decay, commit):
     assert torch.equal(conv, want_conv)
 
 
+@pytest.mark.parametrize("what", ["k", "v", "decay", "beta"])
+@pytest.mark.parametrize("row", [3, 21, 50, 63, 100])
+def test_gdn_chunked_scan_with_a_row_that_is_no_number(ops, what, row):
+    """A NaN in one row's key, value, decay or beta leaves the rows ahead of its eight alone, bit for bit, and the other heads."""
+    nk, nv, d, n = 2, 2, 128, 130
+    conv_dim = 2 * nk * d + nv * d
+    A_log, dtb = torch.zeros(nv, device=DEV), torch.zeros(nv, device=DEV)
+    i32 = lambda v: torch.tensor([v], device=DEV, dtype=torch.int32)
+    ys = []
+    for bad in (False, True):
+        qkv = torch.nn.functional.silu(rnd(n, conv_dim, seed=1).float()).to(torch.bfloat16)
+        proj = rnd(n, conv_dim + nv * d + 2 * nv, seed=2)
+        if bad:
+            to, at = {"k": (qkv, nk * d + 5), "v": (qkv, 2 * nk * d + 5), "decay": (proj, conv_dim + nv * d + nv), "beta": (proj, conv_dim + nv * d)}[what]
+            to[row, at] = float("nan")
+        rec, conv = rnd(1, nv, d, d, scale=0.2, seed=3, dtype=torch.float32), rnd(1, 3, conv_dim, seed=4)
+        ys.append(ops.gdn_rec(qkv, proj, rec, conv, A_log, dtb, i32(0), i32(0), i32(n), nk, nv, d, d, 1e-6, commit=True, chunked=True))
+    ahead = row // 8 * 8
+    assert torch.equal(ys[0][:ahead], ys[1][:ahead]) and torch.equal(ys[0][:, d:], ys[1][:, d:])
+    assert ys[1][row, :d].isnan().any()
+
+
 @pytest.mark.parametrize("nk,nv,d,streams,T,wide", [
     (16, 16, 128, 1, 2, 0), (4, 4, 128, 3, 17, 0), (2, 4, 128, 2, 32, 0), (2, 4, 128, 1, 33, 0), (2, 8, 128, 2, 5, 0), (1, 8, 128, 1, 70, 0),
     (4, 4, 64, 2, 9, 0), (2, 8, 64, 2, 33, 0), (1, 9, 64, 1, 3, 0), (16, 16, 128, 2, 1, 0), (16, 16, 128, 10, 1, 0), (2, 8, 128, 24, 1, 0),
