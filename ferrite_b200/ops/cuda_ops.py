@@ -106,14 +106,16 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
     def _gemm_scratch(self, M: int, N: int, split: int):
         """Workspace and counters of a GEMM call: K splits of few rows, or (split < 0: normal orientation) the last tiles' pieces. The latter belong to the
         current stream, so that a call has the same bits on every one; up to TAIL_STREAMS of them keep theirs (20 MB each: the one that asked
-        first gives its own back to the allocator, in whose order of that stream it is used again). A capture takes buffers of its own."""
+        first gives its own back to the allocator, in whose order of that stream it is used again). A capture takes buffers of its own, but for the
+        steps that the engine captures (up to 64 rows), whose products share what all of its few-row kernels share: every call leaves the
+        counters zero. (Buffers of their own and a fill in front of each product: 20 MB a graph.)"""
         if split >= 0:
             return (self._workspace(self.C.gemm_workspace_bytes(M, N, split)), self._counters) if split > 1 else (None, None)
-        M = max(M, 65)
-        make = lambda: (torch.empty(self.C.gemm_workspace_bytes(M, N, 1) // 4, dtype=torch.float32, device=self.device),
-                        torch.zeros(self.C.gemm_counters(M, N, 1), dtype=torch.int32, device=self.device))
+        rows = max(M, 65)
+        make = lambda: (torch.empty(self.C.gemm_workspace_bytes(rows, N, 1) // 4, dtype=torch.float32, device=self.device),
+                        torch.zeros(self.C.gemm_counters(rows, N, 1), dtype=torch.int32, device=self.device))
         if torch.cuda.is_current_stream_capturing():
-            return make()
+            return (self._workspace(self.C.gemm_workspace_bytes(rows, N, 1)), self._counters) if M <= 64 else make()
         stream = torch.cuda.current_stream(self.device).cuda_stream
         held = self._tails.get(stream)
         if held is None:

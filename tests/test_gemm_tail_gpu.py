@@ -125,6 +125,32 @@ def test_pieces_on_many_streams_and_under_capture(ext):
     assert ops._tails.keys() == held.keys() and ops.status() == 0
 
 
+@pytest.mark.parametrize("M", [33, 64])
+def test_captured_products_of_up_to_64_rows_share_their_scratch(ext, M, monkeypatch):
+    """What a captured step holds: outputs and kernels, no scratch and no fill of a product's own; the bits of the eager call."""
+    from ferrite_b200.ops.cuda_ops import CudaOps
+    ops, N, K = CudaOps(DEV), 1000, 8192
+    x, w = rnd(M, K, seed=1), rnd(N, K, seed=2, scale=K ** -0.5)
+    wq, ws = ops.quantize_weight_fp8(w)
+    want = ops.linear(x, w, out_f32=True), ops.linear_fp8(x, wq, ws)
+    torch.cuda.synchronize()
+    graph, made = torch.cuda.CUDAGraph(), []
+    zeros = torch.zeros
+    with torch.cuda.graph(graph):
+        monkeypatch.setattr(torch, "zeros", lambda *a, **k: made.append(a) or zeros(*a, **k))
+        got = [(ops.linear(x, w, out_f32=True), ops.linear_fp8(x, wq, ws)) for _ in range(4)]
+        monkeypatch.undo()
+    assert not made
+    for _ in range(2):
+        for pair in got:
+            for t in pair:
+                t.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for pair in got for a, b in zip(pair, want))
+    assert ops.status() == 0 and int(ops._counters.count_nonzero()) == 0
+
+
 @pytest.mark.parametrize("N", [24, 100])
 def test_output_on_no_16_bytes(ops, N):
     M, K = 130, 256
