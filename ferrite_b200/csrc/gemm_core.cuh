@@ -93,8 +93,9 @@ struct GemmArgs {
   int stages;
   int split_k;
   int tiles_a, tiles_b;     // tile counts along the A-row and B-row dimensions
-  int acc_cols;             // TMEM columns per accumulator buffer (n_a * bn)
-  int tmem_cols;            // allocated columns (power of two >= 2 * acc_cols)
+  int acc_cols;             // TMEM columns per accumulator (n_a * bn)
+  int chains;               // accumulators that share a work item's k blocks, side by side in a buffer; the epilogue adds them up (see plan_gemm)
+  int tmem_cols;            // allocated columns: a power of two, two buffers where a CTA has more than one work item
   // plain normal orientation: tiles from tail_first on (fewer than the CTAs) are cut along K into tail_split pieces of tail_kb k blocks
   int tail_first, tail_tiles, tail_split, tail_kb;
 };
@@ -347,8 +348,10 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         k_range(w, ks, kb0, kb1);
         if (!mbar_wait_or_flag(&tempty_bar[buf], tphase[buf] ^ 1u, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d0 = tmem_base + (uint32_t)(buf * a.acc_cols);
-        for (int kb = kb0; kb < kb1; ++kb) {
+        uint32_t d0 = tmem_base + (uint32_t)(buf * a.acc_cols * a.chains);
+        const int chain = (kb1 - kb0 + a.chains - 1) / a.chains;
+        for (int kb = kb0, at = 0; kb < kb1; ++kb, ++at) {
+          if (at == chain) { at = 0; d0 += (uint32_t)a.acc_cols; }
           if (!mbar_wait_or_flag(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sa = smem_u32(tiles + (size_t)stage * stage_bytes);
@@ -360,10 +363,10 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             for (int k = 0; k < GM_BK / 16; ++k)
               if (a.fp8)
                 tc_mma_f8f6f4(d0 + (uint32_t)(i * a.bn), da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc,
-                              (kb > kb0 || k > 0) ? 1u : 0u);
+                              (at > 0 || k > 0) ? 1u : 0u);
               else
                 tc_mma_f16(d0 + (uint32_t)(i * a.bn), da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc,
-                           (kb > kb0 || k > 0) ? 1u : 0u);
+                           (at > 0 || k > 0) ? 1u : 0u);
           }
           tc_commit(&empty_bar[stage]);               // frees the smem slot once these MMAs have read it
           if (++stage == a.stages) { stage = 0; phase ^= 1u; }
@@ -400,7 +403,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       if (!ok) break;
       tphase[buf] ^= 1u;
       tc_fence_after();
-      const uint32_t tbase = tmem_base + (uint32_t)(buf * a.acc_cols) + ((uint32_t)(quad * 32) << 16);
+      const uint32_t tbase = tmem_base + (uint32_t)(buf * a.acc_cols * a.chains) + ((uint32_t)(quad * 32) << 16);
       if constexpr (COMM == 1) {
         // Reduce-scatter epilogue (normal orientation, lanes = token rows). Rows owned by other ranks: bf16 partials
         // go through this warp's transpose buffer and leave as 256-byte row pieces for the owner's staging slot of
@@ -542,6 +545,24 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         const uint32_t stage_w = smem_u32(tiles + (size_t)a.stages * stage_bytes + (size_t)quad * GM_EPI_BYTES);
         const int rr = lane >> 2, rc = (lane & 3) * 8;    // bf16 output: row of a group of 8, column of the 32
         const bool wide = (((uintptr_t)a.Y | (uintptr_t)a.res) & 15) == 0;
+        // 32 columns of the item's sums
+        int chains = 1;
+        if (COMM == 0 && a.chains > 1) {
+          int kb0, kb1;
+          k_range(w, ks, kb0, kb1);
+          const int chain = (kb1 - kb0 + a.chains - 1) / a.chains;
+          chains = (kb1 - kb0 + chain - 1) / chain;
+        }
+        auto more_chains = [&](int col, uint32_t (&r)[32]) {
+#pragma unroll 1
+          for (int i = 1; i < chains; ++i) {
+            uint32_t o[32];
+            tmem_ld32(tbase + (uint32_t)(i * a.acc_cols + col), o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(o[j]));
+          }
+        };
         // A piece of a tile (tail of the tile list): 64 accumulator columns at a time go to the workspace as fp32, and the warp that brings a
         // block's last piece sums the pieces in their order and finishes it. The pieces begin at different columns, which spreads the sums over
         // the CTAs; nobody waits.
@@ -560,6 +581,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
               uint32_t r[32];
               tmem_ld32(tbase + (uint32_t)col, r);
               tmem_ld_wait();
+              more_chains(col, r);
               float4* dst = wsp + ks * ws_piece + (size_t)(col / 32) * 1024;
 #pragma unroll
               for (int q = 0; q < 8; ++q)
@@ -614,6 +636,8 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             tmem_ld32(tbase + (uint32_t)c, r0);
             if (a.dual) tmem_ld32(tbase + (uint32_t)(c + a.bn / 2), r1);
             tmem_ld_wait();
+            more_chains(c, r0);
+            if (a.dual) more_chains(c + a.bn / 2, r1);
           }
           // (straight runs of 32 under one test each: a test per element made a lone warp's 32 columns cost 2.7 us)
           float v[32];
@@ -873,6 +897,12 @@ constexpr long GM_TAIL_BYTES = 148L * GM_BM * 256 * (long)sizeof(float);
 constexpr int GM_TAIL_CTRS = 148 * GM_TILE_CTRS;
 inline long gemm_tail_need(const GemmArgs& a) { return (long)a.tail_tiles * a.tail_split * GM_BM * a.bn * (long)sizeof(float); }
 
+// K splits of a product whose rows are the narrow side: work items for every SM, four k blocks each at least.
+inline int gemm_splits(int N, int kblocks, int sm_count) {
+  const int tiles = (N + GM_BM - 1) / GM_BM, want = (sm_count + tiles - 1) / tiles;
+  return max(1, min(kblocks / 4, want));
+}
+
 // Normal orientation, tile width and tail (tail = 1: widths only; 2: the last tiles may be cut along K, workspace and counters are there). A k block
 // of a tile takes 0.26 us + 0.00066 us a column with every SM at work (L2 to shared memory, 50 to 56 bytes a clock and SM, and from 192 columns on
 // the tensor cores close to what the power limit sustains): cost bn + GM_KB_COST per k block and wave. What a fixed width of 256 lost is the last
@@ -882,12 +912,15 @@ inline long gemm_tail_need(const GemmArgs& a) { return (long)a.tail_tiles * a.ta
 // us, width 256 / best width / with pieces: 2048 x 5120 x 17408 348 / 319 / 288, 1111 rows of it 255 / 210 / 177, 300 rows 135 / 104 / 82, 140 rows
 // 128 / 100 / 66; 2048 x 5120 x 2048 53 / 47 / 55 (whole), 140 x 2048 x 4096 38 / 30 / 21. More than four pieces gained nothing.
 // Up to 64 rows are the narrow side of the product (weights on the tensor cores' 128 lanes) and K is cut into split_k, unless split_k < 0 asks for the
-// orientation of more rows.
+// orientation of more rows. Its sums are then no longer than those of these K splits were: the tensor cores cut each sum to the accumulator's scale, an
+// error that grows with the length of the chain (1.0e-6 of 2048 x 4096 in pieces alone, 0.4e-6 so), so that a work item's k blocks go to several
+// accumulators where the pieces are too few.
 static int plan_gemm(GemmPlan& p, int M, int N, int K, int mode, int split_k, int sm_count, int fp8 = 0, int tail = 0) {
   GemmArgs& a = p.a;
   a.fp8 = fp8; a.scale_m = nullptr; a.scale_n = nullptr; a.out_f32 = 0; a.act = ACT_NONE; a.limit = 0.f;
   a.M = M; a.N = N; a.K = K;
   a.dual = mode == 1;
+  a.chains = 1;
   a.swap = M <= 64 && split_k >= 0;
   if (a.swap) {
     a.bn = ((M + 15) / 16) * 16;
@@ -903,6 +936,7 @@ static int plan_gemm(GemmPlan& p, int M, int N, int K, int mode, int split_k, in
     if (tail) {
       const int kb = (K + (fp8 ? 2 * GM_BK : GM_BK) - 1) / (fp8 ? 2 * GM_BK : GM_BK);
       long best = -1;
+      const int longest = M > 64 ? kb : (kb + gemm_splits(N, kb, sm_count) - 1) / gemm_splits(N, kb, sm_count);
       for (int bn = 256; bn >= 64; bn -= a.dual ? 64 : 32) {
         const int cols = a.dual ? bn / 2 : bn;
         const long tiles = (long)((M + GM_BM - 1) / GM_BM) * ((N + cols - 1) / cols);
@@ -910,11 +944,14 @@ static int plan_gemm(GemmPlan& p, int M, int N, int K, int mode, int split_k, in
         const long full = tiles / sm_count * kb * (bn + GM_KB_COST);
         for (int s = 1; s <= GM_TAIL_MAX; ++s) {
           if (s > 1 && (tail < 2 || rest * s > sm_count || kb / s < 4)) break;
-          const int per = (kb + s - 1) / s;
+          const int per = (kb + s - 1) / s, item = tiles < sm_count ? per : kb;      // (the whole tiles' items are the longest)
+          const int chains = (item + longest - 1) / longest;
+          if (chains > 1 && (tiles * s <= sm_count ? 1 : 2) * bn * chains > 512) continue;
           const long cost = full + (rest ? (long)per * (bn + GM_KB_COST) + (s > 1 ? bn * (GM_TAIL_COST + s * GM_PIECE_COST) : 0) : 0);
-          if (best < 0 || cost < best) { best = cost; a.bn = bn; a.tail_split = (kb + per - 1) / per; a.tail_tiles = a.tail_split > 1 ? rest : 0; a.tail_kb = per; }
+          if (best < 0 || cost < best) { best = cost; a.bn = bn; a.tail_split = (kb + per - 1) / per; a.tail_tiles = a.tail_split > 1 ? rest : 0; a.tail_kb = per; a.chains = chains; }
         }
       }
+      if (best < 0) { a.bn = 64; a.tail_tiles = 0; a.chains = 4; }              // (no scratch for pieces: as many as there is room for)
     }
     a.n_a = 1;
     a.n_b = a.dual ? 2 : 1;
@@ -933,8 +970,6 @@ static int plan_gemm(GemmPlan& p, int M, int N, int K, int mode, int split_k, in
     a.split_k = (kblocks + per - 1) / per;
   }
   a.acc_cols = a.n_a * a.bn;
-  a.tmem_cols = round_up_pow2(2 * a.acc_cols);
-  if (a.tmem_cols > 512) return -4;
   int b_bytes = a.n_b * a.b_box_rows * GM_BK * 2;
   int stage_bytes = a.n_a * GM_A_BYTES + ((b_bytes + 1023) & ~1023);
   int budget = 200 * 1024;
@@ -949,6 +984,8 @@ static int plan_gemm(GemmPlan& p, int M, int N, int K, int mode, int split_k, in
   if (a.tail_tiles == 0) { a.tail_first = 0x7fffffff; a.tail_split = 1; }
   total += a.tail_tiles * (a.tail_split - 1);
   p.grid = total < sm_count ? total : sm_count;
+  a.tmem_cols = round_up_pow2((a.chains > 1 && total <= p.grid ? 1 : 2) * a.acc_cols * a.chains);
+  if (a.tmem_cols > 512) return -4;
   return 0;
 }
 

@@ -202,6 +202,12 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         s = max(1, min(kblocks // 4, want))
         return s
 
+    @staticmethod
+    def _narrow(M, y, split):
+        """Whether a GEMM's rows are the narrow side of the product. (Up to 64 rows the other orientation cuts sums as often as these splits do: four
+        pieces and eight accumulators at most.)"""
+        return M <= GEMM_SWAP_ROWS or (M <= 64 and (y.stride(0) % 8 != 0 or split > 32))
+
     def relu2(self, x):
         y = self.empty(x.shape[0], x.shape[1], dtype=self.dtype, device=self.device)
         self.launches += 1
@@ -308,7 +314,8 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         # the wide-M epilogue stores 16-byte row pieces: give odd widths a padded leading dimension
         y = out if out is not None else self.empty(M, (N + 7) // 8 * 8, dtype=torch.float32 if out_f32 else self.dtype,
                                                     device=self.device)[:, :N]
-        split = self._split_k(M, N, K) if M <= (64 if y.stride(0) % 8 else GEMM_SWAP_ROWS) else -1
+        split = self._split_k(M, N, K)
+        split = split if self._narrow(M, y, split) else -1
         ws, cnt = self._gemm_scratch(M, N, split)
         self.launches += 1
         self.C.gemm(y, x, w, res, (1 if swiglu else 0) | (2 if out_f32 else 0) | (4 if act else 0), split, ws, cnt, self.status_word)
@@ -347,7 +354,8 @@ class CudaOps(CudaLatent, CudaMixers, CudaExtras):
         xs = self.empty(M, dtype=torch.float32, device=self.device)
         self.C.quant_fp8(xq, xs, x, norm_w, eps)
         y = self.empty(M, (N + 7) // 8 * 8, dtype=self.dtype, device=self.device)[:, :N]
-        split = self._split_k(M, N, K // 2) if M <= (64 if y.stride(0) % 8 else GEMM_SWAP_ROWS) else -1
+        split = self._split_k(M, N, K // 2)
+        split = split if self._narrow(M, y, split) else -1
         ws, cnt = self._gemm_scratch(M, N, split)
         self.launches += 2
         self.C.gemm_fp8(y, xq, wq, xs, w_scale, res, 1 if swiglu else 0, split, ws, cnt, self.status_word)

@@ -81,6 +81,26 @@ def test_33_to_64_rows_on_either_side(ops, M, N, K, width, swiglu):
     assert ops.status() == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(33, 8224, 5120), (64, 5120, 2048), (64, 2048, 4096), (48, 24, 4096), (40, 640, 8192), (64, 1111, 1032), (50, 17408, 2048),
+                                   (64, 20000, 1024), (36, 256, 16384)])
+def test_sums_of_33_to_64_rows_are_as_exact_as_in_k_splits(ops, M, N, K):
+    """Rows in tiles of 128 against the same rows as the narrow side of the product, K cut into splits: no further off 64 bits (5 % for the sums' chance;
+    chains as long as K, or as a piece of it, are 1.5 to 2.5 times as far off)."""
+    x, w = rnd(M, K, seed=1), rnd(N, K, seed=2, scale=K ** -0.5)
+    want = x.double() @ w.double().t()
+    split = ops._split_k(M, N, K)
+    y = torch.empty(M, (N + 7) // 8 * 8, device=DEV)[:, :N]
+    ws = (torch.empty(ops.C.gemm_workspace_bytes(M, N, split) // 4, device=DEV), torch.zeros(4096, dtype=torch.int32, device=DEV)) if split > 1 else (None, None)
+    ops.C.gemm(y, x, w, None, 2, split, *ws, ops.status_word)
+    off = lambda t: ((t.double() - want).norm() / want.norm()).item()
+    assert off(ops.linear(x, w, out_f32=True)) <= 1.05 * off(y)
+    if split <= 8:                                                                   # without scratch: as many sums as there is room for
+        bare = torch.empty(M, (N + 7) // 8 * 8, device=DEV)[:, :N]
+        ops.C.gemm(bare, x, w, None, 2, -1, None, None, ops.status_word)
+        assert off(bare) <= 1.05 * off(y)
+    assert ops.status() == 0
+
+
 def test_scratch_that_is_too_small_takes_no_pieces(ops):
     """Scratch of any size may come with a call: pieces are taken where they fit it, and nothing past its end is written."""
     M, N, K = 300, 1111, 8192
