@@ -19,9 +19,8 @@
 namespace fb {
 
 constexpr int MLA_WARPS = 4;
-constexpr int MLA_PREP_HEADS = 16;
 
-// grid (rows, 1 + groups of MLA_PREP_HEADS heads), 256 threads; y = 0: the cache row, else the heads' query parts (with a CTA a row, six rows of 128
+// grid (rows, 1 + groups of `per` heads), 256 threads; y = 0: the cache row, else the heads' query parts (with a CTA a row, six rows of 128
 // heads took 12.3 us). kva: [rows][L + R]; q: [rows][nq][dn + R]; qabs: [rows][nq][L + R] (rope tail written here)
 __global__ void __launch_bounds__(256) mla_prep_kernel(__nv_bfloat16* __restrict__ cache, __nv_bfloat16* __restrict__ qabs,
                                                        const __nv_bfloat16* kva, long kva_stride,
@@ -30,7 +29,7 @@ __global__ void __launch_bounds__(256) mla_prep_kernel(__nv_bfloat16* __restrict
                                                        const float* __restrict__ inv_freq, const int* row_slot,
                                                        const int* row_pos, const int* block_table,
                                                        int max_blocks, int kv_block, int nq, int dn, int L, int R,
-                                                       float eps, int* status) {
+                                                       float eps, int* status, int per) {
   __shared__ float red[32];
   const int row = blockIdx.x, tid = threadIdx.x, half = R / 2;
   pdl_launch_dependents();
@@ -40,18 +39,19 @@ __global__ void __launch_bounds__(256) mla_prep_kernel(__nv_bfloat16* __restrict
   const int blk = after_wait(block_table)[(size_t)slot * max_blocks + pos / kv_block];
   if (blk < 0) { if (tid == 0 && blockIdx.y == 0) set_status(status, ST_BOUNDS); return; }
   // pair (i, i + R/2) turned by the row's angle
-  auto rotate = [&](__nv_bfloat16* to, const __nv_bfloat16* from, int i) {
-    float s, c;
-    sincosf((float)pos * inv_freq[i], &s, &c);
+  auto rotate = [&](__nv_bfloat16* to, const __nv_bfloat16* from, int i, float s, float c) {
     const float a = bf2f(from[i]), b = bf2f(from[half + i]);
     to[i] = f2bf(a * c - b * s);
     to[half + i] = f2bf(b * c + a * s);
   };
   if (blockIdx.y > 0) {
-    const int h0 = (blockIdx.y - 1) * MLA_PREP_HEADS, n = min(MLA_PREP_HEADS, nq - h0) * half;
-    for (int idx = tid; idx < n; idx += blockDim.x) {
-      const int h = h0 + idx / half;
-      rotate(qabs + ((size_t)row * nq + h) * (L + R) + L, q + (size_t)row * q_stride + (size_t)h * (dn + R) + dn, idx % half);
+    const int step = max((int)blockDim.x / half, 1);       // heads side by side; a thread's angle is the same for all of its heads
+    if (tid >= step * half) return;
+    for (int i = tid % half; i < half; i += blockDim.x) {
+      float s, c;
+      sincosf((float)pos * inv_freq[i], &s, &c);
+      for (int h = (blockIdx.y - 1) * per + tid / half; h < min((int)blockIdx.y * per, nq); h += step)
+        rotate(qabs + ((size_t)row * nq + h) * (L + R) + L, q + (size_t)row * q_stride + (size_t)h * (dn + R) + dn, i, s, c);
     }
     return;
   }
@@ -62,7 +62,11 @@ __global__ void __launch_bounds__(256) mla_prep_kernel(__nv_bfloat16* __restrict
   ss = block_sum(ss, red);
   const float r = rsqrtf(ss / (float)L + eps);
   for (int i = tid; i < L; i += blockDim.x) crow[i] = f2bf(bf2f(kr[i]) * r * (1.f + bf2f(norm_w[i])));
-  for (int i = tid; i < half; i += blockDim.x) rotate(crow + L, kr + L, i);
+  for (int i = tid; i < half; i += blockDim.x) {
+    float s, c;
+    sincosf((float)pos * inv_freq[i], &s, &c);
+    rotate(crow + L, kr + L, i, s, c);
+  }
 }
 
 // grid (rows, nq, nsplit); D = L + R must be a multiple of 64 with D / 64 <= 9, L a multiple of 64
@@ -234,9 +238,12 @@ extern "C" int fb_mla_prep(void* cache, void* qabs, const void* kva, long kva_st
                            float eps, int* status, cudaStream_t s) {
   if (rows <= 0) return 0;
   if (R % 2) return -1;
-  return (int)launch_pdl(mla_prep_kernel, dim3(rows, 1 + (nq + MLA_PREP_HEADS - 1) / MLA_PREP_HEADS), dim3(256), (size_t)0, s, (__nv_bfloat16*)cache,
+  // heads a CTA: 16 as long as an SM's eight CTAs hold the rows, else 64, which repeat an angle less often. us, a CTA a row / 16 / 64: 64 rows of 128 heads
+  // 13.0 / 5.1 / 6.6, 600 rows 20 / 17 / 12.8, 2048 rows 45 / 52 / 33; of 64 heads 27 / 30 / 21
+  const int per = (long)rows * (1 + (nq + 15) / 16) <= 8 * 148 ? 16 : 64;
+  return (int)launch_pdl(mla_prep_kernel, dim3(rows, 1 + (nq + per - 1) / per), dim3(256), (size_t)0, s, (__nv_bfloat16*)cache,
                          (__nv_bfloat16*)qabs, (const __nv_bfloat16*)kva, kva_stride, (const __nv_bfloat16*)q, q_stride,
-                         (const __nv_bfloat16*)norm_w, inv_freq, row_slot, row_pos, block_table, max_blocks, kv_block, nq, dn, L, R, eps, status);
+                         (const __nv_bfloat16*)norm_w, inv_freq, row_slot, row_pos, block_table, max_blocks, kv_block, nq, dn, L, R, eps, status, per);
 }
 
 // o_part: rows * nq * nsplit * L floats, ml_part: rows * nq * nsplit * 2 floats

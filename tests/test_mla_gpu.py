@@ -252,3 +252,29 @@ def test_mla_engine_gpu(ext):
     kl = torch.nn.functional.kl_div(torch.log_softmax(got, -1), torch.log_softmax(want, -1), log_target=True,
                                     reduction="batchmean").item()
     assert kl < 2e-2, kl
+
+
+@pytest.mark.parametrize("nq,R", [(70, 64), (128, 40), (5, 2)])
+def test_mla_prep_of_many_rows(ops, nq, R):
+    """Rows in one call (a CTA takes up to 64 heads of many rows) have the bits of the same rows in calls of few (16 heads), in the queries' rope parts and
+    in the cache, and are what 64 bits give but for the angle's and the result's roundings."""
+    L, dn, kvb, rows = 64, 24, 64, 600
+    g = torch.Generator(device=DEV).manual_seed(nq)
+    r = lambda *s: torch.randn(*s, generator=g, device=DEV).to(torch.bfloat16)
+    q, kva, norm_w = r(rows, nq * (dn + R)), r(rows, L + R), r(L)
+    inv = (1e4 ** (-torch.arange(R // 2, dtype=torch.float64) / (R // 2))).float().to(DEV)
+    pos, slot = torch.arange(rows, device=DEV, dtype=torch.int32), torch.zeros(rows, device=DEV, dtype=torch.int32)
+    bt = torch.arange((rows + kvb - 1) // kvb, device=DEV, dtype=torch.int32).view(1, -1)
+    caches = [torch.zeros(bt.numel(), kvb, L + R, device=DEV, dtype=torch.bfloat16) for _ in range(2)]
+    call = lambda a, b, cache: ops.mla_prep(q[a:b], kva[a:b], norm_w, None, inv, slot[a:b], pos[a:b], bt, cache, kvb, nq, dn, L, R, 1e-6, absorb=False)[:, :, L:]
+    got = call(0, rows, caches[0])
+    assert torch.equal(got, torch.cat([call(a, min(a + 90, rows), caches[1]) for a in range(0, rows, 90)]))
+    assert torch.equal(caches[0], caches[1])
+    turn = torch.exp(1j * pos.double()[:, None, None] * inv.double())
+    v = q.double().view(rows, nq, dn + R)[:, :, dn:]
+    want = torch.complex(v[..., :R // 2], v[..., R // 2:]) * turn
+    want = torch.cat([want.real, want.imag], -1)
+    # the angle is rounded once (2^-24 of up to 600), a result to bf16 (2^-9 of it), products and sums to 32 bits
+    size = torch.cat([torch.complex(v[..., :R // 2], v[..., R // 2:]).abs()] * 2, -1)
+    assert bool(((got.double() - want).abs() <= 2 ** -8 * want.abs() + (600 * 2 ** -23 + 2 ** -20) * size).all())
+    assert ops.status() == 0
