@@ -319,6 +319,30 @@ def test_gdn_step_operands_at_odd_places(ops, what, T):
     assert ops.status() == 0
 
 
+@pytest.mark.parametrize("share", [3, 5, 6, 7, 8])
+@pytest.mark.parametrize("streams,T", [(1, 1), (1, 6), (2, 17), (30, 1), (30, 2)])
+def test_gdn_step_with_three_to_eight_heads_to_a_key_head(ops, share, streams, T):
+    """Heads that share a key head (one cluster of them, or CTAs by themselves where those find no room at once) give the bits of heads that each have the
+    same key head to themselves, in outputs, states and conv tails."""
+    nk, d, dv = 2, 128, 128
+    nv = nk * share
+    proj = rnd(streams * T, (2 * nk + 2 * nv) * d + 2 * nv, seed=1)
+    conv_w, conv = rnd((2 * nk + nv) * d, 4, scale=0.5, seed=2), rnd(streams, 3, (2 * nk + nv) * d, seed=7)
+    A_log, dtb = rnd(nv, scale=0.3, seed=3, dtype=torch.float32), rnd(nv, scale=0.3, seed=4, dtype=torch.float32)
+    gw, rec = (rnd(d, scale=0.1, seed=5).float() + 1).to(torch.bfloat16), rnd(streams, nv, d, d, scale=0.2, seed=6, dtype=torch.float32)
+    i32 = lambda v: torch.tensor(list(v), device=DEV, dtype=torch.int32)
+    heads = [h * d + i for part in (0, nk) for h in (part + v // share for v in range(nv)) for i in range(d)]
+    own = torch.tensor(heads, device=DEV)                                    # q and k channels with a key head for every head
+    spread = lambda t: torch.cat([t[..., own], t[..., 2 * nk * d:]], -1).contiguous()
+    sides = []
+    for n, p, w, c in ((nk, proj, conv_w, conv), (nv, spread(proj), spread(conv_w.t()).t().contiguous(), spread(conv))):
+        c, r = c.clone(), rec.clone()
+        y = ops.gdn_step(p, w, r, c, A_log, dtb, gw, i32(range(streams)), i32(range(0, streams * T, T)), i32([T] * streams), n, nv, d, dv, 1e-6)
+        sides.append((y, r, c if n == nv else spread(c)))
+    assert all(torch.equal(a, b) for a, b in zip(*sides))
+    assert ops.status() == 0
+
+
 @pytest.mark.parametrize("nk,nv,d", [(2, 18, 128), (2, 32, 64), (1, 40, 64)])
 @pytest.mark.parametrize("T", [1, 2, 5])
 def test_gdn_step_with_many_heads_to_a_key_head(ops, nk, nv, d, T):
