@@ -258,6 +258,13 @@ def test_prompt_experts_from_their_codes(ops, E, K, H, I, T, limit):
     ep.check()
 
 
+@pytest.mark.parametrize("T", [32, 33, 63, 64, 128, 129])
+def test_prompt_experts_at_the_edges_of_an_item(ops, T):
+    """An item is up to 64 rows of an expert, which come in halves of 32: T rows, all of them on the first expert's list, end on either edge and
+    one row beyond it."""
+    test_prompt_experts_from_their_codes(ops, 16, 4, 512, 256, T, 0.0)
+
+
 def test_prompt_experts_with_a_nan_scale(ops):
     """A NaN scale in one expert's down projection reaches the rows that picked this expert, in one column, and no others."""
     from ferrite_b200.ops.qweight import ExpertsFP4
