@@ -191,3 +191,20 @@ def test_scaled_fp8(ops, M, N, K):
     # tensor cores add e4m3 products in 32 bits or a little less; then one rounding to bf16
     got = ops.linear_fp8(x, wq, ws).double()
     assert ((got - want).abs() <= 2 ** -8 * want.abs() + 2 ** -9).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(33, 264, 1040), (48, 5120, 2048), (64, 2048, 8208), (50, 17408, 1024)])
+def test_scaled_fp8_of_33_to_64_rows(ops, M, N, K):
+    """e4m3 rows in tiles of 128, and as the narrow side of the product, against 64 bits."""
+    x, w = rnd(M, K, seed=1), rnd(N, K, seed=2, scale=K ** -0.5)
+    wq, ws = ops.quantize_weight_fp8(w)
+    xq, xs = torch.empty(M, K, dtype=torch.uint8, device=DEV), torch.empty(M, device=DEV)
+    ops.C.quant_fp8(xq, xs, x, None, 1e-6)
+    f8 = lambda q: q.view(torch.float8_e4m3fn).double()
+    want = f8(xq) @ f8(wq).t() * xs.double()[:, None] * ws.double()
+    narrow, split = torch.empty(M, N, dtype=torch.bfloat16, device=DEV), ops._split_k(M, N, K // 2)
+    ops.C.gemm_fp8(narrow, xq, wq, xs, ws, None, 0, split, *ops._gemm_scratch(M, N, split), ops.status_word)
+    for got in (ops.linear_fp8(x, wq, ws), narrow):
+        # tensor cores add e4m3 products in 32 bits or a little less; then one rounding to bf16
+        assert ((got.double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -9).all()
+    assert ops.status() == 0
