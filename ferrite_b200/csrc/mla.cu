@@ -41,8 +41,8 @@ __global__ void __launch_bounds__(256) mla_prep_kernel(__nv_bfloat16* __restrict
   // pair (i, i + R/2) turned by the row's angle
   auto rotate = [&](__nv_bfloat16* to, const __nv_bfloat16* from, int i, float s, float c) {
     const float a = bf2f(from[i]), b = bf2f(from[half + i]);
-    to[i] = f2bf(a * c - b * s);
-    to[half + i] = f2bf(b * c + a * s);
+    to[i] = f2bf(fmaf(a, c, -__fmul_rn(b, s)));       // (spelled out: the compiler's pick of the fused product varies with the code around it)
+    to[half + i] = f2bf(fmaf(b, c, __fmul_rn(a, s)));
   };
   if (blockIdx.y > 0) {
     const int step = max((int)blockDim.x / half, 1);       // heads side by side; a thread's angle is the same for all of its heads
