@@ -60,8 +60,8 @@ __device__ __forceinline__ float tanh_exp(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * 2.885390081777927f));
   return 1.f - __fdividef(2.f, e + 1.f);
 }
-// Two fp32 lanes in one register pair (sm_100: one instruction for both)
 __device__ __forceinline__ float2 bf2f2(uint32_t v) { return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
+// Two fp32 lanes in one register pair (sm_100: one instruction for both)
 __device__ __forceinline__ uint64_t f2_pack(float a, float b) {
   uint64_t v;
   asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
@@ -280,15 +280,7 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint64_t desc_a, uin
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem desc]
-__device__ __forceinline__ void tc_mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
-                                              uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
-}
-// The same from a whole warp, issued by the lane whose `issue` is set (elect_one). Without a branch around it the instruction keeps its
+// D[tmem] (+)= A[tmem] * B[smem desc] from a whole warp, issued by the lane whose `issue` is set (elect_one). Without a branch around it the instruction keeps its
 // operands in uniform registers: 16 cycles from one to the next at N = 32, 64 at N = 128, which is what the tensor cores take; inside a branch
 // for one lane 26 to 95 at N = 32, 74 to 107 at N = 128.
 __device__ __forceinline__ void tc_mma_f16_ts_if(bool issue, uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {

@@ -8,10 +8,10 @@ namespace fb {
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
-// Decode-row fusion of the three kernels above: causal conv + SiLU of this head's q / k / v channels, the delta-rule
-// recurrence, and the gated per-head RMSNorm (y * rsqrt(mean y^2 + eps) * w * silu(z)) in one pass.
+// Causal conv + SiLU of this head's q / k / v channels (gdn_conv_kernel), the delta-rule
+// recurrence (gdn_rec_kernel), and the gated per-head RMSNorm (y * rsqrt(mean y^2 + eps) * w * silu(z)) in one pass.
 // Same arithmetic as the separate kernels (the conv output is rounded to bf16 as it would be when stored), so both
-// paths agree to fp32 rounding of the norm's sum. blockDim = DV * 8 as in gdn_rec_kernel.
+// paths agree to fp32 rounding of the norm's sum.
 // Called by all DV * PARTS threads of a CTA for head h and the segment (n rows from row0, state slot `slot`).
 // The heads that share a key head read the same conv tails, which one of them may rewrite once all have read. CLUSTER: they are the CTAs of one
 // cluster, and the first rewrites behind a barrier of it. Without it, heads that share leave the q / k tail alone: the caller rewrites it
@@ -58,9 +58,10 @@ __device__ __forceinline__ void gdn_step_body(__nv_bfloat16* __restrict__ out, f
   const float gw = bf2f(gnorm_w[col]);
   if (CLUSTER) cluster_arrive();
 
-  // The rows of a segment are sequential, so a row's inputs are fetched while the row before it is computed: without
-  // this every row paid a full global-memory round trip before its first FMA (3.2 us per row on B200, 55 us for a
-  // 17-row verify segment).
+  // The rows of a segment are sequential, so a row's inputs are fetched while the row before it is computed: without this every row paid a
+  // full global-memory round trip before its first FMA (3.2 us a row, 2 with it). Segments of more than one row come here where
+  // gdn_rows_kernel would take several waves of CTAs (many streams), holds no cluster (more than eight heads to a key head) or cannot read
+  // the operands (odd places).
   struct RowIn { float x, b, a, z; };
   auto fetch = [&](int r) {
     RowIn in = {0.f, 0.f, 0.f, 0.f};

@@ -1,4 +1,5 @@
-// Pieces of the products that stream weights through a TMA ring into mma.sync fragments (gemv_stream.cu, moe_stream.cu).
+// Pieces of the products that stream weights through a TMA ring: into mma.sync fragments (gemv_stream.cu), or, 4-bit ones, unpacked as an operand of tcgen05
+// (moe_stream.cu, which takes the unpacking, the waits and the maps from here).
 //
 // A unit of work is 128 weight rows x 128 bytes of K: 64 bf16 or 256 e2m1 values. TMA writes it with the 128-byte swizzle (16-byte chunk c of
 // row r at c ^ (r & 7)); warp w owns 16 of the rows. A dot product does not care about the order of k, so the thread that m16n8k16 makes owner
@@ -22,9 +23,6 @@ namespace fb {
 constexpr int SM_TILE_BYTES = 16384;                  // 128 rows x 128 bytes
 
 __device__ __forceinline__ int sm_row(int g) { return ((g & 1) << 2) | ((g >> 1) & 3); }
-// Pieces that TMA wrote: four boxes of 64 values, piece p of chunk q in box q >> 1 at chunk (q & 1) * 4 + p. Lanes with t >= 2 go through their
-// pieces (and words of codes) in the order 1 0 3 2, and fragment column g is row sm_row4(g): again eight lanes meet eight places.
-__device__ __forceinline__ int sm_row4(int g) { return ((g & 1) << 1) | ((g >> 1) & 1) | (g & 4); }
 __device__ __forceinline__ uint32_t sm_x_bf16(int token, int c) { return (uint32_t)(token * 128 + ((c ^ sm_row(token & 7)) << 4)); }
 __device__ __forceinline__ uint32_t sm_x_fp4(int token, int c) {                // c = k / 8 inside the unit
   const int q = c >> 2, p = c & 3;
@@ -100,13 +98,13 @@ __device__ __forceinline__ void sm_unpack(uint32_t w, uint32_t scale, SmFactors 
   r[3] = sm_mul_bf2(sm_place(h, 0x00f000f0u, f.at4), scale);
 }
 
-// One unit for one warp: acc += the warp's 16 rows x 8 MT tokens (in two sets of sums: products into one set wait for each other), of which
-// the first `live` tiles of 8 hold tokens. `tile`: the weights; `lo`, `hi`: tile rows of fragment rows g and g + 8 of this lane; `xt`: the
-// activations, XT: as TMA wrote them; `sf_lo`, `sf_hi` (e2m1): shared addresses of the rows' scale bytes, SFROW: 16 in a row, otherwise in the
-// first of the unit's four atoms (512 bytes: 128 rows x 4 blocks).
-template <int MT, bool FP4, bool XT, bool SFROW = false>
+// One unit for one warp: acc += the warp's 16 rows x 8 MT tokens (in two sets of sums: products into one set wait for each other).
+// `tile`: the weights; `lo`, `hi`: tile rows of fragment rows g and g + 8 of this lane; `xt`: the activations, XT (bf16 weights): as TMA wrote
+// them; `sf_lo`, `sf_hi` (e2m1): shared addresses of the rows' scale bytes in the first of the unit's four atoms (512 bytes: 128 rows x 4 blocks).
+template <int MT, bool FP4, bool XT>
 __device__ __forceinline__ void sm_unit(float (&acc)[2][MT][4], uint32_t tile, int lo, int hi, uint32_t xt, uint32_t sf_lo, uint32_t sf_hi,
-                                        SmFactors f, int live = MT) {
+                                        SmFactors f) {
+  static_assert(!(FP4 && XT), "");
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -116,19 +114,14 @@ __device__ __forceinline__ void sm_unit(float (&acc)[2][MT][4], uint32_t tile, i
     if constexpr (!FP4) {
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
-        if (mt >= live) break;
         const int r = mt * 8 + sm_row(g);
         const uint4 x = sm_lds(xt + (XT ? (uint32_t)(r * 128 + ((c ^ sm_row(g)) << 4)) : sm_x_bf16(mt * 8 + g, c)));
         sm_mma(acc[0][mt], a.x, b.x, a.y, b.y, x.x, x.y);
         sm_mma(acc[1][mt], a.z, b.z, a.w, b.w, x.z, x.w);
       }
     } else {
-      const uint32_t off = (uint32_t)(SFROW ? c * 2 : (c >> 1) * 512 + ((2 * c) & 3));
+      const uint32_t off = (uint32_t)((c >> 1) * 512 + ((2 * c) & 3));
       const uint2 sa = sm_scales(sm_lds16(sf_lo + off)), sb = sm_scales(sm_lds16(sf_hi + off));
-      if (XT && t >= 2) {
-        a = make_uint4(a.y, a.x, a.w, a.z);
-        b = make_uint4(b.y, b.x, b.w, b.z);
-      }
       const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
       for (int p = 0; p < 4; ++p) {
@@ -137,10 +130,7 @@ __device__ __forceinline__ void sm_unit(float (&acc)[2][MT][4], uint32_t tile, i
         sm_unpack(wb[p], p < 2 ? sb.x : sb.y, f, rb);
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt) {
-          if (mt >= live) break;
-          const int r = sm_row4(g);
-          const uint4 x = sm_lds(xt + (XT ? (uint32_t)((c >> 1) * (MT * 1024) + (mt * 8 + r) * 128 + ((((c & 1) * 4 + (p ^ (t >> 1))) ^ r) << 4))
-                                          : sm_x_fp4(mt * 8 + g, c * 4 + p)));
+          const uint4 x = sm_lds(xt + sm_x_fp4(mt * 8 + g, c * 4 + p));
           sm_mma(acc[0][mt], ra[0], rb[0], ra[1], rb[1], x.x, x.y);
           sm_mma(acc[1][mt], ra[2], rb[2], ra[3], rb[3], x.z, x.w);
         }
