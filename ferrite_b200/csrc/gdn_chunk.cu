@@ -16,8 +16,8 @@
 // The leading terms have sums of their own, since the tensor cores cut what they add to the scale of the largest addend. Off 64 bits (relative, 2-norm;
 // 16 heads, 2048 rows): y 2.0e-7, state 1.6e-7; 1111 rows 2.2e-7 and 1.5e-7; steep decays 2.1e-7 and 1.0e-7. (All in 32-bit FMA: 2.9e-7, 4.0e-7;
 // 3.2e-7, 2.0e-7; 6.1e-7, 4.5e-7.)
-// One layer, prep + scan, us, against both in FMA on the CUDA cores: 2048 rows of 16 heads 80 + 269 -> 26 + 83, 1500 of 32 heads 112 + 387 -> 32 + 98,
-// 64 of 16 heads together 32 -> 14.
+// One layer, prep + scan, us, against both in FMA on the CUDA cores: 2048 rows of 16 heads 80 + 269 -> 26 + 81, 1500 of 32 heads 112 + 387 -> 31 + 104,
+// 64 of 16 heads together 32 -> 15.
 //
 // Counterparts in the reference: `fe_gdn_chunk`, `fe_gdn_chunk_tc`, `fe_gdn_chunk_tc1` (`kernels/k-gdn/src/lib.rs`),
 // `fx_gdn_chunk*` (`kernels/k-fnext/src/gdn.rs`); host wrapper `Gdn::run` (`crates/fe-gdn/src/lib.rs`).
